@@ -97,6 +97,25 @@ int mlcb_launch(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t smem
  * run_kernels (mlc/runtime/executor.py:186-202). */
 int mlcb_launch_many(const mlcb_launch_desc* descs, int n, uint64_t stream, int* failed_at);
 
+/* Dynamic shared memory a kernel may be launched with (above 48 KB it has to be
+ * asked for once). */
+int mlcb_kernel_shared(mlcb_kernel* k, uint32_t bytes);
+
+/* 128-byte tensor map (CUtensorMap) of a 16-bit operand with four dimensions,
+ * innermost first: `strides` are the byte strides of the outer three, `box` the
+ * inner three extents of one 128-byte-swizzled load. */
+int mlcb_tensor_map(void* map, uint64_t address, int bf16, const uint64_t* dims,
+                    const uint64_t* strides, const uint32_t* box);
+
+/* Enqueue one kernel with arbitrary parameters (params[i] points at the i-th
+ * value, read before the call returns) on clusters of `cluster_x` CTAs. */
+int mlcb_launch_ex(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t cluster_x,
+                   uint32_t smem_bytes, void* const* params, uint64_t stream, uint32_t flags);
+
+/* Non-zero when a bounded wait inside one of the module's kernels ran out (their
+ * results are then unusable).  Synchronises with the device. */
+int mlcb_module_fault(mlcb_module* m, uint32_t* code);
+
 #ifdef __cplusplus
 }
 #endif

@@ -95,6 +95,12 @@ class Config:
     #: turn ``mm`` + leading bias add into ``addmm`` (cuBLASLt bias epilogue).  Off by
     #: default: it changes how the matmul is dispatched and rounds once instead of twice
     bias_epilogue: bool = False
+    #: run ``mm`` / ``bmm`` over fp16 / bf16 operands on this package's tensor-core kernels
+    #: (fp32 accumulation, results rounded where the library's are); False: on the library
+    own_matmuls: bool = True
+    #: fold pointwise neighbours into those matmuls and run the attention core as one kernel;
+    #: same values as the separate kernels
+    fuse_matmuls: bool = True
     #: run independent pointwise kernels over the same iteration space as one launch
     #: (BERT's q/k/v bias adds: 36 launches -> 12); bit-identical.  Off by default
     fuse_siblings: bool = False
@@ -113,11 +119,11 @@ class Config:
 
     def as_scheduled(self) -> "Config":
         """The same configuration with every executor-side rewrite off: the schedule
-        runs kernel for kernel and library call for library call as the frontend
-        produced it, on one stream."""
+        runs kernel for kernel and matmul for matmul as the frontend produced it, on
+        one stream."""
         return _replace(self, forward_into_copies=False, write_through_copies=False,
                         sequence_first=False, fold_embeddings=False, bias_epilogue=False,
-                        fuse_siblings=False,
+                        fuse_siblings=False, fuse_matmuls=False,
                         graph_streams=1, dependent_launch="chain")
 
 

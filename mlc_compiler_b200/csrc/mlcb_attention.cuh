@@ -1,0 +1,142 @@
+// One attention tile per CTA: S = Q K^T into TMEM, a generated row functor over the
+// scores (mask, softmax, whatever the schedule's row kernel does), probabilities to
+// shared memory in storage precision, O = P V into TMEM, O to global memory.  Scores and
+// probabilities never leave the SM; both matmuls round where the separate kernels store.
+//
+// A TMEM lane is a query row.  H threads share a row, each with a contiguous part of its
+// keys (warps w, w + 4, ... see the same 32 lanes).  P overlays Q and K, whose matmul is
+// over, and O overlays the scores, which have all been read: [128 x 64] heads over 128
+// keys take 49 KB and 128 TMEM columns, so four CTAs share an SM.
+#pragma once
+
+template <int G_, int T_, int S_, int D_, int H_, int RED_, bool BF16_>
+struct mlcb_att_cfg {
+    static constexpr int G = G_, T = T_, S = S_, D = D_, H = H_, RED = RED_;
+    static constexpr bool BF16 = BF16_;
+    static constexpr int TQ = (T + 127) / 128, S16 = (S + 15) / 16 * 16, S64 = (S + 63) / 64 * 64, DB = D / 64;
+    static constexpr int HALVES = (S16 + 255) / 256;               // a TMA box and an MMA span at most 256 keys
+    static constexpr int KEYS = HALVES == 1 ? S16 : (S16 / 2 + 15) / 16 * 16;   // keys per box
+    static constexpr u32 Q_BYTES = DB * 16384, KV_BYTES = (u32)DB * HALVES * KEYS * 128, P_BYTES = S64 / 64 * 16384;
+    static constexpr u32 QK_BYTES = Q_BYTES + KV_BYTES > P_BYTES ? Q_BYTES + KV_BYTES : P_BYTES;
+    static constexpr u32 SMEM = QK_BYTES + KV_BYTES + 1024;
+    static constexpr int NEED = HALVES * KEYS > D ? HALVES * KEYS : D;
+    static constexpr int COLS = NEED <= 64 ? 64 : NEED <= 128 ? 128 : NEED <= 256 ? 256 : 512;
+    static_assert(D % 64 == 0 && D <= 128 && S <= 512 && H == 4, "attention tile");
+};
+
+template <typename C, typename Rows, typename T>
+__device__ __forceinline__ void mlcb_attention(const mlcb_tmap* tq, const mlcb_tmap* tk, const mlcb_tmap* tv,
+                                               const Rows& rows, T* out, i64 out_g, i64 out_t) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ alignas(8) u64 bars[4];
+    __shared__ u32 tmem_slot;
+    __shared__ volatile u32 dead;
+    __shared__ float red[C::RED];                   // two reductions' worth of partial row results
+    const u32 smem = (mlcb_smem(smem_raw) + 1023u) & ~1023u;
+    const u32 sq = smem, sk = smem + C::Q_BYTES, sp = smem, sv = smem + C::QK_BYTES;
+    const u32 qk_full = mlcb_smem(bars), v_full = qk_full + 8, s_full = qk_full + 16, o_full = qk_full + 24;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int g = blockIdx.x / C::TQ, t0 = (blockIdx.x % C::TQ) * 128;
+
+    if (threadIdx.x == 0) {
+        dead = 0;
+        for (int i = 0; i < 4; ++i) mlcb_bar_init(qk_full + 8 * i, 1);
+        mlcb_bar_fence_init();
+        mlcb_tma_prefetch(tq);
+        mlcb_tma_prefetch(tk);
+        mlcb_tma_prefetch(tv);
+    }
+    if (warp == 0) mlcb_tmem_alloc<1>(mlcb_smem(&tmem_slot), C::COLS);
+    mlcb_tc_before();
+    __syncthreads();
+    mlcb_tc_after();
+    const u32 tmem = tmem_slot;
+    MLCB_GRID_TRIGGER();
+    MLCB_GRID_WAIT();
+
+    if (warp == 0) {
+        const bool elected = mlcb_elect();
+        if (elected) {
+            mlcb_bar_expect(qk_full, C::Q_BYTES + C::KV_BYTES);
+            mlcb_tma_load(sq, tq, qk_full, 0, t0, 0, g);
+#pragma unroll
+            for (int h = 0; h < C::HALVES; ++h)
+                mlcb_tma_load(sk + h * (C::DB * C::KEYS * 128), tk, qk_full, 0, h * C::KEYS, 0, g);
+            mlcb_bar_expect(v_full, C::KV_BYTES);
+#pragma unroll
+            for (int j = 0; j < C::DB; ++j)
+#pragma unroll
+                for (int h = 0; h < C::HALVES; ++h)
+                    mlcb_tma_load(sv + (j * C::HALVES + h) * (C::KEYS * 128), tv, v_full, j * 64, h * C::KEYS, 0, g);
+        }
+        __syncwarp();
+        mlcb_bar_wait(qk_full, 0, &dead);
+        mlcb_tc_after();
+        if (elected) {
+            constexpr u32 idesc = mlcb_idesc(128, C::KEYS, C::BF16, false);
+#pragma unroll
+            for (int h = 0; h < C::HALVES; ++h)
+#pragma unroll
+                for (int j = 0; j < C::DB; ++j)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        mlcb_mma<1>(tmem + h * C::KEYS, mlcb_desc(sq + j * 16384, 16) + k * 2,
+                                    mlcb_desc(sk + (h * C::DB + j) * (C::KEYS * 128), 16) + k * 2, idesc, j > 0 || k > 0);
+            mlcb_mma_commit<1>(s_full);
+        }
+        __syncwarp();
+    }
+    const int quad = warp % 4, part_of_row = warp / 4;
+    const int r = quad * 32 + lane;
+    const u32 lanes = tmem + ((u32)(quad * 32) << 16);
+    rows.run(lanes, sp, g, t0 + r < C::T ? t0 + r : C::T - 1, r, part_of_row, red, s_full, &dead);
+    mlcb_proxy_fence();
+    mlcb_tc_before();
+    __syncthreads();
+    mlcb_tc_after();
+    if (warp == 0) {
+        const bool elected = mlcb_elect();
+        mlcb_bar_wait(v_full, 0, &dead);
+        if (elected) {
+            constexpr u32 idesc = mlcb_idesc(128, C::D, C::BF16, true);
+#pragma unroll
+            for (int k = 0; k < C::S16 / 16; ++k)
+                mlcb_mma<1>(tmem, mlcb_desc(sp + k / 4 * 16384, 16) + (k % 4) * 2,
+                            mlcb_desc(sv, C::HALVES * C::KEYS * 128) + k * 128, idesc, k > 0);
+            mlcb_mma_commit<1>(o_full);
+        }
+        __syncwarp();
+    }
+    mlcb_bar_wait(o_full, 0, &dead);
+    mlcb_tc_after();
+    if (!dead) {
+        // D columns over H threads of the row, at least 16 each
+        constexpr int STEP = C::D / C::H < 16 ? 16 : C::D / C::H;
+#pragma unroll
+        for (int c = 0; c < STEP; c += 16) {
+            const int c0 = part_of_row * STEP + c;
+            float v[16];
+            mlcb_tmem_ld(lanes + c0, v);
+            if (t0 + r < C::T) mlcb_store<T, 16>(out + g * out_g + (t0 + r) * out_t + c0, v);
+            __syncwarp();
+        }
+    } else {
+        mlcb_drain();
+    }
+    mlcb_tc_before();
+    __syncthreads();
+    if (warp == 0) {
+        mlcb_tc_after();
+        mlcb_tmem_free<1>(tmem, C::COLS);
+    }
+}
+
+// eight probabilities of row r, keys [c, c + 8), into the swizzled K-major P tile
+template <typename T>
+__device__ __forceinline__ void mlcb_store_p(u32 sp, int r, int c, const float (&v)[8]) {
+    mlcb_pack<T, 8> u;
+    mlcb_packer<T, 8>::run(u, v);
+    const u32 at = sp + (c / 64) * 16384 + r * 128 + ((((c % 64) * 2) ^ ((r % 8) * 16)));
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                 :: "r"(at), "r"(u.w[0].x), "r"(u.w[0].y), "r"(u.w[0].z), "r"(u.w[0].w) : "memory");
+}

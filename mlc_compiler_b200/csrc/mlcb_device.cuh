@@ -231,6 +231,16 @@ __device__ __forceinline__ void mlcb_store1(T* __restrict__ p, typename mlcb_ele
 // torch.maximum / torch.minimum / amax / amin propagate NaN; fmaxf does not.
 template <typename T> __device__ __forceinline__ T mlcb_max(T a, T b) { return (a > b || a != a) ? a : b; }
 template <typename T> __device__ __forceinline__ T mlcb_min(T a, T b) { return (a < b || a != a) ? a : b; }
+template <> __device__ __forceinline__ float mlcb_max<float>(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+template <> __device__ __forceinline__ float mlcb_min<float>(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
 __device__ __forceinline__ float  mlcb_sigmoid(float x)  { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ double mlcb_sigmoid(double x) { return 1.0 / (1.0 + exp(-x)); }
 __device__ __forceinline__ float  mlcb_rsqrt(float x)  { return 1.0f / sqrtf(x); }

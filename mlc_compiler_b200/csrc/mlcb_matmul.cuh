@@ -1,0 +1,307 @@
+// C = A B over 16-bit operands with fp32 accumulation in TMEM, every element handed
+// to a generated epilogue in registers (mlc_compiler_b200/emit/matmul.py picks the
+// configuration and says why).
+//
+// Warp roles: 0 issues TMA loads, 1 issues MMAs, the rest are the epilogue (one TMEM
+// lane = one row per thread).  A tile is 128 rows x BN columns per CTA; CG = 2 pairs
+// two CTAs on 256 rows so that each fetches only half of B.  SPLIT > 1 divides K over
+// a cluster whose CTAs exchange partial sums through distributed shared memory, in
+// rank order (deterministic), each finishing BN / SPLIT columns.
+#pragma once
+
+// ---------------------------------------------------------------------------
+// Two neighbouring columns per register pair: add, mul and fma of both in one
+// instruction (.f32x2), each half rounded as the scalar form rounds it.  An exact-GELU
+// epilogue is instruction-bound at 28 per element in scalar form.
+// ---------------------------------------------------------------------------
+struct mlcb_f2 {
+    u64 v;
+    __device__ __forceinline__ mlcb_f2() {}
+    __device__ __forceinline__ mlcb_f2(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+    __device__ __forceinline__ mlcb_f2(float both) : mlcb_f2(both, both) {}
+    __device__ __forceinline__ void get(float& lo, float& hi) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+};
+__device__ __forceinline__ mlcb_f2 operator+(mlcb_f2 a, mlcb_f2 b) { mlcb_f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ mlcb_f2 operator*(mlcb_f2 a, mlcb_f2 b) { mlcb_f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ mlcb_f2 operator-(mlcb_f2 a, mlcb_f2 b) { mlcb_f2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ mlcb_f2 mlcb_fma2(mlcb_f2 a, mlcb_f2 b, mlcb_f2 c) { mlcb_f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ mlcb_f2 mlcb_rn_f16(mlcb_f2 a) {
+    float x, y; a.get(x, y);
+    const float2 f = __half22float2(__floats2half2_rn(x, y));
+    return mlcb_f2(f.x, f.y);
+}
+__device__ __forceinline__ mlcb_f2 mlcb_rn_bf16(mlcb_f2 a) {
+    float x, y; a.get(x, y);
+    const float2 f = __bfloat1622float2(__floats2bfloat162_rn(x, y));
+    return mlcb_f2(f.x, f.y);
+}
+__device__ __forceinline__ mlcb_f2 mlcb_ex2(mlcb_f2 a) { float x, y; a.get(x, y); return mlcb_f2(mlcb_ex2(x), mlcb_ex2(y)); }
+__device__ __forceinline__ mlcb_f2 mlcb_rcp_fast(mlcb_f2 a) { float x, y; a.get(x, y); return mlcb_f2(mlcb_rcp_fast(x), mlcb_rcp_fast(y)); }
+// the scalar forms' operations in their order; a negated factor is a negated constant here
+__device__ __forceinline__ mlcb_f2 mlcb_exp_fast(mlcb_f2 x) { return mlcb_ex2(x * 1.4426950408889634f); }
+__device__ __forceinline__ mlcb_f2 mlcb_sigmoid_fast(mlcb_f2 x) { return mlcb_rcp_fast(mlcb_f2(1.0f) + mlcb_ex2(x * -1.4426950408889634f)); }
+__device__ __forceinline__ mlcb_f2 mlcb_tanh_fast(mlcb_f2 x) {
+    return mlcb_fma2(-2.0f, mlcb_rcp_fast(mlcb_f2(1.0f) + mlcb_ex2(x * 2.8853900817779268f)), 1.0f);
+}
+__device__ __forceinline__ mlcb_f2 mlcb_erf_fast(mlcb_f2 x) {
+    float lo, hi; x.get(lo, hi);
+    const mlcb_f2 ax(fabsf(lo), fabsf(hi));
+    const mlcb_f2 t = mlcb_rcp_fast(mlcb_fma2(0.3275911f, ax, 1.0f));
+    mlcb_f2 p = mlcb_fma2(-1.061405429f, t, 1.453152027f);
+    p = mlcb_fma2(p, t, -1.421413741f);
+    p = mlcb_fma2(p, t, 0.284496736f);
+    p = mlcb_fma2(p, t, -0.254829592f);
+    float r0, r1;
+    mlcb_fma2(p * t, mlcb_ex2(ax * ax * -1.4426950408889634f), 1.0f).get(r0, r1);
+    return mlcb_f2(copysignf(r0, lo), copysignf(r1, hi));
+}
+
+template <int M_, int N_, int KBLOCKS_, int KSTEP_, bool A_CUT_, bool B_CUT_, int BN_, int STAGES_, int ACC_, int SPLIT_, int CG_, int GROUPS_,
+          int BATCH_, int EPI_WARPS_, bool B_MN_, bool BF16_, bool B_STABLE_>
+struct mlcb_mm_cfg {
+    static constexpr int M = M_, N = N_, KBLOCKS = KBLOCKS_, KSTEP = KSTEP_, BN = BN_, STAGES = STAGES_, ACC = ACC_, SPLIT = SPLIT_,
+                         CG = CG_, GROUPS = GROUPS_, BATCH = BATCH_, EPI_WARPS = EPI_WARPS_;
+    // K is a whole number of 64-element blocks, addressed as a dimension of its own
+    static constexpr bool A_CUT = A_CUT_, B_CUT = B_CUT_;
+    static constexpr bool B_MN = B_MN_, BF16 = BF16_, B_STABLE = B_STABLE_;
+    static constexpr int TM = (M + 128 * CG - 1) / (128 * CG), TN = (N + BN - 1) / BN;
+    static constexpr int TILES = TM * TN * GROUPS * BATCH;
+    static constexpr int CLUSTER = SPLIT * CG;
+    static constexpr int B_ROWS = BN / CG;                       // rows of B (or columns, MN-major) per CTA
+    static constexpr u32 A_BYTES = KSTEP * 128 * 128, B_BYTES = KSTEP * B_ROWS * 128, STAGE_BYTES = A_BYTES + B_BYTES;
+    static constexpr int COLS_NEEDED = ACC * BN;
+    static constexpr int TMEM_COLS = COLS_NEEDED <= 32 ? 32 : COLS_NEEDED <= 64 ? 64 : COLS_NEEDED <= 128 ? 128
+                                   : COLS_NEEDED <= 256 ? 256 : 512;
+    static_assert(BN % 32 == 0 && BN <= 256 && ACC * BN <= 512, "tile");
+    static_assert(SPLIT == 1 || (BN % (8 * SPLIT) == 0 && (KBLOCKS + KSTEP - 1) / KSTEP >= SPLIT && ACC == 1), "split");
+    static_assert(KSTEP == 1 || (A_CUT && (B_CUT || B_MN)), "several K blocks per copy");
+    static_assert(!B_MN || (BN % 64 == 0 && CG == 1 && KSTEP <= 4), "MN-major B");
+};
+
+template <typename C, typename Epi>
+__device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap* tb0, const mlcb_tmap* tb1,
+                                            const mlcb_tmap* tb2, const mlcb_tmap* tb3, const Epi& epi) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ alignas(8) u64 bars[2 * C::STAGES + 2 * C::ACC];
+    __shared__ u32 tmem_slot;
+    __shared__ volatile u32 dead;
+    const u32 smem = (mlcb_smem(smem_raw) + 1023u) & ~1023u;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const u32 rank = C::CLUSTER > 1 ? mlcb_cta_rank() : 0;
+    const u32 full = mlcb_smem(bars), empty = full + 8 * C::STAGES, acc_full = empty + 8 * C::STAGES,
+              acc_empty = acc_full + 8 * C::ACC;
+
+    if (threadIdx.x == 0) {
+        dead = 0;
+        for (int i = 0; i < C::STAGES; ++i) { mlcb_bar_init(full + 8 * i, 1); mlcb_bar_init(empty + 8 * i, 1); }
+        for (int i = 0; i < C::ACC; ++i) {
+            mlcb_bar_init(acc_full + 8 * i, 1);
+            mlcb_bar_init(acc_empty + 8 * i, C::CG * C::EPI_WARPS);
+        }
+        mlcb_bar_fence_init();
+        mlcb_tma_prefetch(ta);
+        mlcb_tma_prefetch(tb0);
+    }
+    if (warp == 1) mlcb_tmem_alloc<C::CG>(mlcb_smem(&tmem_slot), C::TMEM_COLS);
+    mlcb_tc_before();
+    __syncthreads();
+    if (C::CLUSTER > 1) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }
+    mlcb_tc_after();
+    const u32 tmem = tmem_slot;
+    // the dependent launch may take SM resources from here on: this CTA holds its TMEM
+    MLCB_GRID_TRIGGER();
+
+    const int cluster = blockIdx.x / C::CLUSTER, clusters = gridDim.x / C::CLUSTER;
+    constexpr int KSTEPS = (C::KBLOCKS + C::KSTEP - 1) / C::KSTEP;   // the tail of the last one reads zeros
+    const int pair = C::CG == 2 ? (int)rank & 1 : 0, part = (int)rank / C::CG;
+    const int ks0 = part * KSTEPS / C::SPLIT, ks1 = (part + 1) * KSTEPS / C::SPLIT;
+    constexpr int SLICE = C::BN / C::SPLIT;                  // columns this CTA finishes when K is split
+    const u32 inbox = smem + C::STAGES * C::STAGE_BYTES;     // partial sums other ranks send
+
+    if (warp == 0) {
+        {
+            const bool elected = mlcb_elect();
+            auto load_a = [&](int tile, int ks, int s) {
+                const int m = (tile % C::TM) * (128 * C::CG) + pair * 128;
+                const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
+                const u32 dst = smem + s * C::STAGE_BYTES;
+                const int x = C::A_CUT ? 0 : ks * 64, b = C::A_CUT ? ks * C::KSTEP : 0;
+                if (C::CG == 1) mlcb_tma_load(dst, ta, full + 8 * s, x, m, b, z);
+                else mlcb_tma_load_pair(dst, ta, full + 8 * s, x, m, b, z);
+            };
+            auto load_b = [&](int tile, int ks, int s) {
+                const int nt = (tile / C::TM) % C::TN, g = (tile / (C::TM * C::TN)) % C::GROUPS;
+                const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
+                const mlcb_tmap* tb = C::GROUPS == 1 ? tb0 : g == 0 ? tb0 : g == 1 ? tb1 : g == 2 ? tb2 : tb3;
+                const u32 dst = smem + s * C::STAGE_BYTES + C::A_BYTES;
+                const int x = C::B_CUT ? 0 : ks * 64, b = C::B_CUT ? ks * C::KSTEP : 0;
+                if (C::B_MN) {
+#pragma unroll
+                    for (int j = 0; j < C::BN / 64; ++j)
+                        mlcb_tma_load(dst + j * (C::KSTEP * 8192), tb, full + 8 * s, nt * C::BN + j * 64,
+                                      ks * C::KSTEP * 64, 0, z);
+                } else if (C::CG == 1) {
+                    mlcb_tma_load(dst, tb, full + 8 * s, x, nt * C::BN, b, z);
+                } else {
+                    mlcb_tma_load_pair(dst, tb, full + 8 * s, x, nt * C::BN + pair * C::B_ROWS, b, z);
+                }
+            };
+            // weights do not depend on the launch before this one: the first stages of
+            // them are on their way before the grid-dependency wait
+            int ahead = 0;
+            if (C::B_STABLE && cluster < C::TILES) {
+                for (; ahead < C::STAGES && ks0 + ahead < ks1; ++ahead) {
+                    if (elected) {
+                        if (C::CG == 1 || pair == 0) mlcb_bar_expect(full + 8 * ahead, C::CG * C::STAGE_BYTES);
+                        load_b(cluster, ks0 + ahead, ahead);
+                    }
+                }
+            }
+            MLCB_GRID_WAIT();
+            int s = 0;
+            u32 phase = 1;
+            bool alive = true;
+            for (int tile = cluster; tile < C::TILES && alive; tile += clusters) {
+                for (int ks = ks0; ks < ks1; ++ks) {
+                    const bool both = ahead <= 0;
+                    --ahead;
+                    if (both) {
+                        alive = mlcb_bar_wait(empty + 8 * s, phase, &dead);
+                        if (!alive) break;
+                    }
+                    if (elected) {
+                        if (both) {
+                            if (C::CG == 1 || pair == 0) mlcb_bar_expect(full + 8 * s, C::CG * C::STAGE_BYTES);
+                            load_b(tile, ks, s);
+                        }
+                        load_a(tile, ks, s);
+                    }
+                    __syncwarp();
+                    if (++s == C::STAGES) { s = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (pair == 0) {
+            const bool elected = mlcb_elect();
+            constexpr u32 idesc = mlcb_idesc(128 * C::CG, C::BN, C::BF16, C::B_MN);
+            int s = 0, acc = 0;
+            u32 phase = 0, acc_phase = 1;
+            bool alive = true;
+            for (int tile = cluster; tile < C::TILES && alive; tile += clusters) {
+                alive = mlcb_bar_wait(acc_empty + 8 * acc, acc_phase, &dead);
+                mlcb_tc_after();
+                for (int ks = ks0; ks < ks1 && alive; ++ks) {
+                    alive = mlcb_bar_wait(full + 8 * s, phase, &dead);
+                    if (!alive) break;
+                    mlcb_tc_after();
+                    const u32 a = smem + s * C::STAGE_BYTES;
+                    const u64 da = mlcb_desc(a, 16), db = mlcb_desc(a + C::A_BYTES, C::B_MN ? C::KSTEP * 8192 : 16);
+                    if (elected) {
+#pragma unroll
+                        for (int j = 0; j < C::KSTEP; ++j)
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                mlcb_mma<C::CG>(tmem + acc * C::BN, da + j * 1024 + k * 2,
+                                                db + (C::B_MN ? (j * 4 + k) * 128 : j * (C::B_ROWS * 8) + k * 2), idesc,
+                                                ks > ks0 || j > 0 || k > 0);
+                        mlcb_mma_commit<C::CG>(empty + 8 * s, rank);
+                    }
+                    __syncwarp();
+                    if (++s == C::STAGES) { s = 0; phase ^= 1; }
+                }
+                if (elected) mlcb_mma_commit<C::CG>(acc_full + 8 * acc, rank);
+                __syncwarp();
+                if (++acc == C::ACC) { acc = 0; acc_phase ^= 1; }
+            }
+        }
+    } else {
+        const int quad = warp % 4, half = (warp - 2) / 4;
+        constexpr int HALVES = C::EPI_WARPS / 4;
+        const int r = quad * 32 + lane;
+        const u32 base = tmem + ((u32)(quad * 32) << 16);
+        MLCB_GRID_WAIT();
+        int nth = 0;
+        for (int tile = cluster; tile < C::TILES && !dead; tile += clusters, ++nth) {
+            const int acc = nth % C::ACC;
+            const int tm = tile % C::TM, tn = (tile / C::TM) % C::TN, g = (tile / (C::TM * C::TN)) % C::GROUPS;
+            const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
+            const int row = tm * (128 * C::CG) + pair * 128 + r;
+            mlcb_bar_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+            mlcb_tc_after();
+            if (C::SPLIT > 1) {
+                // partial sums go straight into the shared memory of the CTA that finishes these
+                // columns, as [source rank][column quad][row][4]: conflict-free both ways
+                const u32 mine = inbox + (part * SLICE * 128 + r * 4) * 4;
+#pragma unroll
+                for (int c = half * 16; c < C::BN; c += 16 * HALVES) {
+                    float v[16];
+                    mlcb_tmem_ld(base + c, v);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int col = c + 4 * q;
+                        u32 at;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                                     : "=r"(at) : "r"(mine + (col % SLICE) * 512), "r"((u32)(col / SLICE * C::CG + pair)));
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                                     :: "r"(at), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                                     : "memory");
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int c = half * 32; c < C::BN; c += 32 * HALVES) {
+                    float v[32];
+                    mlcb_tmem_ld(base + acc * C::BN + c, v);
+                    if (c + 32 * HALVES >= C::BN) {
+                        mlcb_tc_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (C::CG == 1) mlcb_bar_arrive(acc_empty + 8 * acc);
+                            else mlcb_bar_arrive_at(acc_empty + 8 * acc, rank & ~1u);
+                        }
+                    }
+                    epi.columns(v, row, tn * C::BN + c, g, z, lane);
+                    __syncwarp();
+                }
+            }
+        }
+    }
+    __syncwarp();
+    if (C::SPLIT > 1) {
+        mlcb_cluster_arrive();
+        mlcb_cluster_wait();
+        if (warp >= 2 && cluster < C::TILES && !dead) {
+            const int quad = warp % 4, half = (warp - 2) / 4;
+            constexpr int HALVES = C::EPI_WARPS / 4;
+            const int r = quad * 32 + lane;
+            const int tm = cluster % C::TM, tn = (cluster / C::TM) % C::TN, g = (cluster / (C::TM * C::TN)) % C::GROUPS;
+            const int z = C::BATCH > 1 ? cluster / (C::TM * C::TN * C::GROUPS) : 0;
+#pragma unroll
+            for (int c = half * 8; c < SLICE; c += 8 * HALVES) {
+                float v[8];
+#pragma unroll
+                for (int p = 0; p < C::SPLIT; ++p)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        float x[4];
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                                     : "r"(inbox + ((p * SLICE + c + 4 * q) * 128 + r * 4) * 4) : "memory");
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) v[4 * q + i] = p ? v[4 * q + i] + x[i] : x[i];
+                    }
+                epi.columns(v, tm * (128 * C::CG) + pair * 128 + r, tn * C::BN + part * SLICE + c, g, z, lane);
+                __syncwarp();
+            }
+        }
+    }
+    mlcb_tc_before();
+    __syncthreads();
+    if (C::CG == 2) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }   // the peer still uses our barriers and TMEM
+    if (dead) mlcb_drain();
+    if (warp == 1) {
+        mlcb_tc_after();
+        mlcb_tmem_free<C::CG>(tmem, C::TMEM_COLS);
+    }
+}

@@ -55,6 +55,13 @@ struct Driver {
     CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned,
                              unsigned, unsigned, CUstream, void**, void**) = nullptr;
     CUresult (*LaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
+    CUresult (*FuncSetAttribute)(CUfunction, CUfunction_attribute, int) = nullptr;
+    CUresult (*ModuleGetGlobal)(CUdeviceptr*, size_t*, CUmodule, const char*) = nullptr;
+    CUresult (*MemcpyDtoH)(void*, CUdeviceptr, size_t) = nullptr;
+    CUresult (*TensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                     const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                     const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill) = nullptr;
     bool ok = false;
 };
 
@@ -88,6 +95,10 @@ void load_driver() {
     ok &= sym(d.lib, MLCB_STR(cuFuncGetAttribute), d.FuncGetAttribute);
     ok &= sym(d.lib, MLCB_STR(cuLaunchKernel), d.LaunchKernel);
     ok &= sym(d.lib, MLCB_STR(cuLaunchKernelEx), d.LaunchKernelEx);
+    ok &= sym(d.lib, MLCB_STR(cuFuncSetAttribute), d.FuncSetAttribute);
+    ok &= sym(d.lib, MLCB_STR(cuModuleGetGlobal), d.ModuleGetGlobal);
+    ok &= sym(d.lib, MLCB_STR(cuMemcpyDtoH), d.MemcpyDtoH);
+    ok &= sym(d.lib, MLCB_STR(cuTensorMapEncodeTiled), d.TensorMapEncodeTiled);
     if (ok && d.Init(0) == CUDA_SUCCESS) d.ok = true;
 }
 
@@ -421,6 +432,83 @@ int mlcb_launch_many(const mlcb_launch_desc* descs, int n, uint64_t stream, int*
             if (failed_at) *failed_at = i;
             return e;
         }
+    }
+    return 0;
+}
+
+int mlcb_kernel_shared(mlcb_kernel* k, uint32_t bytes) {
+    if (!k) return fail(MLCB_ERR_ARGUMENT, "mlcb_kernel_shared: null kernel");
+    if (int e = need_driver()) return e;
+    CtxGuard in_module_context(k->owner->ctx);
+    CUresult r = g_drv.FuncSetAttribute(k->fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)bytes);
+    if (r != CUDA_SUCCESS) return cu_fail(r, "cuFuncSetAttribute(MAX_DYNAMIC_SHARED_SIZE_BYTES)");
+    return 0;
+}
+
+int mlcb_module_fault(mlcb_module* m, uint32_t* code) {
+    if (!m || !code) return fail(MLCB_ERR_ARGUMENT, "mlcb_module_fault: null argument");
+    *code = 0;
+    if (int e = need_driver()) return e;
+    CtxGuard in_module_context(m->ctx);
+    CUdeviceptr p = 0;
+    size_t n = 0;
+    if (g_drv.ModuleGetGlobal(&p, &n, m->mod, "mlcb_fault") != CUDA_SUCCESS) return 0;  // no waits in it
+    CUresult r = g_drv.MemcpyDtoH(code, p, sizeof *code);
+    if (r != CUDA_SUCCESS) return cu_fail(r, "cuMemcpyDtoH(mlcb_fault)");
+    return 0;
+}
+
+int mlcb_tensor_map(void* map, uint64_t address, int bf16, const uint64_t* dims,
+                    const uint64_t* strides, const uint32_t* box) {
+    if (!map || !dims || !strides || !box) return fail(MLCB_ERR_ARGUMENT, "mlcb_tensor_map: null argument");
+    if (int e = need_driver()) return e;
+    const cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]};
+    const cuuint64_t st[3] = {strides[0], strides[1], strides[2]};
+    const cuuint32_t b[4] = {box[0], box[1], box[2], 1};
+    const cuuint32_t step[4] = {1, 1, 1, 1};
+    CUresult r = g_drv.TensorMapEncodeTiled(
+        (CUtensorMap*)map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+        (void*)(uintptr_t)address, d, st, b, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return cu_fail(r, "cuTensorMapEncodeTiled");
+    return 0;
+}
+
+int mlcb_launch_ex(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t cluster_x, uint32_t smem_bytes,
+                   void* const* params, uint64_t stream, uint32_t flags) {
+    if (!k || !params || !grid_x || !block_x || !cluster_x || grid_x % cluster_x)
+        return fail(MLCB_ERR_ARGUMENT, "mlcb_launch_ex: bad argument (kernel=%p grid=%u block=%u cluster=%u)",
+                    (void*)k, grid_x, block_x, cluster_x);
+    if (int e = need_driver()) return e;
+    CUlaunchAttribute attr[2];
+    memset(attr, 0, sizeof attr);
+    unsigned n = 0;
+    if (flags & MLCB_LAUNCH_DEPENDENT) {
+        attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+        attr[n++].value.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster_x > 1) {
+        attr[n].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+        attr[n].value.clusterDim.x = cluster_x;
+        attr[n].value.clusterDim.y = attr[n].value.clusterDim.z = 1;
+        ++n;
+    }
+    CUlaunchConfig cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDimX = grid_x;
+    cfg.gridDimY = cfg.gridDimZ = 1;
+    cfg.blockDimX = block_x;
+    cfg.blockDimY = cfg.blockDimZ = 1;
+    cfg.sharedMemBytes = smem_bytes;
+    cfg.hStream = (CUstream)(uintptr_t)stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    CtxGuard in_module_context(k->owner->ctx);
+    CUresult r = g_drv.LaunchKernelEx(&cfg, k->fn, (void**)params, nullptr);
+    if (r != CUDA_SUCCESS) {
+        char what[256];
+        snprintf(what, sizeof what, "launch of %s <<<%u, %u>>>", k->name.c_str(), grid_x, block_x);
+        return cu_fail(r, what);
     }
     return 0;
 }

@@ -1,0 +1,163 @@
+// Tensor-core side of the device library (sm_100a): bounded barrier waits, TMA
+// tile loads, TMEM allocation and tcgen05 matmuls.  Prepended, after
+// mlcb_device.cuh, to modules that contain matmul or attention kernels.
+//
+// Shared-memory operand tiles are what a 128-byte-swizzled TMA load writes: rows
+// of 64 16-bit elements (128 bytes), eight rows per 1024-byte swizzle atom.  A
+// K-major tile has one row per matrix row; an MN-major tile one row per K.
+#pragma once
+
+typedef unsigned int u32;
+struct alignas(128) mlcb_tmap { u64 opaque[16]; };   // CUtensorMap, passed by value
+
+__device__ __forceinline__ u32 mlcb_smem(const void* p) { return (u32)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ u32 mlcb_cta_rank() { u32 r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+
+// One lane of a converged warp.  The copy and MMA warps run their loops with every lane
+// and only issue under this predicate: addresses, descriptors and counters then stay in
+// uniform registers (four N = 64 MMAs with their wait and commit: 214 cycles against 363
+// when a single lane runs the loop).
+__device__ __forceinline__ bool mlcb_elect() {
+    u32 p;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(p));
+    return p != 0;
+}
+
+// ---------------------------------------------------------------------------
+// Barriers.  Every wait is bounded: after two seconds (three orders above the
+// longest forward) it marks the CTA dead and records a fault code the host can
+// read; a dead CTA skips every later wait and issues no further copies, drains,
+// frees its TMEM and exits.
+// ---------------------------------------------------------------------------
+__device__ unsigned int mlcb_fault = 0;
+
+__device__ __forceinline__ u64 mlcb_now_ns() { u64 t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
+__device__ __forceinline__ void mlcb_bar_init(u32 bar, u32 count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mlcb_bar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void mlcb_bar_arrive(u32 bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
+}
+// arrive on the barrier at the same offset in CTA `rank` of the cluster
+__device__ __forceinline__ void mlcb_bar_arrive_at(u32 bar, u32 rank) {
+    u32 remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(rank));
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(remote) : "memory");
+}
+__device__ __forceinline__ void mlcb_bar_expect(u32 bar, u32 bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mlcb_bar_try(u32 bar, u32 parity) {
+    u32 ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __noinline__ bool mlcb_bar_wait_slow(u32 bar, u32 parity, volatile u32* dead) {
+    const u64 t0 = mlcb_now_ns();
+    while (!mlcb_bar_try(bar, parity)) {
+        if (*dead) return false;
+        if (mlcb_now_ns() - t0 > 2000000000ull) {
+            *dead = 1;
+            atomicExch(&mlcb_fault, 1u);
+            return false;
+        }
+    }
+    return true;
+}
+// false: the CTA is dead
+__device__ __forceinline__ bool mlcb_bar_wait(u32 bar, u32 parity, volatile u32* dead) {
+    if (mlcb_bar_try(bar, parity)) return true;
+    return mlcb_bar_wait_slow(bar, parity, dead);
+}
+__device__ __forceinline__ void mlcb_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void mlcb_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// a dead CTA leaves time for copies already in flight to land before it exits
+__device__ __forceinline__ void mlcb_drain() {
+    const u64 t0 = mlcb_now_ns();
+    while (mlcb_now_ns() - t0 < 20000000ull) __nanosleep(1000);
+}
+
+// ---------------------------------------------------------------------------
+// TMA tile loads.  Every map has four dimensions: 64 contiguous elements (or all of
+// them), rows, blocks of 64 along the contiguous axis, batch -- so that one copy
+// brings several 128-byte-wide blocks, each stored as its own swizzled tile.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void mlcb_tma_prefetch(const mlcb_tmap* m) {
+    asm volatile("prefetch.tensormap [%0];" :: "l"(m) : "memory");
+}
+__device__ __forceinline__ void mlcb_tma_load(u32 dst, const mlcb_tmap* m, u32 bar, int x, int y, int b, int z) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 :: "r"(dst), "l"(m), "r"(bar), "r"(x), "r"(y), "r"(b), "r"(z) : "memory");
+}
+// loads of a CTA pair: the barrier is the one at this offset in the even CTA
+__device__ __forceinline__ void mlcb_tma_load_pair(u32 dst, const mlcb_tmap* m, u32 bar, int x, int y, int b, int z) {
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 :: "r"(dst), "l"(m), "r"(bar & 0xFEFFFFFFu), "r"(x), "r"(y), "r"(b), "r"(z) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// TMEM and tcgen05
+// ---------------------------------------------------------------------------
+template <int CG> __device__ __forceinline__ void mlcb_tmem_alloc(u32 slot, u32 cols) {
+    if (CG == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(slot), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(slot), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+}
+template <int CG> __device__ __forceinline__ void mlcb_tmem_free(u32 addr, u32 cols) {
+    if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(addr), "r"(cols));
+    else         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(addr), "r"(cols));
+}
+__device__ __forceinline__ void mlcb_tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void mlcb_tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void mlcb_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+template <int CG> __device__ __forceinline__ void mlcb_mma(u32 d, u64 a, u64 b, u32 idesc, bool acc) {
+    if (CG == 1)
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+                     " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+                     :: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"((u32)acc) : "memory");
+    else
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+                     " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+                     :: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"((u32)acc) : "memory");
+}
+// signals `bar` (in both CTAs of the pair that cluster rank `rank` belongs to) when every
+// MMA issued so far has finished
+template <int CG> __device__ __forceinline__ void mlcb_mma_commit(u32 bar, u32 rank = 0) {
+    if (CG == 1)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     :: "r"(bar), "h"((unsigned short)(3u << (rank & ~1u))) : "memory");
+}
+// 16 or 32 consecutive fp32 columns of this warp's 32 lanes.  The wait is part of the
+// statement: no use of the registers can be scheduled ahead of it.
+__device__ __forceinline__ void mlcb_tmem_ld(u32 addr, float (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n tcgen05.wait::ld.sync.aligned;"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mlcb_tmem_ld(u32 addr, float (&v)[32]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n tcgen05.wait::ld.sync.aligned;"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31]) : "r"(addr) : "memory");
+}
+
+// Shared-memory matrix descriptor, 128-byte swizzle.  `lbo`: bytes between the
+// 64-wide blocks of an MN-major tile (unused for K-major); eight rows of 128 bytes
+// per atom in both cases.
+__device__ __forceinline__ u64 mlcb_desc(u32 addr, u32 lbo) {
+    return (u64)((addr & 0x3FFFFu) >> 4) | ((u64)(lbo >> 4) << 16) | ((u64)(1024u >> 4) << 32)
+         | ((u64)1 << 46) | ((u64)2 << 61);
+}
+// instruction descriptor of kind::f16: fp32 accumulator, A and B both fp16 or both bf16
+__device__ constexpr u32 mlcb_idesc(int m, int n, bool bf16, bool b_mn) {
+    return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((b_mn ? 1u : 0u) << 16)
+         | ((u32)(n >> 3) << 17) | ((u32)(m >> 4) << 24);
+}

@@ -1,0 +1,290 @@
+"""Attention kernels: the row functor ``csrc/mlcb_attention.cuh`` runs over the scores.
+
+The functor is the schedule's own row kernel (scale, mask, softmax, casts) for the rows
+of one tile, the score entering as the value the separate matmul would have stored.
+Several threads share a row; up to 64 columns each, its values stay in registers, beyond
+that every phase reads the scores from TMEM again.
+"""
+
+from __future__ import annotations
+
+from .. import kir
+from ..fuse import AttentionKernel
+from ..kir import Bind
+from . import expr as X
+from .indexing import check_bounds, classify, needs_64bit, render_offset
+from .matmul import _ceil, operand_map
+from .pointwise import LaunchSpec, algorithmic_bytes, store_code
+from .reduction import _OP, _acc_dtype, _identity, plan_geometry, varying_steps
+
+
+def split_row(k: AttentionKernel, cfg) -> tuple[int, int, int]:
+    """(H, V, G): threads per query row, and the order a row's sums are taken in --
+    column c belongs to lane ``(c // V) % G``, lanes add their columns in order, then a
+    butterfly over the lanes.  That is the stand-alone row kernel's order where it can be:
+    each of the H threads takes G / H neighbouring lanes of every period of ``V * G``
+    columns, so that no lane is divided.  Four threads per row: at one, 128 keys took
+    11.8 us per tile (4 warps cannot hide the latency of a row's chains), at four 3 us."""
+    rows = k.rows
+    operands = [a for a in rows.inputs if a.index.varies_along("col")] + [rows.outputs[0]]
+    geo = plan_geometry(rows.n_rows, rows.n_cols, operands, cfg, False)
+    H = 4
+    if geo.G <= 16 and geo.V * geo.G // H in (16, 32):
+        return H, geo.V, geo.G
+    return H, 8, 8
+
+
+def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[str, list, list]:
+    rows, slot = k.rows, k.slot
+    S, T = rows.n_cols, k.q.shape[1]
+    st = X.STORAGE_T[k.dtype]
+    rn = "mlcb_rn_f16" if k.dtype == "float16" else "mlcb_rn_bf16"
+    out = rows.outputs[0]
+    period, lanes = V * G, G // H
+    width = V * lanes                          # neighbouring columns per thread and period
+    NC = _ceil(S, period) * width              # columns per thread
+    whole = S // period * width                # of them inside the row whatever the thread
+    keep = NC <= 64                            # row values stay in registers between phases
+    extents = [rows.n_rows * S] + [a.index.bounds()[1] + 1 for a in rows.inputs]
+    it = "i64" if needs_64bit(*extents) else "int"
+    vec = varying_steps(rows)
+
+    params, names, L = [], [], []
+    for i, a in enumerate(rows.inputs):
+        if i != slot:
+            r = " __restrict__" if a.buffer in stable else ""
+            params.append(f"const {X.STORAGE_T[a.dtype]}*{r} in{i}")
+            names.append(a.buffer)
+    emit = L.append
+    emit("struct MLCB_KERNEL_NAME_rows {")
+    L += [f"    {p};" for p in params]
+    emit("    __device__ __forceinline__ void run(u32 tm, u32 sp, int g, int t, int r, int h, float* red, u32 ready, "
+         "volatile u32* dead) const {")
+    emit(f"        const {it} row = ({it})g * {T} + t;")
+    emit(f"#define MLCB_COL(j) ((j) / {width} * {period} + h * {width} + (j) % {width})")
+    scalars: dict[str, X.Val] = {}
+    loads: list = []
+    packed: dict[int, bool] = {}
+    for i, a in enumerate(rows.inputs):
+        vdt, ct = X.promoted_load_dtype(a.dtype), X.STORAGE_T[a.dtype]
+        if i == slot:
+            loads.append(X.Val("s[j]", "float32", True, True))
+        elif not a.index.varies_along("col"):
+            emit(f"        const {X.REG_T[a.dtype]} s{i} = mlcb_load1<{ct}>(in{i} + "
+                 f"({render_offset(a.index, {'row': 'row'}, skip=('col',))}));  // {a.name} (per row)")
+            loads.append(X.Val(f"s{i}", vdt))
+        else:
+            emit(f"        const {it} in{i}_r = {render_offset(a.index, {'row': 'row'}, skip=('col',))};")
+            ac = classify(a.index, "col", 8)
+            packed[i] = ac.mode == "contig" and ac.width == 8
+            loads.append(X.Val(f"x{i}[j]", vdt, True, True))
+
+    def fetch(i, lo, n, ind):
+        """Columns ``[lo, lo + n)`` of this thread of operand i, into ``x{i}``."""
+        a, B = rows.inputs[i], []
+        ct = X.STORAGE_T[a.dtype]
+        step = 8 if packed[i] else 1
+        B.append("#pragma unroll")
+        B.append(f"{ind}for (int j = 0; j < {n}; j += {step}) {{")
+        col = f"MLCB_COL({lo} + j)"
+        off = render_offset(a.index, {"col": col}, skip=("row", "base"))
+        guard = f"if ({lo} + j < {whole} || {col} < {S}) " if lo + n > whole else ""
+        if packed[i]:
+            B.append(f"{ind}    {guard}mlcb_load_at<{ct}, 8, {n}>(in{i} + in{i}_r + ({off}), x{i}, j);")
+        else:
+            B.append(f"{ind}    {guard}x{i}[j] = mlcb_load1<{ct}>(in{i} + in{i}_r + ({off}));")
+        B.append(f"{ind}}}")
+        return B
+
+    def scores(lo, n, ind):
+        B = []
+        for c in range(0, n, 16):
+            B.append(f"{ind}{{ float raw[16]; mlcb_tmem_ld(tm + MLCB_COL({lo + c}), raw);")
+            B.append("#pragma unroll")
+            B.append(f"{ind}  for (int i = 0; i < 16; ++i) s[{c} + i] = {rn}(raw[i]); }}")
+        return B
+
+    if keep:
+        for i in packed:
+            emit(f"        {X.REG_T[rows.inputs[i].dtype]} x{i}[{NC}];  // {rows.inputs[i].name}")
+            L += fetch(i, 0, NC, "        ")
+        emit("        mlcb_bar_wait(ready, 0, dead);")
+        emit("        mlcb_tc_after();")
+        emit(f"        float s[{NC}];")
+        L += scores(0, NC, "        ")
+    else:
+        emit("        mlcb_bar_wait(ready, 0, dead);")
+        emit("        mlcb_tc_after();")
+
+    def needed(expr, upto):
+        """Vector binds ``expr`` reads, transitively, in order."""
+        want = set(kir.expr_refs(expr)) & vec
+        for sp in reversed(rows.steps[:upto]):
+            if isinstance(sp, Bind) and sp.name in want:
+                want |= set(kir.expr_refs(sp.expr)) & vec
+        return [sp for sp in rows.steps[:upto] if isinstance(sp, Bind) and sp.name in want]
+
+    done: dict[str, X.Val] = {}                # vector values already in registers (keep)
+
+    def phase(expr, upto, close, elide=frozenset()):
+        """One pass over this thread's columns; ``close(lines, value)`` ends an element."""
+        binds = [b for b in needed(expr, upto) if b.name not in done]
+        step = NC if keep else 16
+        refs = dict(scalars)
+        refs.update(done)
+        body, decl = [], []
+        for b in binds:
+            v = X.render_bind(b.name, b.expr, loads, refs, elide)
+            if keep:
+                decl.append(f"        {X.REG_T[v.dtype]} {b.name}[{NC}];")
+                body.append(f"{b.name}[j] = {v.code};")
+                refs[b.name] = done[b.name] = X.Val(f"{b.name}[j]", v.dtype, v.dim, True)
+            else:
+                body.append(f"const {X.REG_T[v.dtype]} {b.name} = {v.code};")
+                refs[b.name] = X.Val(b.name, v.dtype, v.dim, True)
+        value = X.render(expr, loads, refs)
+        slots = set(kir.expr_loads(expr)).union(*[kir.expr_loads(b.expr) for b in binds]) if binds else \
+            set(kir.expr_loads(expr))
+        for d in decl:
+            emit(d)
+        ind = "        "
+        for lo in range(0, NC, step):
+            if not keep:
+                emit("        {")
+                emit(f"        if (MLCB_COL({lo}) < {S}) {{" if lo + step > whole else "        {")
+                for i in packed:
+                    if i in slots:
+                        emit(f"        {X.REG_T[rows.inputs[i].dtype]} x{i}[16];")
+                        L.extend(fetch(i, lo, 16, ind))
+                emit("        float s[16];")
+                L.extend(scores(lo, 16, ind))
+            close(lo, step, body, value)
+            if not keep:
+                emit("        }}")
+
+    nred = 0
+    for pos, sp in enumerate(rows.steps):
+        if isinstance(sp, Bind):
+            if sp.name not in vec:
+                v = X.render(sp.expr, loads, scalars)
+                emit(f"        const {X.REG_T[v.dtype]} {sp.name} = {v.code};")
+                scalars[sp.name] = X.Val(sp.name, v.dtype, v.dim, False)
+            continue
+        ordered = sp.kind in ("sum", "prod")
+        probe = dict(scalars)
+        probe.update(done)
+        for b in needed(sp.expr, pos):
+            if b.name not in probe:
+                v = X.render(b.expr, loads, probe)
+                probe[b.name] = X.Val(b.name, v.dtype, v.dim, True)
+        rv = X.render(sp.expr, loads, probe)
+        rdt = X.reduce_type(sp.kind, rv.dtype)
+        adt = _acc_dtype(rdt)
+        at, op = X.REG_T[adt], _OP[sp.kind]
+        n = lanes if ordered else 4
+        emit(f"        {at} a_{sp.name}[{n}];")
+        emit("#pragma unroll")
+        emit(f"        for (int i = 0; i < {n}; ++i) a_{sp.name}[i] = {_identity(sp.kind, adt)};")
+
+        def close(lo, step, body, value, sp=sp, at=at, adt=adt, op=op, ordered=ordered):
+            acc = f"a_{sp.name}[{f'({lo} + j) % {width} / {V}' if ordered else 'j % 4'}]"
+            emit("#pragma unroll")
+            emit(f"        for (int j = 0; j < {step}; ++j) {{")
+            for ln in body:
+                emit("            " + ln)
+            guard = f"if ({lo} + j < {whole} || MLCB_COL({lo} + j) < {S}) " if lo + step > whole else ""
+            emit(f"            {guard}{acc} = {op}::f({acc}, ({at}){X.convert(value.code, value.dtype, adt)});")
+            emit("        }")
+        phase(sp.expr, pos, close)
+        # the row's lanes (or its H parts) meet in shared memory, every thread combines them alike
+        if not ordered:
+            emit(f"        a_{sp.name}[0] = {op}::f({op}::f(a_{sp.name}[0], a_{sp.name}[1]), "
+                 f"{op}::f(a_{sp.name}[2], a_{sp.name}[3]));")
+        own, total = (lanes, G) if ordered else (1, H)
+        base = f"red + {(nred % 2) * G * 128} + r"
+        nred += 1
+        emit("#pragma unroll")
+        emit(f"        for (int i = 0; i < {own}; ++i) ({base})[(h * {own} + i) * 128] = a_{sp.name}[i];")
+        emit("        __syncthreads();")
+        emit(f"        {at} b_{sp.name}[{total}];")
+        emit("#pragma unroll")
+        emit(f"        for (int i = 0; i < {total}; ++i) b_{sp.name}[i] = ({base})[i * 128];")
+        emit("#pragma unroll")
+        emit(f"        for (int m = {total // 2}; m > 0; m >>= 1)")
+        emit("#pragma unroll")
+        emit(f"            for (int i = 0; i < m; ++i) b_{sp.name}[i] = {op}::f(b_{sp.name}[i], b_{sp.name}[i + m]);")
+        code = f"b_{sp.name}[0]"
+        if rdt in kir.NARROW_FLOATS:
+            code = X.convert(code, "float32", rdt)
+        emit(f"        const {X.REG_T[rdt]} {sp.name} = {code};")
+        scalars[sp.name] = X.Val(sp.name, rdt, True, False)
+
+    oe = rows.out_expr[out.name]
+    upto = len(rows.steps)
+    elide = X.store_only_casts([(b.name, b.expr) for b in needed(oe, upto) if b.name not in done],
+                               {out.name: oe}, [out])
+
+    def close_store(lo, step, body, value):
+        emit("#pragma unroll")
+        emit(f"        for (int q = 0; q < {step}; q += 8) {{")
+        if lo + step > whole:
+            emit(f"            if ({lo} + q >= {whole} && MLCB_COL({lo} + q) >= {_ceil(S, 16) * 16}) continue;")
+        emit("            float o[8];")
+        emit("#pragma unroll")
+        emit("            for (int i = 0; i < 8; ++i) {")
+        emit("                const int j = q + i;")
+        for ln in body:
+            emit("                " + ln)
+        code = store_code(value, out.dtype)
+        if lo + step > whole:
+            code = f"({lo} + j < {whole} || MLCB_COL({lo} + j) < {S}) ? {code} : 0.0f"
+        emit(f"                o[i] = {code};  // {out.name}")
+        emit("            }")
+        emit(f"            mlcb_store_p<{st}>(sp, r, MLCB_COL({lo} + q), o);")
+        emit("        }")
+    phase(oe, upto, close_store, elide)
+    emit("#undef MLCB_COL")
+    emit("    }")
+    emit("};")
+    return "\n".join(L), params, names
+
+
+def emit_attention(k: AttentionKernel, cfg, buffers, name: str | None = None, stable=frozenset()):
+    name = name or k.name
+    G, T, D = k.q.shape
+    S = k.k.shape[2]
+    H, V, lanes = split_row(k, cfg)
+    for i, a in enumerate(k.rows.inputs):
+        if i != k.slot:
+            check_bounds(a.index, buffers[a.buffer].numel, f"{k.name}:{a.name}")
+    with X.math_mode(X.wants_fast_math(k.rows, cfg)):
+        functor, params, names = _functor(k, cfg, H, V, lanes, stable)
+    st = X.STORAGE_T[k.dtype]
+    s16 = _ceil(S, 16) * 16
+    halves = _ceil(s16, 256)
+    keys = s16 if halves == 1 else _ceil(s16 // 2, 16) * 16
+    db = D // 64
+    tmaps = (operand_map(k.q, k.dtype, -2, -1, 128, db), operand_map(k.k, k.dtype, -1, -2, keys, db),
+             operand_map(k.v, k.dtype, -1, -2, keys))
+    conf = f"mlcb_att_cfg<{G}, {T}, {S}, {D}, {H}, {2 * lanes * 128}, {'true' if k.dtype == 'bfloat16' else 'false'}>"
+    q_bytes, kv_bytes, p_bytes = db * 16384, db * halves * keys * 128, _ceil(S, 64) * 16384
+    smem = max(q_bytes + kv_bytes, p_bytes) + kv_bytes + 1024
+    cols = next(c for c in (64, 128, 256, 512) if c >= max(halves * keys, D))
+    # two CTAs per SM (64 registers) when a thread's share of the row is 32 values
+    resident = 2 if S <= 128 and cols <= 256 else 1
+    sig = ", ".join(["const __grid_constant__ mlcb_tmap tq", "const __grid_constant__ mlcb_tmap tk",
+                     "const __grid_constant__ mlcb_tmap tv"] + params + [f"{st}* out"])
+    fields = ", ".join(p.split()[-1] for p in params)
+    text = "\n".join([
+        functor.replace("MLCB_KERNEL_NAME", name),
+        f'extern "C" __global__ void __launch_bounds__({128 * H}, {resident}) {name}({sig}) {{',
+        f"    // {G} x ([{T}, {D}] x [{D}, {S}] -> rows -> x [{S}, {D}]); {H} thread(s) per query row",
+        f"    const {name}_rows rows{{{fields}}};",
+        f"    mlcb_attention<{conf}>(&tq, &tk, &tv, rows, out + {k.out.offset}, (i64){k.out.strides[0]}, "
+        f"(i64){k.out.strides[1]});",
+        "}"])
+    total = 2 * sum(v.numel for v in (k.q, k.k, k.v, k.out)) + algorithmic_bytes(
+        [a for i, a in enumerate(k.rows.inputs) if i != k.slot], [], k.rows.n_rows * S)
+    spec = LaunchSpec(grid=G * _ceil(T, 128), block=128 * H, smem=smem, alg_bytes=total, tmaps=tmaps,
+                      buffers=tuple(names + [k.out.buffer]))
+    return text, spec

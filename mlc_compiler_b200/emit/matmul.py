@@ -1,0 +1,349 @@
+"""Matmul kernels: the configuration of ``csrc/mlcb_matmul.cuh`` for a shape, and the
+epilogue functor it calls with finished accumulators.
+
+The functor is the text a pointwise kernel would have: operands at the offsets their
+index maps give for ``(row, col)``, the body over a pack of consecutive columns held in
+registers, packed stores.  The accumulator enters as the value the library's matmul
+would have stored (rounded to the storage type), so folding a kernel in changes no
+result.
+"""
+
+from __future__ import annotations
+
+from dataclasses import dataclass
+
+from .. import kir
+from ..fuse import MatmulKernel, tma_layout
+from . import expr as X
+from .indexing import check_bounds, classify, needs_64bit, render_offset
+from .pointwise import LaunchSpec, algorithmic_bytes, store_code
+
+SM_COUNT = 148
+#: dynamic shared memory a CTA may ask for (static barriers take under 1 KB of 227)
+SMEM_MAX = 224 * 1024
+
+
+@dataclass(frozen=True)
+class TensorMap:
+    """What ``cuTensorMapEncodeTiled`` needs for one 16-bit operand: four dimensions,
+    innermost first, byte strides of the outer three, and the box of one load."""
+
+    buffer: str
+    offset: int                 # elements
+    dtype: str
+    dims: tuple[int, int, int, int]
+    strides: tuple[int, int, int]    # bytes
+    box: tuple[int, int, int]
+
+
+def can_cut(v: kir.View, rows_axis: int, k_axis: int) -> bool:
+    """Whether K-major operand ``v`` is a whole number of 64-element blocks along K."""
+    return tma_layout(v, rows_axis, k_axis) == "k" and v.shape[k_axis] % 64 == 0
+
+
+def operand_map(v: kir.View, dtype: str, rows_axis: int, k_axis: int, box_rows: int, blocks: int = 1) -> TensorMap:
+    """128-byte-swizzled loads of a matrix operand: ``box_rows`` rows of 64 elements,
+    ``blocks`` times along K where K is cut into blocks (:func:`can_cut`)."""
+    layout = tma_layout(v, rows_axis, k_axis)
+    inner, outer = (k_axis, rows_axis) if layout == "k" else (rows_axis, k_axis)
+    n, s = v.shape, v.strides
+    z = n[0] if len(n) == 3 else 1
+    row_bytes = 2 * s[outer] if n[outer] > 1 else 16 * -(-n[inner] // 8)
+    z_bytes = 2 * s[0] if z > 1 else row_bytes
+    if can_cut(v, rows_axis, k_axis):
+        return TensorMap(v.buffer, v.offset, dtype, (64, n[outer], n[inner] // 64, z), (row_bytes, 128, z_bytes),
+                         (64, box_rows, blocks))
+    return TensorMap(v.buffer, v.offset, dtype, (n[inner], n[outer], 1, z), (row_bytes, row_bytes, z_bytes),
+                     (64, box_rows, 1))
+
+
+@dataclass(frozen=True)
+class Config:
+    bn: int          # columns per tile
+    stages: int
+    acc: int         # accumulators in TMEM (2: a tile's epilogue overlaps the next one's MMAs)
+    split: int       # CTAs of a cluster that share a tile's K
+    cg: int          # CTAs of a pair (tcgen05 cta_group)
+    epi_warps: int
+    grid: int
+    kstep: int = 1   # 64-element K blocks per stage
+
+    def stage_bytes(self) -> int:
+        return self.kstep * (128 * 128 + self.bn // self.cg * 128)
+
+    def smem(self) -> int:
+        inbox = 128 * self.bn * 4 if self.split > 1 else 0
+        return self.stages * self.stage_bytes() + inbox + 1024
+
+
+def _ceil(a: int, b: int) -> int:
+    return -(-a // b)
+
+
+#: clusters of 2, 4 and 8 CTAs that are resident at once (larger ones do not tile the GPCs)
+_RESIDENT = {1: SM_COUNT, 2: 74, 4: 32, 8: 14}
+
+
+def _estimate(z, m, n, k, groups, b_mn, can_step, splits):
+    """Least estimated time over tiles, pairing and the given splits.
+
+    The estimate is what launches of this kernel measured on a B200 (microseconds,
+    dependent launches, operands in L2).  A 64-element K block takes 0.10 + 0.00075 per
+    column: shared memory moves 128 bytes per clock, and each block's operands cross it
+    twice, in by TMA and out to the tensor cores, which narrow tiles cannot hide behind
+    MMA time.  A pair halves B's share of that and pays 0.4 for keeping in step.  A launch
+    costs 2.1 before and after, and 0.005 per column of its last epilogue; splitting K
+    over a cluster adds the exchange of partial sums."""
+    kb = _ceil(k, 64)
+    best = None
+    for cg in (1, 2):
+        if cg == 2 and (b_mn or m <= 128):
+            continue
+        for bn in (64, 128, 192, 256) if b_mn else (32, 64, 96, 128, 160, 192, 224, 256):
+            if bn > 64 and bn - 32 >= n:
+                continue
+            t = _ceil(m, 128 * cg) * _ceil(n, bn) * groups * z
+            kstep = 2 if bn <= 96 and kb > 1 and can_step else 1
+            for split in splits:
+                if split > 1 and (cg == 2 or bn > 128 or bn % (8 * split) or _ceil(kb, kstep) < split):
+                    continue
+                waves = _ceil(t, _RESIDENT[split * cg])
+                exchange = 0.3 * (split.bit_length() - 1) + 0.012 * bn if split > 1 else 0.0
+                step = 0.10 + 0.00075 * bn if cg == 1 else 0.095 + 0.00065 * bn
+                cost = waves * _ceil(kb, split) * step + 2.1 + 0.4 * (cg - 1) + 0.005 * bn + exchange
+                if best is None or cost < best[0]:
+                    best = (cost, bn, split, cg, t, kstep)
+    return best
+
+
+def split_for(m: int, n: int, k: int, b_mn: bool = False, can_step: bool = True) -> int:
+    """CTAs that share the K of one result tile.  It decides the order in which products
+    are summed, so it depends on the matmul's own shape alone, never on what it shares a
+    launch with.  Up to K = 1024 two halves pay only while the result is small ([128, 768] x
+    [768, 768]: 3.6 us against 3.7, and 4.0 in four parts; N = 2304: 4.3 against 4.2;
+    M = 512: 5.0 against 4.1)."""
+    kb = _ceil(k, 64)
+    if kb <= 16:
+        return 2 if _ceil(m, 128) * n <= 1536 and kb >= 8 and can_step and not b_mn else 1
+    return _estimate(1, m, n, k, 1, b_mn, can_step, (1, 2, 4, 8))[2]
+
+
+def choose(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, can_step: bool = True) -> Config:
+    """Tile, split and pairing for a shape."""
+    split = split_for(m, n, k, b_mn, can_step) if z == 1 else 1
+    found = _estimate(z, m, n, k, groups, b_mn, can_step, (split,))
+    _, bn, split, cg, t, kstep = found
+    persistent = split == 1 and t > SM_COUNT // cg
+    acc = 2 if persistent else 1
+    grid = t * split if split > 1 else min(t, SM_COUNT // cg) * cg
+    probe = Config(bn, 0, acc, split, cg, 8 if bn >= 128 else 4, grid, kstep)
+    steps = _ceil(_ceil(_ceil(k, 64), kstep), split)
+    stages = max(2, min((SMEM_MAX - probe.smem()) // probe.stage_bytes(), 8, steps if not persistent else 8))
+    return Config(bn, stages, acc, split, cg, probe.epi_warps, grid, kstep)
+
+
+# --------------------------------------------------------------------------
+# epilogue functor
+# --------------------------------------------------------------------------
+
+#: functions with a form on register pairs (``mlcb_f2``)
+_PAIRED = {"add", "sub", "mul", "erf", "tanh", "exp", "sigmoid"}
+
+
+def _paired(e, W: int) -> bool:
+    """Whether the epilogue can run on pairs of neighbouring columns."""
+    exprs = [x for _, x in e.body] + list(e.out_expr.values())
+    return (W % 2 == 0 and bool(e.body) and X._FAST
+            and all(a.dtype in kir.NARROW_FLOATS for a in e.outputs)
+            and all(a is None or a.dtype in kir.NARROW_FLOATS + ("float32",) for a in e.inputs)
+            and all(a is None or classify(a.index, "col", W).width == W for a in e.inputs)
+            and all(not isinstance(s, kir.Call) or s.fn in _PAIRED for x in exprs for s in kir.walk(x))
+            and all(not isinstance(s, kir.Cast) or s.dtype in kir.NARROW_FLOATS + ("float32",)
+                    for x in exprs for s in kir.walk(x)))
+
+
+def _pack_width(epilogues, n: int, cap: int) -> int:
+    w = cap
+    while w > 1 and n % w:
+        w //= 2
+    for e in epilogues:
+        for a in e.outputs:
+            ac = classify(a.index, "col", cap)
+            w = min(w, ac.width if ac.mode == "contig" else 1)
+    return w
+
+
+def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, list]:
+    """(struct text, parameter declarations, buffer names in parameter order)."""
+    z, m, n, _ = k.shape
+    e0 = k.epilogues[0]
+    params: list[str] = []
+    buffers: list[str] = []
+    seen: dict[tuple, str] = {}
+
+    def pointer(a, ctype, const):
+        key = (a.buffer, const)
+        if key not in seen:
+            seen[key] = f"p{len(params)}"
+            params.append(f"{'const ' if const else ''}{ctype}* {seen[key]}")
+            buffers.append(a.buffer)
+        return seen[key]
+
+    L: list[str] = ["struct MLCB_KERNEL_NAME_epi {"]
+    fields: list[str] = []
+    selects: list[str] = []
+    for what, ops in (("in", e0.inputs), ("out", e0.outputs)):
+        for i, a in enumerate(ops):
+            if a is None:
+                continue
+            st = X.STORAGE_T[a.dtype]
+            names = [pointer((e.inputs if what == "in" else e.outputs)[i], st, what == "in")
+                     for e in k.epilogues]
+            const = "const " if what == "in" else ""
+            sel = names[-1]
+            for g in range(len(names) - 2, -1, -1):
+                if names[g] != names[-1] or len(set(names)) > 1:
+                    sel = f"(g == {g} ? {names[g]} : {sel})"
+            selects.append(f"        {const}{st}* __restrict__ {what}{i} = {sel};" if what == "in" and all(
+                e.inputs[i].buffer in stable for e in k.epilogues) else f"        {const}{st}* {what}{i} = {sel};")
+    fields = [f"    {p};" for p in params]
+    L += fields
+
+    extents = [z * m * n] + [a.index.bounds()[1] + 1 for e in k.epilogues
+                             for a in [x for x in e.inputs if x is not None] + e.outputs]
+    it = "i64" if needs_64bit(*extents) else "int"
+    nv = 8 if mc.split > 1 else 32
+    W = _pack_width(k.epilogues, n, 8 if nv == 8 else 16)
+    row_expr = "row" if z == 1 else f"(z * {m} + row)"
+    rn = "mlcb_rn_f16" if k.dtype == "float16" else "mlcb_rn_bf16"
+    plain = not e0.body and len(e0.outputs) == 1 and e0.outputs[0].dtype == k.dtype
+
+    L.append("    template <int NV> __device__ __forceinline__ void columns(float (&v)[NV], int row, int col, "
+             "int g, int z, int lane) const {")
+    L += selects
+    if plain and W == 1 and e0.outputs[0].index.axis("col").terms == ((n, 1, 1),) and nv == 32 and z == 1:
+        # rows that start at odd addresses: 32 x 32 elements turn in shared memory so that a
+        # warp writes one row's 32 elements together
+        st = X.STORAGE_T[k.dtype]
+        a = e0.outputs[0]
+        off = render_offset(a.index, {"row": "rr", "col": "(col + lane)"})
+        L.append(f"        __shared__ {st} turn[{mc.epi_warps}][32][34];")
+        L.append(f"        {st} (*t)[34] = turn[threadIdx.x / 32 - 2];")
+        L.append("#pragma unroll")
+        L.append(f"        for (int j = 0; j < 32; ++j) t[lane][j] = mlcb_elem<{st}>::put(v[j]);")
+        L.append("        __syncwarp();")
+        L.append(f"        if (col + lane < {n}) {{")
+        L.append(f"            const int first = row - lane, count = min(32, {m} - first);")
+        L.append("#pragma unroll 8")
+        L.append("            for (int i = 0; i < count; ++i) {")
+        L.append(f"                const {it} rr = first + i;")
+        L.append(f"                out0[{off}] = t[i][lane];")
+        L.append("            }")
+        L.append("        }")
+        L.append("        __syncwarp();")
+    else:
+        L.append(f"        if (row >= {m}) return;")
+        L.append(f"        const {it} r = {row_expr};")
+        for what, ops in (("in", e0.inputs), ("out", e0.outputs)):
+            for i, a in enumerate(ops):
+                if a is not None:
+                    L.append(f"        const {it} {what}{i}_r = {render_offset(a.index, {'row': 'r'}, skip=('col',))};")
+        L.append("#pragma unroll")
+        L.append(f"        for (int c = 0; c < NV; c += {W}) {{")
+        L.append(f"            const int c0 = col + c;")
+        if n % mc.bn or W == 1:
+            L.append(f"            if (c0 >= {n}) break;")
+        loads: list[X.Val] = []
+        late: list[str] = []
+        pairs = _paired(e0, W)
+        for i, a in enumerate(e0.inputs):
+            if a is None and pairs:
+                loads.append(X.Val(f"{rn}(mlcb_f2(v[c + j], v[c + j + 1]))", "float32", True, False))
+                continue
+            if a is None:
+                loads.append(X.Val(f"{rn}(v[c + j])", "float32", True, False, (f"v[c + j]", k.dtype)))
+                continue
+            st, rt = X.STORAGE_T[a.dtype], X.REG_T[a.dtype]
+            ac = classify(a.index, "col", W)
+            off = render_offset(a.index, {"col": "c0"}, skip=("row", "base"))
+            vdt = X.promoted_load_dtype(a.dtype)
+            if ac.mode == "bcast" and ac.width == W:
+                L.append(f"            const {rt} x{i} = mlcb_load1<{st}>(in{i} + in{i}_r + ({off}));  // {a.name}")
+                loads.append(X.Val(f"x{i}", vdt))
+            elif ac.mode == "contig" and ac.width == W and W > 1:
+                L.append(f"            {rt} x{i}[{W}]; mlcb_load<{st}, {W}>(in{i} + in{i}_r + ({off}), x{i});  // {a.name}")
+                loads.append(X.Val(f"mlcb_f2(x{i}[j], x{i}[j + 1])" if pairs else f"x{i}[j]", vdt))
+            else:
+                off = render_offset(a.index, {"col": "(c0 + j)"}, skip=("row", "base"))
+                late.append(f"                const {rt} x{i} = mlcb_load1<{st}>(in{i} + in{i}_r + ({off}));  // {a.name}")
+                loads.append(X.Val(f"x{i}", vdt))
+        for i, a in enumerate(e0.outputs):
+            L.append(f"            {X.REG_T[a.dtype]} o{i}[{W}];")
+        L.append("#pragma unroll")
+        L.append(f"            for (int j = 0; j < {W}; j += {2 if pairs else 1}) {{")
+        L += late
+        refs: dict[str, X.Val] = {}
+        elide = X.store_only_casts(e0.body, e0.out_expr, e0.outputs)
+        for temp, ex in e0.body:
+            v = X.render_bind(temp, ex, loads, refs, elide)
+            L.append(f"                const {'mlcb_f2' if pairs else X.REG_T[v.dtype]} {temp} = {v.code};")
+            refs[temp] = X.Val(temp, v.dtype, v.dim)
+        for i, a in enumerate(e0.outputs):
+            v = X.render(e0.out_expr[a.name], loads, refs)
+            if pairs:
+                L.append(f"                mlcb_f2({store_code(v, a.dtype)}).get(o{i}[j], o{i}[j + 1]);  // {a.name}")
+                continue
+            L.append(f"                o{i}[j] = {store_code(v, a.dtype)};  // {a.name}")
+        L.append("            }")
+        for i, a in enumerate(e0.outputs):
+            off = render_offset(a.index, {"col": "c0"}, skip=("row", "base"))
+            L.append(f"            mlcb_store<{X.STORAGE_T[a.dtype]}, {W}>(out{i} + out{i}_r + ({off}), o{i});")
+        L.append("        }")
+    L.append("    }")
+    L.append("};")
+    return "\n".join(L), params, buffers
+
+
+def emit_matmul(k: MatmulKernel, cfg, buffers, name: str | None = None, stable=frozenset()):
+    """(text, LaunchSpec) of one matmul kernel; the launch passes the tensor maps, then
+    the epilogue's pointers."""
+    name = name or k.name
+    z, m, n, kk = k.shape
+    b_mn = tma_layout(k.bs[0], -1, -2) == "mn"
+    a_cut, b_cut = can_cut(k.a, -2, -1), can_cut(k.bs[0], -1, -2)
+    mc = choose(z, m, n, kk, len(k.bs), b_mn, a_cut and (b_cut or b_mn))
+    for e in k.epilogues:
+        for a in [x for x in e.inputs if x is not None] + e.outputs:
+            check_bounds(a.index, buffers[a.buffer].numel, f"{k.name}:{a.name}")
+
+    class _Outs:                                   # what ``wants_fast_math`` looks at
+        outputs = [a for e in k.epilogues for a in e.outputs]
+    with X.math_mode(X.wants_fast_math(_Outs, cfg)):
+        functor, params, names = _emit_functor(k, cfg, mc, stable)
+    b_stable = all(b.buffer in stable for b in k.bs)
+    flag = lambda x: "true" if x else "false"      # noqa: E731
+    conf = (f"mlcb_mm_cfg<{m}, {n}, {_ceil(kk, 64)}, {mc.kstep}, {flag(a_cut)}, {flag(b_cut)}, {mc.bn}, {mc.stages}, {mc.acc}, {mc.split}, {mc.cg}, "
+            f"{len(k.bs)}, {z}, {mc.epi_warps}, {flag(b_mn)}, {flag(k.dtype == 'bfloat16')}, {flag(b_stable)}>")
+    tmaps = [operand_map(k.a, k.dtype, -2, -1, 128, mc.kstep)]
+    for b in k.bs:
+        tmaps.append(operand_map(b, k.dtype, -1, -2, 64 * mc.kstep if b_mn else mc.bn // mc.cg, mc.kstep))
+    targs = ["ta"] + [f"tb{i}" for i in range(len(k.bs))]
+    threads = 64 + 32 * mc.epi_warps
+    sig = ", ".join([f"const __grid_constant__ mlcb_tmap {t}" for t in targs] + params)
+    fields = ", ".join(p.split("* ")[1] for p in params)
+    tb = [f"&tb{min(i, len(k.bs) - 1)}" for i in range(4)]
+    cluster = mc.split * mc.cg
+    text = "\n".join([
+        functor.replace("MLCB_KERNEL_NAME", name),
+        f'extern "C" __global__ void __launch_bounds__({threads}, 1) {name}({sig}) {{',
+        f"    // {z} x [{m}, {kk}] x [{kk}, {n}] x {len(k.bs)}; tile {128 * mc.cg} x {mc.bn}, {mc.stages} stages, "
+        f"{mc.acc} accumulator(s), split {mc.split}, grid {mc.grid}, cluster {cluster}",
+        f"    const {name}_epi epi{{{fields}}};",
+        f"    mlcb_matmul<{conf}>(&ta, {', '.join(tb)}, epi);",
+        "}"])
+    total = sum(v.numel for v in [k.a] + k.bs) * 2
+    total += sum(algorithmic_bytes([x for x in e.inputs if x is not None], e.outputs, z * m * n)
+                 for e in k.epilogues)
+    spec = LaunchSpec(grid=mc.grid, block=threads, smem=mc.smem(), vector=1, alg_bytes=total, cluster=cluster,
+                      tmaps=tuple(tmaps), buffers=tuple(names))
+    return text, spec

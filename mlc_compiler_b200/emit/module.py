@@ -20,10 +20,14 @@ import re
 from dataclasses import dataclass, field
 
 from .. import kir
+from ..fuse import AttentionKernel, MatmulKernel
+from .attention import emit_attention
+from .matmul import emit_matmul
 from .pointwise import LaunchSpec, emit_pointwise
 from .reduction import emit_reduction
 
-DEVICE_HEADER = pathlib.Path(__file__).resolve().parent.parent / "csrc" / "mlcb_device.cuh"
+CSRC = pathlib.Path(__file__).resolve().parent.parent / "csrc"
+DEVICE_HEADER = CSRC / "mlcb_device.cuh"
 
 BANNER = """// Generated by mlc_compiler_b200 for sm_100a. Do not edit.
 //
@@ -57,11 +61,22 @@ def device_header() -> str:
     return DEVICE_HEADER.read_text()
 
 
+def tensor_headers(kinds: set) -> list[str]:
+    """The tensor-core parts of the device library that kernels of these kinds use."""
+    files = ["mlcb_tensor.cuh"] * bool(kinds & {"mm", "att"}) + ["mlcb_matmul.cuh"] * ("mm" in kinds) \
+        + ["mlcb_attention.cuh"] * ("att" in kinds)
+    return [(CSRC / f).read_text().replace("#pragma once\n", "") for f in files]
+
+
 def emit_kernel(k, cfg, buffers=None, name: str | None = None, stable=frozenset()):
     if isinstance(k, kir.PointwiseKernel):
         return emit_pointwise(k, cfg, buffers, name, stable)
     if isinstance(k, kir.ReductionKernel):
         return emit_reduction(k, cfg, buffers, name, stable)
+    if isinstance(k, MatmulKernel):
+        return emit_matmul(k, cfg, buffers, name, stable)
+    if isinstance(k, AttentionKernel):
+        return emit_attention(k, cfg, buffers, name, stable)
     raise TypeError(f"no CUDA emitter for {type(k).__name__}")
 
 
@@ -86,13 +101,16 @@ def generate_module(schedule, cfg, *, inline_header: bool = True, pdl: bool | No
 
     bodies: dict[str, tuple[str, list[str]]] = {}   # symbol -> (text, users)
     mod = Module(source="")
+    kinds: set[str] = set()
     placeholder = "MLCB_KERNEL_NAME"
     stable = stable_buffers(schedule) if getattr(cfg, "hoist_stable_loads", True) else frozenset()
     for k in schedule.kernels:
         if isinstance(k, kir.ExternKernel):
             continue
         text, spec = emit_kernel(k, cfg, schedule.buffers, placeholder, stable)
-        kind = "pw" if isinstance(k, kir.PointwiseKernel) else "red"
+        kind = {"PointwiseKernel": "pw", "ReductionKernel": "red", "MatmulKernel": "mm",
+                "AttentionKernel": "att"}[type(k).__name__]
+        kinds.add(kind)
         # operand names appear only in comments; identity is the code itself
         code = re.sub(r"[ \t]*//[^\n]*", "", text)
         digest = hashlib.sha256(code.encode()).hexdigest()[:12]
@@ -105,6 +123,7 @@ def generate_module(schedule, cfg, *, inline_header: bool = True, pdl: bool | No
 
     parts = [BANNER, f"#define MLCB_PDL {1 if pdl else 0}\n"]
     parts.append(device_header().replace('#pragma once\n', '') if inline_header else '#include "mlcb_device.cuh"\n')
+    parts += tensor_headers(kinds)
     for sym, (text, users) in bodies.items():
         k0 = schedule.kernel(users[0])
         parts.append(f"// ---- {sym} : {', '.join(users)}\n// {k0.summary()}\n{text}\n")

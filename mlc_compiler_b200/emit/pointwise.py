@@ -32,6 +32,11 @@ class LaunchSpec:
     #: descriptive, for reports: elements per thread-pack and algorithmic bytes
     vector: int = 1
     alg_bytes: int = 0
+    #: CTAs per cluster; tensor maps passed ahead of the pointers; and, where a kernel
+    #: does not take inputs then outputs, the buffers its pointers name
+    cluster: int = 1
+    tmaps: tuple = ()
+    buffers: tuple | None = None
 
     def as_dict(self) -> dict:
         return {"grid": (self.grid,), "block": self.block, "smem": self.smem,

@@ -24,9 +24,9 @@ from typing import Any, Mapping, Sequence
 
 import torch
 
-from . import concurrency, kir, rewrite
+from . import concurrency, fuse, kir, rewrite
 from .config import Config
-from .runtime import BackendError, CudaRuntime, LaunchRun
+from .runtime import BackendError, CudaRuntime, LaunchRun, TensorLaunch
 
 
 class ExecutionError(Exception):
@@ -117,55 +117,27 @@ def run_bound_extern(bound) -> None:
 
 # --------------------------------------------------------------------------
 
-class CompiledModel:
-    """A schedule bound to a device, callable like the module it came from."""
+class _Executable:
+    """One form of a schedule bound to a device: buffers, launch plan, capture."""
 
-    def __init__(self, schedule: kir.Schedule, params: Mapping[str, torch.Tensor] | torch.nn.Module,
-                 cfg: Config | None = None, device: str | torch.device = "cuda") -> None:
+    def _bind_form(self, schedule: kir.Schedule, work: kir.Schedule, params: dict, relaxed: bool) -> None:
+        """``work`` is what runs for ``schedule`` (whose inputs and outputs it keeps)."""
         self.schedule = schedule
-        self.cfg = cfg or Config()
-        self.device = torch.device(device)
-        if self.device.type == "cuda" and self.device.index is None:
-            self.device = torch.device("cuda", torch.cuda.current_device())
-        self.backend = select_backend(self.cfg, self.device)
-
-        # What actually runs.  ``self.schedule`` stays what the frontend produced;
-        # ``self._exec`` may (1) have pointwise producers folded into the copies
-        # that read them and copies folded into the matmul that feeds them, and
-        # (2) be re-ordered by data level with a re-packed
-        # arena, so that independent neighbours (q/k/v projections, embedding
-        # gathers) become parallel branches of the CUDA graph.  Generated and
-        # library kernels are otherwise exactly the scheduled ones.
-        work = rewrite.prepare(schedule, self.cfg)
         self._exec = work
         self._streams = None
         n_streams = int(getattr(self.cfg, "graph_streams", 1) or 1)
         if n_streams > 1 and self.cfg.cuda_graphs and work.plan.mode == "arena":
-            relaxed = concurrency.relax(work)
-            plan = concurrency.assign_streams(concurrency.dependencies(relaxed), n_streams)
-            if plan.forked:
-                self._exec, self._streams = relaxed, plan
+            if not relaxed:
+                work = concurrency.relax(work)
+            plan = concurrency.assign_streams(concurrency.dependencies(work), n_streams)
+            # fused matmuls leave few independent neighbours: a chain whose launches overlap
+            # at their edges beats a fork that only a few of them use
+            if plan.forked > (len(work) // 4 if relaxed else 0):
+                self._exec, self._streams = work, plan
                 self._side = [torch.cuda.Stream(device=self.device) for _ in range(n_streams - 1)]
-
         self._live = self._exec.live_buffers()
-        self.params: dict[str, torch.Tensor] = {}
-        source = _tensor_table(params)
-        for buf, origin in schedule.params.items():
-            if buf not in self._live:
-                continue
-            t = source.get(origin)
-            if t is None:
-                t = source.get(buf)
-            if t is None:
-                raise ExecutionError(f"no tensor supplied for parameter {buf} ({origin})")
-            spec = schedule.buffers[buf]
-            if t.numel() != spec.numel:
-                raise ExecutionError(f"parameter {origin}: schedule wants {spec.shape}, "
-                                     f"got {tuple(t.shape)}")
-            self.params[buf] = (t.detach().to(self.device, kir.torch_dtype(spec.dtype))
-                                .contiguous().reshape(-1))
-
-        self._module = CudaRuntime(self._exec, self.cfg, self.device)
+        self.params = params
+        self._runtime: CudaRuntime | None = None
         self._arena: torch.Tensor | None = None
         self._resident: dict[str, torch.Tensor] | None = None
         self._plan: list | None = None
@@ -173,11 +145,14 @@ class CompiledModel:
         self._graph_replay = None
         self._static_outputs: Any = None
         self._input_views: list[torch.Tensor] = []
-        #: what ``dependent_launch="auto"`` settled on at capture ("chain" or True)
         self.dependent_policy: Any = None
         self.policy_timings_ms: dict[str, float] = {}
-        #: generated-kernel launches per forward (what a bench reports)
-        self.generated_launches = len(self._exec.generated())
+
+    @property
+    def _module(self) -> CudaRuntime:
+        if self._runtime is None:
+            self._runtime = CudaRuntime(self._exec, self.cfg, self.device)
+        return self._runtime
 
     # -- allocation ------------------------------------------------------------
     def _check_inputs(self, inputs: Sequence[torch.Tensor]) -> None:
@@ -255,7 +230,7 @@ class CompiledModel:
                 self._bound[k.name] = ("extern", b)
                 self._per_kernel.append(("extern", b))
                 plan.append(("extern", b))
-            elif isinstance(k, (kir.PointwiseKernel, kir.ReductionKernel)):
+            else:
                 if chain:
                     flags = 1 if tail_generated.get(lane, False) else 0
                 else:
@@ -264,9 +239,11 @@ class CompiledModel:
                 fn = self._module.bind(k, buffers, flags)[0]
                 self._bound[k.name] = ("cuda", fn)
                 self._per_kernel.append(("cuda", fn))
-                run.append(fn)
-            else:
-                raise ExecutionError(f"cannot execute {type(k).__name__}")
+                if isinstance(fn, TensorLaunch):
+                    flush()
+                    plan.append(("cuda", fn))
+                else:
+                    run.append(fn)
         flush()
         return plan
 
@@ -315,10 +292,8 @@ class CompiledModel:
     def run_one(self, k, buffers: dict[str, torch.Tensor]) -> None:
         if isinstance(k, kir.ExternKernel):
             run_bound_extern(bind_extern(k, buffers))
-        elif isinstance(k, (kir.PointwiseKernel, kir.ReductionKernel)):
-            self._module.launch(k, buffers)
         else:
-            raise ExecutionError(f"cannot execute {type(k).__name__}")
+            self._module.launch(k, buffers)
 
     def _run_eager(self, inputs) -> dict[str, torch.Tensor]:
         """The unplanned baseline: allocate each intermediate when it is first
@@ -346,34 +321,9 @@ class CompiledModel:
                 buffers.pop(name, None)
         return buffers
 
-    def forward(self, *inputs: torch.Tensor):
-        if torch.cuda.current_device() != self.device.index:
-            with torch.cuda.device(self.device):
-                return self.forward(*inputs)
-        if self._exec.plan.mode == "eager":
-            return self._collect(self._run_eager(inputs))
-        buffers = self._resident_buffers(inputs)
-        if self._plan is None:
-            self._plan = self._build_plan(buffers)
-        self.run_kernels(buffers)
-        return self._collect(buffers)
-
     def _collect(self, buffers: dict[str, torch.Tensor]):
         outs = [v.as_torch(buffers[v.buffer]) for v in self.schedule.outputs]
         return outs[0] if len(outs) == 1 else tuple(outs)
-
-    def __call__(self, *inputs: torch.Tensor):
-        # everything below enqueues on "the current stream": make that the model's
-        # device's, whichever device the caller has current
-        if torch.cuda.current_device() != self.device.index:
-            with torch.cuda.device(self.device):
-                return self._call(inputs)
-        return self._call(inputs)
-
-    def _call(self, inputs):
-        if self.cfg.cuda_graphs and self.schedule.plan.mode == "arena":
-            return self._call_captured(inputs)
-        return self.forward(*inputs)
 
     # -- CUDA graphs -------------------------------------------------------------
     def _call_captured(self, inputs):
@@ -413,6 +363,8 @@ class CompiledModel:
             for _ in range(3):
                 self.run_kernels(buffers)
         torch.cuda.current_stream(self.device).wait_stream(side)
+        if self._module.loaded.fault():
+            raise BackendError("a bounded wait inside a kernel ran out during warm-up")
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             self.run_kernels(buffers)
@@ -448,15 +400,116 @@ class CompiledModel:
         g, self._plan, self._bound, self._per_kernel = candidates[self.dependent_policy]
         return g
 
-    def replay(self) -> None:
-        """Replay the captured graph on the inputs already resident."""
+    def _forward(self, inputs):
+        if self._exec.plan.mode == "eager":
+            return self._collect(self._run_eager(inputs))
+        buffers = self._resident_buffers(inputs)
+        if self._plan is None:
+            self._plan = self._build_plan(buffers)
+        self.run_kernels(buffers)
+        return self._collect(buffers)
+
+    def _call(self, inputs):
+        if self.cfg.cuda_graphs and self.schedule.plan.mode == "arena":
+            return self._call_captured(inputs)
+        return self._forward(inputs)
+
+    def _replay(self) -> None:
         if self._graph_replay is None:
             raise ExecutionError("nothing captured yet: call the model once")
+        self._graph_replay.replay()
+
+
+
+class _Launched(_Executable):
+    """The fused form of a model's schedule (``fuse.py``): what its calls launch."""
+
+    def __init__(self, schedule, fused, params, cfg, device):
+        self.cfg, self.device = cfg, device
+        self._bind_form(schedule, fused, params, relaxed=True)
+
+
+class CompiledModel(_Executable):
+    """A schedule bound to a device, callable like the module it came from."""
+
+    def __init__(self, schedule: kir.Schedule, params: Mapping[str, torch.Tensor] | torch.nn.Module,
+                 cfg: Config | None = None, device: str | torch.device = "cuda") -> None:
+        self.cfg = cfg or Config()
+        self.device = torch.device(device)
+        if self.device.type == "cuda" and self.device.index is None:
+            self.device = torch.device("cuda", torch.cuda.current_device())
+        self.backend = select_backend(self.cfg, self.device)
+
+        # What the schedule's kernels are.  ``self.schedule`` stays what the frontend produced;
+        # ``self._exec`` may (1) have pointwise producers folded into the copies
+        # that read them and copies folded into the matmul that feeds them, and
+        # (2) be re-ordered by data level with a re-packed
+        # arena, so that independent neighbours (q/k/v projections, embedding
+        # gathers) become parallel branches of the CUDA graph.  Generated and
+        # library kernels are otherwise exactly the scheduled ones.
+        # On top of that (3) calls launch its fused form where there is one.
+        work = rewrite.prepare(schedule, self.cfg)
+        table: dict[str, torch.Tensor] = {}
+        self._bind_form(schedule, work, table, relaxed=False)
+        source = _tensor_table(params)
+        for buf, origin in schedule.params.items():
+            if buf not in self._live:
+                continue
+            t = source.get(origin)
+            if t is None:
+                t = source.get(buf)
+            if t is None:
+                raise ExecutionError(f"no tensor supplied for parameter {buf} ({origin})")
+            spec = schedule.buffers[buf]
+            if t.numel() != spec.numel:
+                raise ExecutionError(f"parameter {origin}: schedule wants {spec.shape}, "
+                                     f"got {tuple(t.shape)}")
+            t = (t.detach().to(self.device, kir.torch_dtype(spec.dtype)).contiguous().reshape(-1))
+            # packed and tensor-map accesses were proven from aligned bases
+            table[buf] = t.clone() if t.data_ptr() % 32 else t
+        fused = fuse.fuse(work, self.cfg)
+        self._launched = None if fused is work else _Launched(schedule, fused, table, self.cfg, self.device)
+        if self._launched is None:
+            self._module             # a schedule that does not compile fails here, not at the first call
+        else:
+            self._launched._module
+        #: generated-kernel launches per forward of the schedule as ``executed_schedule`` has it
+        self.generated_launches = len(self._exec.generated())
+        #: launches of this package's kernels one call makes
+        self.launches_per_call = len((self._launched or self)._exec.generated())
+
+    # -- calls -------------------------------------------------------------------
+    def forward(self, *inputs: torch.Tensor):
+        """One uncaptured pass."""
         if torch.cuda.current_device() != self.device.index:
             with torch.cuda.device(self.device):
-                self._graph_replay.replay()
-            return
-        self._graph_replay.replay()
+                return self.forward(*inputs)
+        return (self._launched or self)._forward(inputs)
+
+    def __call__(self, *inputs: torch.Tensor):
+        # everything below enqueues on "the current stream": make that the model's
+        # device's, whichever device the caller has current
+        if torch.cuda.current_device() != self.device.index:
+            with torch.cuda.device(self.device):
+                return self.__call__(*inputs)
+        run = self._launched
+        if run is None:
+            return self._call(inputs)
+        out = run._call(inputs)
+        self.dependent_policy, self.policy_timings_ms = run.dependent_policy, run.policy_timings_ms
+        return out
+
+    def replay(self) -> None:
+        """Replay the captured graph on the inputs already resident."""
+        if torch.cuda.current_device() != self.device.index:
+            with torch.cuda.device(self.device):
+                return self.replay()
+        (self._launched or self)._replay()
+
+    @property
+    def launched_schedule(self) -> kir.Schedule:
+        """What a call launches: ``executed_schedule`` with matmuls and their neighbours fused."""
+        return (self._launched or self)._exec
 
     # -- profiling -----------------------------------------------------------------
     def profile_kernels(self, inputs, iters: int = 20) -> list[tuple]:

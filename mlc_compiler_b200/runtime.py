@@ -62,6 +62,14 @@ _SIGNATURES = {
                                    ctypes.c_int, ctypes.c_uint64, ctypes.c_uint32]),
     "mlcb_launch_many": (ctypes.c_int, [ctypes.POINTER(_LaunchDesc), ctypes.c_int,
                                         ctypes.c_uint64, ctypes.POINTER(ctypes.c_int)]),
+    "mlcb_kernel_shared": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint32]),
+    "mlcb_module_fault": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint32)]),
+    "mlcb_tensor_map": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int,
+                                       ctypes.POINTER(ctypes.c_uint64), ctypes.POINTER(ctypes.c_uint64),
+                                       ctypes.POINTER(ctypes.c_uint32)]),
+    "mlcb_launch_ex": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32,
+                                      ctypes.c_uint32, ctypes.POINTER(ctypes.c_void_p), ctypes.c_uint64,
+                                      ctypes.c_uint32]),
 }
 
 
@@ -189,6 +197,12 @@ class LoadedModule:
                "mlcb_kernel_info")
         return {"registers": regs.value, "static_smem": smem.value, "max_threads": mt.value}
 
+    def fault(self) -> int:
+        """Non-zero when a bounded wait in one of the kernels ran out."""
+        code = ctypes.c_uint32()
+        _check(self.lib, self.lib.mlcb_module_fault(self.handle, ctypes.byref(code)), "mlcb_module_fault")
+        return code.value
+
     def close(self) -> None:
         if self.handle is not None and self.handle.value:
             self.lib.mlcb_module_unload(self.handle)
@@ -242,6 +256,38 @@ class BoundLaunch:
     def desc(self) -> _LaunchDesc:
         return _LaunchDesc(self.kernel.value, self.grid, self.block, self.smem, self.flags,
                            ctypes.cast(self.ptrs, ctypes.POINTER(ctypes.c_uint64)), self.nptrs, 0)
+
+
+class TensorLaunch(BoundLaunch):
+    """A launch whose parameters are tensor maps (encoded once, at bind time) followed
+    by buffer pointers, on clusters of CTAs."""
+
+    __slots__ = ("cluster", "maps", "params", "mapped")
+
+    def __init__(self, lib, kernel, name, spec, flags, tensors, buffers, device=None):
+        super().__init__(lib, kernel, name, spec.grid, spec.block, spec.smem, flags, tensors, device)
+        self.cluster = spec.cluster
+        self.mapped = tuple(buffers[m.buffer] for m in spec.tmaps)       # keeps the storage alive
+        raw = ctypes.create_string_buffer(128 * len(spec.tmaps) + 128)
+        base = (ctypes.addressof(raw) + 127) & ~127
+        self.maps = raw
+        for i, (m, t) in enumerate(zip(spec.tmaps, self.mapped)):
+            _check(lib, lib.mlcb_tensor_map(
+                base + 128 * i, t.data_ptr() + m.offset * t.element_size(), int(m.dtype == "bfloat16"),
+                (ctypes.c_uint64 * 4)(*m.dims), (ctypes.c_uint64 * 3)(*m.strides),
+                (ctypes.c_uint32 * 3)(*m.box)), f"tensor map of {m.buffer} for {name}")
+        at = ctypes.addressof(self.ptrs)
+        self.params = (ctypes.c_void_p * (len(spec.tmaps) + self.nptrs))(
+            *[base + 128 * i for i in range(len(spec.tmaps))], *[at + 8 * i for i in range(self.nptrs)])
+        if spec.smem:            # above 48 KB together with the static part it has to be asked for
+            _check(lib, lib.mlcb_kernel_shared(kernel, spec.smem), f"shared memory of {name}")
+
+    def __call__(self, *tensors, **consts) -> None:
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        code = self.lib.mlcb_launch_ex(self.kernel, self.grid, self.block, self.cluster, self.smem,
+                                       self.params, stream, self.flags)
+        if code != 0:
+            _check(self.lib, code, f"launch of {self.name}")
 
 
 class LaunchRun:
@@ -306,6 +352,11 @@ class CudaRuntime:
         if self._is_extern(k):
             raise TypeError("extern kernels do not go through the CUDA runtime")
         spec = self.generated.launch[k.name]
+        if spec.tmaps:
+            tensors = tuple(buffers[n] for n in spec.buffers)
+            fn = TensorLaunch(self.lib, self.loaded.kernel(self.generated.symbol[k.name]), k.name, spec,
+                              self.flags if flags is None else flags, tensors, buffers, self.device)
+            return fn, spec.grid, tensors, {}
         tensors = tuple(buffers[n] for n in self._buffer_names(k))
         if flags is None:
             flags = self.flags
