@@ -147,6 +147,8 @@ class _Executable:
         self._input_views: list[torch.Tensor] = []
         self.dependent_policy: Any = None
         self.policy_timings_ms: dict[str, float] = {}
+        #: calls that read the caller's tensors in place, where the schedule allows it
+        self._direct = _DirectCall(self) if _DirectCall.serves(self._exec) else None
 
     @property
     def _module(self) -> CudaRuntime:
@@ -411,14 +413,94 @@ class _Executable:
 
     def _call(self, inputs):
         if self.cfg.cuda_graphs and self.schedule.plan.mode == "arena":
+            if self._direct is not None:
+                out = self._direct(inputs)
+                if out is not None:
+                    return out
             return self._call_captured(inputs)
         return self._forward(inputs)
 
     def _replay(self) -> None:
+        if self._direct is not None and self._direct.last is not None:
+            self._direct(self._direct.last)
+            return
         if self._graph_replay is None:
             raise ExecutionError("nothing captured yet: call the model once")
         self._graph_replay.replay()
 
+
+
+class _DirectCall:
+    """A schedule of one generated kernel, launched on the caller's tensors.
+
+    Captured as a graph such a call is a copy of every input, a graph launch and the
+    kernel; the copies alone move twice the inputs ([4096, 3072] bias + GELU + residual
+    in bf16: 38 us per call, of which the kernel is 13).  Launched directly it is one
+    launch: the input pointers are all that differs between calls.  Inputs the kernel
+    cannot read in place -- another dtype, device or layout, an unaligned start, memory
+    the call writes -- go the captured way (None)."""
+
+    @staticmethod
+    def serves(schedule: kir.Schedule) -> bool:
+        if len(schedule.kernels) != 1 or schedule.plan.mode != "arena":
+            return False
+        k = schedule.kernels[0]
+        ins = [v.buffer for v in schedule.inputs]
+        return (isinstance(k, (kir.PointwiseKernel, kir.ReductionKernel)) and len(set(ins)) == len(ins)
+                and not set(ins) & ({v.buffer for v in schedule.outputs} | set(k.writes())))
+
+    def __init__(self, owner: "_Executable"):
+        self.owner = owner
+        self.launch = None
+        #: inputs of the last call: what ``replay`` runs on
+        self.last = None
+
+    def _bind(self, inputs) -> None:
+        owner = self.owner
+        k = owner._exec.kernels[0]
+        buffers = owner._resident_buffers(inputs)
+        fn = self.launch = owner._module.bind(k, buffers, 0)[0]
+        names = owner._module._buffer_names(k)
+        self.specs = []
+        for v in owner.schedule.inputs:
+            spec = owner._exec.buffers[v.buffer]
+            self.specs.append((torch.Size(v.shape), kir.torch_dtype(spec.dtype), spec.nbytes,
+                               tuple(i for i, n in enumerate(names) if n == v.buffer)))
+        self.written = [(buffers[b].data_ptr(), buffers[b].data_ptr() + owner._exec.buffers[b].nbytes)
+                        for b in set(k.writes())]
+        self.out = owner._collect(buffers)
+        self.args = (fn.kernel, fn.grid, fn.block, fn.smem, fn.ptrs, fn.nptrs)
+        self.run = fn.lib.mlcb_launch
+        self.index = owner.device.index
+
+    def __call__(self, inputs):
+        if self.launch is None:
+            self._bind(inputs)
+        specs = self.specs
+        if len(inputs) != len(specs):
+            return self._refuse()
+        ptrs = self.args[4]
+        for t, (shape, dtype, nbytes, slots) in zip(inputs, specs):
+            if t.shape != shape or t.dtype is not dtype or not t.is_contiguous() or t.get_device() != self.index:
+                return self._refuse()
+            p = t.data_ptr()
+            if p & 31:
+                return self._refuse()
+            for lo, hi in self.written:
+                if p < hi and lo < p + nbytes:
+                    return self._refuse()
+            for i in slots:
+                ptrs[i] = p
+        self.last = inputs
+        code = self.run(*self.args, torch._C._cuda_getCurrentRawStream(self.index), 0)
+        if code != 0:
+            raise BackendError(f"launch of {self.launch.name} failed with code {code}: "
+                               f"{self.launch.lib.mlcb_last_error().decode(errors='replace')}")
+        return self.out
+
+    def _refuse(self):
+        self.last = None
+        return None
 
 
 class _Launched(_Executable):
