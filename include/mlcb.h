@@ -40,6 +40,7 @@ extern "C" {
 
 /* launch flags */
 #define MLCB_LAUNCH_DEPENDENT 1u /* programmatic stream serialisation (PDL) */
+#define MLCB_LAUNCH_CLUSTER(n) ((uint32_t)(n) << 8) /* clusters of n CTAs (0, 1: none) */
 
 typedef struct mlcb_module mlcb_module;
 typedef struct mlcb_kernel mlcb_kernel;

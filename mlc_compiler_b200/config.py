@@ -79,6 +79,10 @@ class Config:
     wide_access_bytes: int = 8 << 20
     #: same for persistent row reductions (0 = never; measured no better than 128-bit)
     wide_reduction_bytes: int = 0
+    #: row reductions over at least this many columns (a third of it
+    #: where rows are not aligned for wide accesses) keep the row in shared memory
+    #: (``emit/staged.py``); 0 = never
+    staged_columns: int = 9000
     #: fold a pointwise producer into the pointwise kernels that only re-read it at
     #: another index (bias add + head-layout copy at batch > 1); bit-identical
     forward_into_copies: bool = True

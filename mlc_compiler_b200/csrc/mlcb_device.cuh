@@ -210,6 +210,9 @@ __device__ __forceinline__ void mlcb_store_at(T* __restrict__ p,
     mlcb_store<T, W>(p, tmp);
 }
 
+// Column of a pack that reaches over the ends of its row: the nearest one inside.
+__device__ __forceinline__ int mlcb_within(int c, int n) { return c < 0 ? 0 : (c >= n ? n - 1 : c); }
+
 // Row id of a gathered operand, forced into the table: an id outside [0, n)
 // reads a wrong row instead of memory that is not the table's.
 __device__ __forceinline__ long long mlcb_clamp_index(long long v, long long n) {

@@ -383,11 +383,20 @@ static int launch_one(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_
     // calling thread had current; `stream` must belong to that context
     CtxGuard in_module_context(k->owner->ctx);
     {
-        if (flags & MLCB_LAUNCH_DEPENDENT) {
-            CUlaunchAttribute attr;
-            memset(&attr, 0, sizeof attr);
-            attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-            attr.value.programmaticStreamSerializationAllowed = 1;
+        if (flags) {
+            CUlaunchAttribute attr[2];
+            memset(attr, 0, sizeof attr);
+            unsigned n = 0;
+            if (flags & MLCB_LAUNCH_DEPENDENT) {
+                attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+                attr[n++].value.programmaticStreamSerializationAllowed = 1;
+            }
+            if (const unsigned cluster = (flags >> 8) & 0xFF; cluster > 1) {
+                attr[n].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+                attr[n].value.clusterDim.x = cluster;
+                attr[n].value.clusterDim.y = attr[n].value.clusterDim.z = 1;
+                ++n;
+            }
             CUlaunchConfig cfg;
             memset(&cfg, 0, sizeof cfg);
             cfg.gridDimX = grid_x;
@@ -396,8 +405,8 @@ static int launch_one(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_
             cfg.blockDimY = cfg.blockDimZ = 1;
             cfg.sharedMemBytes = smem_bytes;
             cfg.hStream = (CUstream)(uintptr_t)stream;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = n;
             r = d.LaunchKernelEx(&cfg, k->fn, args, nullptr);
         } else {
             r = d.LaunchKernel(k->fn, grid_x, 1, 1, block_x, 1, 1, smem_bytes,

@@ -99,6 +99,33 @@ __device__ __forceinline__ void mlcb_tma_load_pair(u32 dst, const mlcb_tmap* m, 
                  :: "r"(dst), "l"(m), "r"(bar & 0xFEFFFFFFu), "r"(x), "r"(y), "r"(b), "r"(z) : "memory");
 }
 
+// untiled copy: both addresses and the size are multiples of 16 bytes
+__device__ __forceinline__ void mlcb_bulk_load(u32 dst, const void* src, u32 bytes, u32 bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// A value per CTA of the cluster, combined in rank order by every thread.  `slot` is not
+// reused by another reduction of the kernel.
+template <typename OP, int C, typename T>
+__device__ __forceinline__ T mlcb_cluster_reduce(T v, u64* slot) {
+    static_assert(sizeof(T) <= 8, "scalar");
+    if (threadIdx.x == 0) *reinterpret_cast<T*>(slot) = v;
+    mlcb_cluster_arrive();
+    mlcb_cluster_wait();
+    T r;
+#pragma unroll
+    for (u32 p = 0; p < C; ++p) {
+        u32 at;
+        u64 bits;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mlcb_smem(slot)), "r"(p));
+        asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(bits) : "r"(at) : "memory");
+        const T x = *reinterpret_cast<T*>(&bits);
+        r = p ? OP::f(r, x) : x;
+    }
+    return r;
+}
+
 // ---------------------------------------------------------------------------
 // TMEM and tcgen05
 // ---------------------------------------------------------------------------

@@ -36,6 +36,7 @@ from dataclasses import dataclass, field
 from .. import kir
 from ..kir import Bind, Reduce
 from . import expr as X
+from . import staged
 from .indexing import (Access, check_bounds, classify, needs_64bit, pow2_ceil,
                        render_offset)
 from .pointwise import (LaunchSpec, algorithmic_bytes, dependent_release, loads_ahead_of_wait,
@@ -89,15 +90,35 @@ class Geometry:
         return self.G > 32
 
 
+def unaligned_rows(k: kir.ReductionKernel) -> list[int] | None:
+    """Input slots that hold this kernel's rows when the rows lie packed one after the
+    other at any alignment (an odd row length): every operand that varies along both axes,
+    the outputs among them, has the same element size and index.  Their 16-byte packs are
+    then cut at the same places, and a row is read by the packs it touches."""
+    outs = [a for a in k.outputs if a.name not in k.row_outputs]
+    slots = [i for i, a in enumerate(k.inputs) if a.index.varies_along("col") and a.index.varies_along("row")]
+    if not outs or not slots or {a.buffer for a in k.inputs} & {a.buffer for a in k.outputs}:
+        return None
+    index, size = outs[0].index, kir.ITEMSIZE[outs[0].dtype]
+    col = index.axis("col")
+    if size not in (2, 4, 8) or col is None or col.terms != ((k.n_cols, 1, 1),) or not index.varies_along("row"):
+        return None
+    same = [k.inputs[i] for i in slots] + outs
+    if any(a.index != index or kir.ITEMSIZE[a.dtype] != size or a.via is not None for a in same):
+        return None
+    return slots
+
+
 def plan_geometry(n_rows: int, n_cols: int, operands, cfg, streamed: bool,
-                  alg_bytes: int = 0) -> Geometry:
-    V = pick_vector(operands, n_cols)
+                  alg_bytes: int = 0, cut: int = 0) -> Geometry:
+    """``cut``: elements per pack of rows that start anywhere in their first pack."""
+    V = cut or pick_vector(operands, n_cols)
     wide = int(getattr(cfg, "wide_reduction_bytes", 0) or 0)
     if wide and alg_bytes >= wide and not streamed:
         V2 = pick_vector(operands, n_cols, cap_bytes=32)
         if V2 > V and all(classify(a.index, "col", V2).width == V2 for a in operands):
             V = V2
-    P = n_cols // V
+    P = n_cols // V if not cut else (n_cols + 2 * V - 2) // V
     want_np = max(1, int(getattr(cfg, "reduction_packs_per_thread", 2)))
     if streamed:
         # eight packs per lane per pass, at least a warp unless the row is shorter
@@ -131,7 +152,7 @@ def plan_geometry(n_rows: int, n_cols: int, operands, cfg, streamed: bool,
             rpb = max(max(1, 32 // G), min(1024 // G, pow2_ceil(want_rows)))
         block = G * rpb
     grid = (n_rows + rpb - 1) // rpb
-    return Geometry(V, P, G, NP, block, rpb, grid, masked=(NP * G != P))
+    return Geometry(V, P, G, NP, block, rpb, grid, masked=(NP * G != P) or bool(cut))
 
 
 # --------------------------------------------------------------------------
@@ -301,8 +322,20 @@ def _col_off(a, var: str) -> str:
 def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset()) -> tuple[str, LaunchSpec]:
     operands = [a for a in k.inputs if a.index.varies_along("col")] + [
         a for a in k.outputs if a.name not in k.row_outputs]
+    # rows at any alignment: the packs a row touches, their elements outside it left out.
+    # One element per lane and access otherwise: softmax over fp16 rows of 1001 / 3001
+    # columns (30 and 60 MB) 23 and 134 us, 17 and 29 in packs; LayerNorm of 3001 146 and
+    # 48.  Short rows of 4 bytes, or with a gain and bias to fetch element by element,
+    # gain nothing ([14985, 1001] fp32 softmax 26 against 27 us).
+    slots = unaligned_rows(k)
+    if slots is not None:
+        extra = [a for a in k.inputs if a.index.varies_along("col") and not a.index.varies_along("row")]
+        size = kir.ITEMSIZE[k.outputs[0].dtype]
+        if pick_vector(operands, k.n_cols) * size > 4 or k.n_cols < (1536 if size > 2 or extra else 256):
+            slots = None
+    cut = 16 // kir.ITEMSIZE[k.inputs[slots[0]].dtype] if slots else 0
     geo = plan_geometry(k.n_rows, k.n_cols, operands or k.inputs + k.outputs, cfg, False,
-                        algorithmic_bytes(k.inputs, k.outputs, k.n_rows * k.n_cols))
+                        algorithmic_bytes(k.inputs, k.outputs, k.n_rows * k.n_cols), cut)
     V, G, NP = geo.V, geo.G, geo.NP
     extents = [k.n_rows * max(1, k.n_cols)] + [a.index.bounds()[1] + 1
                                                for a in k.inputs + k.outputs]
@@ -324,6 +357,8 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
         c.emit(dependent_release(geo.grid, geo.block, cfg))
     _scalar_loads(c, False, scalar_in)
     _row_offsets(c, k.inputs, "in", ahead=False)
+    if cut:
+        c.emit(f"    const int shift = (int)(in{slots[0]}_r % {V});   // of the row in its first pack")
 
     # ---- which phase defines / uses each column-varying value -------------
     phase_of: dict[str, int] = {}
@@ -365,11 +400,12 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
     acc_in: dict[int, Access] = {}
     for i, a in enumerate(k.inputs):
         if a.index.varies_along("col"):
-            acc_in[i] = classify(a.index, "col", V)
+            acc_in[i] = classify(a.index, "col", V) if not cut else \
+                Access("contig", V if i in slots else 1)
     acc_out: dict[int, Access] = {}
     for i, a in enumerate(k.outputs):
         if a.name not in k.row_outputs:
-            ac = classify(a.index, "col", V)
+            ac = classify(a.index, "col", V) if not cut else Access("contig", V)
             acc_out[i] = ac if ac.mode == "contig" else Access("contig", 1)
 
     packed_in = {i for i, ac in acc_in.items() if ac.width > 1}
@@ -391,7 +427,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
     # operands of the first phase -- needed together with the row itself -- last.
     # (A prefetch.global.L1 of the same addresses instead, holding no register, was
     # measured and is far slower on large launches: [4096, 768] 8.1 us against 3.6 us.)
-    candidates = sorted((i for i in packed_in if i in c.ahead and i in load_first
+    candidates = sorted((i for i in packed_in if not cut and i in c.ahead and i in load_first
                          and acc_in[i].mode == "contig" and acc_in[i].width == V),
                         key=lambda i: (-load_first[i], i))
     need = -(-geo.grid // SM_COUNT)
@@ -499,7 +535,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
         c.emit("#pragma unroll")
         c.emit(f"    for (int q = 0; q < {NP}; ++q) {{")
         if geo.masked or first_loads or stores or gathers:
-            c.emit(f"        const int c0 = (lane + q * {G}) * {V};")
+            c.emit(f"        const int c0 = (lane + q * {G}) * {V}{' - shift' if cut else ''};")
         ind = "        "
         if geo.masked:
             c.emit(f"        if (c0 < {k.n_cols}) {{")
@@ -512,6 +548,13 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                 for r_, cc in enumerate(range(0, V, ac.width)):
                     c.emit(f"{ind}v{i}[q][{r_}] = mlcb_load1<{st}>(in{i} + in{i}_r + "
                            f"({_col_off(a, f'(c0 + {cc})')}));")
+            elif cut:
+                c.emit(f"{ind}if (c0 >= 0 && c0 + {V} <= {k.n_cols}) {{ mlcb_load<{st}, {V}>(in{i} + in{i}_r + c0, v{i}[q]); }}")
+                c.emit(f"{ind}else {{")
+                c.emit("#pragma unroll")
+                c.emit(f"{ind}    for (int j = 0; j < {V}; ++j) v{i}[q][j] = (unsigned)(c0 + j) < {k.n_cols}u ? "
+                       f"mlcb_load1<{st}>(in{i} + in{i}_r + c0 + j) : ({X.REG_T[a.dtype]})0;")
+                c.emit(f"{ind}}}")
             elif i in raw_in:
                 c.emit(f"{ind}mlcb_unpack<{st}, {V}>(w{i}[q], v{i}[q]);")
             elif ac.width == V:
@@ -531,7 +574,8 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
             for i in gathers:
                 a = k.inputs[i]
                 c.emit(f"{in2}const {X.REG_T[a.dtype]} g{i} = mlcb_load1<{X.STORAGE_T[a.dtype]}>"
-                       f"(in{i} + in{i}_r + ({_col_off(a, 'col')}));  // {a.name}")
+                       f"(in{i} + in{i}_r + ({_col_off(a, 'mlcb_within(col, %d)' % k.n_cols if cut else 'col')}));"
+                       f"  // {a.name}")
             local = dict(c.scalars)
             local.update(pre_vals)
             for s in vbinds:
@@ -546,7 +590,8 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                 x = X.convert(rv.code, rv.dtype, acc_dt) if rv.dtype not in kir.NARROW_FLOATS \
                     else rv.code
                 t = X.REG_T[acc_dt]
-                c.emit(f"{in2}acc_{red.name} = {_OP[red.kind]}::f<{t}>(acc_{red.name}, {x});")
+                only = f"if ((unsigned)(c0 + j) < {k.n_cols}u) " if cut else ""
+                c.emit(f"{in2}{only}acc_{red.name} = {_OP[red.kind]}::f<{t}>(acc_{red.name}, {x});")
             for i, a in stores:
                 v = X.render(k.out_expr[a.name], loads, local)
                 code = store_code(v, a.dtype)
@@ -558,7 +603,14 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
             c.emit(f"{ind}}}")
         for i, a in out_regs:
             ac, st = acc_out[i], X.STORAGE_T[a.dtype]
-            if ac.width == V:
+            if cut:
+                c.emit(f"{ind}if (live && c0 >= 0 && c0 + {V} <= {k.n_cols}) {{ mlcb_store<{st}, {V}>(out{i} + out{i}_r + c0, o{i}); }}")
+                c.emit(f"{ind}else if (live) {{")
+                c.emit("#pragma unroll")
+                c.emit(f"{ind}    for (int j = 0; j < {V}; ++j) if ((unsigned)(c0 + j) < {k.n_cols}u) "
+                       f"mlcb_store1<{st}>(out{i} + out{i}_r + c0 + j, o{i}[j]);")
+                c.emit(f"{ind}}}")
+            elif ac.width == V:
                 c.emit(f"{ind}if (live) mlcb_store<{st}, {V}>(out{i} + out{i}_r + "
                        f"({_col_off(a, 'c0')}), o{i});")
             else:
@@ -664,12 +716,12 @@ def detect_online_softmax(k: kir.ReductionKernel):
     return (rs[0], rs[1], rs[0].expr)
 
 
-def plan_passes(k: kir.ReductionKernel) -> list[Pass]:
+def plan_passes(k: kir.ReductionKernel, online: bool = True) -> list[Pass]:
     deps = _dependencies(k.steps)
     vec = varying_steps(k)
     by = {s.name: s for s in k.steps}
     order = [s.name for s in k.steps]
-    online = detect_online_softmax(k)
+    online = detect_online_softmax(k) if online else None
 
     def vbinds(needed: set[str]) -> list:
         return [by[n] for n in order if n in needed and isinstance(by[n], Bind) and n in vec]
@@ -927,6 +979,11 @@ def emit_reduction(k: kir.ReductionKernel, cfg, buffers: dict[str, kir.BufferSpe
     if any(a.via is not None for a in k.outputs):
         raise ValueError(f"{k.name}: outputs cannot be gathered")
     name = name or k.name
+    operands = [a for a in k.inputs if a.index.varies_along("col")] + [
+        a for a in k.outputs if a.name not in k.row_outputs]
     with X.math_mode(X.wants_fast_math(k, cfg)):
+        stage = staged.plan(k, cfg, pick_vector(operands or k.inputs + k.outputs, k.n_cols))
+        if stage is not None:
+            return staged.emit_staged(k, cfg, name, stable, stage)
         return (_emit_streamed(k, cfg, name, stable) if k.two_pass
                 else _emit_persistent(k, cfg, name, stable))

@@ -1,0 +1,297 @@
+"""Row reductions whose rows wait in shared memory.
+
+The register form gives a row to one CTA at most and needs aligned rows for wide
+accesses; the streamed form reads the row again in every pass, one load in flight per
+thread.  Here the row is brought into shared memory once, by bulk copies that start at
+the 16-byte boundary before it whatever the row's own alignment, and every pass reads it
+there as 16-byte packs.  A long row, or one of few, is divided over a cluster whose CTAs
+exchange their partial results through distributed shared memory, in rank order.
+
+The copies are issued in blocks of one pack per thread, each with its own barrier: the
+first pass starts on a block while the rest are on their way.  Softmax over
+[512, 50257] fp16 (odd rows, 103 MB) takes 27.8 us (3.7 TB/s), streamed 61.9;
+[2000, 16383] bf16 31 us, 60 in registers; [16, 20001] fp32 5.4 us, 10.4 streamed.
+"""
+
+from __future__ import annotations
+
+from dataclasses import dataclass
+
+from .. import kir
+from ..kir import Reduce
+from . import expr as X
+from .indexing import classify, needs_64bit, pow2_ceil, render_offset
+from .pointwise import LaunchSpec, algorithmic_bytes, dependent_release, store_code
+
+SM_COUNT = 148
+SMEM_MAX = 224 * 1024
+
+
+@dataclass
+class Stage:
+    slots: list      # inputs staged in shared memory
+    V: int           # elements per 16-byte pack
+    aligned: bool    # every row starts on a 16-byte boundary
+    C: int           # CTAs per row
+    T: int           # threads per CTA
+    PC: int          # packs per CTA and operand
+
+    @property
+    def blocks(self) -> int:
+        return -(-self.PC // self.T)
+
+    @property
+    def smem(self) -> int:
+        return len(self.slots) * self.PC * 16
+
+
+def plan(k: kir.ReductionKernel, cfg, vector: int) -> Stage | None:
+    """Whether ``k`` takes this form, and how.  ``vector``: elements per access the
+    register form would get."""
+    from .reduction import unaligned_rows
+
+    least = int(getattr(cfg, "staged_columns", 9000) or 0)
+    slots = unaligned_rows(k)
+    if not least or slots is None or not k.reduces:
+        return None
+    # aligned rows keep the register form to where it needs a whole CTA's registers (60 MB of
+    # fp32 rows of 8000 columns: softmax 21 us against 27 here, of 10000: 39 against 28),
+    # unaligned ones to where its partial packs cost more ([7498, 4001] fp16: 28 against 25)
+    if k.n_cols < (least if k.two_pass or vector * kir.ITEMSIZE[k.outputs[0].dtype] == 16 else least // 3):
+        return None
+    size = kir.ITEMSIZE[k.inputs[slots[0]].dtype]
+    row_bytes = k.n_cols * size
+    V = 16 // size
+    aligned = all(classify(k.inputs[i].index, "col", V).width == V for i in slots)
+    packs = -(-(k.n_cols + (0 if aligned else V - 1)) // V)
+    C = 1
+    # one CTA per row while rows fill the machine and two of them fit an SM; a cluster
+    # where a row is longer than that or rows are few (at least 12 KB per CTA: [60, 9001] fp16 takes 4.0 us
+    # whole and 5.7 in four parts, [16, 20001] fp32 10.4 and 5.4)
+    while C < 8 and (len(slots) * -(-packs // C) * 16 > SMEM_MAX // 2
+                     or (k.n_rows * C < SM_COUNT and row_bytes // (2 * C) >= 12288)):
+        C *= 2
+    PC = -(-packs // C)
+    if len(slots) * PC * 16 > SMEM_MAX:
+        return None
+    T = max(128, min(512, pow2_ceil(-(-PC // 4))))
+    return Stage(slots, V, aligned, C, T, PC)
+
+
+def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tuple[str, LaunchSpec]:
+    from .reduction import _Ctx, _OP, _acc_dtype, _identity, _row_stores, _signature, Geometry, plan_passes
+
+    V, C, T, PC, N = st.V, st.C, st.T, st.PC, k.n_cols
+    grid = k.n_rows * C
+    extents = [k.n_rows * max(1, N)] + [a.index.bounds()[1] + 1 for a in k.inputs + k.outputs]
+    it = "i64" if needs_64bit(*extents) else "int"
+    geo = Geometry(V, PC, T, st.blocks, T, 1, grid, masked=True)
+    c = _Ctx(k, geo, it, stable, cfg)
+    passes = plan_passes(k, online=False)
+    reduces = k.reduces
+    lead = st.slots[0]
+    occ = max(1, min(2048 // T, SMEM_MAX // max(1, st.smem), 65536 // (T * 56)))
+    e = c.emit
+    e(_signature(k, name, T, cfg, occ))
+    e(f"    // staged: {k.n_rows} rows x {N} cols, {C} CTA(s) per row, {PC} packs of {V} each, {len(passes)} passes")
+    e("    extern __shared__ __align__(128) unsigned char staged_raw[];")
+    e(f"    __shared__ alignas(8) u64 bars[{st.blocks}];")
+    e("    __shared__ volatile u32 dead;")
+    e(f"    __shared__ u64 mlcb_red[{max(1, len(reduces))} * 32];")
+    if C > 1:
+        e(f"    __shared__ u64 mlcb_part[{max(1, len(reduces))}];")
+    e(f"    const int rank = {'(int)mlcb_cta_rank()' if C > 1 else '0'}, lane = threadIdx.x;")
+    e(f"    const {it} row = blockIdx.x / {C};")
+    e("    const bool live = true;")
+    e("    if (lane == 0) {")
+    e("        dead = 0;")
+    e(f"        for (int i = 0; i < {st.blocks}; ++i) mlcb_bar_init(mlcb_smem(bars) + 8 * i, 1);")
+    e("        mlcb_bar_fence_init();")
+    e("    }")
+    e("    __syncthreads();")
+    scalar_in: list = [None] * len(k.inputs)
+    e("    MLCB_GRID_WAIT();")
+    for i, a in enumerate(k.inputs):
+        ct, rt = X.STORAGE_T[a.dtype], X.REG_T[a.dtype]
+        off = render_offset(a.index, {"row": "row"}, skip=("col",))
+        if not a.index.varies_along("col"):
+            e(f"    const {rt} s{i} = mlcb_load1<{ct}>(in{i} + ({off}));  // {a.name} (per row)")
+            scalar_in[i] = X.Val(f"s{i}", X.promoted_load_dtype(a.dtype), True, False)
+        else:
+            e(f"    const {it} in{i}_r = {off};")
+    e(f"    const int shift = {'0' if st.aligned else f'(int)(in{lead}_r % {V})'};   // of the row in its first pack")
+    e(f"    const int p0 = rank * {PC}, p1 = min(p0 + {PC}, (shift + {N + V - 1}) / {V});")
+    e(f"    const int whole0 = shift ? 1 : 0, whole1 = (shift + {N}) / {V};   // packs inside the row")
+    e("    if (lane == 0) {")
+    e(f"        for (int i = 0; i < {st.blocks}; ++i) {{")
+    e(f"            const int lo = max(whole0, p0 + i * {T}), hi = min(min(whole1, p1), p0 + (i + 1) * {T});")
+    e("            const u32 bytes = hi > lo ? (hi - lo) * 16 : 0, bar = mlcb_smem(bars) + 8 * i;")
+    e(f"            mlcb_bar_expect(bar, {len(st.slots)} * bytes);")
+    for n, i in enumerate(st.slots):
+        e(f"            if (bytes) mlcb_bulk_load(mlcb_smem(staged_raw) + {n * PC * 16} + (lo - p0) * 16, "
+          f"in{i} + (in{i}_r - shift + lo * {V}), bytes, bar);")
+    e("        }")
+    e("    }")
+    if not st.aligned:
+        # packs the row shares with its neighbours: the thread that owns one fetches its elements
+        e("#pragma unroll")
+        e("    for (int edge = 0; edge < 2; ++edge) {")
+        e("        const int p = edge ? whole1 : 0;")
+        e(f"        if (p >= p0 && p < p1 && (p - p0) % {T} == lane && (edge ? (shift + {N}) % {V} != 0 : shift != 0)) {{")
+        e("#pragma unroll")
+        e(f"            for (int j = 0; j < {V}; ++j) {{")
+        e(f"                const int col = p * {V} - shift + j;")
+        for n, i in enumerate(st.slots):
+            ct = X.STORAGE_T[k.inputs[i].dtype]
+            e(f"                if (col >= 0 && col < {N}) reinterpret_cast<{ct}*>(staged_raw + {n * PC * 16})"
+              f"[(p - p0) * {V} + j] = in{i}[in{i}_r + col];")
+        e("            }")
+        e("        }")
+        e("    }")
+    release = dependent_release(grid, T, cfg)
+    if release:
+        e(release)
+
+    loads: list = []
+    acc_other = {}
+    for i, a in enumerate(k.inputs):
+        dt = X.promoted_load_dtype(a.dtype)
+        if scalar_in[i] is not None:
+            loads.append(scalar_in[i])
+        elif i in st.slots:
+            loads.append(X.Val(f"v{i}[j]", dt, True, True))
+        else:
+            ac = classify(a.index, "col", V)
+            acc_other[i] = st.aligned and ac.mode == "contig" and ac.width == V
+            loads.append(X.Val(f"v{i}[j]" if acc_other[i] else f"g{i}", dt, True, True))
+
+    first = True
+
+    def emit_pass(p) -> None:
+        nonlocal first
+        used: set[int] = set()
+        for b in p.binds:
+            used |= kir.expr_loads(b.expr)
+        for r in p.reduces:
+            used |= kir.expr_loads(r.expr)
+        for nm in p.stores:
+            used |= kir.expr_loads(k.out_expr[nm])
+        probe = dict(c.scalars)
+        for b in p.binds:
+            v = X.render_bind(b.name, b.expr, loads, probe, c.elide)
+            probe[b.name] = X.Val(b.name, v.dtype, v.dim, True)
+        accs = {}
+        for r in p.reduces:
+            rv = X.render(r.expr, loads, probe)
+            rdt = X.reduce_type(r.kind, rv.dtype)
+            adt = _acc_dtype(rdt)
+            accs[r.name] = (adt, rdt)
+            e(f"    {X.REG_T[adt]} acc_{r.name} = {_identity(r.kind, adt)};")
+        stores = [(i, a) for i, a in enumerate(k.outputs) if a.name in p.stores]
+        e("#pragma unroll 1" if st.blocks > 16 else "#pragma unroll 2")
+        e(f"    for (int i = 0; i < {st.blocks}; ++i) {{")
+        e(f"        const int p = p0 + i * {T} + lane;")
+        if first:
+            e("        mlcb_bar_wait(mlcb_smem(bars) + 8 * i, 0, &dead);")
+            first = False
+        e("        if (p < p1) {")
+        ind = "            "
+        e(f"{ind}const int c0 = p * {V} - shift;")
+        for n, i in enumerate(st.slots):
+            if i in used:
+                a = k.inputs[i]
+                ct = X.STORAGE_T[a.dtype]
+                e(f"{ind}{X.REG_T[a.dtype]} v{i}[{V}]; mlcb_load<{ct}, {V}>(reinterpret_cast<const {ct}*>"
+                  f"(staged_raw + {n * PC * 16}) + (p - p0) * {V}, v{i});  // {a.name}")
+        for i, packed in acc_other.items():
+            if i in used and packed:
+                a = k.inputs[i]
+                ct = X.STORAGE_T[a.dtype]
+                off = render_offset(a.index, {"col": "c0"}, skip=("row", "base"))
+                e(f"{ind}{X.REG_T[a.dtype]} v{i}[{V}]; mlcb_load<{ct}, {V}>(in{i} + in{i}_r + ({off}), v{i});")
+        for i, a in stores:
+            e(f"{ind}{X.REG_T[a.dtype]} o{i}[{V}];")
+
+        def body(guarded: bool, ind: str) -> None:
+            e("#pragma unroll")
+            e(f"{ind}for (int j = 0; j < {V}; ++j) {{")
+            ind += "    "
+            if guarded:
+                e(f"{ind}if (c0 + j < 0 || c0 + j >= {N}) continue;")
+            for i, packed in acc_other.items():
+                if i in used and not packed:
+                    a = k.inputs[i]
+                    off = render_offset(a.index, {"col": "(c0 + j)"}, skip=("row", "base"))
+                    e(f"{ind}const {X.REG_T[a.dtype]} g{i} = mlcb_load1<{X.STORAGE_T[a.dtype]}>"
+                      f"(in{i} + in{i}_r + ({off}));  // {a.name}")
+            local = dict(c.scalars)
+            for b in p.binds:
+                v = X.render_bind(b.name, b.expr, loads, local, c.elide)
+                e(f"{ind}const {X.REG_T[v.dtype]} {b.name} = {v.code};")
+                local[b.name] = X.Val(b.name, v.dtype, v.dim, True)
+            for r in p.reduces:
+                adt, _ = accs[r.name]
+                rv = X.render(r.expr, loads, local)
+                x = rv.code if rv.dtype in kir.NARROW_FLOATS else X.convert(rv.code, rv.dtype, adt)
+                e(f"{ind}acc_{r.name} = {_OP[r.kind]}::f<{X.REG_T[adt]}>(acc_{r.name}, {x});")
+            for i, a in stores:
+                code = store_code(X.render(k.out_expr[a.name], loads, local), a.dtype)
+                if guarded:
+                    e(f"{ind}mlcb_store1<{X.STORAGE_T[a.dtype]}>(out{i} + (in{lead}_r + c0 + j), {code});")
+                else:
+                    e(f"{ind}o{i}[j] = {code};  // {a.name}")
+            ind = ind[:-4]
+            e(f"{ind}}}")
+            if not guarded:
+                for i, a in stores:
+                    e(f"{ind}mlcb_store<{X.STORAGE_T[a.dtype]}, {V}>(out{i} + (in{lead}_r + c0), o{i});")
+
+        if st.aligned and N % V == 0:
+            body(False, ind)
+        else:
+            e(f"{ind}if (c0 >= 0 && c0 + {V} <= {N}) {{")
+            body(False, ind + "    ")
+            e(f"{ind}}} else {{")
+            body(True, ind + "    ")
+            e(f"{ind}}}")
+        e("        }")
+        e("    }")
+        for r in p.reduces:
+            adt, rdt = accs[r.name]
+            t, n = X.REG_T[adt], reduces.index(r)
+            red = (f"mlcb_cta_reduce<{_OP[r.kind]}, {T // 32}, {t}>(acc_{r.name}, "
+                   f"reinterpret_cast<{t}*>(mlcb_red + {n} * 32))")
+            if C > 1:
+                red = f"mlcb_cluster_reduce<{_OP[r.kind]}, {C}, {t}>({red}, mlcb_part + {n})"
+            if rdt in kir.NARROW_FLOATS:
+                red = X.convert(red, "float32", rdt)
+            e(f"    const {X.REG_T[rdt]} {r.name} = {red};")
+            c.scalars[r.name] = X.Val(r.name, rdt, True, False)
+
+    by_reduce = {r.name: p for p in passes for r in p.reduces}
+    done: set[int] = set()
+    for s in k.steps:
+        if isinstance(s, Reduce):
+            p = by_reduce[s.name]
+            if id(p) not in done:
+                done.add(id(p))
+                emit_pass(p)
+        elif s.name not in c.vec:
+            v = X.render(s.expr, loads, dict(c.scalars))
+            e(f"    const {X.REG_T[v.dtype]} {s.name} = {v.code};")
+            c.scalars[s.name] = X.Val(s.name, v.dtype, v.dim, False)
+    if C > 1:
+        e("    mlcb_cluster_arrive();        # peers may still read this CTA's partial results".replace("#", "//"))
+    for p in passes:
+        if p.stores and not p.reduces:
+            emit_pass(p)
+    at = len(c.lines)
+    _row_stores(c, loads)
+    c.lines[at:] = [ln.replace("if (live && lane == 0)", "if (rank == 0 && lane == 0)") for ln in c.lines[at:]]
+    if C > 1:
+        e("    mlcb_cluster_wait();")
+    e("    if (dead) mlcb_drain();")
+    e("}")
+    spec = LaunchSpec(grid=grid, block=T, smem=st.smem, vector=V, cluster=C,
+                      alg_bytes=algorithmic_bytes(k.inputs, k.outputs, k.n_rows * N))
+    return "\n".join(c.lines), spec

@@ -470,7 +470,11 @@ class _DirectCall:
                         for b in set(k.writes())]
         self.out = owner._collect(buffers)
         self.args = (fn.kernel, fn.grid, fn.block, fn.smem, fn.ptrs, fn.nptrs)
-        self.run = fn.lib.mlcb_launch
+        self.run, self.flags = fn.lib.mlcb_launch, fn.flags
+        if fn.smem:                  # bounded waits inside: prove them once, as a capture's warm-up does
+            fn[fn.grid]()
+            if owner._module.loaded.fault():
+                raise BackendError("a bounded wait inside a kernel ran out during warm-up")
         self.index = owner.device.index
 
     def __call__(self, inputs):
@@ -492,7 +496,7 @@ class _DirectCall:
             for i in slots:
                 ptrs[i] = p
         self.last = inputs
-        code = self.run(*self.args, torch._C._cuda_getCurrentRawStream(self.index), 0)
+        code = self.run(*self.args, torch._C._cuda_getCurrentRawStream(self.index), self.flags)
         if code != 0:
             raise BackendError(f"launch of {self.launch.name} failed with code {code}: "
                                f"{self.launch.lib.mlcb_last_error().decode(errors='replace')}")

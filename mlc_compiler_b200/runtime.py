@@ -229,6 +229,8 @@ class BoundLaunch:
         #: the device the module lives on: launches go to *its* current stream
         self.device = device
         self.grid, self.block, self.smem, self.flags = int(grid), int(block), int(smem), int(flags)
+        if self.smem:            # above 48 KB together with the static part it has to be asked for
+            _check(lib, lib.mlcb_kernel_shared(kernel, self.smem), f"shared memory of {name}")
         self._set(tuple(tensors))
 
     def _set(self, tensors) -> None:
@@ -279,8 +281,6 @@ class TensorLaunch(BoundLaunch):
         at = ctypes.addressof(self.ptrs)
         self.params = (ctypes.c_void_p * (len(spec.tmaps) + self.nptrs))(
             *[base + 128 * i for i in range(len(spec.tmaps))], *[at + 8 * i for i in range(self.nptrs)])
-        if spec.smem:            # above 48 KB together with the static part it has to be asked for
-            _check(lib, lib.mlcb_kernel_shared(kernel, spec.smem), f"shared memory of {name}")
 
     def __call__(self, *tensors, **consts) -> None:
         stream = torch.cuda.current_stream(self.device).cuda_stream
@@ -360,6 +360,7 @@ class CudaRuntime:
         tensors = tuple(buffers[n] for n in self._buffer_names(k))
         if flags is None:
             flags = self.flags
+        flags |= spec.cluster << 8 if spec.cluster > 1 else 0
         fn = BoundLaunch(self.lib, self.loaded.kernel(self.generated.symbol[k.name]), k.name,
                          spec.grid, spec.block, spec.smem, flags, tensors, self.device)
         return fn, spec.grid, tensors, {}
