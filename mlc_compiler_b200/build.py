@@ -78,6 +78,33 @@ def build_shim(force: bool = False) -> pathlib.Path:
     return LIB
 
 
+CALL = PKG / "_mlcb_call.so"
+
+
+def build_call(force: bool = False) -> pathlib.Path:
+    """Compile ``_mlcb_call.so``, the native call path, against the installed torch."""
+    src = CSRC / "mlcb_call.cpp"
+    if not force and not _stale(CALL, [src]):
+        return CALL
+    import sysconfig
+
+    import torch
+
+    root = pathlib.Path(torch.__file__).parent
+    tmp = CALL.with_suffix(f".so.{os.getpid()}.tmp")
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda_home() / "include",
+           pathlib.Path(sysconfig.get_paths()["include"])]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[x for i in inc for x in ("-isystem", str(i))], str(src), "-o", str(tmp),
+           f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {CALL.name} failed:\n{' '.join(cmd)}\n{r.stderr[-4000:]}")
+    tmp.replace(CALL)
+    return CALL
+
+
 def module_key(source: str, arch: str = ARCH) -> str:
     h = hashlib.sha256()
     h.update(source.encode())

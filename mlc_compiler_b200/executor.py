@@ -20,13 +20,15 @@ no interpreter fallback in this class.
 
 from __future__ import annotations
 
+import ctypes
+import functools
 from typing import Any, Mapping, Sequence
 
 import torch
 
 from . import concurrency, fuse, kir, rewrite
 from .config import Config
-from .runtime import BackendError, CudaRuntime, LaunchRun, TensorLaunch
+from .runtime import BackendError, CudaRuntime, LaunchRun, TensorLaunch, native_call
 
 
 class ExecutionError(Exception):
@@ -430,6 +432,11 @@ class _Executable:
 
 
 
+def _launch_failed(lib, name: str, code: int):
+    raise BackendError(f"launch of {name} failed with code {code}: "
+                       f"{lib.mlcb_last_error().decode(errors='replace')}")
+
+
 class _DirectCall:
     """A schedule of one generated kernel, launched on the caller's tensors.
 
@@ -452,8 +459,9 @@ class _DirectCall:
     def __init__(self, owner: "_Executable"):
         self.owner = owner
         self.launch = None
-        #: inputs of the last call: what ``replay`` runs on
-        self.last = None
+        #: the same call in native code (``csrc/mlcb_call.cpp``), once bound
+        self.native = None
+        self._last = None
 
     def _bind(self, inputs) -> None:
         owner = self.owner
@@ -470,7 +478,19 @@ class _DirectCall:
                         for b in set(k.writes())]
         self.out = owner._collect(buffers)
         self.args = (fn.kernel, fn.grid, fn.block, fn.smem, fn.ptrs, fn.nptrs)
+        if not set(k.reads()) & set(owner.params):
+            # consecutive calls overlap at their edges; a kernel with parameters reads them
+            # ahead of its wait and so starts after whatever the caller enqueued before it
+            fn.flags |= 1
         self.run, self.flags = fn.lib.mlcb_launch, fn.flags
+        native = native_call()
+        if native is not None:
+            address = ctypes.cast(fn.lib.mlcb_launch, ctypes.c_void_p).value
+            dtypes = [torch.empty(0, dtype=d) for _, d, _, _ in self.specs]
+            self.native = native(address, fn.kernel.value, fn.grid, fn.block, fn.smem, fn.flags, owner.device.index,
+                                 list(fn.ptrs)[:fn.nptrs],
+                                 [(tuple(s), d, n, at) for (s, _, n, at), d in zip(self.specs, dtypes)],
+                                 self.written, self.out, functools.partial(_launch_failed, fn.lib, fn.name))
         if fn.smem:                  # bounded waits inside: prove them once, as a capture's warm-up does
             fn[fn.grid]()
             if owner._module.loaded.fault():
@@ -480,6 +500,8 @@ class _DirectCall:
     def __call__(self, inputs):
         if self.launch is None:
             self._bind(inputs)
+        if self.native is not None:
+            return self.native(inputs)
         specs = self.specs
         if len(inputs) != len(specs):
             return self._refuse()
@@ -495,16 +517,20 @@ class _DirectCall:
                     return self._refuse()
             for i in slots:
                 ptrs[i] = p
-        self.last = inputs
+        self._last = inputs
         code = self.run(*self.args, torch._C._cuda_getCurrentRawStream(self.index), self.flags)
         if code != 0:
-            raise BackendError(f"launch of {self.launch.name} failed with code {code}: "
-                               f"{self.launch.lib.mlcb_last_error().decode(errors='replace')}")
+            _launch_failed(self.launch.lib, self.launch.name, code)
         return self.out
 
     def _refuse(self):
-        self.last = None
+        self._last = None
         return None
+
+    @property
+    def last(self):
+        """Inputs of the last call, which ``replay`` runs on; None after a captured one."""
+        return self._last if self.native is None else self.native.last
 
 
 class _Launched(_Executable):
@@ -525,6 +551,7 @@ class CompiledModel(_Executable):
         if self.device.type == "cuda" and self.device.index is None:
             self.device = torch.device("cuda", torch.cuda.current_device())
         self.backend = select_backend(self.cfg, self.device)
+        self._fast = None
 
         # What the schedule's kernels are.  ``self.schedule`` stays what the frontend produced;
         # ``self._exec`` may (1) have pointwise producers folded into the copies
@@ -573,6 +600,10 @@ class CompiledModel(_Executable):
         return (self._launched or self)._forward(inputs)
 
     def __call__(self, *inputs: torch.Tensor):
+        if self._fast is not None:
+            out = self._fast(inputs)
+            if out is not None:
+                return out
         # everything below enqueues on "the current stream": make that the model's
         # device's, whichever device the caller has current
         if torch.cuda.current_device() != self.device.index:
@@ -580,7 +611,10 @@ class CompiledModel(_Executable):
                 return self.__call__(*inputs)
         run = self._launched
         if run is None:
-            return self._call(inputs)
+            out = self._call(inputs)
+            if self._direct is not None and self.cfg.cuda_graphs:
+                self._fast = self._direct.native
+            return out
         out = run._call(inputs)
         self.dependent_policy, self.policy_timings_ms = run.dependent_policy, run.policy_timings_ms
         return out

@@ -97,6 +97,28 @@ def load_library(build_if_missing: bool = True):
     return lib
 
 
+_call_type = False
+
+
+def native_call():
+    """``Call`` of ``_mlcb_call.so`` (``csrc/mlcb_call.cpp``), or None where it has not
+    been built for this torch."""
+    global _call_type
+    if _call_type is False:
+        _call_type = None
+        if _build.CALL.exists():
+            from importlib import machinery, util
+
+            loader = machinery.ExtensionFileLoader("_mlcb_call", str(_build.CALL))
+            try:
+                module = util.module_from_spec(util.spec_from_loader("_mlcb_call", loader))
+                loader.exec_module(module)
+                _call_type = module.Call
+            except ImportError:
+                pass
+    return _call_type
+
+
 def _check(lib, code: int, what: str) -> None:
     if code != 0:
         msg = lib.mlcb_last_error().decode(errors="replace")
