@@ -1,0 +1,281 @@
+// C = A B over fp32 operands on the 16-bit tensor cores, without losing a bit of them.
+//
+// An fp32 value is exactly the sum of three bf16 ones (24 significant bits in three
+// pieces of 8, cut by truncation), so A B is nine bf16 matmuls whose products are exact
+// in fp32 (last times last piece, 2^-32 of the product, is left out).  Sixteen converter
+// warps read the operands a block ahead, cut them and store the pieces as swizzled
+// tiles; the pieces of B lie side by side as one operand, so one MMA multiplies a piece of
+// A with several.  Leading products (first piece times first piece) have accumulators of
+// their own, a new one for every few blocks, and the corrections, 2^-8 of them and less,
+// another: the tensor cores round each addition of 16 products towards zero, and the
+// chain of those is what an error grows with (K = 1024 in one chain: 1.0e-6 of the
+// result's norm; in four: 3e-7; the library's fp32 sum: 5.7e-7).  A result that is not
+// finite is recomputed as a plain fp32 sum (an infinity cut in pieces is Inf - Inf).
+#pragma once
+
+template <int M_, int N_, int K_, int LDA_, int LDB_, i64 ZA_, i64 ZB_, int BN_, int STAGES_, int SPLIT_, int LEADS_,
+          int GROUPS_, int BATCH_, bool B_MN_, int A_VEC_, int B_VEC_, bool B_STABLE_>
+struct mlcb_mm32_cfg {
+    static constexpr int M = M_, N = N_, K = K_, LDA = LDA_, LDB = LDB_, BN = BN_, STAGES = STAGES_, SPLIT = SPLIT_,
+                         LEADS = LEADS_, GROUPS = GROUPS_, BATCH = BATCH_, A_VEC = A_VEC_, B_VEC = B_VEC_;
+    static constexpr i64 ZA = ZA_, ZB = ZB_;
+    static constexpr bool B_MN = B_MN_, B_STABLE = B_STABLE_;
+    static constexpr int TM = (M + 127) / 128, TN = (N + BN - 1) / BN, KB = (K + 63) / 64;
+    static constexpr u32 PLANE_A = 16384, PLANE_B = BN * 128, STAGE = 3 * (PLANE_A + PLANE_B);
+    static constexpr int COLS = (3 + LEADS) * BN <= 128 ? 128 : (3 + LEADS) * BN <= 256 ? 256 : 512;
+    static constexpr int PER_LEAD = ((KB + SPLIT - 1) / SPLIT + LEADS - 1) / LEADS;   // blocks
+    static_assert((3 + LEADS) * BN <= 512, "accumulators");
+    static constexpr int CW = 16, CT = 32 * CW;                                   // converter warps and threads
+    static constexpr int A_CHUNKS = 128 * 16 / CT, B_CHUNKS = BN * 16 / CT;       // of 4 values, per thread
+    static_assert((BN == 32 && !B_MN) || BN == 64, "tile");
+    static_assert(KB >= SPLIT && BN % (8 * SPLIT) == 0, "split");
+};
+
+// four values of row `row` from column `c`; zero outside [0, rows) x [0, cols)
+template <int VEC>
+__device__ __forceinline__ float4 mlcb_fetch4(const float* p, i64 ld, int row, int rows, int c, int cols) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (row < rows) {
+        const float* q = p + row * ld + c;
+        if (VEC == 4) {
+            if (c < cols) v = *reinterpret_cast<const float4*>(q);
+        } else {
+            if (c < cols) v.x = q[0];
+            if (c + 1 < cols) v.y = q[1];
+            if (c + 2 < cols) v.z = q[2];
+            if (c + 3 < cols) v.w = q[3];
+        }
+    }
+    return v;
+}
+
+// the three pieces of four values, to the three planes of a swizzled tile
+__device__ __forceinline__ void mlcb_cut4(float4 v, u32 tile, u32 plane, int row, int chunk) {
+    const u32 at = tile + row * 128 + ((((u32)chunk >> 1) ^ (row & 7)) << 4) + (chunk & 1) * 8;
+    u32 x[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(at + p * plane), "r"(__byte_perm(x[0], x[1], 0x7632)),
+                     "r"(__byte_perm(x[2], x[3], 0x7632)) : "memory");
+        if (p < 2) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                x[i] = __float_as_uint(__uint_as_float(x[i]) - __uint_as_float(x[i] & 0xffff0000u));
+        }
+    }
+}
+
+template <typename C, typename Epi>
+__device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, const float* b1, const float* b2,
+                                              const float* b3, const Epi& epi) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ alignas(8) u64 bars[2 * C::STAGES + 1];
+    __shared__ u32 tmem_slot;
+    __shared__ volatile u32 dead;
+    const u32 smem = (mlcb_smem(smem_raw) + 1023u) & ~1023u;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int part = C::SPLIT > 1 ? (int)mlcb_cta_rank() : 0;
+    const u32 full = mlcb_smem(bars), empty = full + 8 * C::STAGES, done = empty + 8 * C::STAGES;
+
+    if (threadIdx.x == 0) {
+        dead = 0;
+        for (int i = 0; i < C::STAGES; ++i) { mlcb_bar_init(full + 8 * i, C::CW); mlcb_bar_init(empty + 8 * i, 1); }
+        mlcb_bar_init(done, 1);
+        mlcb_bar_fence_init();
+    }
+    if (warp == C::CW) mlcb_tmem_alloc<1>(mlcb_smem(&tmem_slot), C::COLS);
+    mlcb_tc_before();
+    __syncthreads();
+    mlcb_tc_after();
+    const u32 tmem = tmem_slot;
+    MLCB_GRID_TRIGGER();
+
+    const int tile = blockIdx.x / C::SPLIT;
+    const int m0 = tile % C::TM * 128, n0 = tile / C::TM % C::TN * C::BN, g = tile / (C::TM * C::TN) % C::GROUPS;
+    const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
+    const int k0 = part * C::KB / C::SPLIT, k1 = (part + 1) * C::KB / C::SPLIT;
+    a += z * C::ZA;
+    const float* b = (C::GROUPS == 1 ? b0 : g == 0 ? b0 : g == 1 ? b1 : g == 2 ? b2 : b3) + z * C::ZB;
+    constexpr int SLICE = C::BN / C::SPLIT;
+
+    if (warp == C::CW) {
+        const bool elected = mlcb_elect();
+        constexpr u32 one = mlcb_idesc(128, C::BN, true, C::B_MN), two = mlcb_idesc(128, 2 * C::BN, true, C::B_MN),
+                      three = mlcb_idesc(128, 3 * C::BN, true, C::B_MN);
+        int s = 0;
+        u32 phase = 0;
+        for (int kb = k0; kb < k1; ++kb) {
+            if (!mlcb_bar_wait(full + 8 * s, phase, &dead)) break;
+            mlcb_tc_after();
+            const u32 at = smem + s * C::STAGE;
+            const u64 db = mlcb_desc(at + 3 * C::PLANE_A, C::B_MN ? 8192 : 16);
+            if (elected) {
+                const u64 da = mlcb_desc(at, 16);
+                const int i = kb - k0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const u64 ka = da + k * 2, bk = db + k * (C::B_MN ? 128 : 2);
+                    mlcb_mma<1>(tmem, ka + C::PLANE_A / 16, bk, three, i > 0 || k > 0);
+                    mlcb_mma<1>(tmem + (3 + i / C::PER_LEAD) * C::BN, ka, bk, one, i % C::PER_LEAD > 0 || k > 0);
+                    mlcb_mma<1>(tmem + C::BN, ka, bk + C::PLANE_B / 16, two, true);
+                    mlcb_mma<1>(tmem, ka + 2 * C::PLANE_A / 16, bk, two, true);
+                }
+                mlcb_mma_commit<1>(empty + 8 * s);
+            }
+            __syncwarp();
+            if (++s == C::STAGES) { s = 0; phase ^= 1; }
+        }
+        if (elected) mlcb_mma_commit<1>(done);
+        __syncwarp();
+    } else {
+        const int t = threadIdx.x;
+        float4 va[2][C::A_CHUNKS], vb[2][C::B_CHUNKS];
+        auto fetch_b = [&](int kb, float4 (&v)[C::B_CHUNKS]) {
+#pragma unroll
+            for (int j = 0; j < C::B_CHUNKS; ++j) {
+                const int i = t + C::CT * j;
+                v[j] = C::B_MN ? mlcb_fetch4<C::B_VEC>(b, C::LDB, kb * 64 + i / 16, C::K, n0 + i % 16 * 4, C::N)
+                               : mlcb_fetch4<C::B_VEC>(b, C::LDB, n0 + i / 16, C::N, kb * 64 + i % 16 * 4, C::K);
+            }
+        };
+        auto fetch_a = [&](int kb, float4 (&v)[C::A_CHUNKS]) {
+#pragma unroll
+            for (int j = 0; j < C::A_CHUNKS; ++j) {
+                const int i = t + C::CT * j;
+                v[j] = mlcb_fetch4<C::A_VEC>(a, C::LDA, m0 + i / 16, C::M, kb * 64 + i % 16 * 4, C::K);
+            }
+        };
+        if (C::B_STABLE) fetch_b(k0, vb[0]);
+        MLCB_GRID_WAIT();
+        if (!C::B_STABLE) fetch_b(k0, vb[0]);
+        fetch_a(k0, va[0]);
+        int s = 0;
+        u32 phase = 1;
+        bool alive = true;
+        auto block = [&](int kb, float4 (&ca)[C::A_CHUNKS], float4 (&cb)[C::B_CHUNKS], float4 (&na)[C::A_CHUNKS],
+                         float4 (&nb)[C::B_CHUNKS]) {
+            if (kb + 1 < k1) { fetch_b(kb + 1, nb); fetch_a(kb + 1, na); }
+            alive = mlcb_bar_wait(empty + 8 * s, phase, &dead);
+            if (!alive) return;
+            const u32 at = smem + s * C::STAGE;
+#pragma unroll
+            for (int j = 0; j < C::B_CHUNKS; ++j) {
+                const int i = t + C::CT * j;
+                mlcb_cut4(cb[j], at + 3 * C::PLANE_A, C::PLANE_B, i / 16, i % 16);
+            }
+#pragma unroll
+            for (int j = 0; j < C::A_CHUNKS; ++j) {
+                const int i = t + C::CT * j;
+                mlcb_cut4(ca[j], at, C::PLANE_A, i / 16, i % 16);
+            }
+            mlcb_proxy_fence();
+            __syncwarp();
+            if (lane == 0) mlcb_bar_arrive(full + 8 * s);
+            if (++s == C::STAGES) { s = 0; phase ^= 1; }
+        };
+        for (int kb = k0; kb < k1 && alive; kb += 2) {
+            block(kb, va[0], vb[0], va[1], vb[1]);
+            if (kb + 1 < k1 && alive) block(kb + 1, va[1], vb[1], va[0], vb[0]);
+        }
+    }
+    __syncwarp();
+    const int quad = warp % 4, half = warp / 4, r = quad * 32 + lane, row = m0 + r;
+    const u32 base = tmem + ((u32)(quad * 32) << 16);
+    // partial sums of a split K land where the operands were: every CTA of the cluster is past them
+    const u32 inbox = smem;
+    if (warp < C::CW) {
+        mlcb_bar_wait(done, 0, &dead);
+        mlcb_tc_after();
+    }
+    if (C::SPLIT > 1) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }
+    if (warp < C::CW && !dead) {
+        // the four warps that share 32 rows take 16 columns each in turn
+#pragma unroll 1
+        for (int c = half * 16; c < C::BN; c += C::CW * 4) {
+            float v[16], w[16];
+            mlcb_tmem_ld(base + 2 * C::BN + c, v);
+            mlcb_tmem_ld(base + C::BN + c, w);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += w[i];
+            mlcb_tmem_ld(base + c, w);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += w[i];
+            float lead[16];
+            mlcb_tmem_ld(base + 3 * C::BN + c, lead);
+#pragma unroll
+            for (int l = 1; l < C::LEADS; ++l) {
+                if (l * C::PER_LEAD >= k1 - k0) break;
+                mlcb_tmem_ld(base + (3 + l) * C::BN + c, w);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) lead[i] += w[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += lead[i];
+            bool finite = true;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) finite = finite && fabsf(v[i]) <= 3.402823466e38f;
+            if (!finite && row < C::M) {
+#pragma unroll 1
+                for (int i = 0; i < 16; ++i) {
+                    float x = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) x = j == i ? v[j] : x;
+                    if (fabsf(x) <= 3.402823466e38f || n0 + c + i >= C::N) continue;
+                    x = 0.0f;
+                    for (int k = k0 * 64; k < min(C::K, k1 * 64); ++k)
+                        x = fmaf(a[(i64)row * C::LDA + k],
+                                 C::B_MN ? b[(i64)k * C::LDB + n0 + c + i] : b[(i64)(n0 + c + i) * C::LDB + k], x);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = j == i ? x : v[j];
+                }
+            }
+            __syncwarp();
+            if (C::SPLIT == 1) {
+                epi.columns(v, row, n0 + c, g, z, lane);
+                __syncwarp();
+            } else {
+                const u32 mine = inbox + (part * SLICE * 128 + r * 4) * 4;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int col = c + 4 * q;
+                    u32 at;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                                 : "=r"(at) : "r"(mine + (col % SLICE) * 512), "r"((u32)(col / SLICE)));
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+                                 :: "r"(at), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                                 : "memory");
+                }
+            }
+        }
+    }
+    __syncwarp();
+    if (C::SPLIT > 1) {
+        mlcb_cluster_arrive();
+        mlcb_cluster_wait();
+        if (warp < C::CW && !dead) {
+#pragma unroll
+            for (int c = half * 8; c < SLICE; c += C::CW * 2) {
+                float v[8];
+#pragma unroll
+                for (int p = 0; p < C::SPLIT; ++p)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        float x[4];
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                                     : "r"(inbox + ((p * SLICE + c + 4 * q) * 128 + r * 4) * 4) : "memory");
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) v[4 * q + i] = p ? v[4 * q + i] + x[i] : x[i];
+                    }
+                epi.columns(v, row, n0 + part * SLICE + c, g, z, lane);
+                __syncwarp();
+            }
+        }
+    }
+    mlcb_tc_before();
+    __syncthreads();
+    if (warp == C::CW) {
+        mlcb_tc_after();
+        mlcb_tmem_free<1>(tmem, C::COLS);
+    }
+}

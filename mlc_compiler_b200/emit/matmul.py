@@ -68,6 +68,11 @@ class Config:
     grid: int
     kstep: int = 1   # 64-element K blocks per stage
 
+    @property
+    def per_call(self) -> int:
+        """Columns the kernel hands the epilogue at a time."""
+        return 8 if self.split > 1 else 32
+
     def stage_bytes(self) -> int:
         return self.kstep * (128 * 128 + self.bn // self.cg * 128)
 
@@ -212,10 +217,10 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
     extents = [z * m * n] + [a.index.bounds()[1] + 1 for e in k.epilogues
                              for a in [x for x in e.inputs if x is not None] + e.outputs]
     it = "i64" if needs_64bit(*extents) else "int"
-    nv = 8 if mc.split > 1 else 32
+    nv = mc.per_call
     W = _pack_width(k.epilogues, n, 8 if nv == 8 else 16)
     row_expr = "row" if z == 1 else f"(z * {m} + row)"
-    rn = "mlcb_rn_f16" if k.dtype == "float16" else "mlcb_rn_bf16"
+    rn = {"float16": "mlcb_rn_f16", "bfloat16": "mlcb_rn_bf16", "float32": ""}[k.dtype]
     plain = not e0.body and len(e0.outputs) == 1 and e0.outputs[0].dtype == k.dtype
 
     L.append("    template <int NV> __device__ __forceinline__ void columns(float (&v)[NV], int row, int col, "
@@ -261,7 +266,8 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
                 loads.append(X.Val(f"{rn}(mlcb_f2(v[c + j], v[c + j + 1]))", "float32", True, False))
                 continue
             if a is None:
-                loads.append(X.Val(f"{rn}(v[c + j])", "float32", True, False, (f"v[c + j]", k.dtype)))
+                loads.append(X.Val(f"{rn}(v[c + j])", "float32", True, False,
+                                   (f"v[c + j]", k.dtype) if rn else None))
                 continue
             st, rt = X.STORAGE_T[a.dtype], X.REG_T[a.dtype]
             ac = classify(a.index, "col", W)
@@ -308,6 +314,8 @@ def emit_matmul(k: MatmulKernel, cfg, buffers, name: str | None = None, stable=f
     """(text, LaunchSpec) of one matmul kernel; the launch passes the tensor maps, then
     the epilogue's pointers."""
     name = name or k.name
+    if k.dtype == "float32":
+        return emit_matmul32(k, cfg, buffers, name, stable)
     z, m, n, kk = k.shape
     b_mn = tma_layout(k.bs[0], -1, -2) == "mn"
     a_cut, b_cut = can_cut(k.a, -2, -1), can_cut(k.bs[0], -1, -2)
@@ -347,3 +355,87 @@ def emit_matmul(k: MatmulKernel, cfg, buffers, name: str | None = None, stable=f
     spec = LaunchSpec(grid=mc.grid, block=threads, smem=mc.smem(), vector=1, alg_bytes=total, cluster=cluster,
                       tmaps=tuple(tmaps), buffers=tuple(names))
     return text, spec
+
+
+# --------------------------------------------------------------------------
+# fp32 operands (csrc/mlcb_matmul32.cuh)
+# --------------------------------------------------------------------------
+
+@dataclass(frozen=True)
+class Config32:
+    bn: int
+    stages: int
+    split: int
+    grid: int
+    leads: int
+    epi_warps: int = 16
+
+    @property
+    def per_call(self) -> int:
+        return 8 if self.split > 1 else 16
+
+    def smem(self) -> int:
+        return self.stages * 3 * (16384 + self.bn * 128) + 1024
+
+
+def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool) -> Config32:
+    """Least estimated time, in microseconds: a 64-deep block costs 0.75 (32 columns) or 1.0
+    (64), a wave 3 before and after.  Leading products get a new accumulator every four
+    blocks, as far as TMEM goes."""
+    kb = _ceil(k, 64)
+
+    def cost(bn, split, groups):
+        t = _ceil(m, 128) * _ceil(n, bn) * groups * z
+        waves = _ceil(t, _RESIDENT[split])
+        exchange = 0.8 + 0.2 * split if split > 1 else 0.0
+        return waves * (_ceil(kb, split) * (0.75 if bn == 32 else 1.0) + 3.0 + exchange)
+
+    widths = (64,) if b_mn else (32, 64)
+    splits = (1,) if z > 1 else tuple(s for s in (1, 2, 4, 8) if s <= kb)
+    bn, split = min(((bn, s) for bn in widths for s in splits if bn % (8 * s) == 0),
+                    key=lambda c: cost(*c, groups))
+    t = _ceil(m, 128) * _ceil(n, bn) * groups * z
+    return Config32(bn, max(2, min(3, _ceil(kb, split))), split, t * split,
+                    min(5, _ceil(_ceil(kb, split), 4)))
+
+
+def emit_matmul32(k: MatmulKernel, cfg, buffers, name: str, stable):
+    z, m, n, kk = k.shape
+    b0 = k.bs[0]
+    b_mn = b0.strides[-2] != 1
+    mc = choose32(z, m, n, kk, len(k.bs), b_mn)
+    for e in k.epilogues:
+        for a in [x for x in e.inputs if x is not None] + e.outputs:
+            check_bounds(a.index, buffers[a.buffer].numel, f"{k.name}:{a.name}")
+    with X.math_mode(False):
+        functor, params, names = _emit_functor(k, cfg, mc, stable)
+
+    def four(v, rows_axis, inner_axis) -> int:
+        """Values per access: 4 where every row, and its end, is 16-byte aligned."""
+        lead = [v.strides[0]] if len(v.shape) == 3 else []
+        return 4 if all(x % 4 == 0 for x in [v.strides[rows_axis], v.offset, v.shape[inner_axis]] + lead) else 1
+
+    a_vec = four(k.a, -2, -1)
+    b_vec = min(four(b, -2 if b_mn else -1, -1 if b_mn else -2) for b in k.bs)
+    za = k.a.strides[0] if z > 1 else 0
+    zb = b0.strides[0] if z > 1 else 0
+    flag = lambda x: "true" if x else "false"      # noqa: E731
+    b_stable = all(b.buffer in stable for b in k.bs)
+    conf = (f"mlcb_mm32_cfg<{m}, {n}, {kk}, {k.a.strides[-2]}, {b0.strides[-2] if b_mn else b0.strides[-1]}, {za}, {zb}, "
+            f"{mc.bn}, {mc.stages}, {mc.split}, {mc.leads}, {len(k.bs)}, {z}, {flag(b_mn)}, {a_vec}, {b_vec}, {flag(b_stable)}>")
+    ops = ["const float* a"] + [f"const float* b{i}" for i in range(len(k.bs))]
+    bs = [f"b{min(i, len(k.bs) - 1)} + {k.bs[min(i, len(k.bs) - 1)].offset}" for i in range(4)]
+    fields = ", ".join(p.split("* ")[1] for p in params)
+    text = "\n".join([
+        functor.replace("MLCB_KERNEL_NAME", name),
+        f'extern "C" __global__ void __launch_bounds__(544, 1) {name}({", ".join(ops + params)}) {{',
+        f"    // {z} x [{m}, {kk}] x [{kk}, {n}] x {len(k.bs)}, fp32 in three bf16 pieces; tile 128 x {mc.bn}, "
+        f"{mc.stages} stages, split {mc.split}, grid {mc.grid}",
+        f"    const {name}_epi epi{{{fields}}};",
+        f"    mlcb_matmul32<{conf}>(a + {k.a.offset}, {', '.join(bs)}, epi);",
+        "}"])
+    total = sum(v.numel for v in [k.a] + k.bs) * 4
+    total += sum(algorithmic_bytes([x for x in e.inputs if x is not None], e.outputs, z * m * n)
+                 for e in k.epilogues)
+    return text, LaunchSpec(grid=mc.grid, block=544, smem=mc.smem(), alg_bytes=total, cluster=mc.split,
+                            buffers=tuple([k.a.buffer] + [b.buffer for b in k.bs] + names))

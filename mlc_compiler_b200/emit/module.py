@@ -63,8 +63,8 @@ def device_header() -> str:
 
 def tensor_headers(kinds: set) -> list[str]:
     """The tensor-core parts of the device library that kernels of these kinds use."""
-    files = ["mlcb_tensor.cuh"] * bool(kinds & {"mm", "att", "staged"}) + ["mlcb_matmul.cuh"] * ("mm" in kinds) \
-        + ["mlcb_attention.cuh"] * ("att" in kinds)
+    files = ["mlcb_tensor.cuh"] * bool(kinds & {"mm", "mm32", "att", "staged"}) + ["mlcb_matmul.cuh"] * ("mm" in kinds) \
+        + ["mlcb_matmul32.cuh"] * ("mm32" in kinds) + ["mlcb_attention.cuh"] * ("att" in kinds)
     return [(CSRC / f).read_text().replace("#pragma once\n", "") for f in files]
 
 
@@ -110,7 +110,7 @@ def generate_module(schedule, cfg, *, inline_header: bool = True, pdl: bool | No
         text, spec = emit_kernel(k, cfg, schedule.buffers, placeholder, stable)
         kind = {"PointwiseKernel": "pw", "ReductionKernel": "red", "MatmulKernel": "mm",
                 "AttentionKernel": "att"}[type(k).__name__]
-        kinds.add("staged" if "mlcb_bulk_load" in text else kind)
+        kinds.add("mm32" if "mlcb_mm32_cfg" in text else "staged" if "mlcb_bulk_load" in text else kind)
         # operand names appear only in comments; identity is the code itself
         code = re.sub(r"[ \t]*//[^\n]*", "", text)
         digest = hashlib.sha256(code.encode()).hexdigest()[:12]

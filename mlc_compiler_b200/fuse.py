@@ -127,12 +127,19 @@ def _matmul(k, schedule) -> MatmulKernel | None:
         return None
     a, b, out = k.args[0], k.args[1], k.outputs[0]
     dts = {schedule.buffers[v.buffer].dtype for v in (a, b, out)}
-    if len(dts) != 1 or next(iter(dts)) not in kir.NARROW_FLOATS or not out.numel or not a.numel:
+    if len(dts) != 1 or not out.numel or not a.numel:
         return None
-    if tma_layout(a, -2, -1) != "k":
-        return None
-    lb = tma_layout(b, -1, -2)
-    if lb is None or (lb == "mn" and b.shape[-1] < 64):
+    if dts == {"float32"}:
+        if a.strides[-1] != 1 or 1 not in b.strides[-2:] or min(a.strides + b.strides) < 0 \
+                or max(schedule.buffers[v.buffer].numel for v in (a, b)) >= 1 << 31:
+            return None
+    elif dts <= set(kir.NARROW_FLOATS):
+        if tma_layout(a, -2, -1) != "k":
+            return None
+        lb = tma_layout(b, -1, -2)
+        if lb is None or (lb == "mn" and b.shape[-1] < 64):
+            return None
+    else:
         return None
     z = out.shape[0] if len(out.shape) == 3 else 1
     m, n = out.shape[-2:]
@@ -274,7 +281,7 @@ def _attention(i: int, kernels: list, readers: dict, finals: set, schedule) -> t
     """The attention kernel that starts at matmul ``kernels[i]``, and the positions of the
     row kernel and the second matmul it absorbs."""
     a = kernels[i]
-    if a.epilogues[0].body or len(a.bs) != 1 or len(a.a.shape) != 3:
+    if a.epilogues[0].body or len(a.bs) != 1 or len(a.a.shape) != 3 or a.dtype not in kir.NARROW_FLOATS:
         return None
 
     def sole_reader(view):

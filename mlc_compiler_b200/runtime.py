@@ -379,7 +379,7 @@ class CudaRuntime:
             fn = TensorLaunch(self.lib, self.loaded.kernel(self.generated.symbol[k.name]), k.name, spec,
                               self.flags if flags is None else flags, tensors, buffers, self.device)
             return fn, spec.grid, tensors, {}
-        tensors = tuple(buffers[n] for n in self._buffer_names(k))
+        tensors = tuple(buffers[n] for n in spec.buffers or self._buffer_names(k))
         if flags is None:
             flags = self.flags
         flags |= spec.cluster << 8 if spec.cluster > 1 else 0
