@@ -80,16 +80,18 @@ struct mlcb_mm_cfg {
 
 template <typename C, typename Epi>
 __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap* tb0, const mlcb_tmap* tb1,
-                                            const mlcb_tmap* tb2, const mlcb_tmap* tb3, const Epi& epi) {
+                                            const mlcb_tmap* tb2, const mlcb_tmap* tb3, const Epi& epi,
+                                            const mlcb_next& next) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ alignas(8) u64 bars[2 * C::STAGES + 2 * C::ACC];
+    __shared__ alignas(8) u64 bars[2 * C::STAGES + 2 * C::ACC + 1];
     __shared__ u32 tmem_slot;
     __shared__ volatile u32 dead;
     const u32 smem = (mlcb_smem(smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const u32 rank = C::CLUSTER > 1 ? mlcb_cta_rank() : 0;
     const u32 full = mlcb_smem(bars), empty = full + 8 * C::STAGES, acc_full = empty + 8 * C::STAGES,
-              acc_empty = acc_full + 8 * C::ACC;
+              acc_empty = acc_full + 8 * C::ACC,
+              arrived = acc_empty + 8 * C::ACC;
 
     if (threadIdx.x == 0) {
         dead = 0;
@@ -98,6 +100,8 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
             mlcb_bar_init(acc_full + 8 * i, 1);
             mlcb_bar_init(acc_empty + 8 * i, C::CG * C::EPI_WARPS);
         }
+        mlcb_bar_init(arrived, 1);
+        if (C::SPLIT > 1) mlcb_bar_expect(arrived, 128 * C::BN * 4);
         mlcb_bar_fence_init();
         mlcb_tma_prefetch(ta);
         mlcb_tma_prefetch(tb0);
@@ -157,6 +161,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
                     }
                 }
             }
+            if (elected) mlcb_prefetch_next(next);
             MLCB_GRID_WAIT();
             int s = 0;
             u32 phase = 1;
@@ -227,11 +232,19 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
             const int tm = tile % C::TM, tn = (tile / C::TM) % C::TN, g = (tile / (C::TM * C::TN)) % C::GROUPS;
             const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
             const int row = tm * (128 * C::CG) + pair * 128 + r;
-            mlcb_bar_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
-            mlcb_tc_after();
-            if (C::SPLIT > 1) {
+            if constexpr (C::SPLIT > 1) {
+                constexpr int EACH = (SLICE + 8 * HALVES - 1) / (8 * HALVES);
+                // the epilogue's own operands are fetched while the products are still being summed
+                const int first = tn * C::BN + part * SLICE;
+                typename Epi::template Pre<8> pre[EACH];
+#pragma unroll
+                for (int i = 0; i < EACH; ++i)
+                    if ((half + i * HALVES) * 8 < SLICE) epi.fetch(pre[i], row, first + (half + i * HALVES) * 8, g, z);
+                mlcb_bar_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+                mlcb_tc_after();
                 // partial sums go straight into the shared memory of the CTA that finishes these
-                // columns, as [source rank][column quad][row][4]: conflict-free both ways
+                // columns, as [source part][column quad][row][4]: conflict-free both ways.  Its
+                // barrier counts their bytes (a cluster barrier instead took 1270 cycles here)
                 const u32 mine = inbox + (part * SLICE * 128 + r * 4) * 4;
 #pragma unroll
                 for (int c = half * 16; c < C::BN; c += 16 * HALVES) {
@@ -240,18 +253,39 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int col = c + 4 * q;
-                        u32 at;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                                     : "=r"(at) : "r"(mine + (col % SLICE) * 512), "r"((u32)(col / SLICE * C::CG + pair)));
-                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
-                                     :: "r"(at), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
-                                     : "memory");
+                        mlcb_send4(mine + (col % SLICE) * 512, arrived, (u32)(col / SLICE * C::CG + pair),
+                                   v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     }
                 }
+                if (!mlcb_bar_wait(arrived, 0, &dead)) break;
+#pragma unroll
+                for (int i = 0; i < EACH; ++i) {
+                    const int c = (half + i * HALVES) * 8;
+                    if (c >= SLICE) break;
+                    float v[8];
+#pragma unroll
+                    for (int p = 0; p < C::SPLIT; ++p)
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            float x[4];
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                                         : "r"(inbox + ((p * SLICE + c + 4 * q) * 128 + r * 4) * 4) : "memory");
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v[4 * q + j] = p ? v[4 * q + j] + x[j] : x[j];
+                        }
+                    epi.columns(v, pre[i], row, first + c, g, z, lane);
+                    __syncwarp();
+                }
             } else {
+                typename Epi::template Pre<32> pre, ahead;
+                epi.fetch(pre, row, tn * C::BN + half * 32, g, z);
+                mlcb_bar_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+                mlcb_tc_after();
 #pragma unroll 1
                 for (int c = half * 32; c < C::BN; c += 32 * HALVES) {
                     float v[32];
+                    if (c + 32 * HALVES < C::BN) epi.fetch(ahead, row, tn * C::BN + c + 32 * HALVES, g, z);
                     mlcb_tmem_ld(base + acc * C::BN + c, v);
                     if (c + 32 * HALVES >= C::BN) {
                         mlcb_tc_before();
@@ -261,41 +295,14 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
                             else mlcb_bar_arrive_at(acc_empty + 8 * acc, rank & ~1u);
                         }
                     }
-                    epi.columns(v, row, tn * C::BN + c, g, z, lane);
+                    epi.columns(v, pre, row, tn * C::BN + c, g, z, lane);
+                    pre = ahead;
                     __syncwarp();
                 }
             }
         }
     }
     __syncwarp();
-    if (C::SPLIT > 1) {
-        mlcb_cluster_arrive();
-        mlcb_cluster_wait();
-        if (warp >= 2 && cluster < C::TILES && !dead) {
-            const int quad = warp % 4, half = (warp - 2) / 4;
-            constexpr int HALVES = C::EPI_WARPS / 4;
-            const int r = quad * 32 + lane;
-            const int tm = cluster % C::TM, tn = (cluster / C::TM) % C::TN, g = (cluster / (C::TM * C::TN)) % C::GROUPS;
-            const int z = C::BATCH > 1 ? cluster / (C::TM * C::TN * C::GROUPS) : 0;
-#pragma unroll
-            for (int c = half * 8; c < SLICE; c += 8 * HALVES) {
-                float v[8];
-#pragma unroll
-                for (int p = 0; p < C::SPLIT; ++p)
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        float x[4];
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                     : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
-                                     : "r"(inbox + ((p * SLICE + c + 4 * q) * 128 + r * 4) * 4) : "memory");
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) v[4 * q + i] = p ? v[4 * q + i] + x[i] : x[i];
-                    }
-                epi.columns(v, tm * (128 * C::CG) + pair * 128 + r, tn * C::BN + part * SLICE + c, g, z, lane);
-                __syncwarp();
-            }
-        }
-    }
     mlcb_tc_before();
     __syncthreads();
     if (C::CG == 2) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }   // the peer still uses our barriers and TMEM

@@ -67,20 +67,23 @@ __device__ __forceinline__ void mlcb_cut4(float4 v, u32 tile, u32 plane, int row
 
 template <typename C, typename Epi>
 __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, const float* b1, const float* b2,
-                                              const float* b3, const Epi& epi) {
+                                              const float* b3, const Epi& epi, const mlcb_next& next) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ alignas(8) u64 bars[2 * C::STAGES + 1];
+    __shared__ alignas(8) u64 bars[2 * C::STAGES + 2];
     __shared__ u32 tmem_slot;
     __shared__ volatile u32 dead;
     const u32 smem = (mlcb_smem(smem_raw) + 1023u) & ~1023u;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int part = C::SPLIT > 1 ? (int)mlcb_cta_rank() : 0;
-    const u32 full = mlcb_smem(bars), empty = full + 8 * C::STAGES, done = empty + 8 * C::STAGES;
+    const u32 full = mlcb_smem(bars), empty = full + 8 * C::STAGES, done = empty + 8 * C::STAGES,
+              arrived = done + 8;
 
     if (threadIdx.x == 0) {
         dead = 0;
         for (int i = 0; i < C::STAGES; ++i) { mlcb_bar_init(full + 8 * i, C::CW); mlcb_bar_init(empty + 8 * i, 1); }
         mlcb_bar_init(done, 1);
+        mlcb_bar_init(arrived, 1);
+        if (C::SPLIT > 1) mlcb_bar_expect(arrived, 128 * C::BN * 4);
         mlcb_bar_fence_init();
     }
     if (warp == C::CW) mlcb_tmem_alloc<1>(mlcb_smem(&tmem_slot), C::COLS);
@@ -88,6 +91,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     __syncthreads();
     mlcb_tc_after();
     const u32 tmem = tmem_slot;
+    if (C::SPLIT > 1) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }
     MLCB_GRID_TRIGGER();
 
     const int tile = blockIdx.x / C::SPLIT;
@@ -100,6 +104,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
 
     if (warp == C::CW) {
         const bool elected = mlcb_elect();
+        if (elected) mlcb_prefetch_next(next);
         constexpr u32 one = mlcb_idesc(128, C::BN, true, C::B_MN), two = mlcb_idesc(128, 2 * C::BN, true, C::B_MN),
                       three = mlcb_idesc(128, 3 * C::BN, true, C::B_MN);
         int s = 0;
@@ -181,13 +186,18 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     __syncwarp();
     const int quad = warp % 4, half = warp / 4, r = quad * 32 + lane, row = m0 + r;
     const u32 base = tmem + ((u32)(quad * 32) << 16);
-    // partial sums of a split K land where the operands were: every CTA of the cluster is past them
-    const u32 inbox = smem;
+    const u32 inbox = smem + C::STAGES * C::STAGE;     // partial sums of a split K
     if (warp < C::CW) {
         mlcb_bar_wait(done, 0, &dead);
         mlcb_tc_after();
     }
-    if (C::SPLIT > 1) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }
+    constexpr int EACH = (SLICE + C::CW * 2 - 1) / (C::CW * 2);
+    typename Epi::template Pre<8> pre[EACH];
+    if constexpr (C::SPLIT > 1) if (warp < C::CW) {
+#pragma unroll
+        for (int i = 0; i < EACH; ++i)
+            if (half * 8 + i * C::CW * 2 < SLICE) epi.fetch(pre[i], row, n0 + part * SLICE + half * 8 + i * C::CW * 2, g, z);
+    }
     if (warp < C::CW && !dead) {
         // the four warps that share 32 rows take 16 columns each in turn
 #pragma unroll 1
@@ -230,31 +240,29 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
                 }
             }
             __syncwarp();
-            if (C::SPLIT == 1) {
-                epi.columns(v, row, n0 + c, g, z, lane);
+            if constexpr (C::SPLIT == 1) {
+                typename Epi::template Pre<16> own;
+                epi.fetch(own, row, n0 + c, g, z);
+                epi.columns(v, own, row, n0 + c, g, z, lane);
                 __syncwarp();
             } else {
                 const u32 mine = inbox + (part * SLICE * 128 + r * 4) * 4;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int col = c + 4 * q;
-                    u32 at;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                                 : "=r"(at) : "r"(mine + (col % SLICE) * 512), "r"((u32)(col / SLICE)));
-                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
-                                 :: "r"(at), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
-                                 : "memory");
+                    mlcb_send4(mine + (col % SLICE) * 512, arrived, (u32)(col / SLICE),
+                               v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 }
             }
         }
     }
     __syncwarp();
-    if (C::SPLIT > 1) {
-        mlcb_cluster_arrive();
-        mlcb_cluster_wait();
-        if (warp < C::CW && !dead) {
+    if constexpr (C::SPLIT > 1) {
+        if (warp < C::CW && !dead && mlcb_bar_wait(arrived, 0, &dead)) {
 #pragma unroll
-            for (int c = half * 8; c < SLICE; c += C::CW * 2) {
+            for (int i = 0; i < EACH; ++i) {
+                const int c = half * 8 + i * C::CW * 2;
+                if (c >= SLICE) break;
                 float v[8];
 #pragma unroll
                 for (int p = 0; p < C::SPLIT; ++p)
@@ -265,9 +273,9 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
                                      : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
                                      : "r"(inbox + ((p * SLICE + c + 4 * q) * 128 + r * 4) * 4) : "memory");
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) v[4 * q + i] = p ? v[4 * q + i] + x[i] : x[i];
+                        for (int j = 0; j < 4; ++j) v[4 * q + j] = p ? v[4 * q + j] + x[j] : x[j];
                     }
-                epi.columns(v, row, n0 + part * SLICE + c, g, z, lane);
+                epi.columns(v, pre[i], row, n0 + part * SLICE + c, g, z, lane);
                 __syncwarp();
             }
         }

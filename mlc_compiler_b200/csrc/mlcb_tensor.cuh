@@ -105,6 +105,28 @@ __device__ __forceinline__ void mlcb_bulk_load(u32 dst, const void* src, u32 byt
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
+// Weights the next matmul will read, on their way to L2 while this kernel runs: a model
+// larger than L2 streams its weights from memory on every call, and a matmul that starts
+// on cold ones waits a memory latency longer for its first tile (1800 to 2500 cycles
+// after its inputs are ready, 1050 on weights in L2).
+struct mlcb_next { const unsigned char* at[4]; u32 bytes, count; };
+__device__ __forceinline__ void mlcb_prefetch_next(const mlcb_next& next) {
+    const u32 share = (next.bytes / 16 + gridDim.x - 1) / gridDim.x * 16;
+    const u32 lo = blockIdx.x * share, hi = min(lo + share, next.bytes / 16 * 16);
+    for (u32 b = 0; b < next.count; ++b)
+        for (u32 o = lo; o < hi; o += 8192)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(next.at[b] + o), "r"(min(8192u, hi - o)) : "memory");
+}
+
+// four floats to shared memory of a CTA of the cluster, counted by its barrier
+__device__ __forceinline__ void mlcb_send4(u32 dst, u32 bar, u32 rank, float a, float b, float c, float d) {
+    u32 at, there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(dst), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(bar), "r"(rank));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%2, %3, %4, %5}, [%1];"
+                 :: "r"(at), "r"(there), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 // A value per CTA of the cluster, combined in rank order by every thread.  `slot` is not
 // reused by another reduction of the kernel.
 template <typename OP, int C, typename T>

@@ -223,9 +223,36 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
     rn = {"float16": "mlcb_rn_f16", "bfloat16": "mlcb_rn_bf16", "float32": ""}[k.dtype]
     plain = not e0.body and len(e0.outputs) == 1 and e0.outputs[0].dtype == k.dtype
 
-    L.append("    template <int NV> __device__ __forceinline__ void columns(float (&v)[NV], int row, int col, "
+    # operands read in packs are fetched ahead of the accumulator, as packed words
+    packed = {}
+    for i, a in enumerate(e0.inputs):
+        if a is not None:
+            ac = classify(a.index, "col", W)
+            if ac.width == W and (ac.mode == "bcast" or W > 1):
+                packed[i] = ac.mode
+    L.append("    template <int NV> struct Pre {")
+    for i, mode in packed.items():
+        st = X.STORAGE_T[e0.inputs[i].dtype]
+        L.append(f"        mlcb_pack<{st}, {W if mode == 'contig' else 1}> w{i}[NV < {W} ? 1 : NV / {W}];")
+    L.append("    };")
+    L.append("    template <int NV> __device__ __forceinline__ void fetch(Pre<NV>& pre, int row, int col, int g, int z) const {")
+    if packed:
+        L += [s for s in selects if any(f" in{i} " in s for i in packed)]
+        L.append(f"        const {it} r = mlcb_within(row, {m}){f' + ({it})z * {m}' if z > 1 else ''};")
+        L.append("#pragma unroll")
+        L.append(f"        for (int c = 0; c < NV; c += {W}) {{")
+        L.append("            const int c0 = col + c;")
+        L.append(f"            if (c0 >= {n}) break;")
+        for i, mode in packed.items():
+            a = e0.inputs[i]
+            st = X.STORAGE_T[a.dtype]
+            off = render_offset(a.index, {"row": "r", "col": "c0"})
+            L.append(f"            mlcb_load_raw<{st}, {W if mode == 'contig' else 1}>(in{i} + ({off}), pre.w{i}[c / {W}]);  // {a.name}")
+        L.append("        }")
+    L.append("    }")
+    L.append("    template <int NV> __device__ __forceinline__ void columns(float (&v)[NV], const Pre<NV>& pre, int row, int col, "
              "int g, int z, int lane) const {")
-    L += selects
+    L += [s for s in selects if not any(f" in{i} " in s for i in packed)]
     if plain and W == 1 and e0.outputs[0].index.axis("col").terms == ((n, 1, 1),) and nv == 32 and z == 1:
         # rows that start at odd addresses: 32 x 32 elements turn in shared memory so that a
         # warp writes one row's 32 elements together
@@ -251,7 +278,7 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
         L.append(f"        const {it} r = {row_expr};")
         for what, ops in (("in", e0.inputs), ("out", e0.outputs)):
             for i, a in enumerate(ops):
-                if a is not None:
+                if a is not None and not (what == "in" and i in packed):
                     L.append(f"        const {it} {what}{i}_r = {render_offset(a.index, {'row': 'r'}, skip=('col',))};")
         L.append("#pragma unroll")
         L.append(f"        for (int c = 0; c < NV; c += {W}) {{")
@@ -273,11 +300,11 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
             ac = classify(a.index, "col", W)
             off = render_offset(a.index, {"col": "c0"}, skip=("row", "base"))
             vdt = X.promoted_load_dtype(a.dtype)
-            if ac.mode == "bcast" and ac.width == W:
-                L.append(f"            const {rt} x{i} = mlcb_load1<{st}>(in{i} + in{i}_r + ({off}));  // {a.name}")
+            if packed.get(i) == "bcast":
+                L.append(f"            {rt} x{i}_[1]; mlcb_unpack<{st}, 1>(pre.w{i}[c / {W}], x{i}_); const {rt} x{i} = x{i}_[0];  // {a.name}")
                 loads.append(X.Val(f"x{i}", vdt))
-            elif ac.mode == "contig" and ac.width == W and W > 1:
-                L.append(f"            {rt} x{i}[{W}]; mlcb_load<{st}, {W}>(in{i} + in{i}_r + ({off}), x{i});  // {a.name}")
+            elif i in packed:
+                L.append(f"            {rt} x{i}[{W}]; mlcb_unpack<{st}, {W}>(pre.w{i}[c / {W}], x{i});  // {a.name}")
                 loads.append(X.Val(f"mlcb_f2(x{i}[j], x{i}[j + 1])" if pairs else f"x{i}[j]", vdt))
             else:
                 off = render_offset(a.index, {"col": "(c0 + j)"}, skip=("row", "base"))
@@ -337,7 +364,7 @@ def emit_matmul(k: MatmulKernel, cfg, buffers, name: str | None = None, stable=f
         tmaps.append(operand_map(b, k.dtype, -1, -2, 64 * mc.kstep if b_mn else mc.bn // mc.cg, mc.kstep))
     targs = ["ta"] + [f"tb{i}" for i in range(len(k.bs))]
     threads = 64 + 32 * mc.epi_warps
-    sig = ", ".join([f"const __grid_constant__ mlcb_tmap {t}" for t in targs] + params)
+    sig = ", ".join([f"const __grid_constant__ mlcb_tmap {t}" for t in targs] + params + ["const __grid_constant__ mlcb_next next"])
     fields = ", ".join(p.split("* ")[1] for p in params)
     tb = [f"&tb{min(i, len(k.bs) - 1)}" for i in range(4)]
     cluster = mc.split * mc.cg
@@ -347,13 +374,13 @@ def emit_matmul(k: MatmulKernel, cfg, buffers, name: str | None = None, stable=f
         f"    // {z} x [{m}, {kk}] x [{kk}, {n}] x {len(k.bs)}; tile {128 * mc.cg} x {mc.bn}, {mc.stages} stages, "
         f"{mc.acc} accumulator(s), split {mc.split}, grid {mc.grid}, cluster {cluster}",
         f"    const {name}_epi epi{{{fields}}};",
-        f"    mlcb_matmul<{conf}>(&ta, {', '.join(tb)}, epi);",
+        f"    mlcb_matmul<{conf}>(&ta, {', '.join(tb)}, epi, next);",
         "}"])
     total = sum(v.numel for v in [k.a] + k.bs) * 2
     total += sum(algorithmic_bytes([x for x in e.inputs if x is not None], e.outputs, z * m * n)
                  for e in k.epilogues)
     spec = LaunchSpec(grid=mc.grid, block=threads, smem=mc.smem(), vector=1, alg_bytes=total, cluster=cluster,
-                      tmaps=tuple(tmaps), buffers=tuple(names))
+                      tmaps=tuple(tmaps), buffers=tuple(names), next=True)
     return text, spec
 
 
@@ -375,7 +402,8 @@ class Config32:
         return 8 if self.split > 1 else 16
 
     def smem(self) -> int:
-        return self.stages * 3 * (16384 + self.bn * 128) + 1024
+        inbox = 128 * self.bn * 4 if self.split > 1 else 0
+        return self.stages * 3 * (16384 + self.bn * 128) + inbox + 1024
 
 
 def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool) -> Config32:
@@ -395,7 +423,8 @@ def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool) -> Config3
     bn, split = min(((bn, s) for bn in widths for s in splits if bn % (8 * s) == 0),
                     key=lambda c: cost(*c, groups))
     t = _ceil(m, 128) * _ceil(n, bn) * groups * z
-    return Config32(bn, max(2, min(3, _ceil(kb, split))), split, t * split,
+    most = 2 if split > 1 and bn == 64 else 3           # the partial sums' place
+    return Config32(bn, max(2, min(most, _ceil(kb, split))), split, t * split,
                     min(5, _ceil(_ceil(kb, split), 4)))
 
 
@@ -428,14 +457,14 @@ def emit_matmul32(k: MatmulKernel, cfg, buffers, name: str, stable):
     fields = ", ".join(p.split("* ")[1] for p in params)
     text = "\n".join([
         functor.replace("MLCB_KERNEL_NAME", name),
-        f'extern "C" __global__ void __launch_bounds__(544, 1) {name}({", ".join(ops + params)}) {{',
+        f'extern "C" __global__ void __launch_bounds__(544, 1) {name}({", ".join(ops + params + ["const __grid_constant__ mlcb_next next"])}) {{',
         f"    // {z} x [{m}, {kk}] x [{kk}, {n}] x {len(k.bs)}, fp32 in three bf16 pieces; tile 128 x {mc.bn}, "
         f"{mc.stages} stages, split {mc.split}, grid {mc.grid}",
         f"    const {name}_epi epi{{{fields}}};",
-        f"    mlcb_matmul32<{conf}>(a + {k.a.offset}, {', '.join(bs)}, epi);",
+        f"    mlcb_matmul32<{conf}>(a + {k.a.offset}, {', '.join(bs)}, epi, next);",
         "}"])
     total = sum(v.numel for v in [k.a] + k.bs) * 4
     total += sum(algorithmic_bytes([x for x in e.inputs if x is not None], e.outputs, z * m * n)
                  for e in k.epilogues)
     return text, LaunchSpec(grid=mc.grid, block=544, smem=mc.smem(), alg_bytes=total, cluster=mc.split,
-                            buffers=tuple([k.a.buffer] + [b.buffer for b in k.bs] + names))
+                            buffers=tuple([k.a.buffer] + [b.buffer for b in k.bs] + names), next=True)

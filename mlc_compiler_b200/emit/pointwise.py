@@ -37,6 +37,8 @@ class LaunchSpec:
     cluster: int = 1
     tmaps: tuple = ()
     buffers: tuple | None = None
+    #: the last parameter is a ``mlcb_next``: weights to bring to L2 for the next matmul
+    next: bool = False
 
     def as_dict(self) -> dict:
         return {"grid": (self.grid,), "block": self.block, "smem": self.smem,

@@ -240,7 +240,7 @@ class _Executable:
                 else:
                     flags = 1 if policy is True else 0
                 tail_generated[lane] = True
-                fn = self._module.bind(k, buffers, flags)[0]
+                fn = self._module.bind(k, buffers, flags, self._weights_after(j, buffers))[0]
                 self._bound[k.name] = ("cuda", fn)
                 self._per_kernel.append(("cuda", fn))
                 if isinstance(fn, TensorLaunch):
@@ -250,6 +250,16 @@ class _Executable:
                     run.append(fn)
         flush()
         return plan
+
+    def _weights_after(self, j: int, buffers) -> list[torch.Tensor]:
+        """Weights of the first matmul behind kernel ``j`` (of the first one behind the
+        last: the next call begins with it)."""
+        ks = self._exec.kernels
+        if not isinstance(ks[j], fuse.MatmulKernel):
+            return []
+        after = next((k for k in ks[j + 1:] + ks[:j] if isinstance(k, fuse.MatmulKernel)
+                      and all(b.buffer in self.params for b in k.bs)), None)
+        return [] if after is None else [buffers[b.buffer] for b in after.bs]
 
     def run_kernels(self, buffers: dict[str, torch.Tensor] | None = None) -> None:
         if self._plan is None:

@@ -282,14 +282,29 @@ class BoundLaunch:
                            ctypes.cast(self.ptrs, ctypes.POINTER(ctypes.c_uint64)), self.nptrs, 0)
 
 
+class _Next(ctypes.Structure):
+    """``mlcb_next`` (``csrc/mlcb_tensor.cuh``): dense tensors of one size to prefetch."""
+
+    _fields_ = [("at", ctypes.c_uint64 * 4), ("bytes", ctypes.c_uint32), ("count", ctypes.c_uint32)]
+
+    @classmethod
+    def of(cls, tensors):
+        tensors = [t for t in tensors if t.data_ptr() % 16 == 0 and t.numel() * t.element_size() < 1 << 32]
+        size = min((t.numel() * t.element_size() for t in tensors), default=0)
+        if size * len(tensors) > 16 << 20:      # too much of L2 for one kernel's time (a vocabulary)
+            tensors = []
+        return cls((ctypes.c_uint64 * 4)(*[t.data_ptr() for t in tensors[:4]]), size, len(tensors[:4]))
+
+
 class TensorLaunch(BoundLaunch):
     """A launch whose parameters are tensor maps (encoded once, at bind time) followed
     by buffer pointers, on clusters of CTAs."""
 
-    __slots__ = ("cluster", "maps", "params", "mapped")
+    __slots__ = ("cluster", "maps", "params", "mapped", "ahead")
 
-    def __init__(self, lib, kernel, name, spec, flags, tensors, buffers, device=None):
+    def __init__(self, lib, kernel, name, spec, flags, tensors, buffers, device=None, ahead=()):
         super().__init__(lib, kernel, name, spec.grid, spec.block, spec.smem, flags, tensors, device)
+        self.ahead = _Next.of(ahead)
         self.cluster = spec.cluster
         self.mapped = tuple(buffers[m.buffer] for m in spec.tmaps)       # keeps the storage alive
         raw = ctypes.create_string_buffer(128 * len(spec.tmaps) + 128)
@@ -301,8 +316,9 @@ class TensorLaunch(BoundLaunch):
                 (ctypes.c_uint64 * 4)(*m.dims), (ctypes.c_uint64 * 3)(*m.strides),
                 (ctypes.c_uint32 * 3)(*m.box)), f"tensor map of {m.buffer} for {name}")
         at = ctypes.addressof(self.ptrs)
-        self.params = (ctypes.c_void_p * (len(spec.tmaps) + self.nptrs))(
-            *[base + 128 * i for i in range(len(spec.tmaps))], *[at + 8 * i for i in range(self.nptrs)])
+        self.params = (ctypes.c_void_p * (len(spec.tmaps) + self.nptrs + int(spec.next)))(
+            *[base + 128 * i for i in range(len(spec.tmaps))], *[at + 8 * i for i in range(self.nptrs)],
+            *([ctypes.addressof(self.ahead)] if spec.next else []))
 
     def __call__(self, *tensors, **consts) -> None:
         stream = torch.cuda.current_stream(self.device).cuda_stream
@@ -370,14 +386,17 @@ class CudaRuntime:
             names.append(a.buffer if isinstance(a, kir.Operand) else a.value.buffer.name)
         return names
 
-    def bind(self, k, buffers: dict[str, torch.Tensor], flags: int | None = None):
+    def bind(self, k, buffers: dict[str, torch.Tensor], flags: int | None = None, ahead=()):
+        """``ahead``: weights of the matmul after this kernel, for the kernels that can
+        bring them to L2 while they run."""
         if self._is_extern(k):
             raise TypeError("extern kernels do not go through the CUDA runtime")
         spec = self.generated.launch[k.name]
-        if spec.tmaps:
+        if spec.tmaps or spec.next:
             tensors = tuple(buffers[n] for n in spec.buffers)
             fn = TensorLaunch(self.lib, self.loaded.kernel(self.generated.symbol[k.name]), k.name, spec,
-                              self.flags if flags is None else flags, tensors, buffers, self.device)
+                              self.flags if flags is None else flags, tensors, buffers, self.device,
+                              ahead)
             return fn, spec.grid, tensors, {}
         tensors = tuple(buffers[n] for n in spec.buffers or self._buffer_names(k))
         if flags is None:
