@@ -9,53 +9,6 @@
 // rank order (deterministic), each finishing BN / SPLIT columns.
 #pragma once
 
-// ---------------------------------------------------------------------------
-// Two neighbouring columns per register pair: add, mul and fma of both in one
-// instruction (.f32x2), each half rounded as the scalar form rounds it.  An exact-GELU
-// epilogue is instruction-bound at 28 per element in scalar form.
-// ---------------------------------------------------------------------------
-struct mlcb_f2 {
-    u64 v;
-    __device__ __forceinline__ mlcb_f2() {}
-    __device__ __forceinline__ mlcb_f2(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
-    __device__ __forceinline__ mlcb_f2(float both) : mlcb_f2(both, both) {}
-    __device__ __forceinline__ void get(float& lo, float& hi) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-};
-__device__ __forceinline__ mlcb_f2 operator+(mlcb_f2 a, mlcb_f2 b) { mlcb_f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ mlcb_f2 operator*(mlcb_f2 a, mlcb_f2 b) { mlcb_f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ mlcb_f2 operator-(mlcb_f2 a, mlcb_f2 b) { mlcb_f2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ mlcb_f2 mlcb_fma2(mlcb_f2 a, mlcb_f2 b, mlcb_f2 c) { mlcb_f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
-__device__ __forceinline__ mlcb_f2 mlcb_rn_f16(mlcb_f2 a) {
-    float x, y; a.get(x, y);
-    const float2 f = __half22float2(__floats2half2_rn(x, y));
-    return mlcb_f2(f.x, f.y);
-}
-__device__ __forceinline__ mlcb_f2 mlcb_rn_bf16(mlcb_f2 a) {
-    float x, y; a.get(x, y);
-    const float2 f = __bfloat1622float2(__floats2bfloat162_rn(x, y));
-    return mlcb_f2(f.x, f.y);
-}
-__device__ __forceinline__ mlcb_f2 mlcb_ex2(mlcb_f2 a) { float x, y; a.get(x, y); return mlcb_f2(mlcb_ex2(x), mlcb_ex2(y)); }
-__device__ __forceinline__ mlcb_f2 mlcb_rcp_fast(mlcb_f2 a) { float x, y; a.get(x, y); return mlcb_f2(mlcb_rcp_fast(x), mlcb_rcp_fast(y)); }
-// the scalar forms' operations in their order; a negated factor is a negated constant here
-__device__ __forceinline__ mlcb_f2 mlcb_exp_fast(mlcb_f2 x) { return mlcb_ex2(x * 1.4426950408889634f); }
-__device__ __forceinline__ mlcb_f2 mlcb_sigmoid_fast(mlcb_f2 x) { return mlcb_rcp_fast(mlcb_f2(1.0f) + mlcb_ex2(x * -1.4426950408889634f)); }
-__device__ __forceinline__ mlcb_f2 mlcb_tanh_fast(mlcb_f2 x) {
-    return mlcb_fma2(-2.0f, mlcb_rcp_fast(mlcb_f2(1.0f) + mlcb_ex2(x * 2.8853900817779268f)), 1.0f);
-}
-__device__ __forceinline__ mlcb_f2 mlcb_erf_fast(mlcb_f2 x) {
-    float lo, hi; x.get(lo, hi);
-    const mlcb_f2 ax(fabsf(lo), fabsf(hi));
-    const mlcb_f2 t = mlcb_rcp_fast(mlcb_fma2(0.3275911f, ax, 1.0f));
-    mlcb_f2 p = mlcb_fma2(-1.061405429f, t, 1.453152027f);
-    p = mlcb_fma2(p, t, -1.421413741f);
-    p = mlcb_fma2(p, t, 0.284496736f);
-    p = mlcb_fma2(p, t, -0.254829592f);
-    float r0, r1;
-    mlcb_fma2(p * t, mlcb_ex2(ax * ax * -1.4426950408889634f), 1.0f).get(r0, r1);
-    return mlcb_f2(copysignf(r0, lo), copysignf(r1, hi));
-}
-
 template <int M_, int N_, int KBLOCKS_, int KSTEP_, bool A_CUT_, bool B_CUT_, int BN_, int STAGES_, int ACC_, int SPLIT_, int CG_, int GROUPS_,
           int BATCH_, int EPI_WARPS_, bool B_MN_, bool BF16_, bool B_STABLE_>
 struct mlcb_mm_cfg {

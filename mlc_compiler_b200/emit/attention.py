@@ -2,7 +2,7 @@
 
 The functor is the schedule's own row kernel (scale, mask, softmax, casts) for the rows
 of one tile, the score entering as the value the separate matmul would have stored.
-Several threads share a row; up to 64 columns each, its values stay in registers, beyond
+Several threads share a row; up to 96 columns each, its values stay in registers, beyond
 that every phase reads the scores from TMEM again.
 """
 
@@ -34,6 +34,31 @@ def split_row(k: AttentionKernel, cfg) -> tuple[int, int, int]:
     return H, 8, 8
 
 
+def _paired(k: AttentionKernel, V: int) -> bool:
+    """Whether the row kernel runs on pairs of neighbouring columns (``mlcb_f2``): 18
+    instructions per score in scalar form, which is what bounded the kernel."""
+    rows = k.rows
+    vec = varying_steps(rows)
+    cols = {i for i, a in enumerate(rows.inputs) if a.index.varies_along("col")}
+
+    def varies(e):
+        return bool(kir.expr_loads(e) & cols or kir.expr_refs(e) & vec)
+
+    exprs = [s.expr for s in rows.steps if varies(s.expr)] + [rows.out_expr[rows.outputs[0].name]]
+    for e in exprs:
+        for s in kir.walk(e):
+            if isinstance(s, kir.Call) and varies(s):
+                power = isinstance(s.args[-1], kir.Const) and X._is_pow2(s.args[-1].value)
+                if s.fn == "div" and varies(s.args[0]) and (power or not varies(s.args[1])):
+                    continue
+                if s.fn not in ("add", "sub", "mul", "exp", "tanh", "erf", "sigmoid"):
+                    return False
+            if isinstance(s, kir.Cast) and varies(s) and s.dtype not in kir.NARROW_FLOATS + ("float32",):
+                return False
+    return (X._FAST and V % 2 == 0 and all(r.kind in ("sum", "max", "min") for r in rows.reduces)
+            and all(rows.inputs[i].dtype in kir.NARROW_FLOATS + ("float32",) for i in cols))
+
+
 def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[str, list, list]:
     rows, slot = k.rows, k.slot
     S, T = rows.n_cols, k.q.shape[1]
@@ -44,7 +69,11 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
     width = V * lanes                          # neighbouring columns per thread and period
     NC = _ceil(S, period) * width              # columns per thread
     whole = S // period * width                # of them inside the row whatever the thread
-    keep = NC <= 64                            # row values stay in registers between phases
+    keep = NC <= 96                            # row values stay in registers between phases
+    chunk = 32 if width % 32 == 0 else 16      # columns fetched and converted at a time
+    pairs = _paired(k, V)                      # two columns per instruction
+    vt = "mlcb_f2" if pairs else None
+    at_j = "[({} + j) / 2]" if pairs else "[{} + j]"
     extents = [rows.n_rows * S] + [a.index.bounds()[1] + 1 for a in rows.inputs]
     it = "i64" if needs_64bit(*extents) else "int"
     vec = varying_steps(rows)
@@ -68,7 +97,7 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
     for i, a in enumerate(rows.inputs):
         vdt, ct = X.promoted_load_dtype(a.dtype), X.STORAGE_T[a.dtype]
         if i == slot:
-            loads.append(X.Val("s[j]", "float32", True, True))
+            loads.append(X.Val("mlcb_f2(s[j], s[j + 1])" if pairs else "s[j]", "float32", True, True))
         elif not a.index.varies_along("col"):
             emit(f"        const {X.REG_T[a.dtype]} s{i} = mlcb_load1<{ct}>(in{i} + "
                  f"({render_offset(a.index, {'row': 'row'}, skip=('col',))}));  // {a.name} (per row)")
@@ -77,44 +106,41 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
             emit(f"        const {it} in{i}_r = {render_offset(a.index, {'row': 'row'}, skip=('col',))};")
             ac = classify(a.index, "col", 8)
             packed[i] = ac.mode == "contig" and ac.width == 8
-            loads.append(X.Val(f"x{i}[j]", vdt, True, True))
+            loads.append(X.Val(f"mlcb_f2(x{i}[j], x{i}[j + 1])" if pairs else f"x{i}[j]", vdt, True, True))
 
-    def fetch(i, lo, n, ind):
-        """Columns ``[lo, lo + n)`` of this thread of operand i, into ``x{i}``."""
-        a, B = rows.inputs[i], []
+    def fetch(i, lo):
+        """Columns ``[lo, lo + chunk)`` of this thread of operand i, as packed words
+        ``w{i}_{pass}_{lo}`` (or values, where they are not read in packs)."""
+        a = rows.inputs[i]
         ct = X.STORAGE_T[a.dtype]
         step = 8 if packed[i] else 1
-        B.append("#pragma unroll")
-        B.append(f"{ind}for (int j = 0; j < {n}; j += {step}) {{")
+        emit(f"        mlcb_pack<{ct}, {step}> w{i}_{turn[0]}_{lo}[{chunk // step}];  // {a.name}")
+        emit("#pragma unroll")
+        emit(f"        for (int j = 0; j < {chunk}; j += {step}) {{")
         col = f"MLCB_COL({lo} + j)"
         off = render_offset(a.index, {"col": col}, skip=("row", "base"))
-        guard = f"if ({lo} + j < {whole} || {col} < {S}) " if lo + n > whole else ""
-        if packed[i]:
-            B.append(f"{ind}    {guard}mlcb_load_at<{ct}, 8, {n}>(in{i} + in{i}_r + ({off}), x{i}, j);")
+        guard = f"if ({lo} + j < {whole} || {col} < {S}) " if lo + chunk > whole else ""
+        emit(f"            {guard}mlcb_load_raw<{ct}, {step}>(in{i} + in{i}_r + ({off}), w{i}_{turn[0]}_{lo}[j / {step}]);")
+        emit("        }")
+
+    def unpack(i, lo):
+        a = rows.inputs[i]
+        ct, step = X.STORAGE_T[a.dtype], 8 if packed[i] else 1
+        emit(f"        {X.REG_T[a.dtype]} x{i}[{chunk}];")
+        emit("#pragma unroll")
+        emit(f"        for (int j = 0; j < {chunk}; j += {step}) {{ {X.REG_T[a.dtype]} y[{step}]; "
+             f"mlcb_unpack<{ct}, {step}>(w{i}_{turn[0]}_{lo}[j / {step}], y);")
+        emit("#pragma unroll")
+        emit(f"            for (int i = 0; i < {step}; ++i) x{i}[j + i] = y[i]; }}")
+
+    def scores(lo):
+        emit(f"        float s[{chunk}];")
+        emit(f"        mlcb_tmem_ld(tm + MLCB_COL({lo}), s);")
+        emit("#pragma unroll")
+        if pairs:
+            emit(f"        for (int i = 0; i < {chunk}; i += 2) {rn}(mlcb_f2(s[i], s[i + 1])).get(s[i], s[i + 1]);")
         else:
-            B.append(f"{ind}    {guard}x{i}[j] = mlcb_load1<{ct}>(in{i} + in{i}_r + ({off}));")
-        B.append(f"{ind}}}")
-        return B
-
-    def scores(lo, n, ind):
-        B = []
-        for c in range(0, n, 16):
-            B.append(f"{ind}{{ float raw[16]; mlcb_tmem_ld(tm + MLCB_COL({lo + c}), raw);")
-            B.append("#pragma unroll")
-            B.append(f"{ind}  for (int i = 0; i < 16; ++i) s[{c} + i] = {rn}(raw[i]); }}")
-        return B
-
-    if keep:
-        for i in packed:
-            emit(f"        {X.REG_T[rows.inputs[i].dtype]} x{i}[{NC}];  // {rows.inputs[i].name}")
-            L += fetch(i, 0, NC, "        ")
-        emit("        mlcb_bar_wait(ready, 0, dead);")
-        emit("        mlcb_tc_after();")
-        emit(f"        float s[{NC}];")
-        L += scores(0, NC, "        ")
-    else:
-        emit("        mlcb_bar_wait(ready, 0, dead);")
-        emit("        mlcb_tc_after();")
+            emit(f"        for (int i = 0; i < {chunk}; ++i) s[i] = {rn}(s[i]);")
 
     def needed(expr, upto):
         """Vector binds ``expr`` reads, transitively, in order."""
@@ -126,41 +152,51 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
 
     done: dict[str, X.Val] = {}                # vector values already in registers (keep)
 
+    started = [False]
+    turn = [0]                                 # pass being emitted, for names
+
     def phase(expr, upto, close, elide=frozenset()):
-        """One pass over this thread's columns; ``close(lines, value)`` ends an element."""
+        """One pass over this thread's columns; ``close(lo, body, value)`` emits the loop
+        over a chunk of them."""
         binds = [b for b in needed(expr, upto) if b.name not in done]
-        step = NC if keep else 16
-        refs = dict(scalars)
-        refs.update(done)
-        body, decl = [], []
-        for b in binds:
-            v = X.render_bind(b.name, b.expr, loads, refs, elide)
-            if keep:
-                decl.append(f"        {X.REG_T[v.dtype]} {b.name}[{NC}];")
-                body.append(f"{b.name}[j] = {v.code};")
-                refs[b.name] = done[b.name] = X.Val(f"{b.name}[j]", v.dtype, v.dim, True)
-            else:
-                body.append(f"const {X.REG_T[v.dtype]} {b.name} = {v.code};")
-                refs[b.name] = X.Val(b.name, v.dtype, v.dim, True)
-        value = X.render(expr, loads, refs)
-        slots = set(kir.expr_loads(expr)).union(*[kir.expr_loads(b.expr) for b in binds]) if binds else \
-            set(kir.expr_loads(expr))
-        for d in decl:
-            emit(d)
-        ind = "        "
-        for lo in range(0, NC, step):
-            if not keep:
-                emit("        {")
-                emit(f"        if (MLCB_COL({lo}) < {S}) {{" if lo + step > whole else "        {")
-                for i in packed:
-                    if i in slots:
-                        emit(f"        {X.REG_T[rows.inputs[i].dtype]} x{i}[16];")
-                        L.extend(fetch(i, lo, 16, ind))
-                emit("        float s[16];")
-                L.extend(scores(lo, 16, ind))
-            close(lo, step, body, value)
-            if not keep:
-                emit("        }}")
+        slots = set(kir.expr_loads(expr)).union(*[kir.expr_loads(b.expr) for b in binds])
+        if keep:
+            for b in binds:
+                refs = dict(scalars)
+                refs.update(done)
+                v = X.render_bind(b.name, b.expr, loads, refs, elide)
+                emit(f"        {vt or X.REG_T[v.dtype]} {b.name}[{NC // 2 if pairs else NC}];")
+                done[b.name] = X.Val("?", v.dtype, v.dim, True)
+        used = [i for i in packed if i in slots]
+        turn[0] += 1
+        for i in used:
+            fetch(i, 0)                        # the next chunk's operands travel with this one's work
+        if not started[0]:
+            emit("        mlcb_bar_wait(ready, 0, dead);")
+            emit("        mlcb_tc_after();")
+            started[0] = True
+        for lo in range(0, NC, chunk):
+            if lo + chunk < NC:
+                for i in used:
+                    fetch(i, lo + chunk)
+            emit(f"        if (MLCB_COL({lo}) < {S}) {{" if lo + chunk > whole else "        {")
+            for i in used:
+                unpack(i, lo)
+            if slot in slots:
+                scores(lo)
+            refs = dict(scalars)
+            for n, v in done.items():
+                refs[n] = X.Val(n + at_j.format(lo), v.dtype, v.dim, True)
+            body = []
+            for b in binds:
+                v = X.render_bind(b.name, b.expr, loads, refs, elide)
+                if keep:
+                    body.append(f"{b.name}{at_j.format(lo)} = {v.code};")
+                else:
+                    body.append(f"const {vt or X.REG_T[v.dtype]} {b.name} = {v.code};")
+                    refs[b.name] = X.Val(b.name, v.dtype, v.dim, True)
+            close(lo, body, X.render(expr, loads, refs))
+            emit("        }")
 
     nred = 0
     for pos, sp in enumerate(rows.steps):
@@ -186,14 +222,32 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
         emit("#pragma unroll")
         emit(f"        for (int i = 0; i < {n}; ++i) a_{sp.name}[i] = {_identity(sp.kind, adt)};")
 
-        def close(lo, step, body, value, sp=sp, at=at, adt=adt, op=op, ordered=ordered):
-            acc = f"a_{sp.name}[{f'({lo} + j) % {width} / {V}' if ordered else 'j % 4'}]"
+        def close(lo, body, value, sp=sp, at=at, adt=adt, op=op, ordered=ordered):
+            def acc(j):
+                return f"a_{sp.name}[{f'({lo} + {j}) % {width} / {V}' if ordered else f'{j} / 2 % 4'}]"
+
+            def guard(j):
+                return f"({lo} + {j} < {whole} || MLCB_COL({lo} + {j}) < {S})" if lo + chunk > whole else ""
+
             emit("#pragma unroll")
-            emit(f"        for (int j = 0; j < {step}; ++j) {{")
+            emit(f"        for (int j = 0; j < {chunk}; j += {2 if pairs else 1}) {{")
             for ln in body:
                 emit("            " + ln)
-            guard = f"if ({lo} + j < {whole} || MLCB_COL({lo} + j) < {S}) " if lo + step > whole else ""
-            emit(f"            {guard}{acc} = {op}::f({acc}, ({at}){X.convert(value.code, value.dtype, adt)});")
+            if not pairs:
+                g = f"if {guard('j')} " if guard("j") else ""
+                emit(f"            {g}{acc('j')} = {op}::f({acc('j')}, ({at}){X.convert(value.code, value.dtype, adt)});")
+            else:
+                emit(f"            float lo, hi; mlcb_f2({value.code}).get(lo, hi);")
+                if sp.kind in ("max", "min"):
+                    if lo + chunk > whole:
+                        other = "MLCB_NINF_F" if sp.kind == "max" else "MLCB_INF_F"
+                        for v, j in (("lo", "j"), ("hi", "(j + 1)")):
+                            emit(f"            {v} = {guard(j)} ? {v} : {other};")
+                    emit(f"            {acc('j')} = mlcb_{sp.kind}3({acc('j')}, lo, hi);")
+                else:
+                    for v, j in (("lo", "j"), ("hi", "(j + 1)")):
+                        g = f"if {guard(j)} " if guard(j) else ""
+                        emit(f"            {g}{acc(j)} = {op}::f({acc(j)}, {v});")
             emit("        }")
         phase(sp.expr, pos, close)
         # the row's lanes (or its H parts) meet in shared memory, every thread combines them alike
@@ -224,21 +278,26 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
     elide = X.store_only_casts([(b.name, b.expr) for b in needed(oe, upto) if b.name not in done],
                                {out.name: oe}, [out])
 
-    def close_store(lo, step, body, value):
+    def close_store(lo, body, value):
+        edge = lo + chunk > whole
         emit("#pragma unroll")
-        emit(f"        for (int q = 0; q < {step}; q += 8) {{")
-        if lo + step > whole:
+        emit(f"        for (int q = 0; q < {chunk}; q += 8) {{")
+        if edge:
             emit(f"            if ({lo} + q >= {whole} && MLCB_COL({lo} + q) >= {_ceil(S, 16) * 16}) continue;")
         emit("            float o[8];")
         emit("#pragma unroll")
-        emit("            for (int i = 0; i < 8; ++i) {")
+        emit(f"            for (int i = 0; i < 8; i += {2 if pairs else 1}) {{")
         emit("                const int j = q + i;")
         for ln in body:
             emit("                " + ln)
         code = store_code(value, out.dtype)
-        if lo + step > whole:
-            code = f"({lo} + j < {whole} || MLCB_COL({lo} + j) < {S}) ? {code} : 0.0f"
-        emit(f"                o[i] = {code};  // {out.name}")
+        if pairs:
+            emit(f"                mlcb_f2({code}).get(o[i], o[i + 1]);  // {out.name}")
+        else:
+            emit(f"                o[i] = {code};  // {out.name}")
+        for i in ((0, 1) if pairs else (0,)):
+            if edge:
+                emit(f"                if ({lo} + j + {i} >= {whole} && MLCB_COL({lo} + j + {i}) >= {S}) o[i + {i}] = 0.0f;")
         emit("            }")
         emit(f"            mlcb_store_p<{st}>(sp, r, MLCB_COL({lo} + q), o);")
         emit("        }")

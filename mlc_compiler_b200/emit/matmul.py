@@ -110,32 +110,39 @@ def _estimate(z, m, n, k, groups, b_mn, can_step, splits):
             t = _ceil(m, 128 * cg) * _ceil(n, bn) * groups * z
             kstep = 2 if bn <= 96 and kb > 1 and can_step else 1
             for split in splits:
-                if split > 1 and (cg == 2 or bn > 128 or bn % (8 * split) or _ceil(kb, kstep) < split):
+                if split > 1 and (cg == 2 or bn > 128 or bn % (8 * split) or _ceil(kb, kstep) < split
+                                  or (t > _RESIDENT[split] and len(splits) > 1)):
                     continue
                 waves = _ceil(t, _RESIDENT[split * cg])
                 exchange = 0.3 * (split.bit_length() - 1) + 0.012 * bn if split > 1 else 0.0
                 step = 0.10 + 0.00075 * bn if cg == 1 else 0.095 + 0.00065 * bn
-                cost = waves * _ceil(kb, split) * step + 2.1 + 0.4 * (cg - 1) + 0.005 * bn + exchange
+                # a launch that leaves a third of the machine free lets the next one move in: q, k
+                # and v of [231, 768] in 72 CTAs take 1.2 us less inside a model than in 144
+                full = 0.5 if waves == 1 and t * cg > 100 and bn <= 64 else 0.0
+                cost = full + waves * _ceil(kb, split) * step + 2.1 + 0.4 * (cg - 1) + 0.005 * bn + exchange
                 if best is None or cost < best[0]:
                     best = (cost, bn, split, cg, t, kstep)
     return best
 
 
-def split_for(m: int, n: int, k: int, b_mn: bool = False, can_step: bool = True) -> int:
-    """CTAs that share the K of one result tile.  It decides the order in which products
-    are summed, so it depends on the matmul's own shape alone, never on what it shares a
-    launch with.  Up to K = 1024 two halves pay only while the result is small ([128, 768] x
-    [768, 768]: 3.6 us against 3.7, and 4.0 in four parts; N = 2304: 4.3 against 4.2;
-    M = 512: 5.0 against 4.1)."""
+def split_for(m: int, n: int, k: int, groups: int = 1, b_mn: bool = False, can_step: bool = True) -> int:
+    """CTAs that share the K of one result tile.  Up to K = 1024 splitting pays while the
+    parts of all tiles stay under two thirds of the machine, which leaves the next launch
+    room to move in: inside BERT-base b1, [128, 768] x [768, 768] in four parts (96 CTAs)
+    takes 0.4 us less than in two; the three of a layer's q, k, v in one launch take 1.7
+    less whole (72) than in two parts (144)."""
     kb = _ceil(k, 64)
     if kb <= 16:
-        return 2 if _ceil(m, 128) * n <= 1536 and kb >= 8 and can_step and not b_mn else 1
-    return _estimate(1, m, n, k, 1, b_mn, can_step, (1, 2, 4, 8))[2]
+        tiles = _ceil(m, 128) * _ceil(n, 32) * groups
+        if b_mn or not can_step or kb < 8:
+            return 1
+        return next((s for s in (4, 2) if tiles * s <= 96), 1)
+    return _estimate(1, m, n, k, groups, b_mn, can_step, (1, 2, 4, 8))[2]
 
 
 def choose(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, can_step: bool = True) -> Config:
     """Tile, split and pairing for a shape."""
-    split = split_for(m, n, k, b_mn, can_step) if z == 1 else 1
+    split = split_for(m, n, k, groups, b_mn, can_step) if z == 1 else 1
     found = _estimate(z, m, n, k, groups, b_mn, can_step, (split,))
     _, bn, split, cg, t, kstep = found
     persistent = split == 1 and t > SM_COUNT // cg
