@@ -113,6 +113,15 @@ int mlcb_tensor_map(void* map, uint64_t address, int bf16, const uint64_t* dims,
 int mlcb_launch_ex(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t cluster_x,
                    uint32_t smem_bytes, void* const* params, uint64_t stream, uint32_t flags);
 
+/* The node the last launch on a capturing stream became (0: not capturing, or several
+ * streams joined there). */
+int mlcb_capture_node(uint64_t stream, uint64_t* node);
+
+/* New parameter values for one kernel node of an instantiated graph; launches already
+ * enqueued keep the old ones. */
+int mlcb_graph_params(uint64_t exec, uint64_t node, mlcb_kernel* k, uint32_t grid_x, uint32_t block_x,
+                      uint32_t smem_bytes, void* const* params);
+
 /* Non-zero when a bounded wait inside one of the module's kernels ran out (their
  * results are then unusable).  Synchronises with the device. */
 int mlcb_module_fault(mlcb_module* m, uint32_t* code);

@@ -57,6 +57,9 @@ struct Driver {
     CUresult (*LaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
     CUresult (*FuncSetAttribute)(CUfunction, CUfunction_attribute, int) = nullptr;
     CUresult (*ModuleGetGlobal)(CUdeviceptr*, size_t*, CUmodule, const char*) = nullptr;
+    CUresult (*StreamGetCaptureInfo)(CUstream, CUstreamCaptureStatus*, cuuint64_t*, CUgraph*, const CUgraphNode**,
+                                     const CUgraphEdgeData**, size_t*) = nullptr;
+    CUresult (*GraphExecKernelNodeSetParams)(CUgraphExec, CUgraphNode, const CUDA_KERNEL_NODE_PARAMS*) = nullptr;
     CUresult (*MemcpyDtoH)(void*, CUdeviceptr, size_t) = nullptr;
     CUresult (*TensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                      const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -98,6 +101,8 @@ void load_driver() {
     ok &= sym(d.lib, MLCB_STR(cuFuncSetAttribute), d.FuncSetAttribute);
     ok &= sym(d.lib, MLCB_STR(cuModuleGetGlobal), d.ModuleGetGlobal);
     ok &= sym(d.lib, MLCB_STR(cuMemcpyDtoH), d.MemcpyDtoH);
+    ok &= sym(d.lib, MLCB_STR(cuStreamGetCaptureInfo_v3), d.StreamGetCaptureInfo);
+    ok &= sym(d.lib, MLCB_STR(cuGraphExecKernelNodeSetParams), d.GraphExecKernelNodeSetParams);
     ok &= sym(d.lib, MLCB_STR(cuTensorMapEncodeTiled), d.TensorMapEncodeTiled);
     if (ok && d.Init(0) == CUDA_SUCCESS) d.ok = true;
 }
@@ -519,6 +524,41 @@ int mlcb_launch_ex(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t c
         snprintf(what, sizeof what, "launch of %s <<<%u, %u>>>", k->name.c_str(), grid_x, block_x);
         return cu_fail(r, what);
     }
+    return 0;
+}
+
+int mlcb_capture_node(uint64_t stream, uint64_t* node) {
+    if (!node) return fail(MLCB_ERR_ARGUMENT, "mlcb_capture_node: null argument");
+    *node = 0;
+    if (int e = need_driver()) return e;
+    CUstreamCaptureStatus status;
+    cuuint64_t id = 0;
+    CUgraph graph = nullptr;
+    const CUgraphNode* last = nullptr;
+    const CUgraphEdgeData* edges = nullptr;
+    size_t n = 0;
+    CUresult r = g_drv.StreamGetCaptureInfo((CUstream)(uintptr_t)stream, &status, &id, &graph, &last, &edges, &n);
+    if (r != CUDA_SUCCESS) return cu_fail(r, "cuStreamGetCaptureInfo");
+    if (status == CU_STREAM_CAPTURE_STATUS_ACTIVE && n == 1) *node = (uint64_t)(uintptr_t)last[0];
+    return 0;
+}
+
+int mlcb_graph_params(uint64_t exec, uint64_t node, mlcb_kernel* k, uint32_t grid_x, uint32_t block_x,
+                      uint32_t smem_bytes, void* const* params) {
+    if (!exec || !node || !k || !params) return fail(MLCB_ERR_ARGUMENT, "mlcb_graph_params: null argument");
+    if (int e = need_driver()) return e;
+    CUDA_KERNEL_NODE_PARAMS p;
+    memset(&p, 0, sizeof p);
+    p.func = k->fn;
+    p.gridDimX = grid_x;
+    p.gridDimY = p.gridDimZ = 1;
+    p.blockDimX = block_x;
+    p.blockDimY = p.blockDimZ = 1;
+    p.sharedMemBytes = smem_bytes;
+    p.kernelParams = (void**)params;
+    CtxGuard in_module_context(k->owner->ctx);
+    CUresult r = g_drv.GraphExecKernelNodeSetParams((CUgraphExec)(uintptr_t)exec, (CUgraphNode)(uintptr_t)node, &p);
+    if (r != CUDA_SUCCESS) return cu_fail(r, "cuGraphExecKernelNodeSetParams");
     return 0;
 }
 

@@ -126,7 +126,8 @@ def _estimate(z, m, n, k, groups, b_mn, can_step, splits):
 
 
 def split_for(m: int, n: int, k: int, groups: int = 1, b_mn: bool = False, can_step: bool = True) -> int:
-    """CTAs that share the K of one result tile.  Up to K = 1024 splitting pays while the
+    """CTAs that share the K of one result tile: the order of the sum, so a function of the
+    matmul and of what it could share a launch with (``groups``).  Up to K = 1024 splitting pays while the
     parts of all tiles stay under two thirds of the machine, which leaves the next launch
     room to move in: inside BERT-base b1, [128, 768] x [768, 768] in four parts (96 CTAs)
     takes 0.4 us less than in two; the three of a layer's q, k, v in one launch take 1.7
@@ -140,9 +141,10 @@ def split_for(m: int, n: int, k: int, groups: int = 1, b_mn: bool = False, can_s
     return _estimate(1, m, n, k, groups, b_mn, can_step, (1, 2, 4, 8))[2]
 
 
-def choose(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, can_step: bool = True) -> Config:
-    """Tile, split and pairing for a shape."""
-    split = split_for(m, n, k, groups, b_mn, can_step) if z == 1 else 1
+def choose(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, can_step: bool = True,
+           peers: int | None = None) -> Config:
+    """Tile, split and pairing for a shape (``peers``: ``MatmulKernel.peers``)."""
+    split = split_for(m, n, k, peers or groups, b_mn, can_step) if z == 1 else 1
     found = _estimate(z, m, n, k, groups, b_mn, can_step, (split,))
     _, bn, split, cg, t, kstep = found
     persistent = split == 1 and t > SM_COUNT // cg
@@ -353,7 +355,7 @@ def emit_matmul(k: MatmulKernel, cfg, buffers, name: str | None = None, stable=f
     z, m, n, kk = k.shape
     b_mn = tma_layout(k.bs[0], -1, -2) == "mn"
     a_cut, b_cut = can_cut(k.a, -2, -1), can_cut(k.bs[0], -1, -2)
-    mc = choose(z, m, n, kk, len(k.bs), b_mn, a_cut and (b_cut or b_mn))
+    mc = choose(z, m, n, kk, len(k.bs), b_mn, a_cut and (b_cut or b_mn), k.peers)
     for e in k.epilogues:
         for a in [x for x in e.inputs if x is not None] + e.outputs:
             check_bounds(a.index, buffers[a.buffer].numel, f"{k.name}:{a.name}")
@@ -413,7 +415,7 @@ class Config32:
         return self.stages * 3 * (16384 + self.bn * 128) + inbox + 1024
 
 
-def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool) -> Config32:
+def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, peers: int | None = None) -> Config32:
     """Least estimated time, in microseconds: a 64-deep block costs 0.75 (32 columns) or 1.0
     (64), a wave 3 before and after.  Leading products get a new accumulator every four
     blocks, as far as TMEM goes."""
@@ -427,8 +429,9 @@ def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool) -> Config3
 
     widths = (64,) if b_mn else (32, 64)
     splits = (1,) if z > 1 else tuple(s for s in (1, 2, 4, 8) if s <= kb)
-    bn, split = min(((bn, s) for bn in widths for s in splits if bn % (8 * s) == 0),
-                    key=lambda c: cost(*c, groups))
+    _, split = min(((bn, s) for bn in widths for s in splits if bn % (8 * s) == 0),
+                   key=lambda c: cost(*c, peers or groups))
+    bn = min((bn for bn in widths if bn % (8 * split) == 0), key=lambda bn: cost(bn, split, groups))
     t = _ceil(m, 128) * _ceil(n, bn) * groups * z
     most = 2 if split > 1 and bn == 64 else 3           # the partial sums' place
     return Config32(bn, max(2, min(most, _ceil(kb, split))), split, t * split,
@@ -439,7 +442,7 @@ def emit_matmul32(k: MatmulKernel, cfg, buffers, name: str, stable):
     z, m, n, kk = k.shape
     b0 = k.bs[0]
     b_mn = b0.strides[-2] != 1
-    mc = choose32(z, m, n, kk, len(k.bs), b_mn)
+    mc = choose32(z, m, n, kk, len(k.bs), b_mn, k.peers)
     for e in k.epilogues:
         for a in [x for x in e.inputs if x is not None] + e.outputs:
             check_bounds(a.index, buffers[a.buffer].numel, f"{k.name}:{a.name}")

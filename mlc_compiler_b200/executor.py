@@ -261,18 +261,27 @@ class _Executable:
                       and all(b.buffer in self.params for b in k.bs)), None)
         return [] if after is None else [buffers[b.buffer] for b in after.bs]
 
-    def run_kernels(self, buffers: dict[str, torch.Tensor] | None = None) -> None:
+    def run_kernels(self, buffers: dict[str, torch.Tensor] | None = None, after=None) -> None:
+        """``after(j, stream)``: called behind the launch of kernel ``j``."""
         if self._plan is None:
             raise ExecutionError("no launch plan: call the model (or forward) once first")
         if self._streams is not None:
-            return self._run_forked()
+            return self._run_forked(after)
+        if after is not None:
+            for j, (kind, payload) in enumerate(self._per_kernel):
+                if kind == "cuda":
+                    payload[payload.grid]()
+                else:
+                    run_bound_extern(payload)
+                after(j, torch.cuda.current_stream(self.device))
+            return
         for kind, payload in self._plan:
             if kind == "cuda":
                 payload()
             else:
                 run_bound_extern(payload)
 
-    def _run_forked(self) -> None:
+    def _run_forked(self, after=None) -> None:
         """Enqueue the plan over several streams: a kernel goes to the stream the
         plan gave it and waits (by event) for predecessors enqueued elsewhere.
         Under capture the events become edges of the graph; outside capture the
@@ -296,6 +305,8 @@ class _Executable:
                     payload[payload.grid]()
                 else:
                     run_bound_extern(payload)
+            if after is not None:
+                after(j, stream)
             if j in sp.signals:
                 ev = torch.cuda.Event()
                 ev.record(stream)
@@ -350,10 +361,12 @@ class _Executable:
         views = self._input_views
         if len(inputs) != len(views):
             self._check_inputs(inputs)
-        for dst, src in zip(views, inputs):
+        for i, (dst, src) in enumerate(zip(views, inputs)):
             if src.shape != dst.shape:
                 self._check_inputs(inputs)
-            dst.copy_(src, non_blocking=True)
+            if not self._in_place.take(i, src):
+                dst.copy_(src, non_blocking=True)
+        self._in_place.apply(inputs)
         self._graph_replay.replay()
         return self._static_outputs
 
@@ -365,10 +378,10 @@ class _Executable:
             if self._plan is None:
                 self._plan = self._build_plan(buffers)
             g = self._capture_plan(buffers)
-        self._graph_replay = g
+        self._graph_replay, self._in_place = g
         self._static_outputs = self._collect(buffers)
 
-    def _capture_plan(self, buffers) -> torch.cuda.CUDAGraph:
+    def _capture_plan(self, buffers):
         # Warm up off the capture stream: cuBLAS picks algorithms and allocates
         # workspaces on first use, which must not be recorded.
         side = torch.cuda.Stream(device=self.device)
@@ -379,12 +392,16 @@ class _Executable:
         torch.cuda.current_stream(self.device).wait_stream(side)
         if self._module.loaded.fault():
             raise BackendError("a bounded wait inside a kernel ran out during warm-up")
-        g = torch.cuda.CUDAGraph()
+        # the graph is kept: its nodes are how later calls name their inputs
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        in_place = _InPlaceInputs(self, buffers)
         with torch.cuda.graph(g):
-            self.run_kernels(buffers)
-        return g
+            self.run_kernels(buffers, in_place.note)
+        g.instantiate()
+        in_place.ready(g)
+        return g, in_place
 
-    def _capture_best_policy(self, buffers) -> torch.cuda.CUDAGraph:
+    def _capture_best_policy(self, buffers):
         """``dependent_launch="auto"``: capture the schedule twice -- programmatic
         edges only behind generated kernels ("chain"), and behind library kernels
         too -- replay both alternately and keep the faster graph.  Which one wins
@@ -399,7 +416,7 @@ class _Executable:
         end = torch.cuda.Event(enable_timing=True)
         times = {p: [] for p in candidates}
         for _ in range(3):
-            for p, (g, *_rest) in candidates.items():
+            for p, ((g, _), *_rest) in candidates.items():
                 g.replay()
                 start.record()
                 for _ in range(10):
@@ -445,6 +462,97 @@ class _Executable:
 def _launch_failed(lib, name: str, code: int):
     raise BackendError(f"launch of {name} failed with code {code}: "
                        f"{lib.mlcb_last_error().decode(errors='replace')}")
+
+
+class _InPlaceInputs:
+    """Inputs a captured graph reads where the caller has them.
+
+    Copying every input into a fixed buffer costs about 4 us of a call each (a copy
+    kernel and the gaps around it), 8 of the 125 us of a small encoder.  Instead the
+    kernel nodes that read an input get its address, once per change of address: new
+    parameters of a few nodes of the instantiated graph.  An input that cannot be read in
+    place -- another dtype, device or layout, an unaligned start, memory the model
+    writes, a reader that is a library call -- is copied as before, and its nodes point
+    at the fixed buffer again."""
+
+    def __init__(self, owner: "_Executable", buffers: dict[str, torch.Tensor]):
+        sch = owner._exec
+        self.lib, self.index = owner._module.lib, owner.device.index
+        finals = {v.buffer for v in sch.outputs}
+        names = [v.buffer for v in sch.inputs]
+        self.watch: dict[int, list[str]] = {}
+        self.inputs: list = []                   # per input: (buffer, size, dtype) or None
+        for v in sch.inputs:
+            readers = [j for j, k in enumerate(sch.kernels) if v.buffer in k.reads()]
+            spec = sch.buffers[v.buffer]
+            if (v.buffer in finals or names.count(v.buffer) > 1 or not readers or len(readers) > 64
+                    or any(v.buffer in k.writes() for k in sch.kernels)
+                    or any(isinstance(sch.kernels[j], kir.ExternKernel) for j in readers)):
+                self.inputs.append(None)
+                continue
+            self.inputs.append((v.buffer, spec.nbytes, kir.torch_dtype(spec.dtype)))
+            for j in readers:
+                self.watch.setdefault(j, []).append(v.buffer)
+        #: per watched kernel a launch of its own: its parameter values are the node's
+        self.launch = {}
+        for j in self.watch:
+            k = sch.kernels[j]
+            fn = owner._module.bind(k, buffers, 0, owner._weights_after(j, buffers))[0]
+            spec = owner._module.generated.launch[k.name]
+            self.launch[j] = (fn, list(spec.buffers or owner._module._buffer_names(k)), spec.tmaps)
+        self.fixed = {b: buffers[b].data_ptr() for b in names}
+        self.now = dict(self.fixed)
+        self.written = [(buffers[b].data_ptr(), buffers[b].data_ptr() + sch.buffers[b].nbytes) for b in finals]
+        self.node: dict[int, int] = {}
+        self.wanted = dict(self.fixed)
+        self.held = None
+
+    def note(self, j: int, stream) -> None:
+        if j in self.watch:
+            node = ctypes.c_uint64()
+            if self.lib.mlcb_capture_node(stream.cuda_stream, ctypes.byref(node)) == 0 and node.value:
+                self.node[j] = node.value
+
+    def ready(self, graph) -> None:
+        self.exec = int(graph.raw_cuda_graph_exec())
+        lost = {b for j, bs in self.watch.items() if j not in self.node for b in bs}
+        self.inputs = [None if i is None or i[0] in lost else i for i in self.inputs]
+        self.params = {j: fn.parameters() for j, (fn, _, _) in self.launch.items()}
+
+    def take(self, i: int, t: torch.Tensor) -> bool:
+        """Whether input ``i`` is read where ``t`` has it (from ``apply`` on)."""
+        if self.inputs[i] is None:
+            return False
+        buffer, nbytes, dtype = self.inputs[i]
+        p = t.data_ptr() if t.is_cuda else 0
+        if (p == 0 or p & 31 or t.dtype is not dtype or t.get_device() != self.index or not t.is_contiguous()
+                or any(p < hi and lo < p + nbytes for lo, hi in self.written)):
+            self.wanted[buffer] = self.fixed[buffer]
+            return False
+        self.wanted[buffer] = p
+        return True
+
+    def apply(self, inputs) -> None:
+        self.held = inputs                        # a replay reads them again
+        if self.wanted == self.now:
+            return
+        changed = {b for b, p in self.wanted.items() if p != self.now[b]}
+        for j, bs in self.watch.items():
+            if not changed & set(bs) or j not in self.node:
+                continue
+            fn, names, tmaps = self.launch[j]
+            for i, n in enumerate(names):
+                if n in changed:
+                    fn.ptrs[i] = self.wanted[n]
+            for i, m in enumerate(tmaps):
+                if m.buffer in changed:
+                    fn.encode(i, self.wanted[m.buffer])
+            code = self.lib.mlcb_graph_params(self.exec, self.node[j], fn.kernel, fn.grid, fn.block, fn.smem,
+                                              self.params[j])
+            if code != 0:
+                raise BackendError(f"input of {fn.name}: code {code}: "
+                                   f"{self.lib.mlcb_last_error().decode(errors='replace')}")
+        self.now = dict(self.wanted)
 
 
 class _DirectCall:

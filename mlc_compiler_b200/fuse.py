@@ -57,6 +57,10 @@ class MatmulKernel:
     dtype: str
     epilogues: list
     covers: list = field(default_factory=list)
+    #: matmuls of the schedule with this row operand and shape, itself included: what it may
+    #: share a launch with.  How K is split goes by it, so that results do not depend on
+    #: which of them do
+    peers: int = 1
 
     @property
     def shape(self) -> tuple[int, int, int, int]:
@@ -226,7 +230,7 @@ def _with_epilogue(mm: MatmulKernel, p: kir.PointwiseKernel) -> MatmulKernel | N
     except _NoCompose:
         return None
     e = Epilogue(ins, slots[0], outs, list(p.body), dict(p.out_expr))
-    return MatmulKernel(p.name, mm.a, mm.bs, mm.dtype, [e], mm.covers + [p.name])
+    return MatmulKernel(p.name, mm.a, mm.bs, mm.dtype, [e], mm.covers + [p.name], mm.peers)
 
 
 def _same_map(m: kir.IndexMap) -> tuple:
@@ -250,6 +254,11 @@ def _group_key(mm: MatmulKernel, schedule) -> tuple | None:
 MAX_GROUPS = 4
 
 
+def _peer_key(mm: MatmulKernel) -> tuple:
+    a, b = mm.a, mm.bs[0]
+    return a.buffer, a.shape, a.strides, a.offset, b.shape, mm.covers[0] if mm.shape[0] > 1 else ""
+
+
 def _merged(kernels: list, schedule) -> list:
     """Neighbours with equal group keys become one launch at the last one's place.
     Only kernels none of whose operands a kernel in between writes are moved."""
@@ -270,7 +279,8 @@ def _merged(kernels: list, schedule) -> list:
             j += 1
         if len(group) > 1:
             out.append(MatmulKernel(group[0].name, k.a, [g.bs[0] for g in group], k.dtype,
-                                    [g.epilogues[0] for g in group], [c for g in group for c in g.covers]))
+                                    [g.epilogues[0] for g in group], [c for g in group for c in g.covers],
+                                    k.peers))
         else:
             out.append(k)
         i += len(group)
@@ -340,6 +350,13 @@ def fuse(schedule: kir.Schedule, cfg) -> kir.Schedule:
     kernels: list = [_matmul(k, schedule) or k for k in schedule.kernels]
     if not any(isinstance(k, MatmulKernel) for k in kernels):
         return schedule
+    same: dict[tuple, int] = {}
+    for k in kernels:
+        if isinstance(k, MatmulKernel):
+            same[_peer_key(k)] = same.get(_peer_key(k), 0) + 1
+    for k in kernels:
+        if isinstance(k, MatmulKernel):
+            k.peers = min(MAX_GROUPS, same[_peer_key(k)])
     finals = {v.buffer for v in schedule.outputs}
     if fold:
         readers: dict[str, list[int]] = {}

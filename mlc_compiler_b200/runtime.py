@@ -64,6 +64,9 @@ _SIGNATURES = {
                                         ctypes.c_uint64, ctypes.POINTER(ctypes.c_int)]),
     "mlcb_kernel_shared": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint32]),
     "mlcb_module_fault": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint32)]),
+    "mlcb_capture_node": (ctypes.c_int, [ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)]),
+    "mlcb_graph_params": (ctypes.c_int, [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_uint32,
+                                         ctypes.c_uint32, ctypes.c_uint32, ctypes.POINTER(ctypes.c_void_p)]),
     "mlcb_tensor_map": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int,
                                        ctypes.POINTER(ctypes.c_uint64), ctypes.POINTER(ctypes.c_uint64),
                                        ctypes.POINTER(ctypes.c_uint32)]),
@@ -267,6 +270,11 @@ class BoundLaunch:
     def __getitem__(self, grid):
         return self
 
+    def parameters(self):
+        """Addresses of the launch's parameter values, in the kernel's order."""
+        at = ctypes.addressof(self.ptrs)
+        return (ctypes.c_void_p * max(1, self.nptrs))(*[at + 8 * i for i in range(self.nptrs)])
+
     def __call__(self, *tensors, **consts) -> None:
         if tensors and tensors is not self.tensors and \
                 any(a is not b for a, b in zip(tensors, self.tensors)):
@@ -300,7 +308,7 @@ class TensorLaunch(BoundLaunch):
     """A launch whose parameters are tensor maps (encoded once, at bind time) followed
     by buffer pointers, on clusters of CTAs."""
 
-    __slots__ = ("cluster", "maps", "params", "mapped", "ahead")
+    __slots__ = ("cluster", "maps", "tmaps", "params", "mapped", "ahead")
 
     def __init__(self, lib, kernel, name, spec, flags, tensors, buffers, device=None, ahead=()):
         super().__init__(lib, kernel, name, spec.grid, spec.block, spec.smem, flags, tensors, device)
@@ -309,16 +317,25 @@ class TensorLaunch(BoundLaunch):
         self.mapped = tuple(buffers[m.buffer] for m in spec.tmaps)       # keeps the storage alive
         raw = ctypes.create_string_buffer(128 * len(spec.tmaps) + 128)
         base = (ctypes.addressof(raw) + 127) & ~127
-        self.maps = raw
-        for i, (m, t) in enumerate(zip(spec.tmaps, self.mapped)):
-            _check(lib, lib.mlcb_tensor_map(
-                base + 128 * i, t.data_ptr() + m.offset * t.element_size(), int(m.dtype == "bfloat16"),
-                (ctypes.c_uint64 * 4)(*m.dims), (ctypes.c_uint64 * 3)(*m.strides),
-                (ctypes.c_uint32 * 3)(*m.box)), f"tensor map of {m.buffer} for {name}")
+        self.maps, self.tmaps = raw, spec.tmaps
+        for i, t in enumerate(self.mapped):
+            self.encode(i, t.data_ptr())
         at = ctypes.addressof(self.ptrs)
         self.params = (ctypes.c_void_p * (len(spec.tmaps) + self.nptrs + int(spec.next)))(
             *[base + 128 * i for i in range(len(spec.tmaps))], *[at + 8 * i for i in range(self.nptrs)],
             *([ctypes.addressof(self.ahead)] if spec.next else []))
+
+    def encode(self, i: int, address: int) -> None:
+        """Tensor map ``i`` over a buffer at ``address``."""
+        m = self.tmaps[i]
+        base = (ctypes.addressof(self.maps) + 127) & ~127
+        _check(self.lib, self.lib.mlcb_tensor_map(
+            base + 128 * i, address + m.offset * kir.ITEMSIZE[m.dtype], int(m.dtype == "bfloat16"),
+            (ctypes.c_uint64 * 4)(*m.dims), (ctypes.c_uint64 * 3)(*m.strides),
+            (ctypes.c_uint32 * 3)(*m.box)), f"tensor map of {m.buffer} for {self.name}")
+
+    def parameters(self):
+        return self.params
 
     def __call__(self, *tensors, **consts) -> None:
         stream = torch.cuda.current_stream(self.device).cuda_stream
