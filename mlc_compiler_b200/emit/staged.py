@@ -78,6 +78,38 @@ def plan(k: kir.ReductionKernel, cfg, vector: int) -> Stage | None:
     return Stage(slots, V, aligned, C, T, PC)
 
 
+def _paired(k: kir.ReductionKernel) -> bool:
+    """Whether the column-varying work runs on pairs of neighbouring columns
+    (``mlcb_f2``: the same roundings, two columns per instruction)."""
+    from .reduction import varying_steps
+
+    vec = varying_steps(k)
+    cols = {i for i, a in enumerate(k.inputs) if a.index.varies_along("col")}
+    floats = kir.NARROW_FLOATS + ("float32",)
+
+    def varies(e):
+        return bool(kir.expr_loads(e) & cols or kir.expr_refs(e) & vec)
+
+    exprs = [s.expr for s in k.steps if varies(s.expr)] + [
+        k.out_expr[a.name] for a in k.outputs if a.name not in k.row_outputs]
+    for e in exprs:
+        if not varies(e):
+            return False
+        for s in kir.walk(e):
+            if isinstance(s, kir.Call) and varies(s):
+                power = isinstance(s.args[-1], kir.Const) and X._is_pow2(s.args[-1].value)
+                if s.fn in ("add", "sub", "mul") or (s.fn == "div" and varies(s.args[0]) and (
+                        power or (X._FAST and not varies(s.args[1])))):
+                    continue
+                if not (X._FAST and s.fn in ("exp", "tanh", "erf", "sigmoid")):
+                    return False
+            if isinstance(s, kir.Cast) and varies(s) and s.dtype not in floats:
+                return False
+    return (all(r.kind in ("sum", "max", "min") for r in k.reduces)
+            and all(k.inputs[i].dtype in floats for i in cols)
+            and all(a.dtype in floats for a in k.outputs))
+
+
 def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tuple[str, LaunchSpec]:
     from .reduction import _Ctx, _OP, _acc_dtype, _identity, _row_stores, _signature, Geometry, plan_passes
 
@@ -152,6 +184,7 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
     if release:
         e(release)
 
+    pairs = _paired(k)
     loads: list = []
     acc_other = {}
     for i, a in enumerate(k.inputs):
@@ -159,11 +192,12 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
         if scalar_in[i] is not None:
             loads.append(scalar_in[i])
         elif i in st.slots:
-            loads.append(X.Val(f"v{i}[j]", dt, True, True))
+            loads.append(X.Val(f"mlcb_f2(v{i}[j], v{i}[j + 1])" if pairs else f"v{i}[j]", dt, True, True))
         else:
             ac = classify(a.index, "col", V)
             acc_other[i] = st.aligned and ac.mode == "contig" and ac.width == V
-            loads.append(X.Val(f"v{i}[j]" if acc_other[i] else f"g{i}", dt, True, True))
+            loads.append(X.Val((f"mlcb_f2(v{i}[j], v{i}[j + 1])" if pairs else f"v{i}[j]") if acc_other[i]
+                               else f"g{i}", dt, True, True))
 
     first = True
 
@@ -186,7 +220,8 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
             rdt = X.reduce_type(r.kind, rv.dtype)
             adt = _acc_dtype(rdt)
             accs[r.name] = (adt, rdt)
-            e(f"    {X.REG_T[adt]} acc_{r.name} = {_identity(r.kind, adt)};")
+            pair = pairs and r.kind == "sum"       # a partial sum of the even and one of the odd columns
+            e(f"    {'mlcb_f2' if pair else X.REG_T[adt]} acc_{r.name}{'(0.0f)' if pair else f' = {_identity(r.kind, adt)}'};")
         stores = [(i, a) for i, a in enumerate(k.outputs) if a.name in p.stores]
         e("#pragma unroll 1" if st.blocks > 16 else "#pragma unroll 2")
         e(f"    for (int i = 0; i < {st.blocks}; ++i) {{")
@@ -214,29 +249,58 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
 
         def body(guarded: bool, ind: str) -> None:
             e("#pragma unroll")
-            e(f"{ind}for (int j = 0; j < {V}; ++j) {{")
+            e(f"{ind}for (int j = 0; j < {V}; j += {2 if pairs else 1}) {{")
             ind += "    "
             if guarded:
-                e(f"{ind}if (c0 + j < 0 || c0 + j >= {N}) continue;")
+                # a pack over an end of the row: of a pair the half inside counts
+                within = [f"(unsigned)(c0 + j{' + 1' if h else ''}) < {N}u" for h in range(2 if pairs else 1)]
+                e(f"{ind}const bool {', '.join(f'in_{h} = {w}' for h, w in enumerate(within))};")
+                e(f"{ind}if (!({' || '.join(f'in_{h}' for h in range(len(within)))})) continue;")
             for i, packed in acc_other.items():
                 if i in used and not packed:
                     a = k.inputs[i]
-                    off = render_offset(a.index, {"col": "(c0 + j)"}, skip=("row", "base"))
-                    e(f"{ind}const {X.REG_T[a.dtype]} g{i} = mlcb_load1<{X.STORAGE_T[a.dtype]}>"
-                      f"(in{i} + in{i}_r + ({off}));  // {a.name}")
+                    ct = X.STORAGE_T[a.dtype]
+
+                    def at(h):
+                        col = f"(c0 + j{' + 1' if h else ''})"
+                        if guarded:
+                            col = f"mlcb_within({col}, {N})"
+                        return (f"mlcb_load1<{ct}>(in{i} + in{i}_r + "
+                                f"({render_offset(a.index, {'col': col}, skip=('row', 'base'))}))")
+                    if pairs:
+                        e(f"{ind}const mlcb_f2 g{i}({at(0)}, {at(1)});  // {a.name}")
+                    else:
+                        e(f"{ind}const {X.REG_T[a.dtype]} g{i} = {at(0)};  // {a.name}")
             local = dict(c.scalars)
             for b in p.binds:
                 v = X.render_bind(b.name, b.expr, loads, local, c.elide)
-                e(f"{ind}const {X.REG_T[v.dtype]} {b.name} = {v.code};")
+                e(f"{ind}const {'mlcb_f2' if pairs else X.REG_T[v.dtype]} {b.name} = {v.code};")
                 local[b.name] = X.Val(b.name, v.dtype, v.dim, True)
             for r in p.reduces:
                 adt, _ = accs[r.name]
                 rv = X.render(r.expr, loads, local)
+                if pairs:
+                    e(f"{ind}float {r.name}_lo, {r.name}_hi; mlcb_f2({rv.code}).get({r.name}_lo, {r.name}_hi);")
+                    if guarded:
+                        ident = _identity(r.kind, adt)
+                        for h, n in ((0, "lo"), (1, "hi")):
+                            e(f"{ind}{r.name}_{n} = in_{h} ? {r.name}_{n} : {ident};")
+                    if r.kind == "sum":
+                        e(f"{ind}acc_{r.name} = acc_{r.name} + mlcb_f2({r.name}_lo, {r.name}_hi);")
+                    else:
+                        e(f"{ind}acc_{r.name} = mlcb_{r.kind}3(acc_{r.name}, {r.name}_lo, {r.name}_hi);")
+                    continue
                 x = rv.code if rv.dtype in kir.NARROW_FLOATS else X.convert(rv.code, rv.dtype, adt)
                 e(f"{ind}acc_{r.name} = {_OP[r.kind]}::f<{X.REG_T[adt]}>(acc_{r.name}, {x});")
             for i, a in stores:
                 code = store_code(X.render(k.out_expr[a.name], loads, local), a.dtype)
-                if guarded:
+                if pairs:
+                    e(f"{ind}mlcb_f2({code}).get(o{i}[j], o{i}[j + 1]);  // {a.name}")
+                    if guarded:
+                        for h in (0, 1):
+                            e(f"{ind}if (in_{h}) mlcb_store1<{X.STORAGE_T[a.dtype]}>(out{i} + (in{lead}_r + c0 + j + {h}), "
+                              f"o{i}[j + {h}]);")
+                elif guarded:
                     e(f"{ind}mlcb_store1<{X.STORAGE_T[a.dtype]}>(out{i} + (in{lead}_r + c0 + j), {code});")
                 else:
                     e(f"{ind}o{i}[j] = {code};  // {a.name}")
@@ -259,7 +323,10 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
         for r in p.reduces:
             adt, rdt = accs[r.name]
             t, n = X.REG_T[adt], reduces.index(r)
-            red = (f"mlcb_cta_reduce<{_OP[r.kind]}, {T // 32}, {t}>(acc_{r.name}, "
+            if pairs and r.kind == "sum":
+                e(f"    float even_{r.name}, odd_{r.name}; acc_{r.name}.get(even_{r.name}, odd_{r.name});")
+                e(f"    const float both_{r.name} = even_{r.name} + odd_{r.name};")
+            red = (f"mlcb_cta_reduce<{_OP[r.kind]}, {T // 32}, {t}>({'both' if pairs and r.kind == 'sum' else 'acc'}_{r.name}, "
                    f"reinterpret_cast<{t}*>(mlcb_red + {n} * 32))")
             if C > 1:
                 red = f"mlcb_cluster_reduce<{_OP[r.kind]}, {C}, {t}>({red}, mlcb_part + {n})"

@@ -20,6 +20,7 @@ no interpreter fallback in this class.
 
 from __future__ import annotations
 
+import copy
 import ctypes
 import functools
 from typing import Any, Mapping, Sequence
@@ -155,7 +156,14 @@ class _Executable:
     @property
     def _module(self) -> CudaRuntime:
         if self._runtime is None:
-            self._runtime = CudaRuntime(self._exec, self.cfg, self.device)
+            cfg = self.cfg
+            if self._direct is not None and cfg.cuda_graphs:
+                # launched behind whatever the caller enqueued: parameters are read after the
+                # wait like everything else, and the launch can be programmatic ([4096, 3072]
+                # bias + GELU + residual: calls 16.0 us apart with a plain launch)
+                cfg = copy.copy(cfg)
+                cfg.hoist_stable_loads = False
+            self._runtime = CudaRuntime(self._exec, cfg, self.device)
         return self._runtime
 
     # -- allocation ------------------------------------------------------------
@@ -596,10 +604,7 @@ class _DirectCall:
                         for b in set(k.writes())]
         self.out = owner._collect(buffers)
         self.args = (fn.kernel, fn.grid, fn.block, fn.smem, fn.ptrs, fn.nptrs)
-        if not set(k.reads()) & set(owner.params):
-            # consecutive calls overlap at their edges; a kernel with parameters reads them
-            # ahead of its wait and so starts after whatever the caller enqueued before it
-            fn.flags |= 1
+        fn.flags |= 1                # consecutive calls overlap at their edges
         self.run, self.flags = fn.lib.mlcb_launch, fn.flags
         native = native_call()
         if native is not None:
