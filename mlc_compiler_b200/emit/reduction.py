@@ -716,12 +716,12 @@ def detect_online_softmax(k: kir.ReductionKernel):
     return (rs[0], rs[1], rs[0].expr)
 
 
-def plan_passes(k: kir.ReductionKernel, online: bool = True) -> list[Pass]:
+def plan_passes(k: kir.ReductionKernel) -> list[Pass]:
     deps = _dependencies(k.steps)
     vec = varying_steps(k)
     by = {s.name: s for s in k.steps}
     order = [s.name for s in k.steps]
-    online = detect_online_softmax(k) if online else None
+    online = detect_online_softmax(k)
 
     def vbinds(needed: set[str]) -> list:
         return [by[n] for n in order if n in needed and isinstance(by[n], Bind) and n in vec]

@@ -119,7 +119,8 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
     it = "i64" if needs_64bit(*extents) else "int"
     geo = Geometry(V, PC, T, st.blocks, T, 1, grid, masked=True)
     c = _Ctx(k, geo, it, stable, cfg)
-    passes = plan_passes(k, online=False)
+    # softmax: maximum and sum in one pass, which overlaps the arrival of the row
+    passes = plan_passes(k)
     reduces = k.reduces
     lead = st.slots[0]
     occ = max(1, min(2048 // T, SMEM_MAX // max(1, st.smem), 65536 // (T * 56)))
@@ -204,10 +205,14 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
     def emit_pass(p) -> None:
         nonlocal first
         used: set[int] = set()
+        online = p.online
         for b in p.binds:
             used |= kir.expr_loads(b.expr)
-        for r in p.reduces:
+        for r in ([] if online else p.reduces):
             used |= kir.expr_loads(r.expr)
+        if online:
+            used |= kir.expr_loads(online[2])
+            e("    float run_m = MLCB_NINF_F, run_l = 0.0f;")
         for nm in p.stores:
             used |= kir.expr_loads(k.out_expr[nm])
         probe = dict(c.scalars)
@@ -215,7 +220,7 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
             v = X.render_bind(b.name, b.expr, loads, probe, c.elide)
             probe[b.name] = X.Val(b.name, v.dtype, v.dim, True)
         accs = {}
-        for r in p.reduces:
+        for r in ([] if online else p.reduces):
             rv = X.render(r.expr, loads, probe)
             rdt = X.reduce_type(r.kind, rv.dtype)
             adt = _acc_dtype(rdt)
@@ -246,6 +251,8 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
                 e(f"{ind}{X.REG_T[a.dtype]} v{i}[{V}]; mlcb_load<{ct}, {V}>(in{i} + in{i}_r + ({off}), v{i});")
         for i, a in stores:
             e(f"{ind}{X.REG_T[a.dtype]} o{i}[{V}];")
+        if online:
+            e(f"{ind}float xs[{V}];")
 
         def body(guarded: bool, ind: str) -> None:
             e("#pragma unroll")
@@ -255,6 +262,9 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
                 # a pack over an end of the row: of a pair the half inside counts
                 within = [f"(unsigned)(c0 + j{' + 1' if h else ''}) < {N}u" for h in range(2 if pairs else 1)]
                 e(f"{ind}const bool {', '.join(f'in_{h} = {w}' for h, w in enumerate(within))};")
+                if online:
+                    for h in range(len(within)):
+                        e(f"{ind}xs[j + {h}] = MLCB_NINF_F;")
                 e(f"{ind}if (!({' || '.join(f'in_{h}' for h in range(len(within)))})) continue;")
             for i, packed in acc_other.items():
                 if i in used and not packed:
@@ -276,7 +286,16 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
                 v = X.render_bind(b.name, b.expr, loads, local, c.elide)
                 e(f"{ind}const {'mlcb_f2' if pairs else X.REG_T[v.dtype]} {b.name} = {v.code};")
                 local[b.name] = X.Val(b.name, v.dtype, v.dim, True)
-            for r in p.reduces:
+            if online:
+                xv = X.render(online[2], loads, local)
+                if pairs:
+                    e(f"{ind}mlcb_f2({xv.code}).get(xs[j], xs[j + 1]);")
+                    if guarded:
+                        e(f"{ind}if (!in_0) xs[j] = MLCB_NINF_F;")
+                        e(f"{ind}if (!in_1) xs[j + 1] = MLCB_NINF_F;")
+                else:
+                    e(f"{ind}xs[j] = {X.convert(xv.code, xv.dtype, 'float32')};")
+            for r in ([] if online else p.reduces):
                 adt, _ = accs[r.name]
                 rv = X.render(r.expr, loads, local)
                 if pairs:
@@ -318,9 +337,41 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
             e(f"{ind}}} else {{")
             body(True, ind + "    ")
             e(f"{ind}}}")
+        if online:
+            # m' = max(m, max(pack)); l' = l exp(m - m') + sum exp(x - m').  A thread that has
+            # only met -inf keeps l = 0 and never evaluates exp(-inf - -inf)
+            ex = "mlcb_exp_fast" if X._FAST else "expf"
+            e(f"{ind}float nm = run_m;")
+            e("#pragma unroll")
+            e(f"{ind}for (int j = 0; j < {V}; j += 2) nm = mlcb_max3(nm, xs[j], xs[j + 1]);")
+            e(f"{ind}if (nm != MLCB_NINF_F) {{")
+            if X._FAST:
+                e(f"{ind}    mlcb_f2 ps(0.0f);")
+                e("#pragma unroll")
+                e(f"{ind}    for (int j = 0; j < {V}; j += 2) ps = ps + {ex}(mlcb_f2(xs[j], xs[j + 1]) - mlcb_f2(nm));")
+                e(f"{ind}    float p0_, p1_; ps.get(p0_, p1_); const float sum_ = p0_ + p1_;")
+            else:
+                e(f"{ind}    float sum_ = 0.0f;")
+                e("#pragma unroll")
+                e(f"{ind}    for (int j = 0; j < {V}; ++j) sum_ += {ex}(xs[j] - nm);")
+            e(f"{ind}    run_l = run_l * ((run_m == MLCB_NINF_F) ? 0.0f : {ex}(run_m - nm)) + sum_;")
+            e(f"{ind}    run_m = nm;")
+            e(f"{ind}}}")
         e("        }")
         e("    }")
-        for r in p.reduces:
+        if online:
+            mx, sm, _ = online
+            ex = "mlcb_exp_fast" if X._FAST else "expf"
+
+            def whole(op, x, n):
+                code = f"mlcb_cta_reduce<{op}, {T // 32}, float>({x}, reinterpret_cast<float*>(mlcb_red + {n} * 32))"
+                return f"mlcb_cluster_reduce<{op}, {C}, float>({code}, mlcb_part + {n})" if C > 1 else code
+            e(f"    const float {mx.name} = {whole('mlcb_op_max', 'run_m', 0)};")
+            e(f"    const float scaled_l = (run_m == MLCB_NINF_F) ? 0.0f : run_l * {ex}(run_m - {mx.name});")
+            e(f"    const float {sm.name} = {whole('mlcb_op_sum', 'scaled_l', 1)};")
+            for r in (mx, sm):
+                c.scalars[r.name] = X.Val(r.name, "float32", True, False)
+        for r in ([] if online else p.reduces):
             adt, rdt = accs[r.name]
             t, n = X.REG_T[adt], reduces.index(r)
             if pairs and r.kind == "sum":
