@@ -309,18 +309,19 @@ def micro_roofline(dev, peak_gbs: float, batches=(1, 8, 32), launches: int = 64,
 
 
 def in_model_families(cm, dev_inputs, peak_gbs: float, reps: int = 20) -> list[dict]:
-    """Device time of each distinct generated function inside the BERT step: one
+    """Device time of each distinct generated function a call of the model launches: one
     bound launch of it replayed ``reps`` times inside a CUDA graph (in place, so
     it runs out of L2 and is launch-bound at batch 1; reported for context)."""
-    cm(*dev_inputs)
+    cm.forward(*dev_inputs)
     torch.cuda.synchronize()
-    table = cm.launch_table
+    form = cm._launched or cm
+    table = form._module.launch_table
     groups: dict[str, list[str]] = {}
     for name, row in table.items():
         groups.setdefault(row["symbol"], []).append(name)
     out = []
     for sym, names in groups.items():
-        kind, fn = cm._bound[names[0]]
+        kind, fn = form._bound[names[0]]
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -340,7 +341,7 @@ def in_model_families(cm, dev_inputs, peak_gbs: float, reps: int = 20) -> list[d
         torch.cuda.synchronize()
         us = s.elapsed_time(e) * 1e3 / (5 * reps)
         ab = table[names[0]]["alg_bytes"]
-        out.append({"symbol": sym, "kernel": cm.executed_schedule.kernel(names[0]).summary().split(": ", 1)[1][:70],
+        out.append({"symbol": sym, "kernel": cm.launched_schedule.kernel(names[0]).summary().split(": ", 1)[1][:70],
                     "launches_per_forward": len(names), "us_per_launch": round(us, 3),
                     "alg_bytes": ab, "gbs": round(ab / us / 1e3, 1),
                     "frac": round(ab / us / 1e3 / peak_gbs, 4), "l2_resident": True})
@@ -539,7 +540,7 @@ def replica_rows(group, dev, steps: int, flush, cfg_kw, combos=None) -> list[dic
                      "ms_slowest": round(thr["ms_per_forward"], 4),
                      "e2e_seq_per_s": round(32 / (e2e_ms / 1e3), 1), "e2e_ms": round(e2e_ms, 3),
                      "arena_mb_per_gpu": round(sched.arena_bytes / 2 ** 20, 2),
-                     "launches": len(cm.executed_schedule)})
+                     "launches": len(cm.launched_schedule)})
         del cm, host_out, out
     return rows
 
@@ -680,7 +681,7 @@ def run_ours(args) -> int:
 
     config = dict(STATIC_CONFIG)
     config.update({
-        "launched": len(cm.executed_schedule), "generated": cm.generated_launches,
+        "launched": len(cm.launched_schedule), "generated": cm.launches_per_call,
         "arena_kib": round(sched.arena_bytes / 1024, 1),
         "l2": "flushed between steps",
         "graph_streams": cm.cfg.graph_streams, "dependent_policy": str(cm.dependent_policy),
@@ -700,7 +701,7 @@ def run_ours(args) -> int:
         "e2e": {"value": round(e2e_ms, 5), "unit": "ms", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "timing": "host wall clock, drained per step"},
         # generated kernels launched inside the timed region, all ranks together
-        "gpu_launches": cm.generated_launches * steps * world,
+        "gpu_launches": cm.launches_per_call * steps * world,
         "clocks": clocks.summary(),
         "timed_region_wall_s": round(wall, 3),
     }

@@ -95,8 +95,8 @@ def main(argv=None) -> int:
     with torch.no_grad():
         want = model.cuda()(*dev_in)
     err = float((cm(*dev_in).float() - want.float()).abs().max())
-    print(f"{args.schedule}: {len(cm.executed_schedule)} kernels launched "
-          f"({cm.generated_launches} generated), {s.elapsed_time(e) / 50:.4f} ms per call, "
+    print(f"{args.schedule}: {len(cm.launched_schedule)} kernels launched "
+          f"({cm.launches_per_call} generated), {s.elapsed_time(e) / 50:.4f} ms per call, "
           f"max |compiled - eager| = {err:.3e}")
     return 0
 
