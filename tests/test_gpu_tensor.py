@@ -1,0 +1,243 @@
+"""Tensor-core matmuls and attention, rows in shared memory, unaligned rows, and calls
+that read the caller's tensors: at the sizes where each can go wrong, against the same
+mathematics in fp64.  Bounds: ``U`` is the relative error of one rounding to the storage
+type; an fp32 sum of K products is off by at most K * 2^-23 of the sum of magnitudes (the
+tensor cores truncate where they align addends, hence not 2^-24)."""
+
+import ctypes
+
+import pytest
+import torch
+
+from mlc_compiler_b200 import Config, kir
+from mlc_compiler_b200.executor import CompiledModel
+from perf import cases
+
+pytestmark = pytest.mark.gpu
+
+U = {"float16": 2.0 ** -11, "bfloat16": 2.0 ** -8, "float32": 2.0 ** -24}
+
+
+def _dense(shape):
+    strides = [1]
+    for n in reversed(shape[1:]):
+        strides.insert(0, strides[0] * n)
+    return tuple(strides)
+
+
+class _Schedule(kir.Schedule):
+    def buffer(self, name, shape, dtype, kind):
+        self.buffers[name] = kir.BufferSpec(name, shape, dtype, kind)
+        view = kir.View(name, name, shape, _dense(shape))
+        if kind == "param":
+            self.params[name] = name
+        elif kind != "intermediate":
+            getattr(self, kind + "s").append(view)
+        return view
+
+
+def _randn(shape, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    return torch.randn(shape, generator=g).to("cuda", getattr(torch, dtype))
+
+
+def _matmul(z, m, n, k, groups, b_mn, biased, dtype):
+    """``groups`` products of one row operand, each with a bias where ``biased``."""
+    s = _Schedule("matmul")
+    lead = (z,) if z > 1 else ()
+    a = s.buffer("a", lead + (m, k), dtype, "input")
+    for i in range(groups):
+        if b_mn:
+            b = s.buffer(f"b{i}", lead + (k, n), dtype, "param")
+        else:
+            w = s.buffer(f"b{i}", lead + (n, k), dtype, "param")
+            b = kir.View(w.name, w.buffer, lead + (k, n), w.strides[:-2] + (1, k))
+        out = s.buffer(f"c{i}", lead + (m, n), dtype, "intermediate" if biased else "output")
+        s.kernels.append(kir.ExternKernel(f"mm{i}", f"aten.{'bmm' if z > 1 else 'mm'}.default", [a, b], {}, [out]))
+        if biased:
+            s.buffer(f"d{i}", (n,), dtype, "param")
+            s.buffer(f"y{i}", lead + (m, n), dtype, "output")
+            flat = [kir.Operand(x, x, dtype, kir.IndexMap((kir.Axis("idx", z * m * n, ((t, 1, 1),)),)))
+                    for x, t in ((f"c{i}", z * m * n), (f"d{i}", n), (f"y{i}", z * m * n))]
+            s.kernels.append(kir.PointwiseKernel(f"add{i}", (z * m, n), flat[:2], flat[2:],
+                                                 [("t0", kir.Call("add", (kir.Load(0), kir.Load(1))))],
+                                                 {f"y{i}": kir.Ref("t0")}, ["add"]))
+    if biased:
+        cases._plan_arena(s)
+    return s
+
+
+# every split of K, pairs of CTAs, two accumulators, one and two blocks per stage, rows
+# turned through shared memory (odd N), both orders of B, and remainders in M, N and K
+SHAPES = [(1, 1, 8, 8, 1, False, False), (1, 1, 768, 768, 1, False, True), (1, 128, 768, 768, 1, False, True),
+          (1, 127, 760, 3072, 1, False, True), (1, 129, 200, 776, 1, False, False),
+          (1, 256, 520, 768, 1, False, False), (1, 3000, 1003, 256, 1, False, False),
+          (1, 130, 333, 768, 1, False, False), (1, 300, 1003, 256, 1, False, False),
+          (1, 231, 768, 768, 3, False, True), (1, 1024, 768, 768, 3, False, True),
+          (1, 4200, 3000, 136, 1, False, False), (1, 4100, 776, 3072, 1, False, True),
+          (1, 257, 96, 1024, 1, True, False), (12, 77, 64, 136, 1, True, False), (3, 200, 136, 64, 1, False, False)]
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s[:4])) + f"g{s[4]}")
+def test_matmuls_at_the_edges_of_their_tiles(shape, dtype):
+    z, m, n, k, groups, b_mn, biased = shape
+    if dtype == "float32":                       # no alignment is asked of fp32 operands
+        n, k = n + 1, k + 1
+    s = _matmul(z, m, n, k, groups, b_mn, biased, dtype)
+    params = {o: _randn(s.buffers[o].shape, dtype, 7 + i) for i, o in enumerate(s.params)}
+    cm = CompiledModel(s, params, Config(), "cuda")
+    assert len(cm.launched_schedule) == 1 and cm.launches_per_call == 1
+    a = _randn(s.inputs[0].shape, dtype, 3)
+    got = cm(a)
+    got = [got] if groups == 1 else list(got)
+    for i in range(groups):
+        b = params[f"b{i}"].double()
+        b = b if b_mn else b.transpose(-1, -2)
+        mm, mag = a.double() @ b, a.double().abs() @ b.abs()
+        bound = (k + 2) * 2.0 ** -23 * mag + U[dtype] * mm.abs()
+        want = mm
+        if biased:
+            want = mm + params[f"d{i}"].double()
+            bound = bound + U[dtype] * (want.abs() + bound)
+        if dtype == "float16":
+            bound = bound + 2.0 ** -24           # results below the normal range
+        off = (got[i].double() - want).abs() - bound
+        assert float(off.max()) <= 0, f"output {i}: {float(off.max()):.3e} over the bound"
+    assert cm._launched._module.loaded.fault() == 0
+
+
+def test_fp32_matmul_of_values_without_finite_pieces():
+    s = _matmul(1, 130, 70, 100, 1, False, False, "float32")
+    w = _randn((70, 100), "float32", 1)
+    a = _randn((130, 100), "float32", 2)
+    a[0, 3], a[1, 4], a[129, 99], a[5] = float("inf"), float("nan"), -float("inf"), 1e38
+    w[2] = 0.0
+    got = CompiledModel(s, {"b0": w}, Config(), "cuda")(a)
+    want = a.double() @ w.double().T
+    want[want.abs() > torch.finfo(torch.float32).max] *= float("inf")
+    # a sum of products near 1e38 overflows by its order; elsewhere the patterns are equal
+    sure = torch.ones(130, dtype=torch.bool, device="cuda")
+    sure[5] = False
+    assert torch.equal(got[sure].isnan(), want[sure].isnan())
+    assert torch.equal(got[sure].isinf(), want[sure].isinf())
+    inf = want[sure].isinf()
+    assert torch.equal(got[sure][inf].sign().double(), want[sure][inf].sign())
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("groups,queries,keys", [(5, 16, 16), (3, 33, 33), (2, 77, 77), (40, 128, 128), (2, 100, 193),
+                                                 (2, 384, 384), (1, 129, 385), (2, 1, 505), (1, 512, 512)])
+def test_attention_at_the_edges_of_its_tiles(groups, queries, keys, dtype):
+    G, T, S, D, u = groups, queries, keys, 64, U[dtype]
+    s = _Schedule("attention")
+    q = s.buffer("q", (G, T, D), dtype, "input")
+    kb = s.buffer("k", (G, S, D), dtype, "input")
+    v = s.buffer("v", (G, S, D), dtype, "input")
+    s.buffer("mask", (S,), dtype, "input")
+    scores = s.buffer("scores", (G, T, S), dtype, "intermediate")
+    probs = s.buffer("probs", (G, T, S), dtype, "intermediate")
+    out = s.buffer("out", (G, T, D), dtype, "output")
+    s.kernels = [
+        kir.ExternKernel("k0", "aten.bmm.default", [q, kir.View("k", "k", (G, D, S), (S * D, 1, D))], {}, [scores]),
+        cases._softmax("k1", G * T, S, dtype, cases._row("scores", dtype, G * T, S),
+                       cases._row("mask", dtype, G * T, S, []), cases._row("probs", dtype, G * T, S), (G, T)),
+        kir.ExternKernel("k2", "aten.bmm.default", [probs, v], {}, [out])]
+    cases._plan_arena(s)
+    cm = CompiledModel(s, {}, Config(), "cuda")
+    assert len(cm.launched_schedule) == 1
+    q, k, v = (_randn(x, dtype, i) for i, x in enumerate([(G, T, D), (G, S, D), (G, S, D)]))
+    mask = torch.zeros(S, dtype=q.dtype, device="cuda")
+    mask[S - S // 3:] = torch.finfo(q.dtype).min
+    got = cm(q, k, v, mask)
+    x = q.double() @ k.double().transpose(1, 2)
+    p = torch.softmax(x / 8 + mask.double(), -1)
+    want = p @ v.double()
+    # a score rounded by u changes its exponential by u |x| / 8, numerator and sum alike;
+    # the probability and the result round once more each; fp32 work stays below 1e-5
+    bound = (2 * u * float(x.abs().max()) / 8 + u + 1e-5) * (p @ v.double().abs()) + u * want.abs()
+    if dtype == "float16":
+        bound = bound + 2.0 ** -24 * (1 + v.double().abs().sum(1, keepdim=True))     # subnormal probabilities
+    off = (got.double() - want).abs() - bound
+    assert float(off.max()) <= 0, f"{float(off.max()):.3e} over the bound"
+    assert cm._launched._module.loaded.fault() == 0
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("op", ["layernorm", "softmax"])
+@pytest.mark.parametrize("rows,cols", [(300, 257), (1, 1537), (5, 2001), (150, 8999), (3, 9001), (1, 12288),
+                                       (160, 12289), (7, 50257), (2, 65536), (149, 30001)])
+def test_long_and_unaligned_rows(rows, cols, op, dtype):
+    s = cases.rows_schedule(op, rows, cols, dtype)
+    params = {o: _randn((cols,), dtype, 5 + i) for i, o in enumerate(s.params)}
+    x = _randn((rows, cols), dtype, rows)
+    got = CompiledModel(s, params, Config(), "cuda")(x).double()
+    if op == "softmax":
+        want = torch.softmax(x.double(), -1)
+        # fp32: the exponential's argument is exact to 2^-24 of |x - max| < 16, sums to 2^-20
+        bound = (U[dtype] + 4e-6) * want + (2.0 ** -25 if dtype == "float16" else 0.0)
+    else:
+        want = torch.nn.functional.layer_norm(x.double(), (cols,), params["norm.weight"].double(),
+                                              params["norm.bias"].double(), 1e-5)
+        gain = params["norm.weight"].double().abs()
+        bound = U[dtype] * want.abs() + 1e-5 * (1 + gain) * (1 + x.double().abs())
+    off = (got - want).abs() - bound
+    assert float(off.max()) <= 0, f"{float(off.max()):.3e} over the bound"
+
+
+@pytest.mark.parametrize("what", ["one kernel", "model"])
+def test_calls_read_inputs_wherever_they_are(what):
+    """In place where the kernels can, from a copy otherwise: the same bits."""
+    if what == "one kernel":
+        s = cases.rows_schedule("softmax", 33, 96, "float16")
+    else:
+        s = cases.encoder_schedule(2, 33, 4, 1, "float16")
+    params = {o: _randn(s.buffers[b].shape, "float16", 9) * 0.05 for b, o in s.params.items()}
+    cm = CompiledModel(s, params, Config(), "cuda")
+    x = _randn(s.inputs[0].shape, "float16", 1)
+    rest = [torch.zeros(v.shape, dtype=torch.float16, device="cuda") for v in s.inputs[1:]]
+    want = cm(x, *rest).clone()
+    big = torch.zeros(x.numel() + 1, dtype=x.dtype, device="cuda")
+    big[1:] = x.flatten()
+    forms = {"another place": x.clone(), "odd start": big[1:].view(x.shape), "host": x.cpu(), "wide": x.float(),
+             "strided": torch.stack([x, x], -1)[..., 0], "pinned": x.cpu().pin_memory()}
+    for name, t in forms.items():
+        cm(torch.zeros_like(x), *rest)
+        assert torch.equal(cm(t, *rest), want), name
+        cm.replay()
+        assert torch.equal(cm(x, *rest), want), f"after {name}"
+    twice = CompiledModel(s, params, Config(cuda_graphs=False).as_scheduled(), "cuda")(want, *rest).clone()
+    out = cm(x, *rest)
+    assert torch.allclose(cm(out, *rest).float(), twice.float(), rtol=8 * U["float16"], atol=8 * U["float16"]), \
+        "output fed back"
+    with pytest.raises(Exception, match="compiled for|expected"):
+        cm(x[:1], *rest)
+    assert torch.equal(cm(x, *rest), want)
+
+
+def test_a_wait_that_runs_out_is_reported(tmp_path):
+    """The limit on every wait inside a kernel: a barrier nobody signals ends it after two
+    seconds, the module says so, and the device goes on."""
+    from mlc_compiler_b200 import build
+    from mlc_compiler_b200.emit import module
+    from mlc_compiler_b200.runtime import LoadedModule
+
+    source = module.device_header() + "\n".join(module.tensor_headers({"mm"})) + """
+extern "C" __global__ void lonely(u32* seen) {
+    __shared__ alignas(8) u64 bar;
+    __shared__ volatile u32 dead;
+    if (threadIdx.x == 0) { dead = 0; mlcb_bar_init(mlcb_smem(&bar), 1); mlcb_bar_fence_init(); }
+    __syncthreads();
+    const bool met = mlcb_bar_wait(mlcb_smem(&bar), 0, &dead);
+    if (threadIdx.x == 0) seen[0] = met ? 1u : 2u;
+}
+"""
+    build.nvcc_cubin(source, tmp_path / "lonely.cubin")
+    mod = LoadedModule((tmp_path / "lonely.cubin").read_bytes(), 0)
+    assert mod.fault() == 0
+    seen = torch.zeros(4, dtype=torch.int32, device="cuda")
+    ptr = (ctypes.c_uint64 * 1)(seen.data_ptr())
+    assert mod.lib.mlcb_launch(mod.kernel("lonely"), 1, 32, 0, ptr, 1, torch.cuda.current_stream().cuda_stream, 0) == 0
+    torch.cuda.synchronize()
+    assert int(seen[0]) == 2 and mod.fault() != 0
+    assert int((seen + 1)[0]) == 3
