@@ -264,23 +264,30 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
     L.append("    template <int NV> __device__ __forceinline__ void columns(float (&v)[NV], const Pre<NV>& pre, int row, int col, "
              "int g, int z, int lane) const {")
     L += [s for s in selects if not any(f" in{i} " in s for i in packed)]
-    if plain and W == 1 and e0.outputs[0].index.axis("col").terms == ((n, 1, 1),) and nv == 32 and z == 1:
-        # rows that start at odd addresses: 32 x 32 elements turn in shared memory so that a
-        # warp writes one row's 32 elements together
+    if plain and W == 1 and e0.outputs[0].index.axis("col").terms == ((n, 1, 1),) and nv >= 16:
+        # rows that start at odd addresses: 32 rows of nv elements turn in shared memory so
+        # that a warp writes a row's elements together (fp32: two rows' 16, where the stages
+        # were; [511, 64] x [64, 511] x 12 24.0 us a row per lane, 13.8 so)
         st = X.STORAGE_T[k.dtype]
         a = e0.outputs[0]
-        off = render_offset(a.index, {"row": "rr", "col": "(col + lane)"})
-        L.append(f"        __shared__ {st} turn[{mc.epi_warps}][32][34];")
-        L.append(f"        {st} (*t)[34] = turn[threadIdx.x / 32 - 2];")
+        off = render_offset(a.index, {"row": "rr", "col": "(col + c)"})
+        pad, rows = nv + (2 if nv == 32 else 1), 32 // nv
+        if nv == 32:
+            L.append(f"        __shared__ {st} turn[{mc.epi_warps}][32][{pad}];")
+            L.append(f"        {st} (*t)[{pad}] = turn[threadIdx.x / 32 - 2];")
+        else:
+            L.append("        extern __shared__ unsigned char smem_raw[];")
+            L.append(f"        {st} (*t)[{pad}] = reinterpret_cast<{st} (*)[{pad}]>(smem_raw) + threadIdx.x / 32 * 32;")
         L.append("#pragma unroll")
-        L.append(f"        for (int j = 0; j < 32; ++j) t[lane][j] = mlcb_elem<{st}>::put(v[j]);")
+        L.append(f"        for (int j = 0; j < {nv}; ++j) t[lane][j] = mlcb_elem<{st}>::put(v[j]);")
         L.append("        __syncwarp();")
-        L.append(f"        if (col + lane < {n}) {{")
+        L.append(f"        const int c = lane % {nv};")
+        L.append(f"        if (col + c < {n}) {{")
         L.append(f"            const int first = row - lane, count = min(32, {m} - first);")
         L.append("#pragma unroll 8")
-        L.append("            for (int i = 0; i < count; ++i) {")
-        L.append(f"                const {it} rr = first + i;")
-        L.append(f"                out0[{off}] = t[i][lane];")
+        L.append(f"            for (int i = lane / {nv}; i < count; i += {rows}) {{")
+        L.append(f"                const {it} rr = {f'({it})z * {m} + ' if z > 1 else ''}first + i;")
+        L.append(f"                out0[{off}] = t[i][c];")
         L.append("            }")
         L.append("        }")
         L.append("        __syncwarp();")
