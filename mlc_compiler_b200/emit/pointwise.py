@@ -21,6 +21,9 @@ from . import expr as X
 from .indexing import Access, check_bounds, classify, needs_64bit, pow2_ceil, render_offset
 
 
+SM_COUNT = 148
+
+
 @dataclass
 class LaunchSpec:
     """Grid and block of one launch; everything else is baked into the source.
@@ -136,6 +139,8 @@ def _emit_pointwise(k, cfg, buffers, name, stable=frozenset()) -> tuple[str, Lau
     tile = plan_tile(k, V)
     if tile is not None:
         return _emit_tiled(k, cfg, name, V, tile)
+    if ragged(k, V):
+        return _emit_ragged(k, cfg, name)
     # large streaming kernels use 256-bit accesses (two 128-bit packs per thread)
     wide = int(getattr(cfg, "wide_access_bytes", 0) or 0)
     if wide and algorithmic_bytes(k.inputs, k.outputs, numel) >= wide:
@@ -263,6 +268,100 @@ def _emit_pointwise(k, cfg, buffers, name, stable=frozenset()) -> tuple[str, Lau
     spec = LaunchSpec(grid=grid, block=block, vector=V,
                       alg_bytes=algorithmic_bytes(k.inputs, k.outputs, numel))
     return "\n".join(L), spec
+
+
+def _dense(a: kir.Operand, numel: int) -> bool:
+    """Whether the operand is element ``idx`` of a buffer."""
+    return a.via is None and a.index.base == 0 and len(a.index.axes) == 1 \
+        and tuple(map(tuple, a.index.axes[0].terms)) == ((numel, 1, 1),)
+
+
+def ragged(k: kir.PointwiseKernel, V: int) -> bool:
+    """Whether a kernel whose element count is no multiple of a pack runs on packs all the
+    same, its last few elements one per thread.  The line lies at one wave of threads:
+    below it more, shorter threads hide more latency; above it the accesses count."""
+    operands = k.inputs + k.outputs
+    smallest = min((kir.ITEMSIZE[a.dtype] for a in operands), default=4)
+    return bool(V * smallest < 16 and smallest <= 8 and k.inputs and k.numel > SM_COUNT * 1024 * V
+                and all(_dense(a, k.numel) for a in k.outputs) and any(_dense(a, k.numel) for a in k.inputs))
+
+
+def _emit_ragged(k: kir.PointwiseKernel, cfg, name: str) -> tuple[str, LaunchSpec]:
+    """Packs of V elements and, after them, a thread for each element left over.  Operands
+    that are not dense (a bias over rows of odd length) are read element by element: as two
+    packs shifted into place they took 6 % longer.  What bounds the element-wise form is its
+    2-byte accesses: bias + GELU + residual over [6075, 13507] in bf16 (492 MB, 75 us)
+    takes 280 us so and 87 in packs."""
+    numel = k.numel
+    operands = list(k.inputs) + list(k.outputs)
+    wide = int(getattr(cfg, "wide_access_bytes", 0) or 0)
+    smallest = min(kir.ITEMSIZE[a.dtype] for a in operands)
+    big = wide and algorithmic_bytes(k.inputs, k.outputs, numel) >= wide
+    V = (32 if big and all(_dense(a, numel) for a in operands) else 16) // smallest
+    packs, tail = numel // V, numel % V
+    extents = [numel] + [a.index.bounds()[1] + 1 for a in operands]
+    it = "i64" if needs_64bit(*extents) else "int"
+    block = max(32, min(1024, pow2_ceil(max(1, int(getattr(cfg, "pointwise_block", 1024))) // V)))
+    grid = (packs + tail + block - 1) // block
+    aliased = {a.buffer for a in k.inputs} & {a.buffer for a in k.outputs}
+
+    def param(a, what, i):
+        r = "" if a.buffer in aliased else " __restrict__"
+        return f"{'const ' if what == 'in' else ''}{X.STORAGE_T[a.dtype]}*{r} {what}{i}"
+
+    params = [param(a, "in", i) for i, a in enumerate(k.inputs)] + [param(a, "out", i) for i, a in enumerate(k.outputs)]
+    elide = X.store_only_casts(k.body, k.out_expr, k.outputs)
+    L = [f'extern "C" __global__ void __launch_bounds__({block}, {max(1, min(16, 512 // block))}) '
+         f'{name}({", ".join(params)}) {{',
+         f"    // pointwise {list(k.space)} = {numel} elements, {V} per thread and {tail} left over, "
+         f"{grid} x {block} threads",
+         f"    const {it} pack = ({it})blockIdx.x * {block} + threadIdx.x;",
+         "    MLCB_GRID_WAIT();"]
+
+    def element(loads, ind, put) -> None:
+        refs: dict[str, X.Val] = {}
+        for temp, e in k.body:
+            v = X.render_bind(temp, e, loads, refs, elide)
+            L.append(f"{ind}const {X.REG_T[v.dtype]} {temp} = {v.code};")
+            refs[temp] = X.Val(temp, v.dtype, v.dim)
+        for i, a in enumerate(k.outputs):
+            L.append(ind + put(i, a, store_code(X.render(k.out_expr[a.name], loads, refs), a.dtype)))
+
+    def gather(i, a, ind, index) -> str:
+        st, rt = X.STORAGE_T[a.dtype], X.REG_T[a.dtype]
+        return f"{ind}const {rt} x{i} = mlcb_load1<{st}>(in{i} + ({index}));  // {a.name}"
+
+    L.append(f"    if (pack < {packs}) {{")
+    L.append(f"        const {it} i0 = pack * {V};")
+    loads: list[X.Val] = []
+    inner: list[str] = []
+    for i, a in enumerate(k.inputs):
+        st, rt, vdt = X.STORAGE_T[a.dtype], X.REG_T[a.dtype], X.promoted_load_dtype(a.dtype)
+        if _dense(a, numel):
+            L.append(f"        {rt} v{i}[{V}]; mlcb_load<{st}, {V}>(in{i} + i0, v{i});  // {a.name}")
+            loads.append(X.Val(f"v{i}[j]", vdt))
+            continue
+        inner.append(gather(i, a, "            ", render_offset(a.index, {"idx": "(i0 + j)"})))
+        loads.append(X.Val(f"x{i}", vdt))
+    for i, a in enumerate(k.outputs):
+        L.append(f"        {X.REG_T[a.dtype]} o{i}[{V}];")
+    L.append("#pragma unroll")
+    L.append(f"        for (int j = 0; j < {V}; ++j) {{")
+    L += inner
+    element(loads, "            ", lambda i, a, code: f"o{i}[j] = {code};  // {a.name}")
+    L.append("        }")
+    for i, a in enumerate(k.outputs):
+        L.append(f"        mlcb_store<{X.STORAGE_T[a.dtype]}, {V}>(out{i} + i0, o{i});")
+    if tail:
+        L.append(f"    }} else if (pack < {packs + tail}) {{")
+        L.append(f"        const {it} idx = pack + {packs * (V - 1)};")
+        L += [gather(i, a, "        ", render_offset(a.index, {"idx": "idx"})) for i, a in enumerate(k.inputs)]
+        loads = [X.Val(f"x{i}", X.promoted_load_dtype(a.dtype)) for i, a in enumerate(k.inputs)]
+        element(loads, "        ", lambda i, a, code: f"mlcb_store1<{X.STORAGE_T[a.dtype]}>(out{i} + idx, {code});  // {a.name}")
+    L.append("    }")
+    L.append("}")
+    return "\n".join(L), LaunchSpec(grid=grid, block=block, vector=V,
+                                    alg_bytes=algorithmic_bytes(k.inputs, k.outputs, numel))
 
 
 def store_code(v: X.Val, out_dtype: str) -> str:
