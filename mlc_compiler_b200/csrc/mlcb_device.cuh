@@ -213,6 +213,41 @@ __device__ __forceinline__ void mlcb_store_at(T* __restrict__ p,
 // Column of a pack that reaches over the ends of its row: the nearest one inside.
 __device__ __forceinline__ int mlcb_within(int c, int n) { return c < 0 ? 0 : (c >= n ? n - 1 : c); }
 
+// Elements [c, c + W) of the n at p, which lies on a 16-byte boundary while c need not:
+// the two packs that hold them, shifted into place (columns outside [0, n): any element).
+// W loads of one element instead are a multiple of the requests to L1: LayerNorm of 7496
+// fp16 rows of 2001 columns takes 28.3 us with gain and bias so, 26.6 from packs.
+template <typename T, int W>
+__device__ __forceinline__ void mlcb_load_turned(const T* __restrict__ p, int c, int n,
+                                                 typename mlcb_elem<T>::reg (&dst)[W]) {
+    static_assert(W * sizeof(T) == 16, "one 16-byte pack");
+    const int by = c & (W - 1), at = c - by;
+    mlcb_pack<T, W> u[2];
+    if (at >= 0 && at + (by ? 2 * W : W) <= n) {
+        // nothing in here waits for the words: the next loads follow at once
+        mlcb_load_raw<T, W>(p + at, u[0]);
+        if (by) mlcb_load_raw<T, W>(p + at + W, u[1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2 * W; ++i) u[i / W].e[i % W] = p[mlcb_within(at + i, n)];
+    }
+    unsigned int x[8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint4 w = *reinterpret_cast<const uint4*>(u[i].w);
+        x[4 * i] = w.x; x[4 * i + 1] = w.y; x[4 * i + 2] = w.z; x[4 * i + 3] = w.w;
+    }
+    const int words = by * (int)sizeof(T) / 4, bits = by * (int)sizeof(T) % 4 * 8;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) x[i] = (words & 2) ? x[i + 2] : x[i];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) x[i] = (words & 1) ? x[i + 1] : x[i];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = sizeof(T) < 4 ? __funnelshift_r(x[i], x[i + 1], bits) : x[i];
+    *reinterpret_cast<uint4*>(u[0].w) = make_uint4(x[0], x[1], x[2], x[3]);
+    mlcb_unpack<T, W>(u[0], dst);
+}
+
 // Row id of a gathered operand, forced into the table: an id outside [0, n)
 // reads a wrong row instead of memory that is not the table's.
 __device__ __forceinline__ long long mlcb_clamp_index(long long v, long long n) {

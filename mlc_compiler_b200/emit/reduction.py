@@ -109,6 +109,16 @@ def unaligned_rows(k: kir.ReductionKernel) -> list[int] | None:
     return slots
 
 
+def turned(a, n_cols: int, V: int) -> bool:
+    """Whether a row that all rows share can be read in packs of V from any column
+    (``mlcb_load_turned``).  Two-byte elements only: [1000, 12345] fp32 LayerNorm takes 33.2
+    us element by element and 35.1 so."""
+    ax = a.index.axis("col")
+    return (V * kir.ITEMSIZE[a.dtype] == 16 and kir.ITEMSIZE[a.dtype] == 2 and a.via is None
+            and not a.index.varies_along("row") and a.index.base % V == 0
+            and ax is not None and tuple(map(tuple, ax.terms)) == ((n_cols, 1, 1),))
+
+
 def plan_geometry(n_rows: int, n_cols: int, operands, cfg, streamed: bool,
                   alg_bytes: int = 0, cut: int = 0) -> Geometry:
     """``cut``: elements per pack of rows that start anywhere in their first pack."""
@@ -325,13 +335,19 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
     # rows at any alignment: the packs a row touches, their elements outside it left out.
     # One element per lane and access otherwise: softmax over fp16 rows of 1001 / 3001
     # columns (30 and 60 MB) 23 and 134 us, 17 and 29 in packs; LayerNorm of 3001 146 and
-    # 48.  Short rows of 4 bytes, or with a gain and bias to fetch element by element,
-    # gain nothing ([14985, 1001] fp32 softmax 26 against 27 us).
+    # 48.  Rows with a gain and bias, which lie differently in every row, gain from 1536
+    # columns on ([7145, 1001] fp16 LayerNorm 11.0 us element by element, 11.3 in packs).
+    # fp32 softmax: [9000, 513] 13.5 and 9.1 us, [14985, 1001] 25.6 and 22.6; but a small launch
+    # is latency ([300, 701] 1.5 and 2.0), and 769 to 1024 columns fill 256 lanes four times
+    # ([3001, 1001] 5.2 and 5.5).
     slots = unaligned_rows(k)
     if slots is not None:
         extra = [a for a in k.inputs if a.index.varies_along("col") and not a.index.varies_along("row")]
         size = kir.ITEMSIZE[k.outputs[0].dtype]
-        if pick_vector(operands, k.n_cols) * size > 4 or k.n_cols < (1536 if size > 2 or extra else 256):
+        moved = k.n_rows * k.n_cols * size
+        if pick_vector(operands, k.n_cols) * size > 4 or k.n_cols < (1536 if extra or size > 4 else 256):
+            slots = None
+        elif size == 4 and k.n_cols < 1536 and (moved < 4 << 20 or moved < 16 << 20 and 768 < k.n_cols <= 1024):
             slots = None
     cut = 16 // kir.ITEMSIZE[k.inputs[slots[0]].dtype] if slots else 0
     geo = plan_geometry(k.n_rows, k.n_cols, operands or k.inputs + k.outputs, cfg, False,
@@ -409,6 +425,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
             acc_out[i] = ac if ac.mode == "contig" else Access("contig", 1)
 
     packed_in = {i for i, ac in acc_in.items() if ac.width > 1}
+    shifted = {i for i in acc_in if cut and i not in packed_in and turned(k.inputs[i], k.n_cols, V)}
     kept = {nm for nm in c.vec if last_use.get(nm, -1) > phase_of[nm]}
     kept_decl: dict[str, str] = {}
     # registers the row itself occupies: one row in its register type per value that
@@ -417,7 +434,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
     width = max([words(X.promoted_load_dtype(k.inputs[i].dtype)) for i in packed_in] or [1])
     live_rows = max([sum(1 for nm in kept if phase_of[nm] <= b < last_use[nm])
                      for b in range(n_phases)] + [1])
-    row_regs = NP * V * width * live_rows + 16
+    row_regs = NP * V * width * live_rows + 16 + (NP * 4 * len(slots) if cut else 0)
 
     # Stable operands read as whole packs are fetched before the wait as packed words
     # (a quarter of the registers of the widened form) and widened where first used.
@@ -469,11 +486,30 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                 code = f"v{i}[q][j]" if ac.mode == "contig" else f"v{i}[q][j / {ac.width}]"
                 vals.append(X.Val(code, X.promoted_load_dtype(a.dtype), True, True))
             else:
-                vals.append(X.Val(f"g{i}", X.promoted_load_dtype(a.dtype), True, True))
+                vals.append(X.Val(f"u{i}[j]" if i in shifted else f"g{i}", X.promoted_load_dtype(a.dtype), True, True))
         return vals
 
     loads = load_vals(True)
     vec_vals: dict[str, X.Val] = {}
+    if cut:
+        # whole packs, whatever of them belongs to the neighbouring rows: only the last pack
+        # of the buffer may not be there in full.  The words arrive while the next are asked
+        # for; widened inside a branch they were waited for one by one (LayerNorm of 7496 fp16
+        # rows of 2001 columns 26.6 us, 22.4 so)
+        first_tail = k.n_cols // V // G            # packs from lane 0 of this q on may cross the row's end
+        for i in slots:
+            st = X.STORAGE_T[k.inputs[i].dtype]
+            end = k.inputs[i].index.bounds()[1] + 1
+            c.emit(f"    mlcb_pack<{st}, {V}> w{i}[{NP}];  // {k.inputs[i].name}")
+            c.emit("#pragma unroll")
+            c.emit(f"    for (int q = 0; q < {NP}; ++q) {{")
+            c.emit(f"        const int c0 = (lane + q * {G}) * {V} - shift;")
+            c.emit(f"        if (q < {first_tail} || (c0 < {k.n_cols} && in{i}_r + c0 + {V} <= {end})) {{ mlcb_load_raw<{st}, {V}>(in{i} + in{i}_r + c0, w{i}[q]); }}")
+            c.emit(f"        else if (c0 < {k.n_cols}) {{")
+            c.emit("#pragma unroll")
+            c.emit(f"            for (int j = 0; j < {V}; ++j) if (c0 + j < {k.n_cols}) w{i}[q].e[j] = in{i}[in{i}_r + c0 + j];")
+            c.emit("        }")
+            c.emit("    }")
 
     def refs_now() -> dict[str, X.Val]:
         d = dict(c.scalars)
@@ -538,7 +574,10 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
             c.emit(f"        const int c0 = (lane + q * {G}) * {V}{' - shift' if cut else ''};")
         ind = "        "
         if geo.masked:
-            c.emit(f"        if (c0 < {k.n_cols}) {{")
+            # (packs before the row's last ones are inside it whatever the lane: no branch,
+            # so that the loads of several of them are in flight)
+            whole = f"q < {k.n_cols // V // G} || " if cut else ""
+            c.emit(f"        if ({whole}c0 < {k.n_cols}) {{")
             ind = "            "
         for i in first_loads:
             a, ac = k.inputs[i], acc_in[i]
@@ -549,12 +588,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                     c.emit(f"{ind}v{i}[q][{r_}] = mlcb_load1<{st}>(in{i} + in{i}_r + "
                            f"({_col_off(a, f'(c0 + {cc})')}));")
             elif cut:
-                c.emit(f"{ind}if (c0 >= 0 && c0 + {V} <= {k.n_cols}) {{ mlcb_load<{st}, {V}>(in{i} + in{i}_r + c0, v{i}[q]); }}")
-                c.emit(f"{ind}else {{")
-                c.emit("#pragma unroll")
-                c.emit(f"{ind}    for (int j = 0; j < {V}; ++j) v{i}[q][j] = (unsigned)(c0 + j) < {k.n_cols}u ? "
-                       f"mlcb_load1<{st}>(in{i} + in{i}_r + c0 + j) : ({X.REG_T[a.dtype]})0;")
-                c.emit(f"{ind}}}")
+                c.emit(f"{ind}mlcb_unpack<{st}, {V}>(w{i}[q], v{i}[q]);")
             elif i in raw_in:
                 c.emit(f"{ind}mlcb_unpack<{st}, {V}>(w{i}[q], v{i}[q]);")
             elif ac.width == V:
@@ -565,6 +599,12 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                            f"({_col_off(a, f'(c0 + {cc})')}), v{i}[q], {cc});")
         for i, a in out_regs:
             c.emit(f"{ind}{X.REG_T[a.dtype]} o{i}[{V}];")
+        for i in gathers:
+            if i in shifted:
+                a, st = k.inputs[i], X.STORAGE_T[k.inputs[i].dtype]
+                c.emit(f"{ind}{X.REG_T[a.dtype]} u{i}[{V}]; mlcb_load_turned<{st}, {V}>(in{i} + in{i}_r, c0, {k.n_cols}, u{i});"
+                       f"  // {a.name}")
+        gathers = [i for i in gathers if i not in shifted]
         if vbinds or red is not None or stores or gathers:
             c.emit(f"#pragma unroll")
             c.emit(f"{ind}for (int j = 0; j < {V}; ++j) {{")
@@ -590,7 +630,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                 x = X.convert(rv.code, rv.dtype, acc_dt) if rv.dtype not in kir.NARROW_FLOATS \
                     else rv.code
                 t = X.REG_T[acc_dt]
-                only = f"if ((unsigned)(c0 + j) < {k.n_cols}u) " if cut else ""
+                only = f"if ((q > 0 && q < {first_tail}) || (unsigned)(c0 + j) < {k.n_cols}u) " if cut else ""
                 c.emit(f"{in2}{only}acc_{red.name} = {_OP[red.kind]}::f<{t}>(acc_{red.name}, {x});")
             for i, a in stores:
                 v = X.render(k.out_expr[a.name], loads, local)
@@ -604,7 +644,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
         for i, a in out_regs:
             ac, st = acc_out[i], X.STORAGE_T[a.dtype]
             if cut:
-                c.emit(f"{ind}if (live && c0 >= 0 && c0 + {V} <= {k.n_cols}) {{ mlcb_store<{st}, {V}>(out{i} + out{i}_r + c0, o{i}); }}")
+                c.emit(f"{ind}if (live && ((q > 0 && q < {first_tail}) || (c0 >= 0 && c0 + {V} <= {k.n_cols}))) {{ mlcb_store<{st}, {V}>(out{i} + out{i}_r + c0, o{i}); }}")
                 c.emit(f"{ind}else if (live) {{")
                 c.emit("#pragma unroll")
                 c.emit(f"{ind}    for (int j = 0; j < {V}; ++j) if ((unsigned)(c0 + j) < {k.n_cols}u) "

@@ -111,7 +111,7 @@ def _paired(k: kir.ReductionKernel) -> bool:
 
 
 def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tuple[str, LaunchSpec]:
-    from .reduction import _Ctx, _OP, _acc_dtype, _identity, _row_stores, _signature, Geometry, plan_passes
+    from .reduction import _Ctx, _OP, _acc_dtype, _identity, _row_stores, _signature, Geometry, plan_passes, turned
 
     V, C, T, PC, N = st.V, st.C, st.T, st.PC, k.n_cols
     grid = k.n_rows * C
@@ -123,7 +123,10 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
     passes = plan_passes(k)
     reduces = k.reduces
     lead = st.slots[0]
-    occ = max(1, min(2048 // T, SMEM_MAX // max(1, st.smem), 65536 // (T * 56)))
+    # 40 registers, three CTAs of 512 threads per SM, although LayerNorm over rows of odd length
+    # spills a few then: its warps wait for loads most of the time ([1000, 12345] fp16 25.7 us
+    # with two, 23.6 with three)
+    occ = max(1, min(2048 // T, SMEM_MAX // max(1, st.smem), 65536 // (T * 40)))
     e = c.emit
     e(_signature(k, name, T, cfg, occ))
     e(f"    // staged: {k.n_rows} rows x {N} cols, {C} CTA(s) per row, {PC} packs of {V} each, {len(passes)} passes")
@@ -154,10 +157,11 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
             e(f"    const {it} in{i}_r = {off};")
     e(f"    const int shift = {'0' if st.aligned else f'(int)(in{lead}_r % {V})'};   // of the row in its first pack")
     e(f"    const int p0 = rank * {PC}, p1 = min(p0 + {PC}, (shift + {N + V - 1}) / {V});")
-    e(f"    const int whole0 = shift ? 1 : 0, whole1 = (shift + {N}) / {V};   // packs inside the row")
+    end = k.inputs[lead].index.bounds()[1] + 1
+    e(f"    const int whole1 = min((shift + {N + V - 1}) / {V}, (int)(({end} - (in{lead}_r - shift)) / {V}));   // packs the buffer has")
     e("    if (lane == 0) {")
     e(f"        for (int i = 0; i < {st.blocks}; ++i) {{")
-    e(f"            const int lo = max(whole0, p0 + i * {T}), hi = min(min(whole1, p1), p0 + (i + 1) * {T});")
+    e(f"            const int lo = p0 + i * {T}, hi = min(min(whole1, p1), lo + {T});")
     e("            const u32 bytes = hi > lo ? (hi - lo) * 16 : 0, bar = mlcb_smem(bars) + 8 * i;")
     e(f"            mlcb_bar_expect(bar, {len(st.slots)} * bytes);")
     for n, i in enumerate(st.slots):
@@ -165,20 +169,17 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
           f"in{i} + (in{i}_r - shift + lo * {V}), bytes, bar);")
     e("        }")
     e("    }")
-    if not st.aligned:
-        # packs the row shares with its neighbours: the thread that owns one fetches its elements
+    if end % V:
+        # a pack over the end of the buffer (its neighbours' elements of other packs are read
+        # along and left out later): the thread that owns it fetches its elements
+        e(f"    if (whole1 < p1 && whole1 >= p0 && (whole1 - p0) % {T} == lane) {{")
         e("#pragma unroll")
-        e("    for (int edge = 0; edge < 2; ++edge) {")
-        e("        const int p = edge ? whole1 : 0;")
-        e(f"        if (p >= p0 && p < p1 && (p - p0) % {T} == lane && (edge ? (shift + {N}) % {V} != 0 : shift != 0)) {{")
-        e("#pragma unroll")
-        e(f"            for (int j = 0; j < {V}; ++j) {{")
-        e(f"                const int col = p * {V} - shift + j;")
+        e(f"        for (int j = 0; j < {V}; ++j) {{")
+        e(f"            const int col = whole1 * {V} - shift + j;")
         for n, i in enumerate(st.slots):
             ct = X.STORAGE_T[k.inputs[i].dtype]
-            e(f"                if (col >= 0 && col < {N}) reinterpret_cast<{ct}*>(staged_raw + {n * PC * 16})"
-              f"[(p - p0) * {V} + j] = in{i}[in{i}_r + col];")
-        e("            }")
+            e(f"            if (col < {N}) reinterpret_cast<{ct}*>(staged_raw + {n * PC * 16})"
+              f"[(whole1 - p0) * {V} + j] = in{i}[in{i}_r + col];")
         e("        }")
         e("    }")
     release = dependent_release(grid, T, cfg)
@@ -196,7 +197,7 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
             loads.append(X.Val(f"mlcb_f2(v{i}[j], v{i}[j + 1])" if pairs else f"v{i}[j]", dt, True, True))
         else:
             ac = classify(a.index, "col", V)
-            acc_other[i] = st.aligned and ac.mode == "contig" and ac.width == V
+            acc_other[i] = st.aligned and ac.mode == "contig" and ac.width == V or "turned" * turned(a, N, V)
             loads.append(X.Val((f"mlcb_f2(v{i}[j], v{i}[j + 1])" if pairs else f"v{i}[j]") if acc_other[i]
                                else f"g{i}", dt, True, True))
 
@@ -247,6 +248,9 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
             if i in used and packed:
                 a = k.inputs[i]
                 ct = X.STORAGE_T[a.dtype]
+                if packed == "turned":
+                    e(f"{ind}{X.REG_T[a.dtype]} v{i}[{V}]; mlcb_load_turned<{ct}, {V}>(in{i} + in{i}_r, (int)c0, {N}, v{i});")
+                    continue
                 off = render_offset(a.index, {"col": "c0"}, skip=("row", "base"))
                 e(f"{ind}{X.REG_T[a.dtype]} v{i}[{V}]; mlcb_load<{ct}, {V}>(in{i} + in{i}_r + ({off}), v{i});")
         for i, a in stores:

@@ -165,7 +165,7 @@ def test_attention_at_the_edges_of_its_tiles(groups, queries, keys, dtype):
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("op", ["layernorm", "softmax"])
-@pytest.mark.parametrize("rows,cols", [(300, 257), (1, 1537), (5, 2001), (150, 8999), (3, 9001), (1, 12288),
+@pytest.mark.parametrize("rows,cols", [(300, 257), (9000, 513), (4099, 259), (1, 1537), (5, 2001), (150, 8999), (3, 9001), (1, 12288),
                                        (160, 12289), (7, 50257), (2, 65536), (149, 30001)])
 def test_long_and_unaligned_rows(rows, cols, op, dtype):
     s = cases.rows_schedule(op, rows, cols, dtype)
@@ -241,3 +241,19 @@ extern "C" __global__ void lonely(u32* seen) {
     torch.cuda.synchronize()
     assert int(seen[0]) == 2 and mod.fault() != 0
     assert int((seen + 1)[0]) == 3
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("rows,cols", [(777, 1003), (1, 607001), (8, 50001), (601, 1006), (3, 300000)])
+def test_pointwise_over_counts_that_are_no_packs(rows, cols, dtype):
+    s = cases.rows_schedule("gelu", rows, cols, dtype)
+    params = {o: _randn((cols,), dtype, 5) for o in s.params}
+    x, res = _randn((rows, cols), dtype, 1), _randn((rows, cols), dtype, 2)
+    got = CompiledModel(s, params, Config(), "cuda")(x, res).double()
+    h = x.double() + params["bias"].double()
+    g = torch.nn.functional.gelu(h, approximate="tanh")
+    want = res.double() + g
+    # the sum x + bias is fp32, GELU rounds once, the result once; tanh in fp32 is good to 1e-6
+    bound = U[dtype] * (g.abs() + want.abs()) + 4e-6 * (1 + h.abs())
+    off = (got - want).abs() - bound
+    assert float(off.max()) <= 0, f"{float(off.max()):.3e} over the bound"
