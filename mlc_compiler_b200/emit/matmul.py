@@ -264,10 +264,11 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
     L.append("    template <int NV> __device__ __forceinline__ void columns(float (&v)[NV], const Pre<NV>& pre, int row, int col, "
              "int g, int z, int lane) const {")
     L += [s for s in selects if not any(f" in{i} " in s for i in packed)]
-    if plain and W == 1 and e0.outputs[0].index.axis("col").terms == ((n, 1, 1),) and nv >= 16:
-        # rows that start at odd addresses: 32 rows of nv elements turn in shared memory so
+    if plain and W * kir.ITEMSIZE[k.dtype] < 16 and e0.outputs[0].index.axis("col").terms == ((n, 1, 1),) and nv >= 16:
+        # rows that lie on no 16-byte boundary: 32 rows of nv elements turn in shared memory so
         # that a warp writes a row's elements together (fp32: two rows' 16, where the stages
-        # were; [511, 64] x [64, 511] x 12 24.0 us a row per lane, 13.8 so)
+        # were; [511, 64] x [64, 511] x 12 24.0 us a row per lane, 13.8 so; [4096, 768] x
+        # [768, 50258] in fp16 808 us, 257)
         st = X.STORAGE_T[k.dtype]
         a = e0.outputs[0]
         off = render_offset(a.index, {"row": "rr", "col": "(col + c)"})
