@@ -6,10 +6,11 @@ that load a serialised schedule instead of running the reference frontend:
 
 * every buffer is a flat 1-D tensor; planned intermediates are 256-byte aligned
   slices of one ``uint8`` arena (``:119-130``), parameters are uploaded and
-  flattened once (``:52-56``), inputs are copied into fixed buffers so every
-  pointer is stable for the life of the model (``:132-156``);
-* the launch plan is resolved once (``:165-184``); extern kernels go to the ATen
-  ``.out`` overload so cuBLAS writes straight into the arena (``:369-438``);
+  flattened once (``:52-56``); inputs are read where the caller has them, or from
+  copies in fixed buffers (``:132-156``) where the kernels cannot;
+* the launch plan is resolved once (``:165-184``) for the fused form of the schedule
+  (``fuse.py``); extern kernels it leaves go to the ATen ``.out`` overload, which
+  writes straight into the arena (``:369-438``);
 * with ``cfg.cuda_graphs`` the plan is warmed up three times on a side stream,
   captured, and replayed per call (``:269-307``); outputs alias storage the next
   call overwrites (``:244-251``).
@@ -799,7 +800,8 @@ class CompiledModel(_Executable):
     # -- introspection -------------------------------------------------------------
     @property
     def executed_schedule(self) -> kir.Schedule:
-        """The schedule as launched: after producer forwarding and re-ordering."""
+        """The schedule after rewriting, kernel for kernel what ``profile_kernels`` runs; calls
+        launch ``launched_schedule``."""
         return self._exec
 
     def source(self) -> str:
