@@ -111,8 +111,8 @@ def unaligned_rows(k: kir.ReductionKernel) -> list[int] | None:
 
 def turned(a, n_cols: int, V: int) -> bool:
     """Whether a row that all rows share can be read in packs of V from any column
-    (``mlcb_load_turned``).  Two-byte elements only: [1000, 12345] fp32 LayerNorm takes 33.2
-    us element by element and 35.1 so."""
+    (``mlcb_load_turned``): the staged form's gain and bias.  Two-byte elements only: [1000,
+    12345] fp32 LayerNorm takes 33.2 us element by element and 35.1 so."""
     ax = a.index.axis("col")
     return (V * kir.ITEMSIZE[a.dtype] == 16 and kir.ITEMSIZE[a.dtype] == 2 and a.via is None
             and not a.index.varies_along("row") and a.index.base % V == 0
@@ -142,9 +142,26 @@ def plan_geometry(n_rows: int, n_cols: int, operands, cfg, streamed: bool,
         G = min(32, pow2_ceil((P + want_np - 1) // want_np))
         if (P + G - 1) // G > max_np:
             G = min(1024, pow2_ceil((P + 3) // 4))
+        size = max(kir.ITEMSIZE[a.dtype] for a in operands)
+        narrow = V <= 2 and not cut and P > 32 and size <= 4
+        many = n_rows >= 1000
+        # Rows read in ones and twos: as few lanes per row as its registers allow.  A warp per
+        # row needs no barrier, and four of them share a CTA; where a row is too long for
+        # that, four warps rather than two, whose CTAs are too small to be started fast
+        # enough (us, LayerNorm fp16 [4500, 777]: 32 lanes 4.1, 64 5.8, 128 5.0, 256 6.6;
+        # [9000, 1111]: 128 12.7, 512 34.2; softmax fp16 [1000, 2501]: 128 3.2, 1024 11.3)
+        if narrow and many and n_cols <= (512 if size == 4 else 896 if V == 1 else 1024):
+            G = 16 if V == 1 and P <= 112 and n_rows >= 32 * SM_COUNT else 32
+        elif narrow and n_cols > 256:
+            most = (20 if n_rows >= 3000 else 12 if many else 10) if size == 4 else (24 if many else 20)
+            G = 256 if size == 4 and not many and n_cols > 896 else 128
+            while G < 1024 and (P + G - 1) // G > most // V:
+                G *= 2
+        else:
+            narrow = False
         # small problems: spread each row over more lanes until the machine is
         # covered, as long as every lane still has a pack
-        while G < 1024 and G * 2 <= pow2_ceil(P) and n_rows * G < SM_COUNT * 128:
+        while not narrow and G < 1024 and G * 2 <= pow2_ceil(P) and n_rows * G < SM_COUNT * 128:
             G *= 2
     forced = int(getattr(cfg, "reduction_group", 0) or 0)
     if forced:
@@ -333,21 +350,15 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
     operands = [a for a in k.inputs if a.index.varies_along("col")] + [
         a for a in k.outputs if a.name not in k.row_outputs]
     # rows at any alignment: the packs a row touches, their elements outside it left out.
-    # One element per lane and access otherwise: softmax over fp16 rows of 1001 / 3001
-    # columns (30 and 60 MB) 23 and 134 us, 17 and 29 in packs; LayerNorm of 3001 146 and
-    # 48.  Rows with a gain and bias, which lie differently in every row, gain from 1536
-    # columns on ([7145, 1001] fp16 LayerNorm 11.0 us element by element, 11.3 in packs).
-    # fp32 softmax: [9000, 513] 13.5 and 9.1 us, [14985, 1001] 25.6 and 22.6; but a small launch
-    # is latency ([300, 701] 1.5 and 2.0), and 769 to 1024 columns fill 256 lanes four times
-    # ([3001, 1001] 5.2 and 5.5).
+    # Two-byte rows alone gain, long and many of them (softmax fp16 [9000, 1001] 9.0 us
+    # element by element, 7.8 in packs; [3001, 777] 4.2 and 3.0; [1500, 1201] 2.5 and 2.8;
+    # fp32 [9000, 1001] 13.8 and 14.7), and none with a gain and bias, which lie differently
+    # in every row (LayerNorm fp16 [9000, 1001] 11.0 and 15.0).
     slots = unaligned_rows(k)
     if slots is not None:
         extra = [a for a in k.inputs if a.index.varies_along("col") and not a.index.varies_along("row")]
         size = kir.ITEMSIZE[k.outputs[0].dtype]
-        moved = k.n_rows * k.n_cols * size
-        if pick_vector(operands, k.n_cols) * size > 4 or k.n_cols < (1536 if extra or size > 4 else 256):
-            slots = None
-        elif size == 4 and k.n_cols < 1536 and (moved < 4 << 20 or moved < 16 << 20 and 768 < k.n_cols <= 1024):
+        if size != 2 or extra or pick_vector(operands, k.n_cols) > 2 or k.n_cols < 768 or k.n_rows < 2000:
             slots = None
     cut = 16 // kir.ITEMSIZE[k.inputs[slots[0]].dtype] if slots else 0
     geo = plan_geometry(k.n_rows, k.n_cols, operands or k.inputs + k.outputs, cfg, False,
@@ -425,7 +436,6 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
             acc_out[i] = ac if ac.mode == "contig" else Access("contig", 1)
 
     packed_in = {i for i, ac in acc_in.items() if ac.width > 1}
-    shifted = {i for i in acc_in if cut and i not in packed_in and turned(k.inputs[i], k.n_cols, V)}
     kept = {nm for nm in c.vec if last_use.get(nm, -1) > phase_of[nm]}
     kept_decl: dict[str, str] = {}
     # registers the row itself occupies: one row in its register type per value that
@@ -486,7 +496,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                 code = f"v{i}[q][j]" if ac.mode == "contig" else f"v{i}[q][j / {ac.width}]"
                 vals.append(X.Val(code, X.promoted_load_dtype(a.dtype), True, True))
             else:
-                vals.append(X.Val(f"u{i}[j]" if i in shifted else f"g{i}", X.promoted_load_dtype(a.dtype), True, True))
+                vals.append(X.Val(f"g{i}", X.promoted_load_dtype(a.dtype), True, True))
         return vals
 
     loads = load_vals(True)
@@ -494,8 +504,8 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
     if cut:
         # whole packs, whatever of them belongs to the neighbouring rows: only the last pack
         # of the buffer may not be there in full.  The words arrive while the next are asked
-        # for; widened inside a branch they were waited for one by one (LayerNorm of 7496 fp16
-        # rows of 2001 columns 26.6 us, 22.4 so)
+        # for; widened inside a branch they were waited for one by one (softmax of 9000 bf16
+        # rows of 701 columns 6.2 us, 5.1 so)
         first_tail = k.n_cols // V // G            # packs from lane 0 of this q on may cross the row's end
         for i in slots:
             st = X.STORAGE_T[k.inputs[i].dtype]
@@ -599,12 +609,6 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
                            f"({_col_off(a, f'(c0 + {cc})')}), v{i}[q], {cc});")
         for i, a in out_regs:
             c.emit(f"{ind}{X.REG_T[a.dtype]} o{i}[{V}];")
-        for i in gathers:
-            if i in shifted:
-                a, st = k.inputs[i], X.STORAGE_T[k.inputs[i].dtype]
-                c.emit(f"{ind}{X.REG_T[a.dtype]} u{i}[{V}]; mlcb_load_turned<{st}, {V}>(in{i} + in{i}_r, c0, {k.n_cols}, u{i});"
-                       f"  // {a.name}")
-        gathers = [i for i in gathers if i not in shifted]
         if vbinds or red is not None or stores or gathers:
             c.emit(f"#pragma unroll")
             c.emit(f"{ind}for (int j = 0; j < {V}; ++j) {{")
@@ -614,7 +618,7 @@ def _emit_persistent(k: kir.ReductionKernel, cfg, name: str, stable=frozenset())
             for i in gathers:
                 a = k.inputs[i]
                 c.emit(f"{in2}const {X.REG_T[a.dtype]} g{i} = mlcb_load1<{X.STORAGE_T[a.dtype]}>"
-                       f"(in{i} + in{i}_r + ({_col_off(a, 'mlcb_within(col, %d)' % k.n_cols if cut else 'col')}));"
+                       f"(in{i} + in{i}_r + ({_col_off(a, 'col')}));"
                        f"  // {a.name}")
             local = dict(c.scalars)
             local.update(pre_vals)

@@ -54,10 +54,13 @@ def plan(k: kir.ReductionKernel, cfg, vector: int) -> Stage | None:
     slots = unaligned_rows(k)
     if not least or slots is None or not k.reduces:
         return None
-    # aligned rows keep the register form to where it needs a whole CTA's registers (60 MB of
-    # fp32 rows of 8000 columns: softmax 21 us against 27 here, of 10000: 39 against 28),
-    # unaligned ones to where its partial packs cost more ([7498, 4001] fp16: 28 against 25)
-    if k.n_cols < (least if k.two_pass or vector * kir.ITEMSIZE[k.outputs[0].dtype] == 16 else least // 3):
+    # rows keep the register form to where it needs a whole CTA's registers: 60 MB of aligned
+    # fp32 rows of 8000 columns, softmax 21 us against 27 here, of 10000: 39 against 28.
+    # Unaligned ones, read element by element, to two thirds of that where there are many
+    # (fp16 LayerNorm [4000, 5001] 23.3 us against 29.0, [4000, 7053] 43.7 against 37.8; [150,
+    # 7053] 3.9 against 5.4)
+    wide = k.two_pass or vector * kir.ITEMSIZE[k.outputs[0].dtype] == 16 or k.n_rows < 1000
+    if k.n_cols < (least if wide else least * 2 // 3):
         return None
     size = kir.ITEMSIZE[k.inputs[slots[0]].dtype]
     row_bytes = k.n_cols * size

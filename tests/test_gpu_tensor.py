@@ -166,7 +166,7 @@ def test_attention_at_the_edges_of_its_tiles(groups, queries, keys, dtype):
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("op", ["layernorm", "softmax"])
-@pytest.mark.parametrize("rows,cols", [(300, 257), (9000, 513), (4099, 259), (1, 1537), (5, 2001), (150, 8999), (3, 9001), (1, 12288),
+@pytest.mark.parametrize("rows,cols", [(300, 257), (9000, 513), (5000, 101), (2000, 769), (1000, 895), (999, 2501), (40, 4001), (1, 1537), (5, 2001), (150, 8999), (3, 9001), (1, 12288),
                                        (160, 12289), (7, 50257), (2, 65536), (149, 30001)])
 def test_long_and_unaligned_rows(rows, cols, op, dtype):
     s = cases.rows_schedule(op, rows, cols, dtype)
