@@ -431,7 +431,8 @@ class Config32:
 def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, peers: int | None = None) -> Config32:
     """Least estimated time, in microseconds: a 64-deep block costs 0.75 (32 columns) or 1.0
     (64), a wave 3 before and after.  Leading products get a new accumulator every four
-    blocks, as far as TMEM goes."""
+    blocks, as far as TMEM goes.  Batched products split K as others do: two encoder layers
+    of batch 3, sequence 511, 4 heads 170.3 us whole, 159.8 split."""
     kb = _ceil(k, 64)
 
     def cost(bn, split, groups):
@@ -441,7 +442,7 @@ def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, peers: int
         return waves * (_ceil(kb, split) * (0.75 if bn == 32 else 1.0) + 3.0 + exchange)
 
     widths = (64,) if b_mn else (32, 64)
-    splits = (1,) if z > 1 else tuple(s for s in (1, 2, 4, 8) if s <= kb)
+    splits = tuple(s for s in (1, 2, 4, 8) if s <= kb)
     _, split = min(((bn, s) for bn in widths for s in splits if bn % (8 * s) == 0),
                    key=lambda c: cost(*c, peers or groups))
     bn = min((bn for bn in widths if bn % (8 * split) == 0), key=lambda bn: cost(bn, split, groups))

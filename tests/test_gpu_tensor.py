@@ -76,7 +76,8 @@ SHAPES = [(1, 1, 8, 8, 1, False, False), (1, 1, 768, 768, 1, False, True), (1, 1
           (1, 700, 1002, 256, 1, False, False), (2, 130, 68, 64, 1, False, False),
           (1, 231, 768, 768, 3, False, True), (1, 1024, 768, 768, 3, False, True),
           (1, 4200, 3000, 136, 1, False, False), (1, 4100, 776, 3072, 1, False, True),
-          (1, 257, 96, 1024, 1, True, False), (12, 77, 64, 136, 1, True, False), (3, 200, 136, 64, 1, False, False)]
+          (1, 257, 96, 1024, 1, True, False), (12, 77, 64, 136, 1, True, False), (4, 130, 64, 520, 1, True, False),
+          (3, 200, 136, 64, 1, False, False)]
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
