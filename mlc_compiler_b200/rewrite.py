@@ -879,6 +879,7 @@ def sequence_first(schedule: kir.Schedule, replan: bool = True) -> kir.Schedule:
     if anchor is None or anchor[0] == 1:
         return schedule
     B, T, H = anchor
+    Dh = F // H
 
     tables: dict[str, list] = {}
 
@@ -890,26 +891,36 @@ def sequence_first(schedule: kir.Schedule, replan: bool = True) -> kir.Schedule:
         else:
             tables.setdefault(buffer, digits)
 
+    readers: dict[str, list] = {}
+    for k in kernels:
+        for b in k.reads():
+            readers.setdefault(b, []).append(k)
     for k in kernels:
         if not isinstance(k, kir.ExternKernel):
             continue
         if k.op == "aten.bmm.default":
-            for v in list(k.args[:2]) + list(k.outputs):
+            # which axis is tokens goes by its length, and where heads are as wide as the
+            # sequence is long by the role: [T, T] scores stay, of a matmul that makes them
+            # (no copy reads its result) the operands are [T, D/H] and [D/H, T], of one that
+            # takes them the second operand and the result [T, D/H]
+            takes = any(_pure_copy(x) for x in readers.get(k.outputs[0].buffer, []))
+            square = (None, True, True) if takes else (True, False, None)
+            for v, first in zip(list(k.args[:2]) + list(k.outputs), square):
                 if not (_whole_dense(schedule, v) and len(v.shape) == 3):
                     continue
                 G, M, N = v.shape
-                if G != B * H or (M == T) == (N == T):
+                if G != B * H or (M != T and N != T):
                     continue
-                order = (2, 0, 1, 3) if M == T else (3, 0, 1, 2)
+                if M != N:
+                    first = M == T
+                elif first is None or T != Dh:
+                    continue
+                order = (2, 0, 1, 3) if first else (3, 0, 1, 2)
                 propose(v.buffer, L.dense_digits((B, H, M, N), order))
     # a generated kernel's result that only feeds pure copies into moved bmm operands
     # (the bias add in front of the head copies): stored [T, B, H, J, D/H] -- J = 3 for a
     # fused q/k/v projection -- (b, h) is one stride for each of the J slices, the
     # copies become re-addressable and ``read_through_copies`` drops them
-    readers: dict[str, list] = {}
-    for k in kernels:
-        for b in k.reads():
-            readers.setdefault(b, []).append(k)
     for y in [b for b, d in tables.items() if d]:
         w = writer.get(y, [])
         if len(w) != 1 or not _pure_copy(w[0]):

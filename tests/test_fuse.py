@@ -61,3 +61,20 @@ def test_tile_choices_stay_inside_the_machine(m, n):
             assert M.choose(z, m, n, k, 1, b_mn, k % 64 == 0, 3).split == M.choose(z, m, n, k, 3, b_mn, k % 64 == 0, 3).split
             c32 = M.choose32(z, m, n, k, groups, b_mn)
             assert c32.smem() <= M.SMEM_MAX and c32.bn % (8 * c32.split) == 0 and c32.leads * c32.bn + c32.bn <= 512
+
+
+@pytest.mark.parametrize("seq", [63, 64, 65])
+def test_heads_as_wide_as_the_sequence_is_long_fuse_like_others(seq):
+    import kir_oracle as oracle
+    import torch
+
+    from perf import cases
+
+    assert len(fuse(prepare(cases.encoder_schedule(2, seq, 4, 2, "float16"), Config()), Config())) == 14
+    s = cases.encoder_schedule(2, seq, 4, 1, "float32")
+    g = torch.Generator().manual_seed(seq)
+    params = {o: torch.randn(s.buffers[b].shape, generator=g) * 0.05 for b, o in s.params.items()}
+    x = [torch.randn(v.shape, generator=g) for v in s.inputs]
+    want, _ = oracle.run_schedule(s, params, x)
+    got, _ = oracle.run_schedule(prepare(s, Config()), params, x)
+    assert torch.equal(got, want)
