@@ -25,7 +25,7 @@ import math
 from dataclasses import dataclass, field
 
 from . import kir
-from .rewrite import _NoCompose, _replanned, compose
+from .rewrite import _NoCompose, _replanned, _row_major, compose
 
 
 @dataclass
@@ -233,6 +233,18 @@ def _with_epilogue(mm: MatmulKernel, p: kir.PointwiseKernel) -> MatmulKernel | N
     return MatmulKernel(p.name, mm.a, mm.bs, mm.dtype, [e], mm.covers + [p.name], mm.peers)
 
 
+def _result(mm: MatmulKernel) -> bool:
+    """Whether the kernel's one output still is the matmul's result in its own order and
+    type, which is what a reader's index map is inverted against: so before anything is
+    folded in, and behind a copy that moves nothing."""
+    e = mm.epilogues[0]
+    if len(mm.covers) == 1:
+        return True
+    z, m, n, _ = mm.shape
+    return (not e.body and len(e.outputs) == 1 and e.out_expr == {e.outputs[0].name: kir.Load(e.slot)}
+            and e.outputs[0].dtype == mm.dtype and _row_major(e.outputs[0].index, z * m, n))
+
+
 def _same_map(m: kir.IndexMap) -> tuple:
     return tuple((a.var, a.numel, a.terms) for a in m.axes), m.base
 
@@ -369,7 +381,7 @@ def fuse(schedule: kir.Schedule, cfg) -> kir.Schedule:
                 kernels[i] = kernels[found[1]] = None
                 kernels[found[2]] = found[0]
         for i, k in enumerate(kernels):
-            if not isinstance(k, MatmulKernel) or len(k.epilogues[0].body):
+            if not isinstance(k, MatmulKernel) or not _result(k):
                 continue
             dest = k.epilogues[0].outputs[0].buffer
             users = readers.get(dest, [])

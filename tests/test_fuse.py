@@ -1,5 +1,7 @@
 """The launched form of a schedule and the tile configurations it chooses (no GPU)."""
 
+import math
+
 import pytest
 
 from mlc_compiler_b200 import Config, kir, load_schedule
@@ -78,3 +80,102 @@ def test_heads_as_wide_as_the_sequence_is_long_fuse_like_others(seq):
     want, _ = oracle.run_schedule(s, params, x)
     got, _ = oracle.run_schedule(prepare(s, Config()), params, x)
     assert torch.equal(got, want)
+
+
+def _run(kernels, buffers):
+    """The launched form on the CPU, fused matmuls by what their operands and index maps say."""
+    import kir_oracle as oracle
+    import torch
+
+    for k in kernels:
+        if not isinstance(k, MatmulKernel):
+            oracle.run_kernel(k, buffers)
+            continue
+        z, m, n, _ = k.shape
+        at = dict(row=torch.arange(z * m).unsqueeze(1), col=torch.arange(n).unsqueeze(0))
+        done = []
+        for b, e in zip(k.bs, k.epilogues):
+            acc = (k.a.as_torch(buffers[k.a.buffer]) @ b.as_torch(buffers[b.buffer])).reshape(z * m, n)
+            ops = [oracle.widen(acc if a is None else buffers[a.buffer][oracle.offsets(a.index, **at)]) for a in e.inputs]
+            temps = {}
+
+            def value(x):
+                if isinstance(x, kir.Call):
+                    return oracle.OPS[x.fn](*[value(a) for a in x.args])
+                if isinstance(x, kir.Cast):
+                    return value(x.x).to(kir.torch_dtype(x.dtype))
+                if isinstance(x, kir.Const):
+                    return oracle.constant(x, acc)
+                return ops[x.slot] if isinstance(x, kir.Load) else temps[x.name]
+            for name, x in e.body:
+                temps[name] = value(x)
+            done += [(a, value(e.out_expr[a.name])) for a in e.outputs]
+        for a, v in done:
+            dest = buffers[a.buffer]
+            where = oracle.offsets(a.index, **at).expand(z * m, n)
+            dest[where.reshape(-1)] = v.expand(z * m, n).reshape(-1).to(dest.dtype)
+
+
+def _flat(name, n, terms=None, dtype="float32"):
+    return kir.Operand(name, name, dtype, kir.IndexMap((kir.Axis("idx", n, tuple(terms or [(n, 1, 1)])),)))
+
+
+def _schedule(buffers, kernels, dtype="float32"):
+    """Dense buffers ``name: (shape, kind)`` and kernels over them."""
+    from perf import cases
+
+    s = kir.Schedule("hand")
+    for name, (shape, kind) in buffers.items():
+        s.buffers[name] = kir.BufferSpec(name, shape, dtype, kind)
+        view = kir.View(name, name, shape, tuple(math.prod(shape[i + 1:]) for i in range(len(shape))))
+        if kind == "param":
+            s.params[name] = name
+        elif kind != "intermediate":
+            getattr(s, kind + "s").append(view)
+    s.kernels = kernels
+    cases._plan_arena(s)
+    return s
+
+
+def _same_results(s, cfg=None):
+    """``s`` scheduled and as launched, on the CPU; returns the launched form."""
+    import kir_oracle as oracle
+    import torch
+
+    cfg = cfg or Config()
+    g = torch.Generator().manual_seed(1)
+    params = {o: torch.randn(s.buffers[o].shape, generator=g) for o in s.params}
+    x = [torch.randn(v.shape, generator=g) for v in s.inputs]
+    f = fuse(prepare(s, cfg), cfg)
+    _, want = oracle.run_schedule(s, params, x)
+    got = oracle.allocate(f, params, x)
+    _run(f.kernels, got)
+    for v in s.outputs:
+        assert torch.equal(v.as_torch(got[v.buffer]), v.as_torch(want[v.buffer])), v.buffer
+    return f
+
+
+def _mm(name, a, b, out, m, n, k):
+    view = lambda x, shape: kir.View(x, x, shape, (shape[1], 1))       # noqa: E731
+    return kir.ExternKernel(name, "aten.mm.default", [view(a, (m, k)), view(b, (k, n))], {}, [view(out, (m, n))])
+
+
+_ADD = kir.Call("add", (kir.Load(0), kir.Load(1)))
+
+
+@pytest.mark.parametrize("how", ["split heads", "transpose", "as it is"])
+@pytest.mark.parametrize("through", [True, False])
+def test_a_copy_behind_a_matmul_keeps_its_permutation(how, through):
+    """matmul -> copy that moves elements -> pointwise: the second reader goes by the copy's order."""
+    B, S, H, d, k = 2, 8, 4, 16, 24
+    m, n = B * S, H * d
+    N = m * n
+    terms = {"split heads": [(B, S * n, S * n), (H, S * d, d), (S, d, n), (d, 1, 1)],
+             "transpose": [(n, m, 1), (m, 1, n)], "as it is": [(N, 1, 1)]}[how]
+    s = _schedule({"a": ((m, k), "input"), "w": ((k, n), "param"), "c": ((m, n), "intermediate"),
+                   "t": ((N,), "intermediate"), "res": ((N,), "input"), "y": ((N,), "output")},
+                  [_mm("k0", "a", "w", "c", m, n, k),
+                   kir.PointwiseKernel("k1", (N,), [_flat("c", N, terms)], [_flat("t", N)], [], {"t": kir.Load(0)}, ["clone"]),
+                   kir.PointwiseKernel("k2", (N,), [_flat("t", N), _flat("res", N)], [_flat("y", N)],
+                                       [("t0", _ADD)], {"y": kir.Ref("t0")}, ["add"])])
+    _same_results(s, Config(write_through_copies=through))
