@@ -232,7 +232,7 @@ def _emit_functor(k: MatmulKernel, cfg, mc: Config, stable) -> tuple[str, list, 
     W = _pack_width(k.epilogues, n, 8 if nv == 8 else 16)
     row_expr = "row" if z == 1 else f"(z * {m} + row)"
     rn = {"float16": "mlcb_rn_f16", "bfloat16": "mlcb_rn_bf16", "float32": ""}[k.dtype]
-    plain = not e0.body and len(e0.outputs) == 1 and e0.outputs[0].dtype == k.dtype
+    plain = e0.bare and e0.outputs[0].dtype == k.dtype
 
     # operands read in packs are fetched ahead of the accumulator, as packed words
     packed = {}

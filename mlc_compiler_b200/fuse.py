@@ -40,6 +40,11 @@ class Epilogue:
     body: list = field(default_factory=list)
     out_expr: dict = field(default_factory=dict)
 
+    @property
+    def bare(self) -> bool:
+        """Whether it stores the result itself, to one place."""
+        return not self.body and len(self.outputs) == 1 and self.out_expr[self.outputs[0].name] == kir.Load(self.slot)
+
     def reads(self):
         return [a.buffer for a in self.inputs if a is not None]
 
@@ -241,8 +246,7 @@ def _result(mm: MatmulKernel) -> bool:
     if len(mm.covers) == 1:
         return True
     z, m, n, _ = mm.shape
-    return (not e.body and len(e.outputs) == 1 and e.out_expr == {e.outputs[0].name: kir.Load(e.slot)}
-            and e.outputs[0].dtype == mm.dtype and _row_major(e.outputs[0].index, z * m, n))
+    return e.bare and e.outputs[0].dtype == mm.dtype and _row_major(e.outputs[0].index, z * m, n)
 
 
 def _same_map(m: kir.IndexMap) -> tuple:

@@ -179,3 +179,21 @@ def test_a_copy_behind_a_matmul_keeps_its_permutation(how, through):
                    kir.PointwiseKernel("k2", (N,), [_flat("t", N), _flat("res", N)], [_flat("y", N)],
                                        [("t0", _ADD)], {"y": kir.Ref("t0")}, ["add"])])
     _same_results(s, Config(write_through_copies=through))
+
+
+@pytest.mark.parametrize("n", [64, 67])
+def test_an_expression_at_the_store_is_evaluated(n):
+    """A folded kernel without named steps whose stored expression does the work, at a row
+    length that leaves in packs and at one that turns in shared memory."""
+    from mlc_compiler_b200.emit import generate_module
+
+    m, k = 40, 64
+    s = _schedule({"a": ((m, k), "input"), "w": ((k, n), "param"), "c": ((m, n), "intermediate"),
+                   "res": ((m, n), "input"), "y": ((m, n), "output")},
+                  [_mm("k0", "a", "w", "c", m, n, k),
+                   kir.PointwiseKernel("k1", (m, n), [_flat("c", m * n), _flat("res", m * n)], [_flat("y", m * n)],
+                                       [], {"y": _ADD}, ["add"])])
+    f = _same_results(s)
+    assert len(f) == 1
+    body = generate_module(f, Config()).kernel_source("k1").split("void columns")[1]
+    assert " + x1" in body, body
