@@ -249,6 +249,11 @@ def _result(mm: MatmulKernel) -> bool:
     return e.bare and e.outputs[0].dtype == mm.dtype and _row_major(e.outputs[0].index, z * m, n)
 
 
+def _may_move(reads, kernels: list, i: int, j: int) -> bool:
+    """Whether what reads these buffers at position ``i`` reads the same values at ``j``."""
+    return i < j and not any(set(reads) & set(x.writes()) for x in kernels[i + 1:j] if x is not None)
+
+
 def _same_map(m: kir.IndexMap) -> tuple:
     return tuple((a.var, a.numel, a.terms) for a in m.axes), m.base
 
@@ -277,7 +282,7 @@ def _peer_key(mm: MatmulKernel) -> tuple:
 
 def _merged(kernels: list, schedule) -> list:
     """Neighbours with equal group keys become one launch at the last one's place.
-    Only kernels none of whose operands a kernel in between writes are moved."""
+    None of them reads or writes what another writes: a launch has no order inside."""
     out: list = []
     i = 0
     while i < len(kernels):
@@ -289,7 +294,8 @@ def _merged(kernels: list, schedule) -> list:
             nxt = kernels[j]
             if not isinstance(nxt, MatmulKernel) or _group_key(nxt, schedule) != key:
                 break
-            if set(nxt.reads()) & {w for g in group for w in g.writes()}:
+            if set(nxt.reads()) & {w for g in group for w in g.writes()} \
+                    or set(nxt.writes()) & {b for g in group for b in g.reads() + g.writes()}:
                 break
             group.append(nxt)
             j += 1
@@ -334,7 +340,12 @@ def _attention(i: int, kernels: list, readers: dict, finals: set, schedule) -> t
     if any(schedule.buffers[x.buffer].dtype not in kir.FLOAT_DTYPES[:3] for x in r.inputs):
         return None
     users = readers.get(out.buffer, [])
-    if out.buffer in finals or len(users) != 1:
+    if out.buffer in finals or len(users) != 1 or any(x is not r and out.buffer in x.writes()
+                                                      for x in kernels if x is not None):
+        return None
+    extra = [x.buffer for x in r.inputs if x.buffer != scores.buffer]
+    if not i < ri or not _may_move(extra, kernels, ri, users[0]) \
+            or not _may_move(a.reads(), kernels, i, users[0]):
         return None
     b = kernels[users[0]]
     if isinstance(b, MatmulKernel) and not b.epilogues[0].body and len(b.bs) == 1:
@@ -391,7 +402,8 @@ def fuse(schedule: kir.Schedule, cfg) -> kir.Schedule:
             users = readers.get(dest, [])
             if dest in finals or len(users) != 1 or not isinstance(kernels[users[0]], kir.PointwiseKernel):
                 continue
-            if any(dest in x.writes() for x in kernels if x is not None and x is not k):
+            if any(dest in x.writes() for x in kernels if x is not None and x is not k) \
+                    or not _may_move(k.reads(), kernels, i, users[0]):
                 continue
             spec = schedule.buffers[dest]
             view = next(x for x in schedule.kernels if x.name == k.covers[0]).outputs[0]

@@ -197,3 +197,43 @@ def test_an_expression_at_the_store_is_evaluated(n):
     assert len(f) == 1
     body = generate_module(f, Config()).kernel_source("k1").split("void columns")[1]
     assert " + x1" in body, body
+
+
+def test_a_matmul_stays_ahead_of_writes_to_its_operands():
+    """matmul -> an update of its operand in place -> the result's reader: not folded."""
+    m, n, k = 16, 24, 24
+    add_one = kir.Call("add", (kir.Load(0), kir.Const(1.0)))
+    s = _schedule({"x": ((m, k), "input"), "w": ((k, n), "param"), "a": ((m, k), "intermediate"),
+                   "c": ((m, n), "intermediate"), "y": ((m, n), "output"), "z": ((m, k), "output")},
+                  [kir.PointwiseKernel("k0", (m, k), [_flat("x", m * k)], [_flat("a", m * k)],
+                                       [("t0", add_one)], {"a": kir.Ref("t0")}, ["add"]),
+                   _mm("k1", "a", "w", "c", m, n, k),
+                   kir.PointwiseKernel("k2", (m, k), [_flat("a", m * k)], [_flat("a", m * k)],
+                                       [("t0", add_one)], {"a": kir.Ref("t0")}, ["add"]),
+                   kir.PointwiseKernel("k3", (m, n), [_flat("c", m * n), _flat("a", m * n)], [_flat("y", m * n)],
+                                       [("t0", _ADD)], {"y": kir.Ref("t0")}, ["add"]),
+                   kir.PointwiseKernel("k4", (m, k), [_flat("a", m * k)], [_flat("z", m * k)],
+                                       [("t0", add_one)], {"z": kir.Ref("t0")}, ["add"])])
+    _same_results(s)
+
+
+def test_matmuls_of_one_launch_do_not_write_what_another_reads():
+    """Two matmuls of the same rows, one storing over the other's residual: two launches."""
+    m, n, k = 16, 24, 24
+    fold = lambda i, c, r, y: kir.PointwiseKernel(                     # noqa: E731
+        f"p{i}", (m, n), [_flat(c, m * n), _flat(r, m * n)], [_flat(y, m * n)], [("t0", _ADD)], {y: kir.Ref("t0")}, ["add"])
+    s = _schedule({"a": ((m, k), "input"), "w0": ((k, n), "param"), "w1": ((k, n), "param"), "res": ((m, n), "input"),
+                   "c0": ((m, n), "intermediate"), "c1": ((m, n), "intermediate"), "r": ((m, n), "intermediate"),
+                   "y": ((m, n), "output"), "z": ((m, n), "output")},
+                  [kir.PointwiseKernel("k0", (m, n), [_flat("res", m * n)], [_flat("r", m * n)],
+                                       [("t0", kir.Call("neg", (kir.Load(0),)))], {"r": kir.Ref("t0")}, ["neg"]),
+                   _mm("m0", "a", "w0", "c0", m, n, k), _mm("m1", "a", "w1", "c1", m, n, k),
+                   fold(0, "c0", "r", "y"), fold(1, "c1", "res", "r"),
+                   kir.PointwiseKernel("k5", (m, n), [_flat("r", m * n)], [_flat("z", m * n)],
+                                       [("t0", kir.Call("neg", (kir.Load(0),)))], {"z": kir.Ref("t0")}, ["neg"])])
+    f = _same_results(s)
+    for k in f.kernels:
+        reads = [set(e.reads()) for e in getattr(k, "epilogues", [])]
+        writes = [set(e.writes()) for e in getattr(k, "epilogues", [])]
+        for i, r in enumerate(reads):
+            assert not any(r & w for j, w in enumerate(writes) if i != j)
