@@ -308,6 +308,26 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
     return "\n".join(L), params, names
 
 
+#: shared memory a CTA can have, and what of it the barriers and slots take
+SHARED_MAX, SHARED_FIXED = 227 * 1024, 64
+
+
+def shared_bytes(S: int, D: int) -> int:
+    """Dynamic shared memory over S keys: Q and K (the probabilities take their place) and V."""
+    s16, db = _ceil(S, 16) * 16, D // 64
+    halves = _ceil(s16, 256)
+    keys = s16 if halves == 1 else _ceil(s16 // 2, 16) * 16
+    kv = db * halves * keys * 128
+    return max(db * 16384 + kv, _ceil(S, 64) * 16384) + kv + 1024
+
+
+def fits(k: AttentionKernel, cfg) -> bool:
+    """Whether a CTA holds a tile's operands: heads of 64 always, of 128 up to 352 keys (the
+    matmuls and the row kernel stay apart beyond)."""
+    static = 2 * split_row(k, cfg)[2] * 128 * 4          # two reductions' partial row results
+    return shared_bytes(k.k.shape[2], k.q.shape[2]) + static + SHARED_FIXED <= SHARED_MAX
+
+
 def emit_attention(k: AttentionKernel, cfg, buffers, name: str | None = None, stable=frozenset()):
     name = name or k.name
     G, T, D = k.q.shape
@@ -326,8 +346,7 @@ def emit_attention(k: AttentionKernel, cfg, buffers, name: str | None = None, st
     tmaps = (operand_map(k.q, k.dtype, -2, -1, 128, db), operand_map(k.k, k.dtype, -1, -2, keys, db),
              operand_map(k.v, k.dtype, -1, -2, keys))
     conf = f"mlcb_att_cfg<{G}, {T}, {S}, {D}, {H}, {2 * lanes * 128}, {'true' if k.dtype == 'bfloat16' else 'false'}>"
-    q_bytes, kv_bytes, p_bytes = db * 16384, db * halves * keys * 128, _ceil(S, 64) * 16384
-    smem = max(q_bytes + kv_bytes, p_bytes) + kv_bytes + 1024
+    smem = shared_bytes(S, D)
     cols = next(c for c in (64, 128, 256, 512) if c >= max(halves * keys, D))
     # two CTAs per SM (64 registers) when a thread's share of the row is 32 values
     resident = 2 if S <= 128 and cols <= 256 else 1

@@ -309,7 +309,7 @@ def _merged(kernels: list, schedule) -> list:
     return out
 
 
-def _attention(i: int, kernels: list, readers: dict, finals: set, schedule) -> tuple | None:
+def _attention(i: int, kernels: list, readers: dict, finals: set, schedule, cfg) -> tuple | None:
     """The attention kernel that starts at matmul ``kernels[i]``, and the positions of the
     row kernel and the second matmul it absorbs."""
     a = kernels[i]
@@ -366,6 +366,9 @@ def _attention(i: int, kernels: list, readers: dict, finals: set, schedule) -> t
         return None
     att = AttentionKernel(b.name, q, kk, v, dest, r, slots[0], a.dtype,
                           a.covers + [r.name, b.name])
+    from .emit.attention import fits
+    if not fits(att, cfg):
+        return None
     return att, ri, users[0]
 
 
@@ -391,7 +394,7 @@ def fuse(schedule: kir.Schedule, cfg) -> kir.Schedule:
             for b in set(k.reads()):
                 readers.setdefault(b, []).append(i)
         for i, k in enumerate(kernels):
-            found = _attention(i, kernels, readers, finals, schedule) if isinstance(k, MatmulKernel) else None
+            found = _attention(i, kernels, readers, finals, schedule, cfg) if isinstance(k, MatmulKernel) else None
             if found is not None:
                 kernels[i] = kernels[found[1]] = None
                 kernels[found[2]] = found[0]

@@ -133,7 +133,8 @@ def _schedule(buffers, kernels, dtype="float32"):
         elif kind != "intermediate":
             getattr(s, kind + "s").append(view)
     s.kernels = kernels
-    cases._plan_arena(s)
+    if kernels:
+        cases._plan_arena(s)
     return s
 
 
@@ -237,3 +238,41 @@ def test_matmuls_of_one_launch_do_not_write_what_another_reads():
         writes = [set(e.writes()) for e in getattr(k, "epilogues", [])]
         for i, r in enumerate(reads):
             assert not any(r & w for j, w in enumerate(writes) if i != j)
+
+
+def _attention_schedule(G, T, S, D, dtype="float16"):
+    from perf import cases
+
+    s = _schedule({"q": ((G, T, D), "input"), "k": ((G, S, D), "input"), "v": ((G, S, D), "input"),
+                   "scores": ((G, T, S), "intermediate"), "probs": ((G, T, S), "intermediate"),
+                   "out": ((G, T, D), "output")}, [], dtype)
+    view = lambda n: kir.View(n, n, s.buffers[n].shape, tuple(math.prod(s.buffers[n].shape[i + 1:]) for i in range(3)))  # noqa: E731
+    s.kernels = [kir.ExternKernel("k0", "aten.bmm.default", [view("q"), kir.View("k", "k", (G, D, S), (S * D, 1, D))], {},
+                                  [view("scores")]),
+                 cases._softmax("k1", G * T, S, dtype, cases._row("scores", dtype, G * T, S), None,
+                                cases._row("probs", dtype, G * T, S), (G, T)),
+                 kir.ExternKernel("k2", "aten.bmm.default", [view("probs"), view("v")], {}, [view("out")])]
+    cases._plan_arena(s)
+    return s
+
+
+@pytest.mark.parametrize("heads", [64, 128])
+def test_attention_is_fused_where_its_shared_memory_exists(heads):
+    """227 KB per CTA, of which the partial row results and barriers are the static part."""
+    import re
+
+    from mlc_compiler_b200.emit import generate_module
+
+    fused = set()
+    for keys in (16, 128, 256, 304, 336, 352, 353, 368, 384, 385, 400, 448, 512):
+        f = fuse(_attention_schedule(2, 20, keys, heads), Config())
+        mod = generate_module(f, Config())
+        for k in f.kernels:
+            if isinstance(k, kir.ExternKernel):          # probabilities whose rows are no multiple of 16 bytes
+                continue
+            spec, static = mod.launch[k.name], 0
+            if isinstance(k, AttentionKernel):
+                fused.add(keys)
+                static = int(re.search(r"mlcb_att_cfg<\d+, \d+, \d+, \d+, \d+, (\d+)", mod.kernel_source(k.name))[1]) * 4 + 64
+            assert spec.smem + static <= 227 * 1024, (keys, k.name)
+    assert fused >= {16, 128, 256, 304, 336, 352} and (heads == 128 or {384, 512} <= fused)

@@ -131,7 +131,19 @@ def test_fp32_matmul_of_values_without_finite_pieces():
 @pytest.mark.parametrize("groups,queries,keys", [(5, 16, 16), (3, 33, 33), (2, 77, 77), (40, 128, 128), (2, 100, 193),
                                                  (2, 384, 384), (1, 129, 385), (2, 1, 505), (1, 512, 512)])
 def test_attention_at_the_edges_of_its_tiles(groups, queries, keys, dtype):
-    G, T, S, D, u = groups, queries, keys, 64, U[dtype]
+    _attention(groups, queries, keys, 64, dtype, 1)
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("groups,queries,keys,launches", [(3, 33, 48, 1), (2, 130, 256, 1), (2, 77, 272, 1), (1, 129, 352, 1),
+                                                          (2, 100, 360, 3), (1, 130, 512, 3)])
+def test_attention_with_wide_heads(groups, queries, keys, launches, dtype):
+    """Heads of 128: one launch while a CTA's shared memory holds them, three beyond."""
+    _attention(groups, queries, keys, 128, dtype, launches)
+
+
+def _attention(G, T, S, D, dtype, launches):
+    u = U[dtype]
     s = _Schedule("attention")
     q = s.buffer("q", (G, T, D), dtype, "input")
     kb = s.buffer("k", (G, S, D), dtype, "input")
@@ -147,7 +159,7 @@ def test_attention_at_the_edges_of_its_tiles(groups, queries, keys, dtype):
         kir.ExternKernel("k2", "aten.bmm.default", [probs, v], {}, [out])]
     cases._plan_arena(s)
     cm = CompiledModel(s, {}, Config(), "cuda")
-    assert len(cm.launched_schedule) == 1
+    assert len(cm.launched_schedule) == launches
     q, k, v = (_randn(x, dtype, i) for i, x in enumerate([(G, T, D), (G, S, D), (G, S, D)]))
     mask = torch.zeros(S, dtype=q.dtype, device="cuda")
     mask[S - S // 3:] = torch.finfo(q.dtype).min
