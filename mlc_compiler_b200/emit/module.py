@@ -45,6 +45,9 @@ class Module:
     launch: dict[str, LaunchSpec] = field(default_factory=dict)
     #: schedule kernel name -> symbol of the function that implements it
     symbol: dict[str, str] = field(default_factory=dict)
+    #: the kernels wait for the launch before them themselves: only then may one be launched
+    #: with programmatic serialisation
+    waits: bool = False
 
     def launch_table(self) -> dict[str, dict]:
         return {n: dict(s.as_dict(), symbol=self.symbol[n]) for n, s in self.launch.items()}
@@ -100,7 +103,7 @@ def generate_module(schedule, cfg, *, inline_header: bool = True, pdl: bool | No
         pdl = bool(getattr(cfg, "dependent_launch", False))   # True, "chain" or "auto"
 
     bodies: dict[str, tuple[str, list[str]]] = {}   # symbol -> (text, users)
-    mod = Module(source="")
+    mod = Module(source="", waits=pdl)
     kinds: set[str] = set()
     placeholder = "MLCB_KERNEL_NAME"
     stable = stable_buffers(schedule) if getattr(cfg, "hoist_stable_loads", True) else frozenset()

@@ -588,6 +588,12 @@ class _DirectCall:
         cfg.hoist_stable_loads = False
         return cfg
 
+    @staticmethod
+    def launch_flags(module) -> int:
+        """Programmatic where the kernel has the wait that makes it safe: consecutive calls
+        overlap at their edges."""
+        return 1 if module.waits else 0
+
     def __init__(self, owner: "_Executable"):
         self.owner = owner
         self.launch = None
@@ -610,7 +616,7 @@ class _DirectCall:
                         for b in set(k.writes())]
         self.out = owner._collect(buffers)
         self.args = (fn.kernel, fn.grid, fn.block, fn.smem, fn.ptrs, fn.nptrs)
-        fn.flags |= 1                # consecutive calls overlap at their edges
+        fn.flags |= self.launch_flags(owner._module.generated)
         self.run, self.flags = fn.lib.mlcb_launch, fn.flags
         native = native_call()
         if native is not None:

@@ -357,3 +357,20 @@ def test_float64_streamed_softmax_keeps_two_float64_passes():
     src = generate_module(wide, Config()).source
     assert "run_m" not in src and "float acc_" not in src
     assert "double acc_" in src and "exp(" in src
+
+
+@pytest.mark.parametrize("dependent", [False, True, "chain", "auto"])
+@pytest.mark.parametrize("op,rows,cols", [("layernorm", 128, 768), ("softmax", 40, 1001), ("softmax", 3001, 1001),
+                                          ("softmax", 64, 50257), ("gelu", 33, 96), ("gelu", 777, 1003)])
+def test_direct_calls_are_programmatic_only_with_the_wait(op, rows, cols, dependent):
+    """A lone kernel launched on the caller's tensors may start while what produces them
+    drains: only if it waits before it touches any of them, parameters included."""
+    from mlc_compiler_b200.executor import _DirectCall
+    from perf import cases
+
+    s = cases.rows_schedule(op, rows, cols, "float16")
+    cfg = _DirectCall.module_config(Config(dependent_launch=dependent))
+    mod = generate_module(s, cfg)
+    assert bool(_DirectCall.launch_flags(mod)) == ("#define MLCB_PDL 1" in mod.source) == bool(dependent)
+    head, _ = _before_and_after_the_wait(mod.kernel_source("k0"))
+    assert not any(x in head for x in ("mlcb_load", "mlcb_store", "mlcb_bulk_load"))
