@@ -130,7 +130,7 @@ PyObject* call_call(PyObject* self, PyObject* args, PyObject*) {
             t.sizes() != at::IntArrayRef(in.shape) || !t.is_contiguous() || t.get_device() != c->device)
             return refuse(c);
         const uint64_t p = (uint64_t)(uintptr_t)t.data_ptr();
-        if (p & 31) return refuse(c);
+        if (!p || (p & 31)) return refuse(c);          // (null: a tensor without memory of its own)
         for (const auto& w : *c->written)
             if (p < w.second && w.first < p + in.bytes) return refuse(c);
         for (int s : in.slots) ptrs[s] = p;

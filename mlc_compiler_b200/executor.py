@@ -645,7 +645,7 @@ class _DirectCall:
             if t.shape != shape or t.dtype is not dtype or not t.is_contiguous() or t.get_device() != self.index:
                 return self._refuse()
             p = t.data_ptr()
-            if p & 31:
+            if p == 0 or p & 31:         # 0: a tensor without memory of its own
                 return self._refuse()
             for lo, hi in self.written:
                 if p < hi and lo < p + nbytes:

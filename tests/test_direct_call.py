@@ -1,0 +1,66 @@
+"""The direct call's checks of its inputs, in native code and in Python: what is refused
+goes the general way (no GPU: a stand-in takes the launch)."""
+
+import ctypes
+import subprocess
+import sys
+
+import pytest
+import torch
+
+from mlc_compiler_b200.executor import _DirectCall
+from mlc_compiler_b200.runtime import native_call
+
+SHAPE, WRITTEN = (4, 8), (0x10000, 0x10040)
+
+_SETUP = """
+import ctypes, torch
+from mlc_compiler_b200.runtime import native_call
+launched = []
+LAUNCH = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32,
+                          ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64, ctypes.c_uint32)
+stand_in = LAUNCH(lambda *a: launched.append(a) or 0)
+address = ctypes.cast(stand_in, ctypes.c_void_p).value
+def make(inputs, ptrs=(0, 64)):
+    return native_call()(address, 0, 1, 32, 0, 0, 0, list(ptrs), inputs, [(0x10000, 0x10040)], "out", print)
+half = torch.empty(0, dtype=torch.float16)
+call = make([((4, 8), half, 64, (0,))])
+"""
+
+
+def native(code: str) -> str:
+    """Run ``code`` in a process of its own: at an entry without a guard a C++ exception
+    ends the process."""
+    if native_call() is None:
+        pytest.skip("_mlcb_call.so is not built")
+    r = subprocess.run([sys.executable, "-W", "ignore", "-c", _SETUP + code], capture_output=True, text=True,
+                       cwd=str(__import__("conftest").ROOT))
+    assert r.returncode == 0, r.stderr[-2000:]
+    return r.stdout.strip()
+
+
+def in_python():
+    """The Python form with the same input, on a launch that records."""
+    d = _DirectCall.__new__(_DirectCall)
+    d.native, d.index, d.launch, d.out, d.flags, d._last = None, 0, object(), "out", 0, None
+    d.specs = [(torch.Size(SHAPE), torch.float16, 64, (0,))]
+    d.written = [WRITTEN]
+    d.args = (0, 1, 32, 0, (ctypes.c_uint64 * 64)(), 2)
+    d.run = lambda *a: pytest.fail("launched")
+    return d
+
+
+def test_an_input_without_memory_is_refused():
+    got = native("""
+from torch._subclasses import FakeTensorMode
+with FakeTensorMode():
+    t = torch.empty(4, 8, dtype=torch.float16, device="cuda:0")
+print(call((t,)), call.last, launched)
+""")
+    assert got == "None None []"
+    from torch._subclasses import FakeTensorMode
+    with FakeTensorMode():
+        t = torch.empty(*SHAPE, dtype=torch.float16, device="cuda:0")
+    d = in_python()
+    d._last = (t,)
+    assert d((t,)) is None and d.last is None
