@@ -9,6 +9,7 @@
 #include <Python.h>
 
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
@@ -55,6 +56,7 @@ void call_free(PyObject* self) {
 // Call(launch, kernel, grid, block, smem, flags, device, ptrs, inputs, written, out, fail)
 // inputs: [(shape, exemplar tensor, bytes, slots)], written: [(begin, end)]
 PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
+    HANDLE_TH_ERRORS
     unsigned long long launch, kernel;
     unsigned grid, block, smem, flags;
     int device;
@@ -81,13 +83,23 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
         unsigned long long bytes;
         if (!PyArg_ParseTuple(PyList_GET_ITEM(inputs, i), "O!OKO!", &PyTuple_Type, &shape, &exemplar, &bytes,
                               &PyTuple_Type, &slots)) { Py_DECREF(c); return nullptr; }
+        if (!THPVariable_Check(exemplar)) {
+            PyErr_SetString(PyExc_TypeError, "expected a tensor that names the input's type");
+            Py_DECREF(c);
+            return nullptr;
+        }
         Input in;
         for (Py_ssize_t j = 0; j < PyTuple_GET_SIZE(shape); ++j)
             in.shape.push_back(PyLong_AsLongLong(PyTuple_GET_ITEM(shape, j)));
         in.dtype = (int)THPVariable_Unpack(exemplar).scalar_type();
         in.bytes = bytes;
-        for (Py_ssize_t j = 0; j < PyTuple_GET_SIZE(slots); ++j)
-            in.slots.push_back((int)PyLong_AsLong(PyTuple_GET_ITEM(slots, j)));
+        for (Py_ssize_t j = 0; j < PyTuple_GET_SIZE(slots); ++j) {
+            const long slot = PyLong_AsLong(PyTuple_GET_ITEM(slots, j));
+            if (!PyErr_Occurred() && (slot < 0 || (size_t)slot >= c->ptrs->size()))
+                PyErr_SetString(PyExc_ValueError, "an input's slot is none of the pointers");
+            if (PyErr_Occurred()) { Py_DECREF(c); return nullptr; }
+            in.slots.push_back((int)slot);
+        }
         c->inputs->push_back(std::move(in));
     }
     for (Py_ssize_t i = 0; i < PyList_GET_SIZE(written); ++i) {
@@ -101,6 +113,7 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
         return nullptr;
     }
     return (PyObject*)c;
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* refuse(Call* c) {
@@ -109,8 +122,26 @@ PyObject* refuse(Call* c) {
     Py_RETURN_NONE;
 }
 
+// Whether input `in` can be read where `t` has it, and where that is.  Asking a tensor that
+// stands for another one (a wrapper, a nested or batched tensor) throws: it cannot.
+bool in_place(const Call* c, const Input& in, const at::Tensor& t, uint64_t& p) {
+    try {
+        if (!t.is_cuda() || t.layout() != at::kStrided || (int)t.scalar_type() != in.dtype || t.is_neg() ||
+            t.sizes() != at::IntArrayRef(in.shape) || !t.is_contiguous() || t.get_device() != c->device)
+            return false;
+        p = (uint64_t)(uintptr_t)t.data_ptr();
+    } catch (const std::exception&) {
+        return false;
+    }
+    if (!p || (p & 31)) return false;                  // (null: a tensor without memory of its own)
+    for (const auto& w : *c->written)
+        if (p < w.second && w.first < p + in.bytes) return false;
+    return true;
+}
+
 // call(inputs tuple) -> output, or None when these inputs cannot be read in place
 PyObject* call_call(PyObject* self, PyObject* args, PyObject*) {
+    HANDLE_TH_ERRORS
     Call* c = (Call*)self;
     PyObject* tuple;
     if (PyTuple_GET_SIZE(args) != 1 || !PyTuple_Check(tuple = PyTuple_GET_ITEM(args, 0))) {
@@ -125,14 +156,8 @@ PyObject* call_call(PyObject* self, PyObject* args, PyObject*) {
         const Input& in = (*c->inputs)[i];
         PyObject* o = PyTuple_GET_ITEM(tuple, (Py_ssize_t)i);
         if (!THPVariable_Check(o)) return refuse(c);
-        const at::Tensor& t = THPVariable_Unpack(o);
-        if (!t.is_cuda() || t.layout() != at::kStrided || (int)t.scalar_type() != in.dtype || t.is_neg() ||
-            t.sizes() != at::IntArrayRef(in.shape) || !t.is_contiguous() || t.get_device() != c->device)
-            return refuse(c);
-        const uint64_t p = (uint64_t)(uintptr_t)t.data_ptr();
-        if (!p || (p & 31)) return refuse(c);          // (null: a tensor without memory of its own)
-        for (const auto& w : *c->written)
-            if (p < w.second && w.first < p + in.bytes) return refuse(c);
+        uint64_t p = 0;
+        if (!in_place(c, in, THPVariable_Unpack(o), p)) return refuse(c);
         for (int s : in.slots) ptrs[s] = p;
     }
     const uint64_t stream = (uint64_t)(uintptr_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)c->device).stream();
@@ -142,6 +167,7 @@ PyObject* call_call(PyObject* self, PyObject* args, PyObject*) {
     Py_SETREF(c->last, tuple);
     Py_INCREF(c->out);
     return c->out;
+    END_HANDLE_TH_ERRORS
 }
 
 PyObject* call_last(PyObject* self, void*) {

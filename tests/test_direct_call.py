@@ -64,3 +64,40 @@ print(call((t,)), call.last, launched)
     d = in_python()
     d._last = (t,)
     assert d((t,)) is None and d.last is None
+
+
+def test_a_tensor_that_answers_with_an_exception_is_refused():
+    """A batched tensor has no data pointer to give: asking for it throws."""
+    got = native("""
+from torch._subclasses import FakeTensorMode
+seen = []
+def one(x):
+    try:
+        x.data_ptr()
+        seen.append("has one")
+    except RuntimeError:
+        pass
+    seen.append(call((x,)))
+    return x
+with FakeTensorMode():
+    torch.func.vmap(one)(torch.empty(3, 4, 8, dtype=torch.float16, device="cuda:0"))
+print(seen, call.last, launched)
+""")
+    assert got == "[None] None []"
+
+
+def test_arguments_a_call_cannot_be_made_of_raise():
+    """Nothing a constructor or a call is given ends the process."""
+    got = native("""
+for what in (lambda: make([((4, 8), 3, 64, (0,))]), lambda: make([((4, 8), half, 64, (2,))]),
+             lambda: make([((4, 8), half, 64, (-1,))]), lambda: make([((4, "x"), half, 64, (0,))]),
+             lambda: make([], ["x"]), lambda: make([], [0] * 65), lambda: call(1), lambda: call()):
+    try:
+        what()
+        print("accepted")
+    except (TypeError, ValueError) as e:
+        print(type(e).__name__)
+print(call(()), call((1,)), call((torch.zeros(4, 8),)), launched)
+""")
+    assert got.splitlines() == ["TypeError", "ValueError", "ValueError", "TypeError", "TypeError", "ValueError",
+                                "TypeError", "TypeError", "None None None []"]
