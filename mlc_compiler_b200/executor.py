@@ -530,7 +530,7 @@ class _InPlaceInputs:
             return False
         buffer, nbytes, dtype = self.inputs[i]
         p = t.data_ptr() if t.is_cuda else 0
-        if (p == 0 or p & 31 or t.dtype is not dtype or t.get_device() != self.index or not t.is_contiguous()
+        if (p == 0 or p & 31 or t.dtype is not dtype or t.get_device() != self.index or not t.is_contiguous() or t.is_neg()
                 or any(p < hi and lo < p + nbytes for lo, hi in self.written)):
             self.wanted[buffer] = self.fixed[buffer]
             return False
@@ -642,7 +642,8 @@ class _DirectCall:
             return self._refuse()
         ptrs = self.args[4]
         for t, (shape, dtype, nbytes, slots) in zip(inputs, specs):
-            if t.shape != shape or t.dtype is not dtype or not t.is_contiguous() or t.get_device() != self.index:
+            if t.shape != shape or t.dtype is not dtype or not t.is_contiguous() or t.is_neg() \
+                    or t.get_device() != self.index:
                 return self._refuse()
             p = t.data_ptr()
             if p == 0 or p & 31:         # 0: a tensor without memory of its own

@@ -101,3 +101,21 @@ print(call(()), call((1,)), call((torch.zeros(4, 8),)), launched)
 """)
     assert got.splitlines() == ["TypeError", "ValueError", "ValueError", "TypeError", "TypeError", "ValueError",
                                 "TypeError", "TypeError", "None None None []"]
+
+
+def test_a_negated_view_is_refused():
+    """Its memory holds the values before the sign."""
+    d = in_python()
+    d.index = -1                                       # host memory stands in for the device's
+    ran = []
+    d.run = lambda *a: ran.append(a) or 0
+    x = torch.ones(SHAPE, dtype=torch.float16)
+    torch._C._cuda_getCurrentRawStream, real = (lambda index: 0), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    try:
+        assert d((x,)) == "out" and len(ran) == 1 and d.args[4][0] == x.data_ptr()
+        assert d((torch._neg_view(x),)) is None and len(ran) == 1
+    finally:
+        if real is None:
+            del torch._C._cuda_getCurrentRawStream
+        else:
+            torch._C._cuda_getCurrentRawStream = real

@@ -229,6 +229,19 @@ def test_calls_read_inputs_wherever_they_are(what):
     assert torch.equal(cm(x, *rest), want)
 
 
+@pytest.mark.parametrize("what", ["one kernel", "model"])
+def test_calls_read_negated_views_with_their_sign(what):
+    s = cases.rows_schedule("softmax", 33, 96, "float16") if what == "one kernel" else \
+        cases.encoder_schedule(2, 33, 4, 1, "float16")
+    params = {o: _randn(s.buffers[b].shape, "float16", 9) * 0.05 for b, o in s.params.items()}
+    cm = CompiledModel(s, params, Config(), "cuda")
+    x = _randn(s.inputs[0].shape, "float16", 1)
+    rest = [torch.zeros(v.shape, dtype=torch.float16, device="cuda") for v in s.inputs[1:]]
+    want = cm(-x, *rest).clone()
+    cm(x, *rest)
+    assert torch.equal(cm(torch._neg_view(x), *rest), want)
+
+
 def test_a_wait_that_runs_out_is_reported(tmp_path):
     """The limit on every wait inside a kernel: a barrier nobody signals ends it after two
     seconds, the module says so, and the device goes on."""
