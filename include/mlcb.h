@@ -123,8 +123,12 @@ int mlcb_graph_params(uint64_t exec, uint64_t node, mlcb_kernel* k, uint32_t gri
                       uint32_t smem_bytes, void* const* params);
 
 /* Non-zero when a bounded wait inside one of the module's kernels ran out (their
- * results are then unusable).  Synchronises with the device. */
+ * results are then unusable).  Waits for everything enqueued on the device, on any stream. */
 int mlcb_module_fault(mlcb_module* m, uint32_t* code);
+
+/* The host word behind it (null: no kernel of the module waits), for hosts that look at it
+ * before each call without waiting; writing 0 clears it.  Valid until the module is unloaded. */
+volatile uint32_t* mlcb_module_fault_word(mlcb_module* m);
 
 #ifdef __cplusplus
 }

@@ -36,8 +36,9 @@ struct Call {
     std::vector<Input>* inputs;
     std::vector<std::pair<uint64_t, uint64_t>>* written;
     PyObject* out;    // what a call returns
-    PyObject* fail;   // called with a launch's error code
+    PyObject* fail;   // called with a launch's error code, with 0 when `fault` is set
     PyObject* last;   // inputs of the last call, or None
+    volatile uint32_t* fault;   // set when a wait inside the kernel has run out; null: it has none
 };
 
 void call_free(PyObject* self) {
@@ -53,16 +54,16 @@ void call_free(PyObject* self) {
     Py_DECREF(t);
 }
 
-// Call(launch, kernel, grid, block, smem, flags, device, ptrs, inputs, written, out, fail)
+// Call(launch, kernel, grid, block, smem, flags, device, ptrs, inputs, written, out, fail, fault)
 // inputs: [(shape, exemplar tensor, bytes, slots)], written: [(begin, end)]
 PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
     HANDLE_TH_ERRORS
-    unsigned long long launch, kernel;
+    unsigned long long launch, kernel, fault;
     unsigned grid, block, smem, flags;
     int device;
     PyObject *ptrs, *inputs, *written, *out, *fail;
-    if (!PyArg_ParseTuple(args, "KKIIIIiO!O!O!OO", &launch, &kernel, &grid, &block, &smem, &flags, &device,
-                          &PyList_Type, &ptrs, &PyList_Type, &inputs, &PyList_Type, &written, &out, &fail))
+    if (!PyArg_ParseTuple(args, "KKIIIIiO!O!O!OOK", &launch, &kernel, &grid, &block, &smem, &flags, &device,
+                          &PyList_Type, &ptrs, &PyList_Type, &inputs, &PyList_Type, &written, &out, &fail, &fault))
         return nullptr;
     Call* c = (Call*)type->tp_alloc(type, 0);
     if (!c) return nullptr;
@@ -70,6 +71,7 @@ PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
     c->kernel = (void*)(uintptr_t)kernel;
     c->grid = grid; c->block = block; c->smem = smem; c->flags = flags;
     c->device = device;
+    c->fault = (volatile uint32_t*)(uintptr_t)fault;
     c->ptrs = new std::vector<uint64_t>();
     c->inputs = new std::vector<Input>();
     c->written = new std::vector<std::pair<uint64_t, uint64_t>>();
@@ -148,6 +150,7 @@ PyObject* call_call(PyObject* self, PyObject* args, PyObject*) {
         PyErr_SetString(PyExc_TypeError, "expected one tuple of tensors");
         return nullptr;
     }
+    if (c->fault && *c->fault) return PyObject_CallFunction(c->fail, "i", 0);
     const size_t n = c->inputs->size();
     if ((size_t)PyTuple_GET_SIZE(tuple) != n) return refuse(c);
     uint64_t ptrs[64];

@@ -60,7 +60,11 @@ struct Driver {
     CUresult (*StreamGetCaptureInfo)(CUstream, CUstreamCaptureStatus*, cuuint64_t*, CUgraph*, const CUgraphNode**,
                                      const CUgraphEdgeData**, size_t*) = nullptr;
     CUresult (*GraphExecKernelNodeSetParams)(CUgraphExec, CUgraphNode, const CUDA_KERNEL_NODE_PARAMS*) = nullptr;
-    CUresult (*MemcpyDtoH)(void*, CUdeviceptr, size_t) = nullptr;
+    CUresult (*MemcpyHtoD)(CUdeviceptr, const void*, size_t) = nullptr;
+    CUresult (*MemHostAlloc)(void**, size_t, unsigned) = nullptr;
+    CUresult (*MemHostGetDevicePointer)(CUdeviceptr*, void*, unsigned) = nullptr;
+    CUresult (*MemFreeHost)(void*) = nullptr;
+    CUresult (*CtxSynchronize)() = nullptr;
     CUresult (*TensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                      const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                      const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -100,7 +104,11 @@ void load_driver() {
     ok &= sym(d.lib, MLCB_STR(cuLaunchKernelEx), d.LaunchKernelEx);
     ok &= sym(d.lib, MLCB_STR(cuFuncSetAttribute), d.FuncSetAttribute);
     ok &= sym(d.lib, MLCB_STR(cuModuleGetGlobal), d.ModuleGetGlobal);
-    ok &= sym(d.lib, MLCB_STR(cuMemcpyDtoH), d.MemcpyDtoH);
+    ok &= sym(d.lib, MLCB_STR(cuMemcpyHtoD), d.MemcpyHtoD);
+    ok &= sym(d.lib, MLCB_STR(cuMemHostAlloc), d.MemHostAlloc);
+    ok &= sym(d.lib, MLCB_STR(cuMemHostGetDevicePointer), d.MemHostGetDevicePointer);
+    ok &= sym(d.lib, MLCB_STR(cuMemFreeHost), d.MemFreeHost);
+    ok &= sym(d.lib, MLCB_STR(cuCtxSynchronize), d.CtxSynchronize);
     ok &= sym(d.lib, MLCB_STR(cuStreamGetCaptureInfo_v3), d.StreamGetCaptureInfo);
     ok &= sym(d.lib, MLCB_STR(cuGraphExecKernelNodeSetParams), d.GraphExecKernelNodeSetParams);
     ok &= sym(d.lib, MLCB_STR(cuTensorMapEncodeTiled), d.TensorMapEncodeTiled);
@@ -209,6 +217,7 @@ struct mlcb_module {
     CUmodule mod = nullptr;
     CUcontext ctx = nullptr;
     CUdevice dev = 0;
+    volatile uint32_t* fault = nullptr;   // host word that waits which run out set; null: no waits
     std::vector<mlcb_kernel*> kernels;
 };
 
@@ -302,13 +311,32 @@ int mlcb_module_load(const void* image, size_t size, int device, mlcb_module** o
     }
     CUmodule mod = nullptr;
     r = d.ModuleLoadData(&mod, image);
+    const char* what = "cuModuleLoadData";
+    void* word = nullptr;
+    CUdeviceptr at = 0;
+    size_t n = 0;
+    if (r == CUDA_SUCCESS && d.ModuleGetGlobal(&at, &n, mod, "mlcb_fault") == CUDA_SUCCESS) {
+        CUdeviceptr seen = 0;
+        what = "the fault word";
+        r = d.MemHostAlloc(&word, sizeof(uint32_t), CU_MEMHOSTALLOC_PORTABLE | CU_MEMHOSTALLOC_DEVICEMAP);
+        if (r == CUDA_SUCCESS) {
+            *(volatile uint32_t*)word = 0;
+            r = d.MemHostGetDevicePointer(&seen, word, 0);
+        }
+        if (r == CUDA_SUCCESS) r = d.MemcpyHtoD(at, &seen, sizeof seen);
+        if (r != CUDA_SUCCESS) {
+            if (word) d.MemFreeHost(word);
+            d.ModuleUnload(mod);
+        }
+    }
     CUcontext popped = nullptr;
     d.CtxPopCurrent(&popped);
     if (r != CUDA_SUCCESS) {
         d.PrimaryCtxRelease(dev);
-        return cu_fail(r, "cuModuleLoadData");
+        return cu_fail(r, what);
     }
     mlcb_module* m = new mlcb_module();
+    m->fault = (volatile uint32_t*)word;
     m->mod = mod;
     m->ctx = ctx;
     m->dev = dev;
@@ -322,6 +350,7 @@ int mlcb_module_unload(mlcb_module* m) {
     if (g_drv.ok && m->mod) {
         g_drv.CtxPushCurrent(m->ctx);
         CUresult r = g_drv.ModuleUnload(m->mod);
+        if (m->fault) g_drv.MemFreeHost((void*)m->fault);
         CUcontext popped = nullptr;
         g_drv.CtxPopCurrent(&popped);
         g_drv.PrimaryCtxRelease(m->dev);
@@ -464,13 +493,13 @@ int mlcb_module_fault(mlcb_module* m, uint32_t* code) {
     *code = 0;
     if (int e = need_driver()) return e;
     CtxGuard in_module_context(m->ctx);
-    CUdeviceptr p = 0;
-    size_t n = 0;
-    if (g_drv.ModuleGetGlobal(&p, &n, m->mod, "mlcb_fault") != CUDA_SUCCESS) return 0;  // no waits in it
-    CUresult r = g_drv.MemcpyDtoH(code, p, sizeof *code);
-    if (r != CUDA_SUCCESS) return cu_fail(r, "cuMemcpyDtoH(mlcb_fault)");
+    CUresult r = g_drv.CtxSynchronize();
+    if (r != CUDA_SUCCESS) return cu_fail(r, "cuCtxSynchronize");
+    if (m->fault) *code = *m->fault;
     return 0;
 }
+
+volatile uint32_t* mlcb_module_fault_word(mlcb_module* m) { return m ? m->fault : nullptr; }
 
 int mlcb_tensor_map(void* map, uint64_t address, int bf16, const uint64_t* dims,
                     const uint64_t* strides, const uint32_t* box) {

@@ -29,7 +29,15 @@ __device__ __forceinline__ bool mlcb_elect() {
 // read; a dead CTA skips every later wait and issues no further copies, drains,
 // frees its TMEM and exits.
 // ---------------------------------------------------------------------------
-__device__ unsigned int mlcb_fault = 0;
+// The word is host memory (the loader puts its address here): a host sees a wait that ran
+// out without a copy of its own, at its next call.
+__device__ unsigned int* mlcb_fault = nullptr;
+__device__ __forceinline__ void mlcb_report() {
+    if (mlcb_fault) {
+        *reinterpret_cast<volatile unsigned int*>(mlcb_fault) = 1u;
+        __threadfence_system();
+    }
+}
 
 __device__ __forceinline__ u64 mlcb_now_ns() { u64 t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
 __device__ __forceinline__ void mlcb_bar_init(u32 bar, u32 count) {
@@ -60,7 +68,7 @@ __device__ __noinline__ bool mlcb_bar_wait_slow(u32 bar, u32 parity, volatile u3
         if (*dead) return false;
         if (mlcb_now_ns() - t0 > 2000000000ull) {
             *dead = 1;
-            atomicExch(&mlcb_fault, 1u);
+            mlcb_report();
             return false;
         }
     }

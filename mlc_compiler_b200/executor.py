@@ -142,6 +142,8 @@ class _Executable:
         self._live = self._exec.live_buffers()
         self.params = params
         self._runtime: CudaRuntime | None = None
+        #: host word that a kernel's bounded wait sets when it runs out (None: no waits)
+        self._fault = None
         self._arena: torch.Tensor | None = None
         self._resident: dict[str, torch.Tensor] | None = None
         self._plan: list | None = None
@@ -161,6 +163,7 @@ class _Executable:
             if self._direct is not None and cfg.cuda_graphs:
                 cfg = _DirectCall.module_config(cfg)
             self._runtime = CudaRuntime(self._exec, cfg, self.device)
+            self._fault = self._runtime.loaded.word
         return self._runtime
 
     # -- allocation ------------------------------------------------------------
@@ -363,6 +366,8 @@ class _Executable:
             # one shape check and one copy per input, then the replay
             self._input_views = [dst.view(tuple(v.shape))
                                  for dst, v in zip(self._static_inputs, self.schedule.inputs)]
+        if self._fault is not None and self._fault.value:
+            self._module.loaded.check()
         views = self._input_views
         if len(inputs) != len(views):
             self._check_inputs(inputs)
@@ -395,8 +400,7 @@ class _Executable:
             for _ in range(3):
                 self.run_kernels(buffers)
         torch.cuda.current_stream(self.device).wait_stream(side)
-        if self._module.loaded.fault():
-            raise BackendError("a bounded wait inside a kernel ran out during warm-up")
+        self._settled()
         # the graph is kept: its nodes are how later calls name their inputs
         g = torch.cuda.CUDAGraph(keep_graph=True)
         in_place = _InPlaceInputs(self, buffers)
@@ -436,7 +440,15 @@ class _Executable:
         g, self._plan, self._bound, self._per_kernel = candidates[self.dependent_policy]
         return g
 
+    def _settled(self) -> None:
+        """Wait for what is enqueued and raise if one of its waits ran out."""
+        if self._fault is not None:
+            self._module.loaded.fault()
+            self._module.loaded.check()
+
     def _forward(self, inputs):
+        if self._fault is not None and self._fault.value:
+            self._module.loaded.check()
         if self._exec.plan.mode == "eager":
             return self._collect(self._run_eager(inputs))
         buffers = self._resident_buffers(inputs)
@@ -460,11 +472,15 @@ class _Executable:
             return
         if self._graph_replay is None:
             raise ExecutionError("nothing captured yet: call the model once")
+        if self._fault is not None and self._fault.value:
+            self._module.loaded.check()
         self._graph_replay.replay()
 
 
 
-def _launch_failed(lib, name: str, code: int):
+def _launch_failed(lib, name: str, loaded, code: int):
+    if code == 0:                # not the launch: a wait of an earlier one ran out
+        loaded.check()
     raise BackendError(f"launch of {name} failed with code {code}: "
                        f"{lib.mlcb_last_error().decode(errors='replace')}")
 
@@ -615,6 +631,7 @@ class _DirectCall:
         self.written = [(buffers[b].data_ptr(), buffers[b].data_ptr() + owner._exec.buffers[b].nbytes)
                         for b in set(k.writes())]
         self.out = owner._collect(buffers)
+        self.fault = owner._fault
         self.args = (fn.kernel, fn.grid, fn.block, fn.smem, fn.ptrs, fn.nptrs)
         fn.flags |= self.launch_flags(owner._module.generated)
         self.run, self.flags = fn.lib.mlcb_launch, fn.flags
@@ -625,11 +642,12 @@ class _DirectCall:
             self.native = native(address, fn.kernel.value, fn.grid, fn.block, fn.smem, fn.flags, owner.device.index,
                                  list(fn.ptrs)[:fn.nptrs],
                                  [(tuple(s), d, n, at) for (s, _, n, at), d in zip(self.specs, dtypes)],
-                                 self.written, self.out, functools.partial(_launch_failed, fn.lib, fn.name))
+                                 self.written, self.out,
+                                 functools.partial(_launch_failed, fn.lib, fn.name, owner._module.loaded),
+                                 0 if owner._fault is None else ctypes.addressof(owner._fault))
         if fn.smem:                  # bounded waits inside: prove them once, as a capture's warm-up does
             fn[fn.grid]()
-            if owner._module.loaded.fault():
-                raise BackendError("a bounded wait inside a kernel ran out during warm-up")
+            owner._settled()
         self.index = owner.device.index
 
     def __call__(self, inputs):
@@ -637,6 +655,8 @@ class _DirectCall:
             self._bind(inputs)
         if self.native is not None:
             return self.native(inputs)
+        if self.fault is not None and self.fault.value:
+            self.owner._module.loaded.check()
         specs = self.specs
         if len(inputs) != len(specs):
             return self._refuse()
@@ -656,7 +676,7 @@ class _DirectCall:
         self._last = inputs
         code = self.run(*self.args, torch._C._cuda_getCurrentRawStream(self.index), self.flags)
         if code != 0:
-            _launch_failed(self.launch.lib, self.launch.name, code)
+            _launch_failed(self.launch.lib, self.launch.name, self.owner._module.loaded, code)
         return self.out
 
     def _refuse(self):
@@ -761,6 +781,18 @@ class CompiledModel(_Executable):
             with torch.cuda.device(self.device):
                 return self.replay()
         (self._launched or self)._replay()
+
+    def check(self) -> None:
+        """Wait for the device and raise ``BackendError`` if a wait inside a kernel ran out
+        since the last report.  Every wait between the warps and CTAs of a kernel is bounded
+        (two seconds); what such a kernel leaves is unusable.  Calls report it by themselves,
+        but only what has finished when they begin: whoever reads the last result of a series
+        synchronises, and can do so here."""
+        with torch.cuda.device(self.device):
+            torch.cuda.synchronize(self.device)
+            for form in (self, self._launched):
+                if form is not None:
+                    form._settled()
 
     @property
     def launched_schedule(self) -> kir.Schedule:

@@ -64,6 +64,7 @@ _SIGNATURES = {
                                         ctypes.c_uint64, ctypes.POINTER(ctypes.c_int)]),
     "mlcb_kernel_shared": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint32]),
     "mlcb_module_fault": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint32)]),
+    "mlcb_module_fault_word": (ctypes.c_void_p, [ctypes.c_void_p]),
     "mlcb_capture_node": (ctypes.c_int, [ctypes.c_uint64, ctypes.POINTER(ctypes.c_uint64)]),
     "mlcb_graph_params": (ctypes.c_int, [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_uint32,
                                          ctypes.c_uint32, ctypes.c_uint32, ctypes.POINTER(ctypes.c_void_p)]),
@@ -205,6 +206,9 @@ class LoadedModule:
                                                    ctypes.byref(h)), "mlcb_module_load")
         self.handle = h
         self._kernels: dict[str, ctypes.c_void_p] = {}
+        word = self.lib.mlcb_module_fault_word(h)
+        #: host word that a bounded wait which ran out sets, None where no kernel waits
+        self.word = ctypes.c_uint32.from_address(word) if word else None
 
     def kernel(self, symbol: str) -> ctypes.c_void_p:
         k = self._kernels.get(symbol)
@@ -222,14 +226,24 @@ class LoadedModule:
                "mlcb_kernel_info")
         return {"registers": regs.value, "static_smem": smem.value, "max_threads": mt.value}
 
+    def check(self) -> None:
+        """Raise, once, if a wait has been seen to run out: what has finished since the last
+        check, nothing is waited for."""
+        if self.word is not None and self.word.value:
+            self.word.value = 0
+            raise BackendError("a bounded wait inside a kernel ran out: results since the last "
+                               "check are unusable")
+
     def fault(self) -> int:
-        """Non-zero when a bounded wait in one of the kernels ran out."""
+        """Non-zero when a bounded wait in one of the kernels ran out, everything enqueued on
+        the device included."""
         code = ctypes.c_uint32()
         _check(self.lib, self.lib.mlcb_module_fault(self.handle, ctypes.byref(code)), "mlcb_module_fault")
         return code.value
 
     def close(self) -> None:
         if self.handle is not None and self.handle.value:
+            self.word = None
             self.lib.mlcb_module_unload(self.handle)
             self.handle = None
 

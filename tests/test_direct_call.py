@@ -21,8 +21,12 @@ LAUNCH = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_uint32, ctypes
                           ctypes.c_void_p, ctypes.c_int, ctypes.c_uint64, ctypes.c_uint32)
 stand_in = LAUNCH(lambda *a: launched.append(a) or 0)
 address = ctypes.cast(stand_in, ctypes.c_void_p).value
+word = ctypes.c_uint32(0)
+def fail(code):
+    raise RuntimeError(f"code {code}")
 def make(inputs, ptrs=(0, 64)):
-    return native_call()(address, 0, 1, 32, 0, 0, 0, list(ptrs), inputs, [(0x10000, 0x10040)], "out", print)
+    return native_call()(address, 0, 1, 32, 0, 0, 0, list(ptrs), inputs, [(0x10000, 0x10040)], "out", fail,
+                         ctypes.addressof(word))
 half = torch.empty(0, dtype=torch.float16)
 call = make([((4, 8), half, 64, (0,))])
 """
@@ -44,7 +48,7 @@ def in_python():
     d = _DirectCall.__new__(_DirectCall)
     d.native, d.index, d.launch, d.out, d.flags, d._last = None, 0, object(), "out", 0, None
     d.specs = [(torch.Size(SHAPE), torch.float16, 64, (0,))]
-    d.written = [WRITTEN]
+    d.written, d.fault = [WRITTEN], None
     d.args = (0, 1, 32, 0, (ctypes.c_uint64 * 64)(), 2)
     d.run = lambda *a: pytest.fail("launched")
     return d
@@ -119,3 +123,23 @@ def test_a_negated_view_is_refused():
             del torch._C._cuda_getCurrentRawStream
         else:
             torch._C._cuda_getCurrentRawStream = real
+
+
+def test_a_wait_that_ran_out_is_reported_at_the_next_call():
+    got = native("""
+print(call((torch.zeros(4, 8),)))
+word.value = 1
+try:
+    call((torch.zeros(4, 8),))
+    print("not reported")
+except RuntimeError as e:
+    print(e)
+""")
+    assert got.splitlines() == ["None", "code 0"]
+    from mlc_compiler_b200.runtime import BackendError, LoadedModule
+
+    loaded = LoadedModule.__new__(LoadedModule)
+    loaded.handle, loaded.word = None, ctypes.c_uint32(1)
+    with pytest.raises(BackendError, match="ran out"):
+        loaded.check()
+    loaded.check()                                     # reported once

@@ -242,9 +242,8 @@ def test_calls_read_negated_views_with_their_sign(what):
     assert torch.equal(cm(torch._neg_view(x), *rest), want)
 
 
-def test_a_wait_that_runs_out_is_reported(tmp_path):
-    """The limit on every wait inside a kernel: a barrier nobody signals ends it after two
-    seconds, the module says so, and the device goes on."""
+def _lonely(tmp_path):
+    """A module whose one kernel waits for a barrier that nobody signals."""
     from mlc_compiler_b200 import build
     from mlc_compiler_b200.emit import module
     from mlc_compiler_b200.runtime import LoadedModule
@@ -260,7 +259,13 @@ extern "C" __global__ void lonely(u32* seen) {
 }
 """
     build.nvcc_cubin(source, tmp_path / "lonely.cubin")
-    mod = LoadedModule((tmp_path / "lonely.cubin").read_bytes(), 0)
+    return LoadedModule((tmp_path / "lonely.cubin").read_bytes(), 0)
+
+
+def test_a_wait_that_runs_out_is_reported(tmp_path):
+    """The limit on every wait inside a kernel: a barrier nobody signals ends it after two
+    seconds, the module says so, and the device goes on."""
+    mod = _lonely(tmp_path)
     assert mod.fault() == 0
     seen = torch.zeros(4, dtype=torch.int32, device="cuda")
     ptr = (ctypes.c_uint64 * 1)(seen.data_ptr())
@@ -268,6 +273,44 @@ extern "C" __global__ void lonely(u32* seen) {
     torch.cuda.synchronize()
     assert int(seen[0]) == 2 and mod.fault() != 0
     assert int((seen + 1)[0]) == 3
+
+
+def test_a_wait_that_runs_out_on_a_side_stream_is_seen(tmp_path):
+    """The report covers what any stream has enqueued, and is made once."""
+    from mlc_compiler_b200.runtime import BackendError
+
+    mod = _lonely(tmp_path)
+    seen = torch.zeros(4, dtype=torch.int32, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    ptr = (ctypes.c_uint64 * 1)(seen.data_ptr())
+    assert mod.lib.mlcb_launch(mod.kernel("lonely"), 1, 32, 0, ptr, 1, side.cuda_stream, 0) == 0
+    assert mod.fault() != 0
+    with pytest.raises(BackendError, match="ran out"):
+        mod.check()
+    mod.check()
+    assert mod.fault() == 0 and int(seen[0]) == 2
+
+
+@pytest.mark.parametrize("what", ["one kernel", "model"])
+def test_calls_report_a_wait_that_ran_out(what):
+    """Whatever comes next says it, once: a call, a replay, a check."""
+    from mlc_compiler_b200.runtime import BackendError
+
+    s = cases.rows_schedule("softmax", 3, 50257, "float16") if what == "one kernel" else \
+        cases.encoder_schedule(2, 33, 4, 1, "float16")
+    params = {o: _randn(s.buffers[b].shape, "float16", 9) * 0.05 for b, o in s.params.items()}
+    cm = CompiledModel(s, params, Config(), "cuda")
+    x = [_randn(v.shape, "float16", 1) if i == 0 else torch.zeros(v.shape, dtype=torch.float16, device="cuda")
+         for i, v in enumerate(s.inputs)]
+    want = cm(*x).clone()
+    word = (cm._launched or cm)._module.loaded.word
+    for report in (lambda: cm(*x), cm.replay, cm.check, lambda: cm.forward(*x)):
+        word.value = 1                                 # as a kernel would
+        with pytest.raises(BackendError, match="ran out"):
+            report()
+        assert torch.equal(cm(*x), want)
+        report()
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
