@@ -143,6 +143,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
         if (pair == 0) {
             const bool elected = mlcb_elect();
             constexpr u32 idesc = mlcb_idesc(128 * C::CG, C::BN, C::BF16, C::B_MN);
+            MLCB_GRID_WAIT();                 // the limit of the waits below is this launch's own time
             int s = 0, acc = 0;
             u32 phase = 0, acc_phase = 1;
             bool alive = true;

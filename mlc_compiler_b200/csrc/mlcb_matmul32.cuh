@@ -105,6 +105,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     if (warp == C::CW) {
         const bool elected = mlcb_elect();
         if (elected) mlcb_prefetch_next(next);
+        MLCB_GRID_WAIT();                     // the limit of the waits below is this launch's own time
         constexpr u32 one = mlcb_idesc(128, C::BN, true, C::B_MN), two = mlcb_idesc(128, 2 * C::BN, true, C::B_MN),
                       three = mlcb_idesc(128, 3 * C::BN, true, C::B_MN);
         int s = 0;

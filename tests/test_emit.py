@@ -374,3 +374,20 @@ def test_direct_calls_are_programmatic_only_with_the_wait(op, rows, cols, depend
     assert bool(_DirectCall.launch_flags(mod)) == ("#define MLCB_PDL 1" in mod.source) == bool(dependent)
     head, _ = _before_and_after_the_wait(mod.kernel_source("k0"))
     assert not any(x in head for x in ("mlcb_load", "mlcb_store", "mlcb_bulk_load"))
+
+
+def test_waits_with_a_limit_come_behind_the_grid_wait():
+    """Their clock is the launch's own time: a warp that reaches a bounded wait has waited for
+    the launch before this one first, or it would count how long that one takes."""
+    from mlc_compiler_b200.emit.module import CSRC
+
+    for f, roles in (("mlcb_matmul.cuh", 3), ("mlcb_matmul32.cuh", 2), ("mlcb_attention.cuh", 1)):
+        text = (CSRC / f).read_text().split("__device__ __forceinline__ void mlcb_", 1)[1]
+        # the roles' code in order: each waits for the grid before its first bounded wait
+        parts = re.split(r"MLCB_GRID_WAIT\(\);", text)
+        assert len(parts) == roles + 1, f
+        assert "mlcb_bar_wait" not in parts[0] and "mlcb_warp_wait" not in parts[0]
+        for part in parts[1:-1]:
+            role = re.split(r"\} else (?:if \(warp == \S+\) )?\{", part)
+            assert len(role) >= 2, f
+            assert not any(re.search(r"mlcb_(bar|warp)_wait\(", r) for r in role[1:]), f
