@@ -70,9 +70,9 @@ __device__ __forceinline__ void mlcb_attention(const mlcb_tmap* tq, const mlcb_t
                     mlcb_tma_load(sv + (j * C::HALVES + h) * (C::KEYS * 128), tv, v_full, j * 64, h * C::KEYS, 0, g);
         }
         __syncwarp();
-        mlcb_bar_wait(qk_full, 0, &dead);
+        const bool alive = mlcb_bar_wait(qk_full, 0, &dead);
         mlcb_tc_after();
-        if (elected) {
+        if (elected && alive) {
             constexpr u32 idesc = mlcb_idesc(128, C::KEYS, C::BF16, false);
 #pragma unroll
             for (int h = 0; h < C::HALVES; ++h)
@@ -96,8 +96,8 @@ __device__ __forceinline__ void mlcb_attention(const mlcb_tmap* tq, const mlcb_t
     mlcb_tc_after();
     if (warp == 0) {
         const bool elected = mlcb_elect();
-        mlcb_bar_wait(v_full, 0, &dead);
-        if (elected) {
+        const bool alive = mlcb_bar_wait(v_full, 0, &dead);
+        if (elected && alive) {
             constexpr u32 idesc = mlcb_idesc(128, C::D, C::BF16, true);
 #pragma unroll
             for (int k = 0; k < C::S16 / 16; ++k)
@@ -107,9 +107,9 @@ __device__ __forceinline__ void mlcb_attention(const mlcb_tmap* tq, const mlcb_t
         }
         __syncwarp();
     }
-    mlcb_bar_wait(o_full, 0, &dead);
+    const bool alive = mlcb_warp_wait(o_full, 0, &dead);
     mlcb_tc_after();
-    if (!dead) {
+    if (alive) {
         // D columns over H threads of the row, at least 16 each
         constexpr int STEP = C::D / C::H < 16 ? 16 : C::D / C::H;
 #pragma unroll
@@ -120,11 +120,10 @@ __device__ __forceinline__ void mlcb_attention(const mlcb_tmap* tq, const mlcb_t
             if (t0 + r < C::T) mlcb_store<T, 16>(out + g * out_g + (t0 + r) * out_t + c0, v);
             __syncwarp();
         }
-    } else {
-        mlcb_drain();
     }
     mlcb_tc_before();
     __syncthreads();
+    mlcb_leave<1>(&dead);
     if (warp == 0) {
         mlcb_tc_after();
         mlcb_tmem_free<1>(tmem, C::COLS);

@@ -169,7 +169,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
                     __syncwarp();
                     if (++s == C::STAGES) { s = 0; phase ^= 1; }
                 }
-                if (elected) mlcb_mma_commit<C::CG>(acc_full + 8 * acc, rank);
+                if (elected && alive) mlcb_mma_commit<C::CG>(acc_full + 8 * acc, rank);
                 __syncwarp();
                 if (++acc == C::ACC) { acc = 0; acc_phase ^= 1; }
             }
@@ -181,7 +181,8 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
         const u32 base = tmem + ((u32)(quad * 32) << 16);
         MLCB_GRID_WAIT();
         int nth = 0;
-        for (int tile = cluster; tile < C::TILES && !dead; tile += clusters, ++nth) {
+        bool alive = true;
+        for (int tile = cluster; tile < C::TILES && alive; tile += clusters, ++nth) {
             const int acc = nth % C::ACC;
             const int tm = tile % C::TM, tn = (tile / C::TM) % C::TN, g = (tile / (C::TM * C::TN)) % C::GROUPS;
             const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
@@ -194,7 +195,8 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
 #pragma unroll
                 for (int i = 0; i < EACH; ++i)
                     if ((half + i * HALVES) * 8 < SLICE) epi.fetch(pre[i], row, first + (half + i * HALVES) * 8, g, z);
-                mlcb_bar_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+                alive = mlcb_warp_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+                if (!alive) break;
                 mlcb_tc_after();
                 // partial sums go straight into the shared memory of the CTA that finishes these
                 // columns, as [source part][column quad][row][4]: conflict-free both ways.  Its
@@ -211,7 +213,8 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
                                    v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     }
                 }
-                if (!mlcb_bar_wait(arrived, 0, &dead)) break;
+                alive = mlcb_warp_wait(arrived, 0, &dead);
+                if (!alive) break;
 #pragma unroll
                 for (int i = 0; i < EACH; ++i) {
                     const int c = (half + i * HALVES) * 8;
@@ -234,7 +237,8 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
             } else {
                 typename Epi::template Pre<32> pre, ahead;
                 epi.fetch(pre, row, tn * C::BN + half * 32, g, z);
-                mlcb_bar_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+                alive = mlcb_warp_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
+                if (!alive) break;
                 mlcb_tc_after();
 #pragma unroll 1
                 for (int c = half * 32; c < C::BN; c += 32 * HALVES) {
@@ -260,7 +264,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
     mlcb_tc_before();
     __syncthreads();
     if (C::CG == 2) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }   // the peer still uses our barriers and TMEM
-    if (dead) mlcb_drain();
+    mlcb_leave<C::CG == 2 ? 1 : C::CLUSTER>(&dead);
     if (warp == 1) {
         mlcb_tc_after();
         mlcb_tmem_free<C::CG>(tmem, C::TMEM_COLS);

@@ -110,8 +110,10 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
                       three = mlcb_idesc(128, 3 * C::BN, true, C::B_MN);
         int s = 0;
         u32 phase = 0;
+        bool alive = true;
         for (int kb = k0; kb < k1; ++kb) {
-            if (!mlcb_bar_wait(full + 8 * s, phase, &dead)) break;
+            alive = mlcb_bar_wait(full + 8 * s, phase, &dead);
+            if (!alive) break;
             mlcb_tc_after();
             const u32 at = smem + s * C::STAGE;
             const u64 db = mlcb_desc(at + 3 * C::PLANE_A, C::B_MN ? 8192 : 16);
@@ -131,7 +133,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
             __syncwarp();
             if (++s == C::STAGES) { s = 0; phase ^= 1; }
         }
-        if (elected) mlcb_mma_commit<1>(done);
+        if (elected && alive) mlcb_mma_commit<1>(done);
         __syncwarp();
     } else {
         const int t = threadIdx.x;
@@ -188,8 +190,9 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     const int quad = warp % 4, half = warp / 4, r = quad * 32 + lane, row = m0 + r;
     const u32 base = tmem + ((u32)(quad * 32) << 16);
     const u32 inbox = smem + C::STAGES * C::STAGE;     // partial sums of a split K
-    if (warp < C::CW) {
-        mlcb_bar_wait(done, 0, &dead);
+    bool alive = warp < C::CW;
+    if (alive) {
+        alive = mlcb_warp_wait(done, 0, &dead);
         mlcb_tc_after();
     }
     constexpr int EACH = (SLICE + C::CW * 2 - 1) / (C::CW * 2);
@@ -199,7 +202,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
         for (int i = 0; i < EACH; ++i)
             if (half * 8 + i * C::CW * 2 < SLICE) epi.fetch(pre[i], row, n0 + part * SLICE + half * 8 + i * C::CW * 2, g, z);
     }
-    if (warp < C::CW && !dead) {
+    if (alive) {
         // the four warps that share 32 rows take 16 columns each in turn
 #pragma unroll 1
         for (int c = half * 16; c < C::BN; c += C::CW * 4) {
@@ -259,7 +262,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     }
     __syncwarp();
     if constexpr (C::SPLIT > 1) {
-        if (warp < C::CW && !dead && mlcb_bar_wait(arrived, 0, &dead)) {
+        if (alive && mlcb_warp_wait(arrived, 0, &dead)) {
 #pragma unroll
             for (int i = 0; i < EACH; ++i) {
                 const int c = half * 8 + i * C::CW * 2;
@@ -283,6 +286,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     }
     mlcb_tc_before();
     __syncthreads();
+    mlcb_leave<C::SPLIT>(&dead);
     if (warp == C::CW) {
         mlcb_tc_after();
         mlcb_tmem_free<1>(tmem, C::COLS);

@@ -81,8 +81,18 @@ __device__ __forceinline__ bool mlcb_bar_wait(u32 bar, u32 parity, volatile u32*
 }
 __device__ __forceinline__ void mlcb_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mlcb_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// a dead CTA leaves time for copies already in flight to land before it exits
-__device__ __forceinline__ void mlcb_drain() {
+// The same answer in every lane of a converged warp: for waits that TMEM loads follow, which
+// the whole warp executes or none of it.
+__device__ __forceinline__ bool mlcb_warp_wait(u32 bar, u32 parity, volatile u32* dead) {
+    return __all_sync(0xffffffffu, mlcb_bar_wait(bar, parity, dead));
+}
+// How a CTA ends (CLUSTER > 1: behind a barrier of all its threads).  One whose waits ran out stays until
+// every other CTA of its cluster has done the same or exited (their waits are bounded too, and
+// a barrier of the cluster does not wait for exited threads): a late partner may still be
+// sending to its shared memory.  Then it leaves time for copies in flight to land.
+template <int CLUSTER> __device__ __forceinline__ void mlcb_leave(volatile u32* dead) {
+    if (!*dead) return;
+    if (CLUSTER > 1) { mlcb_cluster_arrive(); mlcb_cluster_wait(); }
     const u64 t0 = mlcb_now_ns();
     while (mlcb_now_ns() - t0 < 20000000ull) __nanosleep(1000);
 }

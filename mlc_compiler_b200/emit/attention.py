@@ -172,7 +172,7 @@ def _functor(k: AttentionKernel, cfg, H: int, V: int, G: int, stable) -> tuple[s
         for i in used:
             fetch(i, 0)                        # the next chunk's operands travel with this one's work
         if not started[0]:
-            emit("        mlcb_bar_wait(ready, 0, dead);")
+            emit("        mlcb_warp_wait(ready, 0, dead);")
             emit("        mlcb_tc_after();")
             started[0] = True
         for lo in range(0, NC, chunk):

@@ -415,7 +415,7 @@ def emit_staged(k: kir.ReductionKernel, cfg, name: str, stable, st: Stage) -> tu
     c.lines[at:] = [ln.replace("if (live && lane == 0)", "if (rank == 0 && lane == 0)") for ln in c.lines[at:]]
     if C > 1:
         e("    mlcb_cluster_wait();")
-    e("    if (dead) mlcb_drain();")
+    e("    mlcb_leave<1>(&dead);")
     e("}")
     spec = LaunchSpec(grid=grid, block=T, smem=st.smem, vector=V, cluster=C,
                       alg_bytes=algorithmic_bytes(k.inputs, k.outputs, k.n_rows * N))

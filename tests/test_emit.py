@@ -391,3 +391,20 @@ def test_waits_with_a_limit_come_behind_the_grid_wait():
             role = re.split(r"\} else (?:if \(warp == \S+\) )?\{", part)
             assert len(role) >= 2, f
             assert not any(re.search(r"mlcb_(bar|warp)_wait\(", r) for r in role[1:]), f
+
+
+def test_split_matmuls_leave_with_their_cluster():
+    """Every kernel ends through ``mlcb_leave``, those whose CTAs send one another partial
+    sums with the size of the cluster."""
+    from mlc_compiler_b200.emit.module import CSRC
+    from perf import cases
+
+    for f, size in (("mlcb_matmul.cuh", "C::CG == 2 ? 1 : C::CLUSTER"), ("mlcb_matmul32.cuh", "C::SPLIT"),
+                    ("mlcb_attention.cuh", "1")):
+        text = (CSRC / f).read_text()
+        end = text.index(f"mlcb_leave<{size}>(&dead);")
+        # behind the last barrier of all threads, ahead of giving TMEM back
+        assert text.rindex("__syncthreads();", 0, end) > text.rindex("mlcb_warp_wait(", 0, end)
+        assert text.index("mlcb_tmem_free<", end) > end
+    s = cases.rows_schedule("softmax", 3, 50257, "float16")
+    assert "mlcb_leave<1>(&dead);" in generate_module(s, Config()).kernel_source("k0")

@@ -242,13 +242,20 @@ def test_calls_read_negated_views_with_their_sign(what):
     assert torch.equal(cm(torch._neg_view(x), *rest), want)
 
 
-def _lonely(tmp_path):
-    """A module whose one kernel waits for a barrier that nobody signals."""
+def _built(tmp_path, kernel):
+    """A module of the device library and ``kernel``."""
     from mlc_compiler_b200 import build
     from mlc_compiler_b200.emit import module
     from mlc_compiler_b200.runtime import LoadedModule
 
-    source = module.device_header() + "\n".join(module.tensor_headers({"mm"})) + """
+    image = tmp_path / "kernel.cubin"
+    build.nvcc_cubin(module.device_header() + "\n".join(module.tensor_headers({"mm"})) + kernel, image)
+    return LoadedModule(image.read_bytes(), 0)
+
+
+def _lonely(tmp_path):
+    """A module whose one kernel waits for a barrier that nobody signals."""
+    return _built(tmp_path, """
 extern "C" __global__ void lonely(u32* seen) {
     __shared__ alignas(8) u64 bar;
     __shared__ volatile u32 dead;
@@ -257,9 +264,7 @@ extern "C" __global__ void lonely(u32* seen) {
     const bool met = mlcb_bar_wait(mlcb_smem(&bar), 0, &dead);
     if (threadIdx.x == 0) seen[0] = met ? 1u : 2u;
 }
-"""
-    build.nvcc_cubin(source, tmp_path / "lonely.cubin")
-    return LoadedModule((tmp_path / "lonely.cubin").read_bytes(), 0)
+""")
 
 
 def test_a_wait_that_runs_out_is_reported(tmp_path):
@@ -290,6 +295,33 @@ def test_a_wait_that_runs_out_on_a_side_stream_is_seen(tmp_path):
         mod.check()
     mod.check()
     assert mod.fault() == 0 and int(seen[0]) == 2
+
+
+def test_a_cta_whose_wait_ran_out_outlives_its_partner(tmp_path):
+    """A cluster of two: one gives up after two seconds, the other works half a second longer
+    and is the first to leave (its partial sums would have found the memory they go to)."""
+    mod = _built(tmp_path, """
+extern "C" __global__ void partners(u64* left) {
+    __shared__ alignas(8) u64 bar;
+    __shared__ volatile u32 dead;
+    if (threadIdx.x == 0) { dead = 0; mlcb_bar_init(mlcb_smem(&bar), 1); mlcb_bar_fence_init(); }
+    __syncthreads();
+    const u32 rank = mlcb_cta_rank();
+    const u64 t0 = mlcb_now_ns();
+    if (rank == 0) mlcb_warp_wait(mlcb_smem(&bar), 0, &dead);
+    else while (mlcb_now_ns() - t0 < 2500000000ull) __nanosleep(1000);
+    __syncthreads();
+    mlcb_leave<2>(&dead);
+    if (threadIdx.x == 0) left[rank] = mlcb_now_ns();
+}
+""")
+    left = torch.zeros(2, dtype=torch.int64, device="cuda")
+    ptr = (ctypes.c_uint64 * 1)(left.data_ptr())
+    stream = torch.cuda.current_stream().cuda_stream
+    assert mod.lib.mlcb_launch(mod.kernel("partners"), 2, 64, 0, ptr, 1, stream, 2 << 8) == 0
+    assert mod.fault() != 0
+    gave_up, worked = left.tolist()
+    assert gave_up >= worked > 0
 
 
 @pytest.mark.parametrize("what", ["one kernel", "model"])
