@@ -1,7 +1,8 @@
 // C = A B over fp32 operands on the 16-bit tensor cores, without losing a bit of them.
 //
 // An fp32 value is exactly the sum of three bf16 ones (24 significant bits in three
-// pieces of 8, cut by truncation), so A B is nine bf16 matmuls whose products are exact
+// pieces of 8, cut by truncation; below 2^-110 the last piece has no bf16 left to be, and
+// what is lost is below 2^-133), so A B is nine bf16 matmuls whose products are exact
 // in fp32 (last times last piece, 2^-32 of the product, is left out).  Sixteen converter
 // warps read the operands a block ahead, cut them and store the pieces as swizzled
 // tiles; the pieces of B lie side by side as one operand, so one MMA multiplies a piece of

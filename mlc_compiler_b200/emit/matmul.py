@@ -428,10 +428,23 @@ class Config32:
         return self.stages * 3 * (16384 + self.bn * 128) + inbox + 1024
 
 
+#: 64-element blocks of K that one accumulator of an fp32 product may sum, and accumulators.
+#: Every addition truncates, so an error grows with the chain's length: over normal operands
+#: [1024, K] x [K, 768] is off by 4.2e-7 of the result's norm at seven blocks a chain (the
+#: library's fp32: 8.1e-7 at that K), by 1.8e-6 at 26 (3.2e-6, but 6.6e-7 where it splits K);
+#: over positive ones, whose errors all point one way, by 7.0e-7 and 4.0e-6 (6.0e-7, 2.4e-6)
+LEAD_BLOCKS, LEADS = 7, 5
+
+
+def whole32(k: int) -> bool:
+    """Whether chains stay that short in the parts of the widest split (K up to 17920)."""
+    return _ceil(k, 64) <= 8 * LEADS * LEAD_BLOCKS
+
+
 def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, peers: int | None = None) -> Config32:
     """Least estimated time, in microseconds: a 64-deep block costs 0.75 (32 columns) or 1.0
     (64), a wave 3 before and after.  Leading products get a new accumulator every four
-    blocks, as far as TMEM goes.  Batched products split K as others do: two encoder layers
+    blocks, as far as TMEM goes (five), and K is split until none sums more than seven.  Batched products split K as others do: two encoder layers
     of batch 3, sequence 511, 4 heads 170.3 us whole, 159.8 split."""
     kb = _ceil(k, 64)
 
@@ -442,14 +455,14 @@ def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, peers: int
         return waves * (_ceil(kb, split) * (0.75 if bn == 32 else 1.0) + 3.0 + exchange)
 
     widths = (64,) if b_mn else (32, 64)
-    splits = tuple(s for s in (1, 2, 4, 8) if s <= kb)
+    splits = tuple(s for s in (1, 2, 4, 8) if s <= kb and _ceil(kb, s) <= LEADS * LEAD_BLOCKS)
     _, split = min(((bn, s) for bn in widths for s in splits if bn % (8 * s) == 0),
                    key=lambda c: cost(*c, peers or groups))
     bn = min((bn for bn in widths if bn % (8 * split) == 0), key=lambda bn: cost(bn, split, groups))
     t = _ceil(m, 128) * _ceil(n, bn) * groups * z
     most = 2 if split > 1 and bn == 64 else 3           # the partial sums' place
     return Config32(bn, max(2, min(most, _ceil(kb, split))), split, t * split,
-                    min(5, _ceil(_ceil(kb, split), 4)))
+                    min(LEADS, _ceil(_ceil(kb, split), 4)))
 
 
 def emit_matmul32(k: MatmulKernel, cfg, buffers, name: str, stable):

@@ -132,6 +132,8 @@ def tma_layout(v: kir.View, rows_axis: int, k_axis: int) -> str | None:
 
 def _matmul(k, schedule) -> MatmulKernel | None:
     """The tensor-core form of a library matmul, result stored as the library would."""
+    from .emit.matmul import whole32
+
     if not isinstance(k, kir.ExternKernel) or k.op not in ("aten.mm.default", "aten.bmm.default") or k.kwargs:
         return None
     a, b, out = k.args[0], k.args[1], k.outputs[0]
@@ -140,7 +142,7 @@ def _matmul(k, schedule) -> MatmulKernel | None:
         return None
     if dts == {"float32"}:
         if a.strides[-1] != 1 or 1 not in b.strides[-2:] or min(a.strides + b.strides) < 0 \
-                or max(schedule.buffers[v.buffer].numel for v in (a, b)) >= 1 << 31:
+                or max(schedule.buffers[v.buffer].numel for v in (a, b)) >= 1 << 31 or not whole32(a.shape[-1]):
             return None
     elif dts <= set(kir.NARROW_FLOATS):
         if tma_layout(a, -2, -1) != "k":

@@ -133,7 +133,7 @@ def _schedule(buffers, kernels, dtype="float32"):
         elif kind != "intermediate":
             getattr(s, kind + "s").append(view)
     s.kernels = kernels
-    if kernels:
+    if any(kind == "intermediate" for _, kind in buffers.values()) and kernels:
         cases._plan_arena(s)
     return s
 
@@ -276,3 +276,20 @@ def test_attention_is_fused_where_its_shared_memory_exists(heads):
                 static = int(re.search(r"mlcb_att_cfg<\d+, \d+, \d+, \d+, \d+, (\d+)", mod.kernel_source(k.name))[1]) * 4 + 64
             assert spec.smem + static <= 227 * 1024, (keys, k.name)
     assert fused >= {16, 128, 256, 304, 336, 352} and (heads == 128 or {384, 512} <= fused)
+
+
+@pytest.mark.parametrize("k", [64, 448, 449, 2240, 2241, 3072, 4096, 4481, 8192, 8961, 17919, 17920, 17921, 65536])
+def test_fp32_sums_are_taken_in_short_chains(k):
+    """At most seven blocks of K per accumulator; a K that the widest split cannot cut that
+    short stays with the library."""
+    for m in (1, 128, 1024, 4096, 16384):
+        for n in (64, 768, 3072):
+            s = _schedule({"a": ((m, k), "input"), "w": ((k, n), "param"), "c": ((m, n), "output")},
+                          [_mm("k0", "a", "w", "c", m, n, k)])
+            own = isinstance(fuse(s, Config()).kernels[0], MatmulKernel)
+            assert own == (k <= 17920 and k * max(m, n) < 1 << 31)
+            if own:
+                for b_mn in (False, True):
+                    c = M.choose32(1, m, n, k, 1, b_mn)
+                    assert -(-(-(-(-(-k // 64)) // c.split)) // c.leads) <= 7 and (3 + c.leads) * c.bn <= 512
+                    assert c.smem() <= M.SMEM_MAX and c.bn % (8 * c.split) == 0

@@ -109,6 +109,27 @@ def test_matmuls_at_the_edges_of_their_tiles(shape, dtype):
     assert cm._launched._module.loaded.fault() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(128, 768, 3072), (1024, 768, 2048), (1387, 768, 3072), (1110, 1024, 4096), (128, 64, 8192),
+                                   (1024, 64, 8961), (130, 72, 17920)])
+def test_fp32_matmul_errors_do_not_grow_with_k(m, n, k):
+    """Sums of any length within what a chain of seven blocks loses.  An accumulator takes four
+    additions of 16 products per block, each truncated to 24 bits: 28 * 2^-23 of the magnitudes;
+    adding up five of those, the corrections and the parts of a split K rounds 16 times more.
+    One chain over K = 8192 would make 512.  And no further off than the library's fp32 sum,
+    where neither sum's errors point one way."""
+    w = {"even": _randn((n, k), "float32", 2), "positive": torch.rand((n, k), device="cuda") + 0.5}
+    a = {"even": _randn((m, k), "float32", 3), "positive": _randn((m, k), "float32", 3).relu()}
+    for how in w:
+        cm = CompiledModel(_matmul(1, m, n, k, 1, False, False, "float32"), {"b0": w[how]}, Config(), "cuda")
+        assert cm.launches_per_call == 1
+        got, want = cm(a[how]).double(), a[how].double() @ w[how].double().T
+        off = (got - want).abs() - (28 + 16) * 2.0 ** -23 * (a[how].double().abs() @ w[how].double().abs().T)
+        assert float(off.max()) <= 0, f"{how}: {float(off.max()):.3e} over the bound"
+        if how == "even":
+            library = (a[how] @ w[how].T).double()
+            assert float((got - want).norm()) <= float((library - want).norm())
+
+
 def test_fp32_matmul_of_values_without_finite_pieces():
     s = _matmul(1, 130, 70, 100, 1, False, False, "float32")
     w = _randn((70, 100), "float32", 1)
