@@ -149,20 +149,20 @@ std::once_flag g_rtc_once;
 
 void load_rtc() {
     Rtc& r = g_rtc;
-    const char* names[] = {"libnvrtc.so.12", "libnvrtc.so", "libnvrtc.so.13"};
-    for (const char* n : names) {
-        r.lib = dlopen(n, RTLD_NOW | RTLD_GLOBAL);
+    // The toolkit's own first, whose headers the modules include.  By name alone a process that
+    // has loaded torch gets torch's, and 12.8 knows neither 256-bit accesses nor three-operand
+    // maxima: every module with one went through nvcc (seconds), or nowhere without nvcc.
+    const char* homes[] = {getenv("CUDA_HOME"), getenv("CUDA_PATH"), "/usr/local/cuda"};
+    for (const char* h : homes) {
+        if (!h) continue;
+        std::string p = std::string(h) + "/lib64/libnvrtc.so";
+        r.lib = dlopen(p.c_str(), RTLD_NOW | RTLD_LOCAL | RTLD_DEEPBIND);
         if (r.lib) break;
     }
-    if (!r.lib) {
-        // a toolkit that is installed but not on the loader path
-        const char* homes[] = {getenv("CUDA_HOME"), getenv("CUDA_PATH"), "/usr/local/cuda"};
-        for (const char* h : homes) {
-            if (!h) continue;
-            std::string p = std::string(h) + "/lib64/libnvrtc.so";
-            r.lib = dlopen(p.c_str(), RTLD_NOW | RTLD_GLOBAL);
-            if (r.lib) break;
-        }
+    const char* names[] = {"libnvrtc.so.12", "libnvrtc.so", "libnvrtc.so.13"};
+    for (const char* n : names) {
+        if (r.lib) break;
+        r.lib = dlopen(n, RTLD_NOW | RTLD_GLOBAL);
     }
     if (!r.lib) return;
     bool ok = true;

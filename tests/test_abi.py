@@ -57,3 +57,30 @@ def test_nvrtc_produces_an_sm100a_image_without_a_gpu():
     except runtime.BackendError as e:  # pragma: no cover
         pytest.skip(str(e))
     assert image[:4] == b"\x7fELF"
+
+
+def test_nvrtc_compiles_what_calls_launch():
+    """In a process that has torch loaded (whose own NVRTC may be older than the toolkit):
+    256-bit accesses, three-operand maxima, tcgen05."""
+    import torch  # noqa: F401
+
+    from mlc_compiler_b200 import Config
+    from mlc_compiler_b200.emit import generate_module
+    from mlc_compiler_b200.fuse import fuse
+    from mlc_compiler_b200.rewrite import prepare
+    from perf import cases
+
+    lib = runtime.load_library()
+    opts = [o.encode() for o in B.NVRTC_FLAGS] + [f"-I{B.cuda_home() / 'include'}".encode()]
+    arr = (ctypes.c_char_p * len(opts))(*opts)
+    for s in (fuse(prepare(cases.encoder_schedule(2, 77, 4, 1, "float16"), Config()), Config()),
+              cases.rows_schedule("gelu", 4096, 3072, "bfloat16")):
+        image, size = ctypes.c_void_p(), ctypes.c_size_t()
+        log = ctypes.create_string_buffer(1 << 14)
+        code = lib.mlcb_compile(generate_module(s, Config()).source.encode(), B.ARCH.encode(), arr, len(opts),
+                                ctypes.byref(image), ctypes.byref(size), log, len(log))
+        if code == 200001:
+            pytest.skip("NVRTC not installed on this machine")
+        assert code == 0, log.value.decode()[:2000]
+        assert ctypes.string_at(image.value, 4) == b"\x7fELF"
+        lib.mlcb_free_image(image)
