@@ -185,19 +185,20 @@ class _Executable:
             self._arena = torch.empty(need, dtype=torch.uint8, device=self.device)
         return self._arena
 
-    def _resident_buffers(self, inputs: Sequence[torch.Tensor]) -> dict[str, torch.Tensor]:
-        self._check_inputs(inputs)
+    def _storage(self) -> dict[str, torch.Tensor]:
+        """Every buffer but the inputs (which are in it from the first call that copies them)."""
         if self._resident is None:
             sch = self._exec
             buffers = dict(self.params)
+            inputs = {v.buffer for v in sch.inputs}
             for b in sch.buffers.values():
-                if b.name in buffers or b.plannable or b.name not in self._live:
+                if b.name in buffers or b.plannable or b.name not in self._live or b.name in inputs:
                     continue
                 buffers[b.name] = self._empty(b)
             offsets = sch.plan.offsets if sch.plan.mode == "arena" else {}
             arena = self._get_arena()
             for b in sch.buffers.values():
-                if b.name in buffers or b.name not in self._live:
+                if b.name in buffers or b.name not in self._live or b.name in inputs:
                     continue
                 off = offsets.get(b.name)
                 if off is None:
@@ -205,7 +206,17 @@ class _Executable:
                 else:
                     buffers[b.name] = arena[off:off + b.nbytes].view(kir.torch_dtype(b.dtype))
             self._resident = buffers
-            self._static_inputs = [buffers[v.buffer] for v in sch.inputs]
+        return self._resident
+
+    def _resident_buffers(self, inputs: Sequence[torch.Tensor]) -> dict[str, torch.Tensor]:
+        """Every buffer, the inputs' with the values of these."""
+        self._check_inputs(inputs)
+        buffers = self._storage()
+        if self._static_inputs is None:
+            for v in self._exec.inputs:
+                if v.buffer not in buffers:
+                    buffers[v.buffer] = self._empty(self._exec.buffers[v.buffer])
+            self._static_inputs = [buffers[v.buffer] for v in self._exec.inputs]
         for dst, t in zip(self._static_inputs, inputs):
             dst.copy_(t.reshape(-1), non_blocking=True)
         return self._resident
@@ -616,11 +627,17 @@ class _DirectCall:
         #: the same call in native code (``csrc/mlcb_call.cpp``), once bound
         self.native = None
         self._last = None
+        #: whether a launch has finished and its waits were met
+        self.proved = False
 
     def _bind(self, inputs) -> None:
         owner = self.owner
         k = owner._exec.kernels[0]
-        buffers = owner._resident_buffers(inputs)
+        owner._check_inputs(inputs)
+        buffers = dict(owner._storage())
+        nowhere = torch.empty(0, device=owner.device)      # every launch gets the caller's addresses
+        for v in owner.schedule.inputs:
+            buffers.setdefault(v.buffer, nowhere)
         fn = self.launch = owner._module.bind(k, buffers, 0)[0]
         names = owner._module._buffer_names(k)
         self.specs = []
@@ -645,16 +662,19 @@ class _DirectCall:
                                  self.written, self.out,
                                  functools.partial(_launch_failed, fn.lib, fn.name, owner._module.loaded),
                                  0 if owner._fault is None else ctypes.addressof(owner._fault))
-        if fn.smem:                  # bounded waits inside: prove them once, as a capture's warm-up does
-            fn[fn.grid]()
-            owner._settled()
         self.index = owner.device.index
 
     def __call__(self, inputs):
         if self.launch is None:
             self._bind(inputs)
-        if self.native is not None:
-            return self.native(inputs)
+        out = self.native(inputs) if self.native is not None else self._run(inputs)
+        if out is not None and not self.proved:
+            # bounded waits inside: seen to end once, as a capture's warm-up does
+            self.owner._settled()
+            self.proved = True
+        return out
+
+    def _run(self, inputs):
         if self.fault is not None and self.fault.value:
             self.owner._module.loaded.check()
         specs = self.specs
@@ -768,7 +788,7 @@ class CompiledModel(_Executable):
         run = self._launched
         if run is None:
             out = self._call(inputs)
-            if self._direct is not None and self.cfg.cuda_graphs:
+            if self._direct is not None and self._direct.proved:
                 self._fast = self._direct.native
             return out
         out = run._call(inputs)

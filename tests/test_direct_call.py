@@ -48,7 +48,7 @@ def in_python():
     d = _DirectCall.__new__(_DirectCall)
     d.native, d.index, d.launch, d.out, d.flags, d._last = None, 0, object(), "out", 0, None
     d.specs = [(torch.Size(SHAPE), torch.float16, 64, (0,))]
-    d.written, d.fault = [WRITTEN], None
+    d.written, d.fault, d.proved = [WRITTEN], None, True
     d.args = (0, 1, 32, 0, (ctypes.c_uint64 * 64)(), 2)
     d.run = lambda *a: pytest.fail("launched")
     return d
@@ -143,3 +143,21 @@ except RuntimeError as e:
     with pytest.raises(BackendError, match="ran out"):
         loaded.check()
     loaded.check()                                     # reported once
+
+
+def test_a_direct_call_needs_no_buffers_for_its_inputs():
+    """They exist from the first call that copies an input; results stay where they are."""
+    from mlc_compiler_b200 import Config
+    from mlc_compiler_b200.executor import _Executable
+    from perf import cases
+
+    s = cases.rows_schedule("gelu", 8, 64, "float16")
+    form = _Executable.__new__(_Executable)
+    form.cfg, form.device = Config(), torch.device("cpu")
+    form._bind_form(s, s, {"bias": torch.zeros(64, dtype=torch.float16)}, relaxed=False)
+    first = dict(form._storage())
+    assert "y" in first and not {"x", "res"} & set(first)
+    x, res = torch.ones(8, 64), torch.zeros(8, 64, dtype=torch.float16)
+    after = form._resident_buffers([x, res])
+    assert torch.equal(after["x"], torch.ones(512, dtype=torch.float16)) and after["y"] is first["y"]
+    assert form._resident_buffers([x * 2, res])["x"] is after["x"] and int(after["x"][0]) == 2
