@@ -487,6 +487,56 @@ class _Executable:
             self._module.loaded.check()
         self._graph_replay.replay()
 
+    # -- profiling -----------------------------------------------------------------
+    def profile_kernels(self, inputs, iters: int = 20) -> list[tuple]:
+        """Per-kernel device time of this form over the bound plan, in place
+        (``executor.py:309-352``): (name, summary, milliseconds)."""
+        if torch.cuda.current_device() != self.device.index:
+            with torch.cuda.device(self.device):
+                return self.profile_kernels(inputs, iters)
+        buffers = self._resident_buffers(inputs)
+        if self._plan is None:
+            self._plan = self._build_plan(buffers)
+        for _ in range(3):
+            _Executable.run_kernels(self, buffers)
+        torch.cuda.synchronize(self.device)
+
+        def run(entry):
+            kind, payload = entry
+            if kind == "cuda":
+                payload[payload.grid]()
+            else:
+                run_bound_extern(payload)
+
+        start = torch.cuda.Event(enable_timing=True)
+        end = torch.cuda.Event(enable_timing=True)
+        out = []
+        for k in self._exec.kernels:
+            entry = self._bound[k.name]
+            for _ in range(3):
+                run(entry)
+            torch.cuda.synchronize(self.device)
+            start.record()
+            for _ in range(iters):
+                run(entry)
+            end.record()
+            end.synchronize()
+            out.append((k.name, k.summary(), start.elapsed_time(end) / iters))
+        return out
+
+    # -- source ----------------------------------------------------------------------
+    def source(self) -> str:
+        return self._module.source
+
+    def source_path(self):
+        return self._module.path
+
+    def kernel_source(self, name: str) -> str:
+        return self._module.generated.kernel_source(name)
+
+    @property
+    def launch_table(self) -> dict:
+        return self._module.launch_table
 
 
 def _launch_failed(lib, name: str, loaded, code: int):
@@ -795,8 +845,15 @@ class CompiledModel(_Executable):
         self.dependent_policy, self.policy_timings_ms = run.dependent_policy, run.policy_timings_ms
         return out
 
+    def run_kernels(self, buffers: dict[str, torch.Tensor] | None = None, after=None) -> None:
+        """What a call launches, once more on the buffers it left (uncaptured)."""
+        if self._launched is not None:
+            return self._launched.run_kernels(buffers, after)
+        return super().run_kernels(buffers, after)
+
     def replay(self) -> None:
-        """Replay the captured graph on the inputs already resident."""
+        """Run the last call again, on its inputs: those read in place are read where the
+        caller has them (the model holds on to them), with the values they have now."""
         if torch.cuda.current_device() != self.device.index:
             with torch.cuda.device(self.device):
                 return self.replay()
@@ -815,66 +872,23 @@ class CompiledModel(_Executable):
                     form._settled()
 
     @property
+    def launched(self) -> "_Executable":
+        """The form that calls launch, to look at: ``profile_kernels``, ``source``,
+        ``kernel_source`` and ``launch_table`` of it describe ``launched_schedule``, those of
+        the model itself ``executed_schedule``."""
+        return self._launched or self
+
+    @property
     def launched_schedule(self) -> kir.Schedule:
         """What a call launches: ``executed_schedule`` with matmuls and their neighbours fused."""
-        return (self._launched or self)._exec
-
-    # -- profiling -----------------------------------------------------------------
-    def profile_kernels(self, inputs, iters: int = 20) -> list[tuple]:
-        """Per-kernel device time over the bound plan, in place
-        (``executor.py:309-352``): (name, summary, milliseconds)."""
-        if torch.cuda.current_device() != self.device.index:
-            with torch.cuda.device(self.device):
-                return self.profile_kernels(inputs, iters)
-        buffers = self._resident_buffers(inputs)
-        if self._plan is None:
-            self._plan = self._build_plan(buffers)
-        for _ in range(3):
-            self.run_kernels(buffers)
-        torch.cuda.synchronize(self.device)
-
-        def run(entry):
-            kind, payload = entry
-            if kind == "cuda":
-                payload[payload.grid]()
-            else:
-                run_bound_extern(payload)
-
-        start = torch.cuda.Event(enable_timing=True)
-        end = torch.cuda.Event(enable_timing=True)
-        out = []
-        for k in self._exec.kernels:
-            entry = self._bound[k.name]
-            for _ in range(3):
-                run(entry)
-            torch.cuda.synchronize(self.device)
-            start.record()
-            for _ in range(iters):
-                run(entry)
-            end.record()
-            end.synchronize()
-            out.append((k.name, k.summary(), start.elapsed_time(end) / iters))
-        return out
+        return self.launched._exec
 
     # -- introspection -------------------------------------------------------------
     @property
     def executed_schedule(self) -> kir.Schedule:
-        """The schedule after rewriting, kernel for kernel what ``profile_kernels`` runs; calls
-        launch ``launched_schedule``."""
+        """The schedule after rewriting, kernel for kernel what the model's ``profile_kernels``
+        runs; calls launch ``launched_schedule``."""
         return self._exec
-
-    def source(self) -> str:
-        return self._module.source
-
-    def source_path(self):
-        return self._module.path
-
-    def kernel_source(self, name: str) -> str:
-        return self._module.generated.kernel_source(name)
-
-    @property
-    def launch_table(self) -> dict:
-        return self._module.launch_table
 
     def __repr__(self) -> str:  # pragma: no cover
         return (f"CompiledModel({self.schedule.name}, {len(self.schedule)} kernels, "

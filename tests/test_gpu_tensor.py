@@ -366,6 +366,30 @@ def test_calls_report_a_wait_that_ran_out(what):
         report()
 
 
+def test_what_calls_launch_can_be_looked_at_and_run_again():
+    """The launched form's kernels by name, their source and times, beside the scheduled ones."""
+    s = cases.encoder_schedule(2, 33, 4, 1, "float16")
+    params = {o: _randn(s.buffers[b].shape, "float16", 9) * 0.05 for b, o in s.params.items()}
+    cm = CompiledModel(s, params, Config(), "cuda")
+    x = [_randn(v.shape, "float16", 1) if i == 0 else torch.zeros(v.shape, dtype=torch.float16, device="cuda")
+         for i, v in enumerate(s.inputs)]
+    with pytest.raises(Exception, match="no launch plan"):
+        cm.run_kernels()
+    out = cm(*x)
+    want = out.clone()
+    assert [r[0] for r in cm.profile_kernels(x, iters=2)] == [k.name for k in cm.executed_schedule.kernels]
+    rows = cm.launched.profile_kernels(x, iters=2)
+    assert [r[0] for r in rows] == [k.name for k in cm.launched_schedule.kernels] and all(r[2] > 0 for r in rows)
+    assert len(rows) == cm.launches_per_call < len(cm.executed_schedule)
+    assert set(cm.launched.launch_table) == {r[0] for r in rows}
+    for name, _, _ in rows:
+        assert "__launch_bounds__" in cm.launched.kernel_source(name)
+    assert "mlcb_attention" in cm.launched.source() and "mlcb_attention" not in cm.source()
+    out.zero_()
+    cm.run_kernels()
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("rows,cols", [(777, 1003), (1, 607001), (8, 50001), (601, 1006), (3, 300000)])
 def test_pointwise_over_counts_that_are_no_packs(rows, cols, dtype):
