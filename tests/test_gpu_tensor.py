@@ -391,6 +391,70 @@ def test_what_calls_launch_can_be_looked_at_and_run_again():
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("m,n,k", [(128, 768, 768), (100, 96, 1536), (1, 64, 4096)])
+def test_a_split_matmul_of_a_graph_reads_its_input_at_other_addresses(m, n, k, dtype):
+    """New parameters of a captured node keep its cluster: partial sums meet as before."""
+    from mlc_compiler_b200.emit import matmul as M
+
+    s = _matmul(1, m, n, k, 1, False, False, dtype)
+    c = M.choose32(1, m, n, k, 1, False) if dtype == "float32" else M.choose(1, m, n, k, 1, False)
+    assert c.split > 1
+    cm = CompiledModel(s, {"b0": _randn((n, k), dtype, 2)}, Config(), "cuda")
+    x = _randn((m, k), dtype, 3)
+    want = cm(x).clone()
+    assert cm._launched._in_place.inputs[0] is not None          # read where the caller has it
+    places = [x.clone() for _ in range(3)]
+    for t in (*places, x, places[1]):
+        cm(-x)
+        assert torch.equal(cm(t), want)
+        assert cm._launched._in_place.now["a"] == t.data_ptr()
+
+
+@pytest.mark.parametrize("how", ["no dependent launches", "no native call", "neither"])
+@pytest.mark.parametrize("op,cols", [("layernorm", 768), ("softmax", 1001), ("softmax", 50257), ("gelu", 515)])
+def test_direct_calls_without_their_helpers_give_the_same(op, cols, how, monkeypatch):
+    """Launched plainly, or by the Python form of the call: the same bits, at every address."""
+    from mlc_compiler_b200 import executor
+
+    if how != "no dependent launches":
+        monkeypatch.setattr(executor, "native_call", lambda: None)
+    cfg = Config(dependent_launch=False) if how != "no native call" else Config()
+    s = cases.rows_schedule(op, 33, cols, "float16")
+    params = {o: _randn((cols,), "float16", 5 + i) for i, o in enumerate(s.params)}
+    x = [_randn(v.shape, "float16", 1 + i) for i, v in enumerate(s.inputs)]
+    cm, usual = CompiledModel(s, params, cfg, "cuda"), CompiledModel(s, params, Config(), "cuda")
+    want = usual(*x).clone()
+    for t in ([y.clone() for y in x], x):
+        cm(*[-y for y in t])
+        for _ in range(3):
+            assert torch.equal(cm(*t), want)
+    assert (cm._direct.native is None) == (how != "no dependent launches")
+    assert (cm._direct.flags & 1 == 0) == (how != "no native call") and usual._direct.flags & 1
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("batch,seq,heads", [(1, 128, 4), (2, 33, 6), (3, 64, 4), (1, 200, 12)])
+def test_a_fused_model_gives_what_its_kernels_give_apart(batch, seq, heads, dtype):
+    """The same encoder with its matmuls unfused, and with them in the library.  A layer stores
+    ten tensors (q, k, v, scores, probabilities, context, projection, norm, activation, result);
+    sums taken in another order can round each the other way, off by at most U of its norm, and
+    LayerNorm keeps such a difference what it is relative to its rows.  In fp32 the sums
+    themselves differ, by less than 1e-6 of their norms each."""
+    layers = 2
+    s = cases.encoder_schedule(batch, seq, heads, layers, dtype)
+    params = {o: _randn(s.buffers[b].shape, dtype, 9 + i) * 0.02 + (o.endswith("norm.weight"))
+              for i, (b, o) in enumerate(s.params.items())}
+    x = _randn(s.inputs[0].shape, dtype, 1)
+    mask = torch.zeros(s.inputs[1].shape, dtype=x.dtype, device="cuda")
+    mask[..., seq - seq // 4:] = torch.finfo(x.dtype).min
+    fused = CompiledModel(s, params, Config(), "cuda")(x, mask).double()
+    for cfg in (Config(fuse_matmuls=False), Config(own_matmuls=False), Config().as_scheduled()):
+        apart = CompiledModel(s, params, cfg, "cuda")(x, mask).double()
+        off = float((fused - apart).norm() / apart.norm())
+        assert off <= layers * 10 * (U[dtype] if dtype != "float32" else 1e-6), off
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("rows,cols", [(777, 1003), (1, 607001), (8, 50001), (601, 1006), (3, 300000)])
 def test_pointwise_over_counts_that_are_no_packs(rows, cols, dtype):
     s = cases.rows_schedule("gelu", rows, cols, dtype)
