@@ -130,6 +130,20 @@ def tma_layout(v: kir.View, rows_axis: int, k_axis: int) -> str | None:
     return None
 
 
+#: with TF32 allowed, products of more operations than this stay with the library: exact ones
+#: take 13 us there against 12 ([512, 768] x [768, 768], [128, 768] x [768, 3072]), 8.8 against
+#: 12.0 at a quarter of it, 529.8 against 105.3 at [2048, 4096] x [4096, 4096]
+TF32_FLOPS = 6e8
+
+
+def _tf32() -> bool:
+    """Whether the caller lets fp32 matmuls of the library round their operands to TF32."""
+    import torch
+
+    m = torch.backends.cuda.matmul
+    return m.fp32_precision == "tf32" if hasattr(m, "fp32_precision") else bool(m.allow_tf32)
+
+
 def _matmul(k, schedule) -> MatmulKernel | None:
     """The tensor-core form of a library matmul, result stored as the library would."""
     from .emit.matmul import whole32
@@ -142,7 +156,8 @@ def _matmul(k, schedule) -> MatmulKernel | None:
         return None
     if dts == {"float32"}:
         if a.strides[-1] != 1 or 1 not in b.strides[-2:] or min(a.strides + b.strides) < 0 \
-                or max(schedule.buffers[v.buffer].numel for v in (a, b)) >= 1 << 31 or not whole32(a.shape[-1]):
+                or max(schedule.buffers[v.buffer].numel for v in (a, b)) >= 1 << 31 or not whole32(a.shape[-1]) \
+                or (_tf32() and 2 * out.numel * a.shape[-1] > TF32_FLOPS):
             return None
     elif dts <= set(kir.NARROW_FLOATS):
         if tma_layout(a, -2, -1) != "k":

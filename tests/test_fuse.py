@@ -293,3 +293,21 @@ def test_fp32_sums_are_taken_in_short_chains(k):
                     c = M.choose32(1, m, n, k, 1, b_mn)
                     assert -(-(-(-(-(-k // 64)) // c.split)) // c.leads) <= 7 and (3 + c.leads) * c.bn <= 512
                     assert c.smem() <= M.SMEM_MAX and c.bn % (8 * c.split) == 0
+
+
+def test_fp32_matmuls_stay_with_the_library_where_tf32_is_allowed():
+    """Large ones: the caller asked for the faster sum.  Set back, they are this package's."""
+    import torch
+
+    def own(m, n, k):
+        s = _schedule({"a": ((m, k), "input"), "w": ((k, n), "param"), "c": ((m, n), "output")},
+                      [_mm("k0", "a", "w", "c", m, n, k)])
+        return isinstance(fuse(s, Config()).kernels[0], MatmulKernel)
+
+    assert own(512, 768, 3072) and own(128, 768, 768)
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        assert not own(512, 768, 3072) and own(128, 768, 768)
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = False
+    assert own(512, 768, 3072)
