@@ -441,6 +441,20 @@ def whole32(k: int) -> bool:
     return _ceil(k, 64) <= 8 * LEADS * LEAD_BLOCKS
 
 
+def padded32(z: int, m: int, n: int, k: int) -> bool:
+    """Whether an fp32 product has so few rows for so many tiles that most of their 128 rows
+    is work for nothing, and the library's kernels for such shapes are faster.  In microseconds,
+    here and there: up to 64 rows and eight waves of tiles (384 x [64, 64] x [64, 512] 86.4,
+    68.3; 512 x [64, 64] x [64, 64], 3.5 waves, 17.1, 19.6), up to 32 rows and two and a half
+    (512 x [16, 16] x [16, 64] 14.8, 10.7; [32, 768] x [768, 50257] 86.7, 72.7; [8, 512] x
+    [512, 20000], 2.1 waves, 29.3, 30.5), up to 4 and one ([2, 768] x [768, 10000] 26.5, 14.5;
+    one of batched ones 21.0, 15.0 only from 2.5), a single one and 700 64-deep blocks
+    ([1, 2048] x [2048, 2048] 14.7, 10.8; [1, 3072] x [3072, 768], 576 of them, 12.8, 14.5)."""
+    tiles = z * _ceil(n, 64)
+    return (m <= 64 and tiles > 8 * SM_COUNT or m <= 32 and 2 * tiles > 5 * SM_COUNT
+            or m <= 4 and z == 1 and tiles > SM_COUNT or m == 1 and tiles * _ceil(k, 64) > 700)
+
+
 def choose32(z: int, m: int, n: int, k: int, groups: int, b_mn: bool, peers: int | None = None) -> Config32:
     """Least estimated time, in microseconds: a 64-deep block costs 0.75 (32 columns) or 1.0
     (64), a wave 3 before and after.  Leading products get a new accumulator every four

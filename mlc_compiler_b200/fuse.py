@@ -146,7 +146,7 @@ def _tf32() -> bool:
 
 def _matmul(k, schedule) -> MatmulKernel | None:
     """The tensor-core form of a library matmul, result stored as the library would."""
-    from .emit.matmul import whole32
+    from .emit.matmul import padded32, whole32
 
     if not isinstance(k, kir.ExternKernel) or k.op not in ("aten.mm.default", "aten.bmm.default") or k.kwargs:
         return None
@@ -169,7 +169,7 @@ def _matmul(k, schedule) -> MatmulKernel | None:
         return None
     z = out.shape[0] if len(out.shape) == 3 else 1
     m, n = out.shape[-2:]
-    if z * m * n >= 1 << 31:
+    if z * m * n >= 1 << 31 or (dts == {"float32"} and padded32(z, m, n, a.shape[-1])):
         return None
     rows = [(z, m, out.strides[0])] * (z > 1) + [(m, 1, out.strides[-2])] * (m > 1)
     dest = kir.Operand(out.name, out.buffer, next(iter(dts)), kir.IndexMap(

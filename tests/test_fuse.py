@@ -287,7 +287,7 @@ def test_fp32_sums_are_taken_in_short_chains(k):
             s = _schedule({"a": ((m, k), "input"), "w": ((k, n), "param"), "c": ((m, n), "output")},
                           [_mm("k0", "a", "w", "c", m, n, k)])
             own = isinstance(fuse(s, Config()).kernels[0], MatmulKernel)
-            assert own == (k <= 17920 and k * max(m, n) < 1 << 31)
+            assert own == (k <= 17920 and k * max(m, n) < 1 << 31 and not M.padded32(1, m, n, k))
             if own:
                 for b_mn in (False, True):
                     c = M.choose32(1, m, n, k, 1, b_mn)
@@ -311,3 +311,16 @@ def test_fp32_matmuls_stay_with_the_library_where_tf32_is_allowed():
     finally:
         torch.backends.cuda.matmul.allow_tf32 = False
     assert own(512, 768, 3072)
+
+
+@pytest.mark.parametrize("z,m,n,k,own", [(1, 1, 768, 3072, True), (1, 1, 2048, 2048, False), (1, 2, 2048, 2048, True),
+                                         (1, 2, 10000, 768, False), (1, 8, 20000, 512, True), (1, 32, 50257, 768, False),
+                                         (1, 40, 50257, 768, True), (96, 4, 64, 64, True), (512, 16, 16, 64, False),
+                                         (512, 64, 64, 64, True), (384, 64, 512, 64, False), (384, 65, 512, 64, True)])
+def test_fp32_products_of_few_rows_stay_with_the_library(z, m, n, k, own):
+    """Where most of a tile's 128 rows would be padding and there are waves of them."""
+    lead = (z,) if z > 1 else ()
+    s = _schedule({"a": (lead + (m, k), "input"), "w": (lead + (k, n), "param"), "c": (lead + (m, n), "output")}, [])
+    view = lambda b: kir.View(b, b, s.buffers[b].shape, tuple(math.prod(s.buffers[b].shape[i + 1:]) for i in range(len(s.buffers[b].shape))))  # noqa: E731
+    s.kernels = [kir.ExternKernel("k0", f"aten.{'bmm' if z > 1 else 'mm'}.default", [view("a"), view("w")], {}, [view("c")])]
+    assert isinstance(fuse(s, Config()).kernels[0], MatmulKernel) == own
