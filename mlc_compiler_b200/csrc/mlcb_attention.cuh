@@ -107,19 +107,17 @@ __device__ __forceinline__ void mlcb_attention(const mlcb_tmap* tq, const mlcb_t
         }
         __syncwarp();
     }
-    const bool alive = mlcb_warp_wait(o_full, 0, &dead);
+    mlcb_warp_wait(o_full, 0, &dead);
     mlcb_tc_after();
-    if (alive) {
-        // D columns over H threads of the row, at least 16 each
-        constexpr int STEP = C::D / C::H < 16 ? 16 : C::D / C::H;
+    // D columns over H threads of the row, at least 16 each
+    constexpr int STEP = C::D / C::H < 16 ? 16 : C::D / C::H;
 #pragma unroll
-        for (int c = 0; c < STEP; c += 16) {
-            const int c0 = part_of_row * STEP + c;
-            float v[16];
-            mlcb_tmem_ld(lanes + c0, v);
-            if (t0 + r < C::T) mlcb_store<T, 16>(out + g * out_g + (t0 + r) * out_t + c0, v);
-            __syncwarp();
-        }
+    for (int c = 0; c < STEP; c += 16) {
+        const int c0 = part_of_row * STEP + c;
+        float v[16];
+        mlcb_tmem_ld(lanes + c0, v);
+        if (t0 + r < C::T) mlcb_store<T, 16>(out + g * out_g + (t0 + r) * out_t + c0, v);
+        __syncwarp();
     }
     mlcb_tc_before();
     __syncthreads();

@@ -181,8 +181,8 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
         const u32 base = tmem + ((u32)(quad * 32) << 16);
         MLCB_GRID_WAIT();
         int nth = 0;
-        bool alive = true;
-        for (int tile = cluster; tile < C::TILES && alive; tile += clusters, ++nth) {
+        for (int tile = cluster; tile < C::TILES; tile += clusters, ++nth) {
+            if (nth > 0 && __any_sync(0xffffffffu, dead)) break;
             const int acc = nth % C::ACC;
             const int tm = tile % C::TM, tn = (tile / C::TM) % C::TN, g = (tile / (C::TM * C::TN)) % C::GROUPS;
             const int z = C::BATCH > 1 ? tile / (C::TM * C::TN * C::GROUPS) : 0;
@@ -195,8 +195,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
 #pragma unroll
                 for (int i = 0; i < EACH; ++i)
                     if ((half + i * HALVES) * 8 < SLICE) epi.fetch(pre[i], row, first + (half + i * HALVES) * 8, g, z);
-                alive = mlcb_warp_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
-                if (!alive) break;
+                mlcb_warp_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
                 mlcb_tc_after();
                 // partial sums go straight into the shared memory of the CTA that finishes these
                 // columns, as [source part][column quad][row][4]: conflict-free both ways.  Its
@@ -213,8 +212,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
                                    v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                     }
                 }
-                alive = mlcb_warp_wait(arrived, 0, &dead);
-                if (!alive) break;
+                mlcb_warp_wait(arrived, 0, &dead);
 #pragma unroll
                 for (int i = 0; i < EACH; ++i) {
                     const int c = (half + i * HALVES) * 8;
@@ -237,8 +235,7 @@ __device__ __forceinline__ void mlcb_matmul(const mlcb_tmap* ta, const mlcb_tmap
             } else {
                 typename Epi::template Pre<32> pre, ahead;
                 epi.fetch(pre, row, tn * C::BN + half * 32, g, z);
-                alive = mlcb_warp_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
-                if (!alive) break;
+                mlcb_warp_wait(acc_full + 8 * acc, (nth / C::ACC) & 1, &dead);
                 mlcb_tc_after();
 #pragma unroll 1
                 for (int c = half * 32; c < C::BN; c += 32 * HALVES) {

@@ -191,9 +191,8 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     const int quad = warp % 4, half = warp / 4, r = quad * 32 + lane, row = m0 + r;
     const u32 base = tmem + ((u32)(quad * 32) << 16);
     const u32 inbox = smem + C::STAGES * C::STAGE;     // partial sums of a split K
-    bool alive = warp < C::CW;
-    if (alive) {
-        alive = mlcb_warp_wait(done, 0, &dead);
+    if (warp < C::CW) {
+        mlcb_warp_wait(done, 0, &dead);
         mlcb_tc_after();
     }
     constexpr int EACH = (SLICE + C::CW * 2 - 1) / (C::CW * 2);
@@ -203,7 +202,7 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
         for (int i = 0; i < EACH; ++i)
             if (half * 8 + i * C::CW * 2 < SLICE) epi.fetch(pre[i], row, n0 + part * SLICE + half * 8 + i * C::CW * 2, g, z);
     }
-    if (alive) {
+    if (warp < C::CW) {
         // the four warps that share 32 rows take 16 columns each in turn
 #pragma unroll 1
         for (int c = half * 16; c < C::BN; c += C::CW * 4) {
@@ -263,7 +262,8 @@ __device__ __forceinline__ void mlcb_matmul32(const float* a, const float* b0, c
     }
     __syncwarp();
     if constexpr (C::SPLIT > 1) {
-        if (alive && mlcb_warp_wait(arrived, 0, &dead)) {
+        if (warp < C::CW) {
+            mlcb_warp_wait(arrived, 0, &dead);
 #pragma unroll
             for (int i = 0; i < EACH; ++i) {
                 const int c = half * 8 + i * C::CW * 2;
