@@ -454,6 +454,72 @@ def test_a_fused_model_gives_what_its_kernels_give_apart(batch, seq, heads, dtyp
         assert off <= layers * 10 * (U[dtype] if dtype != "float32" else 1e-6), off
 
 
+def _same_values(got, want, bound):
+    """Equal where not finite; elsewhere within ``bound`` of the value or of one."""
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf() * got.sign(), want.isinf() * want.sign())
+    fin = want.isfinite()
+    assert float(((got - want).abs() - bound * (1 + want.abs()))[fin].max()) <= 0
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
+@pytest.mark.parametrize("op", ["layernorm", "softmax", "gelu"])
+@pytest.mark.parametrize("rows,cols", [(9, 50257), (9, 12289), (2500, 801), (9000, 513), (999, 2501), (40, 64), (160, 9216)])
+def test_values_that_are_not_finite_stay_in_their_rows(rows, cols, op, dtype):
+    """Rows of -inf in part and whole, with +inf, with NaN, and of the type's lowest value."""
+    s = cases.rows_schedule(op, rows, cols, dtype)
+    params = {o: _randn((cols,), dtype, 5 + i) for i, o in enumerate(s.params)}
+    x = _randn((rows, cols), dtype, rows)
+    low = torch.finfo(x.dtype).min
+    x[0, 1:], x[1], x[2, cols - 1], x[3, 0], x[5], x[6, : cols - 1] = -float("inf"), -float("inf"), float("inf"), float("nan"), low, low
+    res = _randn((rows, cols), dtype, 2)
+    args = (x, res) if op == "gelu" else (x,)
+    got = CompiledModel(s, params, Config(), "cuda")(*args).double()
+    d = x.double()
+    if op == "softmax":
+        want = torch.softmax(d, -1)
+    elif op == "layernorm":
+        want = torch.nn.functional.layer_norm(d, (cols,), params["norm.weight"].double(), params["norm.bias"].double(), 1e-5)
+    else:
+        want = d + params["bias"].double()
+        want = res.double() + torch.nn.functional.gelu(want, approximate="tanh")
+    # squares and cubes of the lowest values overflow in 32 bits, and 0.5 x (1 + tanh) is NaN at -inf
+    keep = [r for r in range(rows) if not (op != "softmax" and r in (0, 1, 5, 6))]
+    # the result's rounding and the steps in 32 bits before it: sums of up to 50257 columns to
+    # 2^-20, of a LayerNorm's to 1e-5 (as above) times 1 + gain and 1 + x, below 16 together
+    _same_values(got[keep], want[keep], U[dtype] + (1.6e-4 if op == "layernorm" else 1e-5))
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+@pytest.mark.parametrize("keys", [48, 128, 200, 512])
+def test_attention_masked_with_minus_infinity(keys, dtype):
+    """Some keys, and for one batch entry all of them: NaN there, and only there."""
+    G, T, S, D = 3, 40, keys, 64
+    s = _Schedule("attention")
+    q = s.buffer("q", (G, T, D), dtype, "input")
+    s.buffer("k", (G, S, D), dtype, "input")
+    v = s.buffer("v", (G, S, D), dtype, "input")
+    s.buffer("mask", (G, S), dtype, "input")
+    scores, probs = (s.buffer(n, (G, T, S), dtype, "intermediate") for n in ("scores", "probs"))
+    out = s.buffer("out", (G, T, D), dtype, "output")
+    s.kernels = [
+        kir.ExternKernel("k0", "aten.bmm.default", [q, kir.View("k", "k", (G, D, S), (S * D, 1, D))], {}, [scores]),
+        cases._softmax("k1", G * T, S, dtype, cases._row("scores", dtype, G * T, S),
+                       cases._row("mask", dtype, G * T, S, [(G, T, S)]), cases._row("probs", dtype, G * T, S), (G, T)),
+        kir.ExternKernel("k2", "aten.bmm.default", [probs, v], {}, [out])]
+    cases._plan_arena(s)
+    cm = CompiledModel(s, {}, Config(), "cuda")
+    assert len(cm.launched_schedule) == 1
+    q, k, v = (_randn(x, dtype, i) for i, x in enumerate([(G, T, D), (G, S, D), (G, S, D)]))
+    mask = torch.zeros((G, S), dtype=q.dtype, device="cuda")
+    mask[0, 5:], mask[1], mask[2, : S - 1] = -float("inf"), -float("inf"), -float("inf")
+    got = cm(q, k, v, mask).double()
+    x = q.double() @ k.double().transpose(1, 2) / 8 + mask.double()[:, None]
+    want = torch.softmax(x, -1) @ v.double()
+    # a score's rounding moves its exponential by u |x| / 8 < 8 u, numerator and sum alike
+    _same_values(got, want, U[dtype] * 18)
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16", "float32"])
 @pytest.mark.parametrize("rows,cols", [(777, 1003), (1, 607001), (8, 50001), (601, 1006), (3, 300000)])
 def test_pointwise_over_counts_that_are_no_packs(rows, cols, dtype):
