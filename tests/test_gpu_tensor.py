@@ -486,8 +486,9 @@ def test_values_that_are_not_finite_stay_in_their_rows(rows, cols, op, dtype):
     # squares and cubes of the lowest values overflow in 32 bits, and 0.5 x (1 + tanh) is NaN at -inf
     keep = [r for r in range(rows) if not (op != "softmax" and r in (0, 1, 5, 6))]
     # the result's rounding and the steps in 32 bits before it: sums of up to 50257 columns to
-    # 2^-20, of a LayerNorm's to 1e-5 (as above) times 1 + gain and 1 + x, below 16 together
-    _same_values(got[keep], want[keep], U[dtype] + (1.6e-4 if op == "layernorm" else 1e-5))
+    # 2^-20, of a LayerNorm's to 1e-5 (as above) times 1 + gain and 1 + x, below 16 together;
+    # GELU rounds its own result too, up to 9 here, which the residual may cancel
+    _same_values(got[keep], want[keep], U[dtype] * (10 if op == "gelu" else 1) + (1.6e-4 if op == "layernorm" else 1e-5))
 
 
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
