@@ -398,6 +398,35 @@ int mlcb_kernel_info(mlcb_kernel* k, int* regs, int* static_smem, int* max_threa
     return 0;
 }
 
+// A launch on clusters of `cluster` CTAs (0, 1: none), programmatic where the flags say so;
+// `attr` has room for two attributes and outlives the result.
+static CUlaunchConfig launch_config(CUlaunchAttribute* attr, uint32_t grid_x, uint32_t block_x, uint32_t cluster,
+                                    uint32_t smem_bytes, uint64_t stream, uint32_t flags) {
+    memset(attr, 0, 2 * sizeof *attr);
+    unsigned n = 0;
+    if (flags & MLCB_LAUNCH_DEPENDENT) {
+        attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+        attr[n++].value.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+        attr[n].value.clusterDim.x = cluster;
+        attr[n].value.clusterDim.y = attr[n].value.clusterDim.z = 1;
+        ++n;
+    }
+    CUlaunchConfig cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDimX = grid_x;
+    cfg.gridDimY = cfg.gridDimZ = 1;
+    cfg.blockDimX = block_x;
+    cfg.blockDimY = cfg.blockDimZ = 1;
+    cfg.sharedMemBytes = smem_bytes;
+    cfg.hStream = (CUstream)(uintptr_t)stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cfg;
+}
+
 static int launch_one(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t smem_bytes,
                       const uint64_t* device_ptrs, int nptrs, uint64_t stream, uint32_t flags) {
     enum { MAX_PTRS = 64 };
@@ -419,28 +448,7 @@ static int launch_one(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_
     {
         if (flags) {
             CUlaunchAttribute attr[2];
-            memset(attr, 0, sizeof attr);
-            unsigned n = 0;
-            if (flags & MLCB_LAUNCH_DEPENDENT) {
-                attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-                attr[n++].value.programmaticStreamSerializationAllowed = 1;
-            }
-            if (const unsigned cluster = (flags >> 8) & 0xFF; cluster > 1) {
-                attr[n].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
-                attr[n].value.clusterDim.x = cluster;
-                attr[n].value.clusterDim.y = attr[n].value.clusterDim.z = 1;
-                ++n;
-            }
-            CUlaunchConfig cfg;
-            memset(&cfg, 0, sizeof cfg);
-            cfg.gridDimX = grid_x;
-            cfg.gridDimY = cfg.gridDimZ = 1;
-            cfg.blockDimX = block_x;
-            cfg.blockDimY = cfg.blockDimZ = 1;
-            cfg.sharedMemBytes = smem_bytes;
-            cfg.hStream = (CUstream)(uintptr_t)stream;
-            cfg.attrs = attr;
-            cfg.numAttrs = n;
+            const CUlaunchConfig cfg = launch_config(attr, grid_x, block_x, (flags >> 8) & 0xFF, smem_bytes, stream, flags);
             r = d.LaunchKernelEx(&cfg, k->fn, args, nullptr);
         } else {
             r = d.LaunchKernel(k->fn, grid_x, 1, 1, block_x, 1, 1, smem_bytes,
@@ -524,28 +532,7 @@ int mlcb_launch_ex(mlcb_kernel* k, uint32_t grid_x, uint32_t block_x, uint32_t c
                     (void*)k, grid_x, block_x, cluster_x);
     if (int e = need_driver()) return e;
     CUlaunchAttribute attr[2];
-    memset(attr, 0, sizeof attr);
-    unsigned n = 0;
-    if (flags & MLCB_LAUNCH_DEPENDENT) {
-        attr[n].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-        attr[n++].value.programmaticStreamSerializationAllowed = 1;
-    }
-    if (cluster_x > 1) {
-        attr[n].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
-        attr[n].value.clusterDim.x = cluster_x;
-        attr[n].value.clusterDim.y = attr[n].value.clusterDim.z = 1;
-        ++n;
-    }
-    CUlaunchConfig cfg;
-    memset(&cfg, 0, sizeof cfg);
-    cfg.gridDimX = grid_x;
-    cfg.gridDimY = cfg.gridDimZ = 1;
-    cfg.blockDimX = block_x;
-    cfg.blockDimY = cfg.blockDimZ = 1;
-    cfg.sharedMemBytes = smem_bytes;
-    cfg.hStream = (CUstream)(uintptr_t)stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = n;
+    const CUlaunchConfig cfg = launch_config(attr, grid_x, block_x, cluster_x, smem_bytes, stream, flags);
     CtxGuard in_module_context(k->owner->ctx);
     CUresult r = g_drv.LaunchKernelEx(&cfg, k->fn, (void**)params, nullptr);
     if (r != CUDA_SUCCESS) {
