@@ -145,9 +145,9 @@ EXAMPLE = CSRC / "examples" / "bert-base_b8_s128_float16.cu"
 
 
 def example_source() -> str:
-    """The translation unit the executor compiles for BERT-base fp16 at batch 8
-    (after producer forwarding): every kernel family in one readable file.  A
-    copy is kept under ``csrc/examples`` so that the generated CUDA can be read
+    """The pointwise and row-reduction kernels of BERT-base fp16 at batch 8 (after
+    producer forwarding, before matmuls are fused: ``CompiledModel.launched.source()``
+    prints what calls launch): those families in one readable file.  A copy is kept under ``csrc/examples`` so that the generated CUDA can be read
     without running anything; ``write_example`` refreshes it and a test keeps it
     honest."""
     from .config import Config

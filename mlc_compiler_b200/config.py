@@ -79,9 +79,9 @@ class Config:
     wide_access_bytes: int = 8 << 20
     #: same for persistent row reductions (0 = never; measured no better than 128-bit)
     wide_reduction_bytes: int = 0
-    #: row reductions over at least this many columns (a third of it
-    #: where rows are not aligned for wide accesses) keep the row in shared memory
-    #: (``emit/staged.py``); 0 = never
+    #: row reductions over at least this many columns keep the row in shared memory
+    #: (``emit/staged.py``), from two thirds of it where there are 1000 rows or more that are
+    #: neither streamed nor aligned for 128-bit accesses; 0 = never
     staged_columns: int = 9000
     #: fold a pointwise producer into the pointwise kernels that only re-read it at
     #: another index (bias add + head-layout copy at batch > 1); bit-identical
@@ -99,11 +99,13 @@ class Config:
     #: turn ``mm`` + leading bias add into ``addmm`` (cuBLASLt bias epilogue).  Off by
     #: default: it changes how the matmul is dispatched and rounds once instead of twice
     bias_epilogue: bool = False
-    #: run ``mm`` / ``bmm`` over fp16 / bf16 operands on this package's tensor-core kernels
-    #: (fp32 accumulation, results rounded where the library's are); False: on the library
+    #: run ``mm`` / ``bmm`` over fp16, bf16 or fp32 operands on this package's tensor-core
+    #: kernels (fp32 accumulation, results rounded where the library's are; fp32 operands in
+    #: three exact pieces, but for shapes ``fuse.py`` leaves to the library); False: all there
     own_matmuls: bool = True
-    #: fold pointwise neighbours into those matmuls and run the attention core as one kernel;
-    #: same values as the separate kernels
+    #: fold pointwise neighbours into those matmuls and run the attention core of 16-bit models
+    #: as one kernel, rounded where the separate kernels round.  The values are theirs but for
+    #: the order of a softmax's sums where ``emit/attention.py`` cannot keep it
     fuse_matmuls: bool = True
     #: run independent pointwise kernels over the same iteration space as one launch
     #: (BERT's q/k/v bias adds: 36 launches -> 12); bit-identical.  Off by default
@@ -124,7 +126,8 @@ class Config:
     def as_scheduled(self) -> "Config":
         """The same configuration with every executor-side rewrite off: the schedule
         runs kernel for kernel and matmul for matmul as the frontend produced it, on
-        one stream."""
+        one stream (the matmuls on this package's kernels; with ``own_matmuls=False``
+        besides, through the library calls of the schedule)."""
         return _replace(self, forward_into_copies=False, write_through_copies=False,
                         sequence_first=False, fold_embeddings=False, bias_epilogue=False,
                         fuse_siblings=False, fuse_matmuls=False,

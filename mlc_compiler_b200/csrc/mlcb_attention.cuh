@@ -6,7 +6,7 @@
 // A TMEM lane is a query row.  H threads share a row, each with a contiguous part of its
 // keys (warps w, w + 4, ... see the same 32 lanes).  P overlays Q and K, whose matmul is
 // over, and O overlays the scores, which have all been read: [128 x 64] heads over 128
-// keys take 49 KB and 128 TMEM columns, so four CTAs share an SM.
+// keys take 49 KB and 128 TMEM columns; two such CTAs of 512 threads share an SM (64 registers).
 #pragma once
 
 template <int G_, int T_, int S_, int D_, int H_, int RED_, bool BF16_>

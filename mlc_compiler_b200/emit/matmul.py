@@ -417,7 +417,6 @@ class Config32:
     split: int
     grid: int
     leads: int
-    epi_warps: int = 16
 
     @property
     def per_call(self) -> int:

@@ -9,7 +9,7 @@ exchange their partial results through distributed shared memory, in rank order.
 
 The copies are issued in blocks of one pack per thread, each with its own barrier: the
 first pass starts on a block while the rest are on their way.  Softmax over
-[512, 50257] fp16 (odd rows, 103 MB) takes 27.8 us (3.7 TB/s), streamed 61.9;
+[512, 50257] fp16 (odd rows, 103 MB) takes 25.4 us (4.1 TB/s), streamed 61.9;
 [2000, 16383] bf16 31 us, 60 in registers; [16, 20001] fp32 5.4 us, 10.4 streamed.
 """
 

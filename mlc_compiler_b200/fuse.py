@@ -6,12 +6,13 @@ after them and produces what a captured call launches: a schedule whose kernels 
 the generated pointwise and row-reduction kernels, :class:`MatmulKernel` and
 :class:`AttentionKernel`, plus whatever stays with the library.
 
-* ``mm`` / ``bmm`` over 16-bit operands becomes a :class:`MatmulKernel`; a pointwise
+* ``mm`` / ``bmm`` over 16-bit or fp32 operands becomes a :class:`MatmulKernel` (fp32
+  ones of very long K, of few rows, or where the caller allows TF32 stay); a pointwise
   kernel that is the only reader of the result becomes its epilogue (bias add, GELU,
   residual), evaluated on the accumulator after the rounding the separate matmul
   would have stored, so the values are the ones the two kernels would produce;
 * matmuls of the same rows with the same shape and epilogue (q, k, v) share a launch;
-* ``bmm`` -> row softmax -> ``bmm`` becomes one :class:`AttentionKernel` that keeps
+* 16-bit ``bmm`` -> row softmax -> ``bmm`` becomes one :class:`AttentionKernel` that keeps
   scores and probabilities on the SM, rounded where the three kernels round them.
 
 A buffer that disappears into a fused kernel is one nothing else reads.  The arena is
